@@ -35,7 +35,8 @@ void free_all(ws::Workspace &w) {
                     w.n2t_val_alt, w.n2t_offset, w.row_pair_cols, w.row_pair_cnts, w.row_pair_first,
                     w.row_entry_first, w.pair_val, w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene, w.half_slot_up,
                     w.half_slot_lo, w.row_cnt_up, w.row_cnt_lo, w.row_first, w.rowptr, w.col_key, w.col_val,
-                    w.col_key_alt, w.col_val_alt, w.colidx, w.item_ptr, w.item_info, w.item_col, w.sym_blocks, w.contrib, w.pcg_warp_groups, w.pcg_unit_info, w.pcg_tickets, w.mf_ux, w.inv_diag, w.diag64, w.jtr, w.x, w.r, w.q,
+                    w.col_key_alt, w.col_val_alt, w.colidx, w.item_ptr, w.item_info, w.item_col, w.sym_blocks, w.contrib, w.pcg_warp_groups, w.pcg_unit_info, w.pcg_words, w.pcg_send,
+                    w.pcg_send_count, w.pcg_halo, w.pcg_tickets, w.mf_ux, w.inv_diag, w.diag64, w.jtr, w.x, w.r, w.q,
                     w.sd0, w.sd1, w.se3, w.centers, w.chunk_partial, w.scene_scalars, w.scene_counter,
                     w.error_flag};
     for (void *p : ptrs)
@@ -214,6 +215,11 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
         A(dalloc(&w.pcg_warp_groups, (size_t)ws::kPcgUnitsPerWarp * w.pcg_grid * ws::pcg_warps_per_block() + 2));
         A(dalloc(&w.pcg_unit_info, 2 * (size_t)ws::kPcgUnitsPerWarp * w.pcg_grid * ws::pcg_warps_per_block()));
         A(dalloc(&w.pcg_tickets, 4));
+        w.pcg_cluster = ws::pcg_cluster_max(&w.pcg_clusters_active);
+        A(dalloc(&w.pcg_words, w.cap_items));
+        A(dalloc(&w.pcg_send, w.cap_half));
+        A(dalloc(&w.pcg_send_count, w.cap_nodes));
+        A(dalloc(&w.pcg_halo, 16ull * w.cap_scenes));   // kResMaxCluster each
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -324,6 +330,13 @@ int ws_set_batch(ws_solver *h, const ws_inputs *scenes, int num_scenes) {
         fb += in.num_features;
         tb += nt;
         cb += nc;
+    }
+    {
+        // k_pcg_cluster starts the batch's largest scenes first
+        std::vector<int> order(num_scenes);
+        for (int s = 0; s < num_scenes; ++s) order[s] = s;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return hs[a].num_nodes > hs[b].num_nodes; });
+        for (int s = 0; s < num_scenes; ++s) hs[s].pcg_order = order[s];
     }
     w.h_scenes.assign(hs, hs + num_scenes);
     w.num_scenes = num_scenes;
@@ -445,7 +458,8 @@ int ws_solve_graph(ws_solver *h, int gn_iters, int pcg_iters, void *stream) {
     w.last_stream = st;
     const uint64_t key[] = {(uint64_t)gn_iters, (uint64_t)pcg_iters, (uint64_t)w.num_scenes, w.total_nodes,
                             w.total_edges, w.total_tiles, w.total_chunks, (uint64_t)w.node_bits,
-                            (uint64_t)w.dense_channels, (uint64_t)ws::pcg_split_group(w)};
+                            (uint64_t)w.dense_channels, (uint64_t)ws::pcg_split_group(w),
+                            (uint64_t)ws::pcg_cluster_size(w)};
     constexpr size_t kKey = sizeof(key) / sizeof(key[0]);
     bool same = w.graph_exec && w.graph_key.size() == kKey && std::equal(key, key + kKey, w.graph_key.begin());
     if (same) {
@@ -652,7 +666,11 @@ int ws_autotune(ws_solver *h, int pcg_iters, void *stream, ws_tuning *out) {
     const int max_per_sm = std::max(1, std::min(8, w.pcg_grid / std::max(1, w.num_sms)));
     int best_b = max_per_sm;
     float bb = 1e30f;
-    for (int b = 1; b <= max_per_sm; ++b) {
+    if (ws::pcg_cluster_size(w) > 0) {   // clusters run these inputs: blocks per SM stays at its bound
+        w.tune.pcg_blocks_per_sm = max_per_sm;
+        out->pcg_ms[max_per_sm - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });
+    }
+    for (int b = 1; b <= max_per_sm && ws::pcg_cluster_size(w) == 0; ++b) {
         w.tune.pcg_blocks_per_sm = b;
         ws::pcg_ranges(w, st);
         out->pcg_ms[b - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });

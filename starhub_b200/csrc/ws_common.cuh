@@ -68,6 +68,7 @@ struct Scene {
     float lam_depth, lam_of, lam_reg, lam_node, lam_feat;
     int tile_base, num_tiles;          // pixel tiles of this scene
     int chunk_base, num_chunks;        // PCG row groups (kRowsPerGroup nodes) of this scene
+    int pcg_order;                     // entry k of the batch's table: the scene with the k-th most nodes
 };
 
 // Per-scene counts derived on the device during the index build.

@@ -672,6 +672,7 @@ void index_build(Workspace &w, cudaStream_t st) {
                                                              w.colidx, w.item_info, w.item_col, w.error_flag);
     count_launch(w, 2);
     pcg_ranges(w, st);
+    pcg_plan(w, st);
 }
 
 void pcg_ranges(Workspace &w, cudaStream_t st) {

@@ -22,6 +22,8 @@ struct Workspace {
     int device = 0;
     int num_sms = 0;
     int pcg_grid = 0;           // co-resident blocks for the persistent PCG kernel
+    int pcg_cluster = 0;        // blocks per cluster of k_pcg_cluster on this device (16, 8; 0: none)
+    int pcg_clusters_active = 0;   // such clusters that run at once
     // launch shapes picked by ws_autotune (defaults until then); none of them changes a result
     struct Tuning {
         int node_threads = 128;     // threads per block of the node assembly (64, 128, 256)
@@ -103,6 +105,10 @@ struct Workspace {
                                                              // first row group of every PCG work unit, the
                                                              // group count, the first half's unit count
     uint4 *pcg_unit_info = nullptr;                          // [2 * PCG work units]: groups, rows, items, scenes
+    // work distribution of the cluster PCG (ResPlan): item words [cap_items], send lists [cap_half],
+    // sends per row [cap_nodes], halo rows per block [cap_scenes * 16]
+    uint2 *pcg_words = nullptr;
+    uint32_t *pcg_send = nullptr, *pcg_send_count = nullptr, *pcg_halo = nullptr;
     uint32_t *pcg_tickets = nullptr;                         // [4]: [0] PCG work-unit tickets, zeroed per launch
     float *mf_ux = nullptr;             // matrix-free SpMV scratch: J x per dense term and edge (float4),
                                         // allocated on first use
@@ -158,6 +164,9 @@ cudaError_t gn_pcg(Workspace &w, int pcg_iters, cudaStream_t st);
 void init_warp(Workspace &w, cudaStream_t st);
 // Occupancy of the persistent PCG kernel.
 int pcg_max_blocks(int device);
+int pcg_cluster_max(int *active);
+int pcg_cluster_size(const Workspace &w);
+cudaError_t pcg_plan(Workspace &w, cudaStream_t st);
 int pcg_launch_blocks(const Workspace &w);
 void pcg_ranges(Workspace &w, cudaStream_t st);
 // First row group of the second half of the scenes in the PCG's schedule (a scene boundary).

@@ -1,0 +1,68 @@
+"""The cluster PCG against the persistent one: a lone small scene runs on a cluster, the same scene in a
+batch of many on k_pcg, and both must give the same bits (the kernels do the same arithmetic)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _cut(scene, nodes, seed):
+    """The scene on `nodes` of its nodes (anchors included): surfels skinned to four distinct ones near their
+    own, the graph a band (a pair then has at most one smoothness term per direction)."""
+    import dataclasses
+    keep = np.sort(np.random.default_rng(seed).permutation(scene.num_nodes)[:nodes])
+    near = np.searchsorted(keep, scene.surfel_knn.astype(int)[:, 0]).clip(0, nodes - 1)
+    k = min(8, (nodes - 1) // 2)
+    i = np.arange(nodes)[:, None]
+    edges = np.stack(np.broadcast_arrays(i, (i + np.arange(k)) % nodes, np.arange(k)), -1)
+    return dataclasses.replace(scene, nodes=scene.nodes[keep], graph_k=k, node_cw=np.ones((nodes, k), np.float32),
+                               surfel_knn=((near[:, None] + np.arange(4)) % nodes).astype(np.uint16),
+                               edges=edges.reshape(-1, 3).astype(np.uint16))
+
+
+# nodes: one group, a partial group, fewer groups than blocks, one more than a block each, a whole scene
+@pytest.mark.parametrize("nodes,gn,pcg,precision", [(5, 2, 3, 0), (16, 1, 1, 0), (17, 2, 4, 0), (255, 2, 5, 0),
+                                                    (257, 2, 5, 1), (900, 1, 0, 0), (900, 2, 2, 0), (1500, 3, 10, 0)])
+def test_cluster_equals_persistent(ws, small_scene_k8, nodes, gn, pcg, precision):
+    import torch
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    nodes = min(nodes, small_scene_k8.num_nodes)
+    sc = small_scene_k8 if nodes == small_scene_k8.num_nodes else _cut(small_scene_k8, nodes, 3)
+    ds = DeviceScene.from_scene(sc)
+    copies = 72   # far past the batch size where k_pcg takes over
+    out = []
+    for n in (1, copies):
+        s = WarpSolver(max_nodes=n * ds.num_nodes, max_pixels=n * ds.num_pixels, max_edges=n * ds.num_edges, max_scenes=n,
+                       precision=precision)
+        s.SetBatchInputs([ds] * n)
+        s.SolveStreamed(gn, pcg, stream=torch.cuda.Stream())
+        s.Sync()
+        out.append([s.SolvedNodeSE3(i).cpu().numpy().copy() for i in {0, n // 2, n - 1}])
+    assert np.isfinite(out[0][0]).all()
+    for b in out[1]:
+        np.testing.assert_array_equal(out[0][0], b)
+
+
+def test_scattered_node_order(ws, small_scene_k8):
+    """Node ids in random order: every block's halo is most of the scene."""
+    import dataclasses
+    import torch
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    n = small_scene_k8.num_nodes
+    order = np.random.default_rng(9).permutation(n)
+    new_id = np.empty(n, int)
+    new_id[order] = np.arange(n)
+    e = small_scene_k8.edges.astype(int).reshape(n, 8, 3)[order]
+    e = np.stack([new_id[e[..., 0]], new_id[e[..., 1]], e[..., 2]], -1).reshape(-1, 3)
+    sc = dataclasses.replace(small_scene_k8, nodes=small_scene_k8.nodes[order], node_cw=small_scene_k8.node_cw[order],
+                             surfel_knn=new_id[small_scene_k8.surfel_knn.astype(int)].astype(np.uint16),
+                             edges=e.astype(np.uint16))
+    ds = DeviceScene.from_scene(sc)
+    out = []
+    for c in (1, 72):
+        s = WarpSolver(max_nodes=c * n, max_pixels=c * ds.num_pixels, max_edges=c * ds.num_edges, max_scenes=c)
+        s.SetBatchInputs([ds] * c)
+        s.SolveStreamed(2, 10, stream=torch.cuda.Stream())
+        s.Sync()
+        out.append(s.SolvedNodeSE3(c - 1).cpu().numpy().copy())
+    np.testing.assert_array_equal(out[0], out[1])
