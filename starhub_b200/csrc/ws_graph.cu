@@ -54,9 +54,39 @@ struct Heap {
         }
         refresh();
     }
+    // Ascending order.  Distinct distances have one: a sorting network in registers.  With ties the
+    // order is that of the reference's quicksort.
+    __device__ __forceinline__ void sort() {
+        float s[CAP];
+        uint16_t k[CAP];
+#pragma unroll
+        for (int i = 0; i < CAP; ++i) { s[i] = d[i]; k[i] = id[i]; }
+#pragma unroll
+        for (int round = 0; round < CAP; ++round)   // odd-even transposition
+#pragma unroll
+            for (int i = round & 1; i + 1 < CAP; i += 2) {
+                const bool swap = s[i + 1] < s[i];
+                const float a = s[i], b = s[i + 1];
+                const uint16_t ka = k[i], kb = k[i + 1];
+                s[i] = swap ? b : a;
+                s[i + 1] = swap ? a : b;
+                k[i] = swap ? kb : ka;
+                k[i + 1] = swap ? ka : kb;
+            }
+        bool strict = true;
+#pragma unroll
+        for (int i = 0; i + 1 < CAP; ++i) strict = strict && s[i] < s[i + 1];
+        if (strict) {
+#pragma unroll
+            for (int i = 0; i < CAP; ++i) { d[i] = s[i]; id[i] = k[i]; }
+        } else {
+            quicksort(d, id);
+        }
+    }
     // Lomuto quicksort on strict <, iterative form of the reference's recursion
-    // (same partitions in the same order).
-    __device__ void sort() {
+    // (same partitions in the same order); kept out of line, since its run-time indices put the arrays in
+    // local memory.
+    static __device__ __noinline__ void quicksort_arrays(float *d, uint16_t *id) {
         int lo_stack[2 * CAP + 2], hi_stack[2 * CAP + 2];
         int top = 0;
         lo_stack[0] = 0;
@@ -82,6 +112,15 @@ struct Heap {
             lo_stack[top] = pi + 1; hi_stack[top] = high; ++top;
             lo_stack[top] = low; hi_stack[top] = pi - 1; ++top;
         }
+    }
+    static __device__ __forceinline__ void quicksort(float (&d)[CAP], uint16_t (&id)[CAP]) {
+        float ld[CAP];
+        uint16_t li[CAP];
+#pragma unroll
+        for (int i = 0; i < CAP; ++i) { ld[i] = d[i]; li[i] = id[i]; }
+        quicksort_arrays(ld, li);
+#pragma unroll
+        for (int i = 0; i < CAP; ++i) { d[i] = ld[i]; id[i] = li[i]; }
     }
 };
 
@@ -534,6 +573,224 @@ __global__ void __launch_bounds__(256) k_skinning(const float4 *nodes, const uin
     cw[v] = make_float4(1.f, 1.f, 1.f, 1.f);
 }
 
+// Full skinning over a grid of the nodes.  k_skinning tests every node for every surfel; here a surfel tests
+// the nodes of the 3 x 3 x 3 cells around it, about 40.  1.2M surfels: 8.4k nodes 13422 -> 361 us, 31k
+// nodes 46298 -> 2814 us, 525 nodes 1078 -> 236 us; 3000 surfels on 8.4k nodes 934 -> 45 us.  What bounds it now is shared memory: 16
+// random bytes a lane and candidate, and warps that wait for their longest row of cells.
+//
+// Every block builds the same grid in its shared memory: kSkinCells cells (coordinates wrap, which only
+// adds far candidates) and the nodes in cell order.  The cell size starts at 1.75 node radii and is
+// halved or doubled until a node shares its cell with a few others, whatever the radius says.  More than
+// kSkinGridNodes nodes go through in chunks, a surfel's five nearest kept from one to the next.
+// Result: exactly k_skinning's.  When the four nearest found are strictly below the fifth and below
+// every node outside the cells (by the distance to their faces, with a margin of a hundredth of a cell
+// for the rounding of the scaled coordinates, |cell| <= 4096), and differ from one another, the ordered
+// scan ends with the same four in the same order.  Otherwise (ties, far or few nodes, NaN) the surfel's
+// warp repeats the ordered scan itself, 32 nodes at a time with the heap updates in node order.
+constexpr int kSkinThreads = 1024;
+constexpr int kSkinCellsX = 32, kSkinCellsY = 32, kSkinCellsZ = 16;
+constexpr int kSkinCells = kSkinCellsX * kSkinCellsY * kSkinCellsZ;
+constexpr int kSkinGridNodes = 10240;   // 16 bytes a node and 4 a cell fill a block's shared memory
+static_assert(kSkinCells % kSkinThreads == 0, "whole cells per thread");
+
+__device__ __forceinline__ float skin_scaled(float v, float inv_h) {
+    return fminf(fmaxf(__fmul_rn(v, inv_h), -262144.f), 262144.f);
+}
+__device__ __forceinline__ int skin_cell(int x, int y, int z) {
+    return (x & (kSkinCellsX - 1)) | ((y & (kSkinCellsY - 1)) * kSkinCellsX) |
+           ((z & (kSkinCellsZ - 1)) * (kSkinCellsX * kSkinCellsY));
+}
+__device__ __forceinline__ int skin_cell_of(float4 q, float inv_h) {
+    return skin_cell(__float2int_rd(skin_scaled(q.x, inv_h)), __float2int_rd(skin_scaled(q.y, inv_h)),
+                     __float2int_rd(skin_scaled(q.z, inv_h)));
+}
+
+// Grid of nodes n0 .. n1 - 1 in the block's shared memory; returns the cell size.
+__device__ float skin_grid_build(const float4 *nodes, const uint2 *status, int n0, int n1, float h, float4 *cell_nodes,
+                                 uint32_t *cell_end) {
+    __shared__ unsigned long long sm64[kSkinThreads / 32];
+    __shared__ uint32_t sm32[32];
+    const int tid = threadIdx.x, n = n1 - n0;
+    constexpr int kPer = kSkinCells / kSkinThreads;
+    int dir = 0;
+    for (int trial = 0;; ++trial) {   // uniform: every thread sees the same sums
+        const float inv_h = 1.0f / h;
+        __syncthreads();
+        for (int c = tid; c < kSkinCells; c += kSkinThreads) cell_end[c] = 0;
+        __syncthreads();
+        for (int i = n0 + tid; i < n1; i += kSkinThreads)
+            // a deleted node enters no heap: its distance is the heap's initial 1e6
+            if (!node_deleted(status, i)) atomicAdd(&cell_end[skin_cell_of(nodes[i], inv_h)], 1u);
+        __syncthreads();
+        unsigned long long sq = 0;
+        for (int c = tid; c < kSkinCells; c += kSkinThreads) sq += (unsigned long long)cell_end[c] * cell_end[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if ((tid & 31) == 0) sm64[tid >> 5] = sq;
+        __syncthreads();
+        sq = 0;
+        for (int i = 0; i < kSkinThreads / 32; ++i) sq += sm64[i];
+        // nodes that share a node's cell, itself among them: 1.5 to 16 on average
+        const int want = sq > 16ull * n ? -1 : (2ull * sq < 3ull * n ? 1 : 0);
+        const float next = want < 0 ? 0.5f * h : 2.0f * h;
+        if (want == 0 || trial == 12 || (dir != 0 && want != dir) || !(next > 1e-12f && next < 1e12f)) break;
+        dir = want;
+        h = next;
+    }
+    {   // counts -> first positions (thread t owns cells kPer t ..); placing the nodes moves them to the ends
+        uint32_t v[kPer], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) { v[k] = cell_end[kPer * tid + k]; sum += v[k]; }
+        uint32_t at = block_excl_scan_u32(sum, nullptr, sm32);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) { cell_end[kPer * tid + k] = at; at += v[k]; }
+    }
+    __syncthreads();
+    const float inv_h = 1.0f / h;
+    for (int i = n0 + tid; i < n1; i += kSkinThreads) {
+        if (node_deleted(status, i)) continue;
+        const float4 q = nodes[i];
+        cell_nodes[atomicAdd(&cell_end[skin_cell_of(q, inv_h)], 1u)] = make_float4(q.x, q.y, q.z, __int_as_float(i));
+    }
+    __syncthreads();
+    return h;
+}
+
+// One surfel's search: its five nearest so far, ascending, with the ids of four, and the distance up to
+// which every node has been seen.
+struct SkinNearest {
+    float d[5] = {1e6f, 1e6f, 1e6f, 1e6f, 1e6f};
+    int id[4] = {0, 0, 0, 0};
+    float reach = 1e30f;
+};
+
+__device__ __forceinline__ void skin_grid_search(float4 p, float h, const float4 *cell_nodes, const uint32_t *cell_end,
+                                                 SkinNearest &b) {
+    const float inv_h = 1.0f / h;
+    const float sx = skin_scaled(p.x, inv_h), sy = skin_scaled(p.y, inv_h), sz = skin_scaled(p.z, inv_h);
+    const int cx = __float2int_rd(sx), cy = __float2int_rd(sy), cz = __float2int_rd(sz);
+    const int x0 = (cx - 1) & (kSkinCellsX - 1), x1 = (cx + 1) & (kSkinCellsX - 1);
+    for (int row = 0; row < 9; ++row) {
+        // the row's three cells: one range, or two where x wraps
+        const int c0 = skin_cell(0, cy + row % 3 - 1, cz + row / 3 - 1);
+        for (int part = 0; part < (x0 <= x1 ? 1 : 2); ++part) {
+            const int lo = c0 + (x0 <= x1 || part == 0 ? x0 : 0);
+            const int hi = c0 + (x0 <= x1 || part == 1 ? x1 : kSkinCellsX - 1);
+            const uint32_t e = cell_end[hi];
+            for (uint32_t k = lo > 0 ? cell_end[lo - 1] : 0u; k < e; ++k) {
+                const float4 q = cell_nodes[k];
+                const float dist = sq3_fused(p.x - q.x, p.y - q.y, p.z - q.z);
+                if (dist < b.d[4]) {
+                    const int id = __float_as_int(q.w);
+                    const bool b0 = dist < b.d[0], b1 = dist < b.d[1], b2 = dist < b.d[2], b3 = dist < b.d[3];
+                    b.d[4] = b3 ? b.d[3] : dist;
+                    b.d[3] = b2 ? b.d[2] : (b3 ? dist : b.d[3]);
+                    b.id[3] = b2 ? b.id[2] : (b3 ? id : b.id[3]);
+                    b.d[2] = b1 ? b.d[1] : (b2 ? dist : b.d[2]);
+                    b.id[2] = b1 ? b.id[1] : (b2 ? id : b.id[2]);
+                    b.d[1] = b0 ? b.d[0] : (b1 ? dist : b.d[1]);
+                    b.id[1] = b0 ? b.id[0] : (b1 ? id : b.id[1]);
+                    b.d[0] = b0 ? dist : b.d[0];
+                    b.id[0] = b0 ? id : b.id[0];
+                }
+            }
+        }
+    }
+    // distance to the nearest face of the 3 x 3 x 3 cells, less the margin
+    const float fx = sx - floorf(sx), fy = sy - floorf(sy), fz = sz - floorf(sz);
+    const float inside = fminf(fminf(fminf(fx, 1.f - fx), fminf(fy, 1.f - fy)), fminf(fz, 1.f - fz));
+    const bool near = fmaxf(fmaxf(fabsf(sx), fabsf(sy)), fabsf(sz)) <= 4096.f;
+    b.reach = near ? fminf(b.reach, (0.99f + inside) * h) : -1.f;
+}
+
+// The surfels of a warp (lane's surfel v at p): the ordered scan where the search does not settle the
+// result, then ids and weights.
+__device__ __forceinline__ void skin_grid_finish(const float4 *nodes, const uint2 *status, int n_nodes, float4 p, int v,
+                                                 bool live, SkinNearest &b, float r2, int normalize, ushort4 *knn,
+                                                 float4 *sw, float4 *cw) {
+    const int lane = threadIdx.x & 31;
+    const bool sure = b.d[0] < b.d[1] && b.d[1] < b.d[2] && b.d[2] < b.d[3] && b.d[3] < b.d[4] && b.reach > 0.f &&
+                      b.d[3] < b.reach * b.reach;
+    unsigned open = __ballot_sync(0xffffffffu, live && !sure);
+    while (open) {
+        const int who = __ffs(open) - 1;
+        open &= open - 1;
+        const float px = __shfl_sync(0xffffffffu, p.x, who), py = __shfl_sync(0xffffffffu, p.y, who),
+                    pz = __shfl_sync(0xffffffffu, p.z, who);
+        Heap<4> heap;
+        heap.init(1e6f);
+        for (int i0 = 0; i0 < n_nodes; i0 += 32) {
+            const int i = i0 + lane;
+            float dist = 1e6f;
+            if (i < n_nodes && !node_deleted(status, i)) {
+                const float4 q = nodes[i];
+                dist = sq3_fused(px - q.x, py - q.y, pz - q.z);
+            }
+            for (unsigned m = __ballot_sync(0xffffffffu, dist < heap.max_d); m; m &= m - 1) {
+                const int l = __ffs(m) - 1;
+                heap.update((uint16_t)(i0 + l), __shfl_sync(0xffffffffu, dist, l));
+            }
+        }
+        heap.sort();
+        if (lane == who) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                b.id[i] = heap.id[i];
+                const float4 q = nodes[min(b.id[i], n_nodes - 1)];
+                b.d[i] = sq3_fused(p.x - q.x, p.y - q.y, p.z - q.z);
+            }
+        }
+    }
+    if (!live) return;
+    float wv[4], sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        wv[i] = __expf(-b.d[i] / (2.f * r2));
+        sum += wv[i];
+    }
+    const float inv = 1.f / sum;
+    knn[v] = make_ushort4((uint16_t)b.id[0], (uint16_t)b.id[1], (uint16_t)b.id[2], (uint16_t)b.id[3]);
+    sw[v] = normalize ? make_float4(inv * wv[0], inv * wv[1], inv * wv[2], inv * wv[3])
+                      : make_float4(wv[0], wv[1], wv[2], wv[3]);
+    cw[v] = make_float4(1.f, 1.f, 1.f, 1.f);
+}
+
+// kChunked: more than kSkinGridNodes nodes; a launch then covers at most 32 surfels a warp.
+template <bool kChunked>
+__global__ void __launch_bounds__(kSkinThreads, 1) k_skinning_grid(const float4 *nodes, const uint2 *status, int n_nodes,
+                                                                   const float4 *verts, int first_vert, int n_verts,
+                                                                   float radius, float r2, int normalize, ushort4 *knn,
+                                                                   float4 *sw, float4 *cw) {
+    extern __shared__ __align__(16) unsigned char skin_smem[];
+    float4 *cell_nodes = reinterpret_cast<float4 *>(skin_smem);                                    // one chunk's
+    uint32_t *cell_end = reinterpret_cast<uint32_t *>(skin_smem + 16 * (size_t)min(n_nodes, kSkinGridNodes));
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (kSkinThreads / 32);
+    const int first = first_vert + 32 * (blockIdx.x * (kSkinThreads / 32) + (threadIdx.x >> 5));
+    if constexpr (kChunked) {
+        const int v = first + lane;
+        const bool live = v < n_verts;
+        const float4 p = live ? verts[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+        SkinNearest b;
+        for (int n0 = 0; n0 < n_nodes; n0 += kSkinGridNodes) {
+            const float h = skin_grid_build(nodes, status, n0, min(n_nodes, n0 + kSkinGridNodes), 1.75f * radius,
+                                            cell_nodes, cell_end);
+            if (live) skin_grid_search(p, h, cell_nodes, cell_end, b);
+        }
+        skin_grid_finish(nodes, status, n_nodes, p, v, live, b, r2, normalize, knn, sw, cw);
+    } else {
+        const float h = skin_grid_build(nodes, status, 0, n_nodes, 1.75f * radius, cell_nodes, cell_end);
+        for (int base = first; base < n_verts; base += 32 * warps) {
+            const int v = base + lane;
+            const bool live = v < n_verts;
+            const float4 p = live ? verts[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+            SkinNearest b;
+            if (live) skin_grid_search(p, h, cell_nodes, cell_end, b);
+            skin_grid_finish(nodes, status, n_nodes, p, v, live, b, r2, normalize, knn, sw, cw);
+        }
+    }
+}
+
 // ForwardWarpVertexAndNodeKernel (libs/star/geometry/surfel/SurfelNodeDeformer.cu:13-79) with
 // averageDualQuaternion<4> (libs/star/math/DualQuaternion.hpp:288-306).
 __global__ void k_forward_warp(const float *se3, int num_nodes, const float4 *verts, const float4 *normals, int n,
@@ -981,6 +1238,11 @@ int ws_build_node_graph(const float *nodes, int n, int k, float node_radius, uin
     return ws_build_node_graph_ex(nodes, nullptr, n, k, node_radius, 1, knn, w, edges, stream);
 }
 
+// Nodes from which a full skinning goes over the grid (building it takes about 20 us; both sides measured,
+// k_skinning / grid, at 3000 and 260k surfels: 104 nodes 18 / 40 and 64 / 72 us, 248 nodes 36 / 42 and
+// 134 / 74 us, 305 nodes 42 / 40 and 161 / 71 us, 525 nodes 68 / 38 and 259 / 68 us).
+constexpr int kSkinGridFrom = 300;
+
 int ws_skinning_incremental(const float *nodes, const uint32_t *node_status, int num_nodes, int num_prev_nodes,
                             const float *verts, int num_verts, int num_remaining_surfels, float node_radius,
                             int normalize_weights, uint16_t *knn, float *sw, float *cw, void *stream) {
@@ -992,7 +1254,30 @@ int ws_skinning_incremental(const float *nodes, const uint32_t *node_status, int
     if (count == 0) return WS_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float r2 = node_radius * node_radius;
-    ws::k_skinning<<<(count + 255) / 256, 256, 0, st>>>(
+    if (num_prev_nodes == 0 && num_nodes >= kSkinGridFrom && node_radius > 1e-6f && node_radius < 1e6f) {
+        const bool chunked = num_nodes > ws::kSkinGridNodes;
+        const size_t smem = 16 * (size_t)std::min(num_nodes, ws::kSkinGridNodes) + 4 * (size_t)ws::kSkinCells;
+        constexpr int kMaxSmem = 16 * ws::kSkinGridNodes + 4 * ws::kSkinCells;   // one value, whichever thread calls
+        auto kernel = chunked ? ws::k_skinning_grid<true> : ws::k_skinning_grid<false>;
+        int dev = 0, sms = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
+            cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return WS_ERR_CUDA;
+        const int slab = chunked ? sms * ws::kSkinThreads : count;   // surfels of a launch
+        for (long long v0 = num_remaining_surfels; v0 < num_verts; v0 += slab) {
+            const int v1 = (int)std::min<long long>(num_verts, v0 + slab);
+            const int grid = (int)std::min<long long>(sms, (v1 - v0 + ws::kSkinThreads - 1) / ws::kSkinThreads);
+            kernel<<<grid, ws::kSkinThreads, smem, st>>>(
+                reinterpret_cast<const float4 *>(nodes), reinterpret_cast<const uint2 *>(node_status), num_nodes,
+                reinterpret_cast<const float4 *>(verts), (int)v0, v1, node_radius, r2, normalize_weights ? 1 : 0,
+                reinterpret_cast<ushort4 *>(knn), reinterpret_cast<float4 *>(sw), reinterpret_cast<float4 *>(cw));
+        }
+        return cudaGetLastError() == cudaSuccess ? WS_OK : WS_ERR_CUDA;
+    }
+    // small sets in small blocks: 3001 new surfels are 12 blocks of 256 threads, 47 of 64
+    const int threads = count <= 148 * 256 ? 64 : 256;
+    ws::k_skinning<<<(count + threads - 1) / threads, threads, 0, st>>>(
         reinterpret_cast<const float4 *>(nodes), reinterpret_cast<const uint2 *>(node_status), num_nodes,
         num_prev_nodes, reinterpret_cast<const float4 *>(verts), num_remaining_surfels, num_verts, r2,
         normalize_weights ? 1 : 0, reinterpret_cast<ushort4 *>(knn), reinterpret_cast<float4 *>(sw),
