@@ -575,7 +575,7 @@ int ws_selftest_wait_timeout(void *stream) {
 
 int ws_selftest_grid_barrier_timeout(void *stream) {
     int flags = 0;
-    if (ws::grid_barrier_selftest(&flags, (cudaStream_t)stream) != cudaSuccess) return WS_ERR_CUDA;
+    if (ws::dedup_wait_selftest(&flags, (cudaStream_t)stream) != cudaSuccess) return WS_ERR_CUDA;
     return (flags & 4) ? WS_ERR_TIMEOUT : WS_OK;
 }
 

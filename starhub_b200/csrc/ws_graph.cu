@@ -180,80 +180,78 @@ __global__ void k_voxel_sample(const uint32_t *keys, const uint32_t *perm, const
 // candidates in order and keeps one when no candidate kept before it lies within 0.85 R
 // (squared distance <= (0.85 R)^2, summed as ((dx*dx + dy*dy) + dz*dz) + dw*dw with dw = 0).
 // That is the lexicographically first maximal independent set of the graph that joins
-// candidates within 0.85 R, and it comes out of rounds: a candidate is rejected once one of
-// its earlier neighbours is kept, and kept once all of them are rejected.  Every decision is
-// final and equals the sequential loop's (by induction on the index), and each round decides
-// at least the lowest undecided candidate, so at most nv rounds run.
+// candidates within 0.85 R: a candidate is rejected once one of its earlier neighbours is kept, and
+// kept once all of them are rejected.  Every decision is final and equals the sequential loop's (by
+// induction on the index), and the lowest undecided candidate can always be decided.
 
 // Dedup grid: cells of 1.125 x the overlap radius.  Two candidates that pass the distance test
 // differ by at most r (1 + 2^-22) per axis, i.e. 0.889 cells; the scaled coordinates are
 // clamped to +-2^18 cells, where a float resolves 1/32 of a cell, so their rounding adds at most
-// 1/32 and such candidates lie in the same or adjacent cells.  Cell coordinates wrap at 1024
-// per axis, which only adds far candidates that the distance test turns away.
+// 1/32 and such candidates lie in the same or adjacent cells.  Cell coordinates wrap at
+// kDedupCells per axis, which only adds far candidates that the distance test turns away.  The
+// candidates are put in cell order by counting (a table of all cells, counts, a scan, placement): their
+// order within a cell is left open, since no decision depends on it.  Sorting them by a 30-bit cell key
+// and searching it took 13 launches and 18 binary searches a candidate.
 constexpr float kDedupCellScale = 1.125f;
+constexpr int kDedupCells = 64;                                              // per axis
+constexpr uint32_t kDedupTable = kDedupCells * kDedupCells * kDedupCells;
 
 __device__ __forceinline__ int dedup_cell(float v, float inv_cell) {
     return __float2int_rd(fminf(fmaxf(__fmul_rn(v, inv_cell), -262144.f), 262144.f));
 }
 
 __device__ __forceinline__ uint32_t dedup_key(int x, int y, int z) {
-    return (uint32_t)(x & 1023) | ((uint32_t)(y & 1023) << 10) | ((uint32_t)(z & 1023) << 20);
+    constexpr int m = kDedupCells - 1;
+    return (uint32_t)(x & m) + kDedupCells * ((uint32_t)(y & m) + kDedupCells * (uint32_t)(z & m));
+}
+__device__ __forceinline__ uint32_t dedup_key_of(float4 p, float inv_cell) {
+    return dedup_key(dedup_cell(p.x, inv_cell), dedup_cell(p.y, inv_cell), dedup_cell(p.z, inv_cell));
 }
 
-__global__ void k_dedup_keys(const float4 *cand, uint32_t nv, float inv_cell, uint32_t *keys, uint32_t *ids, int *err) {
+__global__ void k_dedup_count(const float4 *cand, uint32_t nv, float inv_cell, uint32_t *table, int *err) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
         const float4 p = cand[i];
         if (isnan(p.x) || isnan(p.y) || isnan(p.z)) atomicOr(err, 1);
-        keys[i] = dedup_key(dedup_cell(p.x, inv_cell), dedup_cell(p.y, inv_cell), dedup_cell(p.z, inv_cell));
-        ids[i] = i;
+        atomicAdd(table + dedup_key_of(p, inv_cell), 1u);
     }
 }
 
-__device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t n, uint32_t key) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
+// table: first position of every cell; on return the end of every cell (the next one's first).
+__global__ void k_dedup_place(const float4 *cand, uint32_t nv, float inv_cell, uint32_t *table, float4 *placed) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
+        const float4 p = cand[i];
+        placed[atomicAdd(table + dedup_key_of(p, inv_cell), 1u)] = make_float4(p.x, p.y, p.z, __uint_as_float(i));
     }
-    return lo;
 }
 
 // Earlier candidates that overlap candidate i, found in the 3 x 3 rows of three cells around
-// it (a row is one key range unless its x wraps).  kFill = false counts them into `cnt`;
+// it (a row is one range unless its x wraps).  kFill = false counts them into `cnt`;
 // kFill = true writes their indices from offset `cnt[i]` of `nbr`.
 template <bool kFill>
-__global__ void k_dedup_neighbours(const float4 *cand, const uint32_t *cell_keys, const uint32_t *cell_ids, uint32_t nv,
-                                   float inv_cell, float thr, uint32_t *cnt, uint32_t *nbr) {
+__global__ void k_dedup_neighbours(const float4 *cand, const uint32_t *cell_end, const float4 *placed, uint32_t nv,
+                                   float inv_cell, float thr, uint32_t *cnt, uint32_t *nbr, uint32_t cap, int *err) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
         const float4 p = cand[i];
         const int cx = dedup_cell(p.x, inv_cell), cy = dedup_cell(p.y, inv_cell), cz = dedup_cell(p.z, inv_cell);
-        const int x0 = (cx - 1) & 1023, x1 = (cx + 1) & 1023;
+        const uint32_t x0 = (uint32_t)(cx - 1) & (kDedupCells - 1), x1 = (uint32_t)(cx + 1) & (kDedupCells - 1);
+        const int ranges = x0 < x1 ? 1 : 2;
         uint32_t c = 0, out = kFill ? cnt[i] : 0u;
-        for (int dz = -1; dz <= 1; ++dz) {
-            for (int dy = -1; dy <= 1; ++dy) {
-                uint32_t lo_key[2], hi_key[2];
-                int ranges = 1;
-                if (x0 < x1) {
-                    lo_key[0] = dedup_key(x0, cy + dy, cz + dz);
-                    hi_key[0] = dedup_key(x1, cy + dy, cz + dz);
-                } else {
-                    lo_key[0] = dedup_key(x0, cy + dy, cz + dz);
-                    hi_key[0] = dedup_key(1023, cy + dy, cz + dz);
-                    lo_key[1] = dedup_key(0, cy + dy, cz + dz);
-                    hi_key[1] = dedup_key(x1, cy + dy, cz + dz);
-                    ranges = 2;
-                }
-                for (int q = 0; q < ranges; ++q) {
-                    for (uint32_t b = lower_bound_u32(cell_keys, nv, lo_key[q]); b < nv && __ldg(cell_keys + b) <= hi_key[q];
-                         ++b) {
-                        const uint32_t j = __ldg(cell_ids + b);
-                        if (j >= i) continue;
-                        const float4 o = cand[j];
-                        const float ex = o.x - p.x, ey = o.y - p.y, ez = o.z - p.z;
-                        const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
-                        if (d2 <= thr) {
-                            if (kFill) nbr[out++] = j; else ++c;
-                        }
+        for (int row = 0; row < 9; ++row) {
+            const uint32_t c0 = dedup_key(0, cy + row % 3 - 1, cz + row / 3 - 1);
+            for (int q = 0; q < ranges; ++q) {
+                const uint32_t lo = c0 + (ranges == 1 || q == 0 ? x0 : 0u);
+                const uint32_t hi = c0 + (ranges == 1 || q == 1 ? x1 : (uint32_t)(kDedupCells - 1));
+                const uint32_t e = __ldg(cell_end + hi);
+                for (uint32_t b = lo > 0 ? __ldg(cell_end + lo - 1) : 0u; b < e; ++b) {
+                    const float4 o = placed[b];
+                    const uint32_t j = __float_as_uint(o.w);
+                    if (j >= i) continue;
+                    const float ex = o.x - p.x, ey = o.y - p.y, ez = o.z - p.z;
+                    const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
+                    if (d2 <= thr) {
+                        if (!kFill) ++c;
+                        else if (out < cap) nbr[out++] = j;
+                        else atomicOr(err, 8);
                     }
                 }
             }
@@ -261,147 +259,95 @@ __global__ void k_dedup_neighbours(const float4 *cand, const uint32_t *cell_keys
         if (!kFill) cnt[i] = c;
     }
 }
+// Overlapping pairs per candidate: a candidate is the only one of its voxel (0.7 R), and a ball of 0.85 R
+// around one meets at most 4^3 voxels, so it has at most 63 neighbours and half of them are earlier.  (Far
+// from the origin, where floats are coarser than that, `err` gets 8 and the lists are made again as long as
+// they need to be.)
+constexpr uint32_t kDedupPairsPerCandidate = 32;
 
-// The rounds for small candidate sets (at most kDedupOneBlockMax), in one block of 1024
-// threads.  Decisions (0 open, 1 kept, 2 rejected) live in shared memory, one byte per
-// candidate, and are read volatile, so a decision taken earlier in the same round is used at
-// once.  Thread t walks candidates t, t + 1024, ... from the first one it has not yet settled.
-// On return `decision` holds every decision; `err` is set only if nv + 1 rounds left a
-// candidate open, which the argument above excludes.
-constexpr int kDedupThreads = 1024;
-constexpr uint32_t kDedupOneBlockMax = 16384;
+// The decisions, without rounds: thread t takes candidates t, t + T, ... (T threads in all) in turn and
+// re-reads a candidate's open earlier neighbours until one is kept (rejected) or none is open (kept).
+// Decisions (0 open, 1 kept, 2 rejected; zeroed before the launch) are final and read volatile from L2.
+// All blocks are resident (a cooperative launch) and a thread's earlier candidates are settled, so the
+// lowest open candidate is always being polled and can be decided.  What bounds it is the longest chain
+// of candidates that wait for one another, at an L2 round trip each; a round behind a grid barrier cost
+// about 15 us each (89k candidates, 361 rounds: 5429 -> 179 us; 5k candidates, in one block: 470 -> 50 us).
+// A candidate's wait is bounded: after kDedupFreePolls polls it sleeps between polls, and gives up after
+// about two seconds of requested sleep, or when another has: `err` gets 4 and the thread leaves.
+constexpr int kDedupThreads = 128;
+constexpr int kDedupFreePolls = 4096;
+constexpr unsigned kDedupSleepNs = 256;
+constexpr unsigned long long kDedupTimeoutNs = 2000000000ull;
 
-__global__ void __launch_bounds__(kDedupThreads) k_dedup_greedy(const uint32_t *nbr_ptr, const uint32_t *nbr, uint32_t nv,
-                                                                uint8_t *decision, int *err) {
-    extern __shared__ uint8_t s_decision[];
-    volatile uint8_t *dec = s_decision;
-    for (uint32_t i = threadIdx.x; i < nv; i += kDedupThreads) dec[i] = 0;
-    __syncthreads();
-    uint32_t first = threadIdx.x;
-    bool done = false;
-    for (uint32_t round = 0; round <= nv && !done; ++round) {   // uniform: `done` comes from a block vote
-        int open = 0;
-        bool settled_prefix = true;
-        for (uint32_t i = first; i < nv; i += kDedupThreads) {
-            uint8_t d = dec[i];
-            if (d == 0) {
-                d = 1;
-                for (uint32_t k = __ldg(nbr_ptr + i), e = __ldg(nbr_ptr + i + 1); k < e; ++k) {
-                    const uint8_t t = dec[__ldg(nbr + k)];
-                    if (t == 1) { d = 2; break; }
-                    if (t == 0) d = 0;
-                }
-                if (d != 0) dec[i] = d;
-            }
-            if (d == 0) {
-                open = 1;
-                settled_prefix = false;
-            } else if (settled_prefix) {
-                first = i + kDedupThreads;
-            }
+__device__ void dedup_decide(const uint32_t *nbr_ptr, const uint32_t *nbr, uint32_t cap, uint32_t first, uint32_t nv,
+                             uint32_t step, volatile uint8_t *dec, int *err) {
+    constexpr int kBatch = 8;   // neighbours polled side by side; few candidates have more
+    uint32_t i = first, b = 0, e = 0;
+    uint32_t id[kBatch];
+    auto load = [&]() {
+        if (i >= nv) return;
+        b = __ldg(nbr_ptr + i);
+        e = min(__ldg(nbr_ptr + i + 1), cap);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) id[k] = b + k < e ? __ldg(nbr + b + k) : 0u;
+    };
+    load();
+    int polls = 0;
+    unsigned long long waited_ns = 0;
+    while (i < nv) {
+        uint8_t t[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) t[k] = b + k < e ? dec[id[k]] : (uint8_t)2;
+        bool kept = false, open = false;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            kept = kept || t[k] == 1;
+            open = open || t[k] == 0;
         }
-        done = !__syncthreads_or(open);
-    }
-    if (!done && threadIdx.x == 0) atomicOr(err, 2);
-    for (uint32_t i = threadIdx.x; i < nv; i += kDedupThreads) decision[i] = s_decision[i];
-}
-
-// The same rounds over the whole GPU, for large candidate sets.  One launch whose blocks are
-// all resident (a cooperative launch); thread t takes candidates t, t + T, ... (T threads in
-// all); decisions in global memory (zeroed before the launch), read volatile; a barrier of our
-// own between rounds.  sync[0] counts a barrier's arrivals, sync[1] is its generation, and
-// sync[2 + r % 2] says whether round r left a candidate open: every write to it comes before
-// round r's barrier, so all threads read the same value after it, and the barrier's last
-// arrival clears the other word for round r + 1 (its readers, in round r - 1, have all arrived).
-// A barrier wait sleeps with backoff and gives up after about two seconds of requested sleep,
-// or at once when another block has: `err` gets 4 and the blocks leave.
-constexpr int kDedupGridThreads = 512;
-constexpr unsigned long long kDedupBarrierTimeoutNs = 2000000000ull;
-
-__device__ bool dedup_grid_barrier(unsigned *sync, unsigned clear_word, int *err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ok = 1;
-        volatile unsigned *gen = sync + 1;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(sync, 1u) == gridDim.x - 1) {
-            atomicExch(sync + clear_word, 0u);
-            atomicExch(sync, 0u);
-            __threadfence();
-            atomicAdd(sync + 1, 1u);
-        } else {
-            unsigned long long waited_ns = 0;
-            unsigned sleep_ns = 32;
-            while (*gen == g) {
-                if (waited_ns > kDedupBarrierTimeoutNs || (*reinterpret_cast<volatile int *>(err) & 4) != 0) {
-                    atomicOr(err, 4);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(sleep_ns);
-                waited_ns += sleep_ns;
-                sleep_ns = min(sleep_ns * 2u, 256u);
-            }
+        for (uint32_t k = b + kBatch; k < e && !kept; ++k) {
+            const uint8_t u = dec[__ldg(nbr + k)];
+            kept = u == 1;
+            open = open || u == 0;
         }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
-__global__ void __launch_bounds__(kDedupGridThreads) k_dedup_greedy_grid(const uint32_t *nbr_ptr, const uint32_t *nbr,
-                                                                        uint32_t nv, uint8_t *decision, unsigned *sync,
-                                                                        int *err) {
-    volatile uint8_t *dec = decision;
-    const uint32_t threads = gridDim.x * blockDim.x;
-    uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint32_t round = 0; round <= nv; ++round) {   // uniform: the exit reads a word written before the barrier
-        int open = 0;
-        bool settled_prefix = true;
-        for (uint32_t i = first; i < nv; i += threads) {
-            uint8_t d = dec[i];
-            if (d == 0) {
-                d = 1;
-                for (uint32_t k = __ldg(nbr_ptr + i), e = __ldg(nbr_ptr + i + 1); k < e; ++k) {
-                    const uint8_t t = dec[__ldg(nbr + k)];
-                    if (t == 1) { d = 2; break; }
-                    if (t == 0) d = 0;
-                }
-                if (d != 0) dec[i] = d;
+        if (kept || !open) {
+            dec[i] = kept ? 2 : 1;
+            i += step;
+            load();
+            polls = 0;
+            waited_ns = 0;
+        } else if (++polls > kDedupFreePolls) {
+            if (waited_ns > kDedupTimeoutNs || (*reinterpret_cast<volatile int *>(err) & 4) != 0) {
+                atomicOr(err, 4);
+                return;
             }
-            if (d == 0) {
-                open = 1;
-                settled_prefix = false;
-            } else if (settled_prefix) {
-                first = i + threads;
-            }
+            __nanosleep(kDedupSleepNs);
+            waited_ns += kDedupSleepNs;
         }
-        volatile unsigned *flag = sync + 2 + (round & 1);
-        if (open) *flag = 1u;
-        if (!dedup_grid_barrier(sync, 2 + ((round + 1) & 1), err)) return;
-        if (*flag == 0u) return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, 2);
 }
 
-// Failure-detection self-test of the barrier above: two blocks launched, only block 0 arrives,
-// so the generation never advances and block 0 must give up after about two seconds of
-// requested sleep with bit 2 of err set, and return.
-__global__ void k_barrier_selftest(unsigned *sync, int *err) {
-    if (blockIdx.x == 0) dedup_grid_barrier(sync, 2, err);
+__global__ void __launch_bounds__(kDedupThreads) k_dedup_decide(const uint32_t *nbr_ptr, const uint32_t *nbr, uint32_t cap,
+                                                                uint32_t nv, uint8_t *decision, int *err) {
+    dedup_decide(nbr_ptr, nbr, cap, blockIdx.x * kDedupThreads + threadIdx.x, nv, gridDim.x * kDedupThreads, decision,
+                 err);
 }
 
-cudaError_t grid_barrier_selftest(int *flags, cudaStream_t st) {
-    unsigned *words = nullptr;   // sync[0..3], err
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&words), 5 * sizeof(unsigned), st);
+// Failure-detection self-test of the wait above: one thread takes candidate 1, whose earlier neighbour 0
+// nobody decides, and must give up after about two seconds of requested sleep with bit 2 of err set.
+__global__ void k_dedup_wait_selftest(const uint32_t *nbr_ptr, const uint32_t *nbr, uint8_t *decision, int *err) {
+    dedup_decide(nbr_ptr, nbr, 1, 1, 2, 2, decision, err);
+}
+
+cudaError_t dedup_wait_selftest(int *flags, cudaStream_t st) {
+    const uint32_t host[8] = {0, 0, 1, 0, 0, 0, 0, 0};   // nbr_ptr[0..2], nbr[0], decisions, err
+    uint32_t *words = nullptr;
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&words), sizeof(host), st);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(words, 0, 5 * sizeof(unsigned), st);
-    int *err = reinterpret_cast<int *>(words + 4);
+    e = cudaMemcpyAsync(words, host, sizeof(host), cudaMemcpyHostToDevice, st);
+    int *err = reinterpret_cast<int *>(words + 5);
     int flag = 0;
     if (e == cudaSuccess) {
-        k_barrier_selftest<<<2, 32, 0, st>>>(words, err);
+        k_dedup_wait_selftest<<<1, 1, 0, st>>>(words, words + 3, reinterpret_cast<uint8_t *>(words + 4), err);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, err, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -1052,7 +998,7 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
     uint32_t *keys = mem.get<uint32_t>(4ull * (n + 1)), *vals = mem.get<uint32_t>(4ull * (n + 1));
     uint32_t *keys2 = mem.get<uint32_t>(4ull * (n + 1)), *vals2 = mem.get<uint32_t>(4ull * (n + 1));
     uint32_t *heads = mem.get<uint32_t>(4ull * (n + 1));
-    uint32_t *tmp = mem.get<uint32_t>(4ull * (n / ws::kScanTile + 4));
+    uint32_t *tmp = mem.get<uint32_t>(4ull * (std::max(n, ws::kDedupTable) / ws::kScanTile + 4));
     uint32_t *hist = mem.get<uint32_t>(4ull * 256 * ws::sort_max_tiles(n));
     uint32_t *digit = mem.get<uint32_t>(4ull * 256);
     float4 *cand = mem.get<float4>(16ull * n);
@@ -1077,69 +1023,63 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
     const float r = 0.85f * node_radius;
     const float thr = r * r;
     const float inv_cell = 1.0f / (ws::kDedupCellScale * r);
-    uint32_t *cnt = heads;   // free again: the candidates are written
-    uint32_t total = 0;
-    int flag = 0;
-    const uint32_t *ck = nullptr, *ci = nullptr;
-    uint32_t *spare_keys = nullptr, *spare_vals = nullptr;
-    {
-        if (cudaMemsetAsync(err, 0, 4, st) != cudaSuccess) return WS_ERR_CUDA;
-        ws::k_dedup_keys<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, keys, vals, err);
-        const bool alt = ws::radix_sort<uint32_t>(keys, vals, keys2, vals2, nullptr, nv, nv, 30, hist, digit, st);
-        ck = alt ? keys2 : keys;
-        ci = alt ? vals2 : vals;
-        spare_keys = alt ? keys : keys2;
-        spare_vals = alt ? vals : vals2;
-        ws::k_dedup_neighbours<false><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, ck, ci, nv, inv_cell, thr, cnt, nullptr);
-        ws::exclusive_scan(cnt, cnt, nullptr, nv, nv, tmp, st);
-        if (cudaMemcpyAsync(&total, cnt + nv, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    uint32_t *cnt = heads, *pos = vals2;   // free again: the candidates are written
+    uint32_t pairs = (uint32_t)std::min<uint64_t>((uint64_t)ws::kDedupPairsPerCandidate * nv, 0xFFFFFFF0ull);
+    uint32_t *table = mem.get<uint32_t>(4ull * (ws::kDedupTable + 1));
+    float4 *placed = mem.get<float4>(16ull * nv);
+    uint32_t *nbr = mem.get<uint32_t>(4ull * pairs);
+    uint8_t *decision = mem.get<uint8_t>(nv);
+    int dev = 0, sms = 0, per_sm = 0, coop = 0, flag = 0;
+    if (mem.err != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ws::k_dedup_decide, ws::kDedupThreads, 0) != cudaSuccess ||
+        per_sm < 1)
+        return WS_ERR_CUDA;
+    if (cudaMemsetAsync(err, 0, 4, st) != cudaSuccess || cudaMemsetAsync(decision, 0, nv, st) != cudaSuccess ||
+        cudaMemsetAsync(table, 0, 4ull * ws::kDedupTable, st) != cudaSuccess)
+        return WS_ERR_CUDA;
+    ws::k_dedup_count<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, table, err);
+    ws::exclusive_scan(table, table, nullptr, ws::kDedupTable, ws::kDedupTable, tmp, st);
+    ws::k_dedup_place<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, table, placed);
+    ws::k_dedup_neighbours<false><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, thr, cnt,
+                                                                       nullptr, 0, err);
+    ws::exclusive_scan(cnt, cnt, nullptr, nv, nv, tmp, st);
+    uint32_t count = 0;
+    for (int attempt = 0;; ++attempt) {
+        ws::k_dedup_neighbours<true><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, thr, cnt,
+                                                                          nbr, pairs, err);
+        const long long want = ((long long)nv + ws::kDedupThreads - 1) / ws::kDedupThreads;
+        const int grid = (int)std::min<long long>(want, (long long)per_sm * sms);
+        const uint32_t *nbr_ptr = cnt;
+        uint32_t nv_arg = nv;
+        void *args[] = {(void *)&nbr_ptr, (void *)&nbr, (void *)&pairs, (void *)&nv_arg, (void *)&decision, (void *)&err};
+        if (cudaLaunchCooperativeKernel((const void *)ws::k_dedup_decide, dim3(grid), dim3(ws::kDedupThreads), args, 0,
+                                        st) != cudaSuccess) {
+            cudaGetLastError();   // a refused launch leaves no sticky error for later checks
+            return WS_ERR_CUDA;
+        }
+        ws::k_dedup_flags<<<ws::grid_of(nv, 256), 256, 0, st>>>(decision, nv, pos);
+        ws::exclusive_scan(pos, pos, nullptr, nv, nv, tmp, st);
+        ws::k_dedup_emit<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, decision, pos, nv, *nodes);
+        if (cudaGetLastError() != cudaSuccess) return WS_ERR_CUDA;
+        uint32_t total = 0;
+        if (cudaMemcpyAsync(&count, pos + nv, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaMemcpyAsync(&total, cnt + nv, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaMemcpyAsync(&flag, err, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return WS_ERR_CUDA;
         // AppendNodeFromVertexHost stops on a NaN candidate (LOG(FATAL)).
         if (flag & 1) return WS_ERR_INVALID_ARGUMENT;
+        if (!(flag & 8)) break;
+        if (attempt > 0) return WS_ERR_CUDA;
+        pairs = total;
+        nbr = mem.get<uint32_t>(4ull * pairs);
+        if (mem.err != cudaSuccess || cudaMemsetAsync(err, 0, 4, st) != cudaSuccess ||
+            cudaMemsetAsync(decision, 0, nv, st) != cudaSuccess)
+            return WS_ERR_CUDA;
     }
-    uint32_t *nbr = mem.get<uint32_t>(4ull * total);
-    if (mem.err != cudaSuccess) return WS_ERR_CUDA;
-    ws::k_dedup_neighbours<true><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, ck, ci, nv, inv_cell, thr, cnt, nbr);
-    uint8_t *decision = reinterpret_cast<uint8_t *>(spare_keys);
-    if (nv <= ws::kDedupOneBlockMax) {   // 16 KB of shared memory at most
-        ws::k_dedup_greedy<<<1, ws::kDedupThreads, nv, st>>>(cnt, nbr, nv, decision, err);
-    } else {
-        unsigned *sync = mem.get<unsigned>(16);
-        int dev = 0, sms = 0, per_sm = 0, coop = 0;
-        if (mem.err != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ws::k_dedup_greedy_grid, ws::kDedupGridThreads, 0) !=
-                cudaSuccess ||
-            per_sm < 1)
-            return WS_ERR_CUDA;
-        const long long want = ((long long)nv + ws::kDedupGridThreads - 1) / ws::kDedupGridThreads;
-        const int grid = (int)std::min<long long>(want, (long long)per_sm * sms);
-        if (cudaMemsetAsync(decision, 0, nv, st) != cudaSuccess || cudaMemsetAsync(sync, 0, 16, st) != cudaSuccess)
-            return WS_ERR_CUDA;
-        const uint32_t *nbr_ptr = cnt;
-        uint32_t nv_arg = nv;
-        void *args[] = {(void *)&nbr_ptr, (void *)&nbr, (void *)&nv_arg, (void *)&decision, (void *)&sync, (void *)&err};
-        if (cudaLaunchCooperativeKernel((const void *)ws::k_dedup_greedy_grid, dim3(grid), dim3(ws::kDedupGridThreads),
-                                        args, 0, st) != cudaSuccess) {
-            cudaGetLastError();   // a refused launch leaves no sticky error for later checks
-            return WS_ERR_CUDA;
-        }
-    }
-    uint32_t *pos = spare_vals;
-    ws::k_dedup_flags<<<ws::grid_of(nv, 256), 256, 0, st>>>(decision, nv, pos);
-    ws::exclusive_scan(pos, pos, nullptr, nv, nv, tmp, st);
-    ws::k_dedup_emit<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, decision, pos, nv, *nodes);
-    if (cudaGetLastError() != cudaSuccess) return WS_ERR_CUDA;
-    uint32_t count = 0;
-    if (cudaMemcpyAsync(&count, pos + nv, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaMemcpyAsync(&flag, err, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return WS_ERR_CUDA;
     if (flag & 4) return WS_ERR_TIMEOUT;
-    if (flag & 2) return WS_ERR_CUDA;
     *kept = count;
     return WS_OK;
 }
