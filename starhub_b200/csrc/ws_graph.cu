@@ -376,40 +376,13 @@ __global__ void k_fill_u32(uint32_t *a, uint32_t n, uint32_t v) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = v;
 }
 
-// Bounding boxes of runs of kGraphRun consecutive nodes (lo in boxes[0, runs), hi after).
-// NaN coordinates stay out of a box: fminf/fmaxf return the other operand.
-constexpr int kGraphRun = 32;
-
-__global__ void k_node_boxes(const float4 *nodes, int n, float4 *lo, float4 *hi) {
-    const int runs = (n + kGraphRun - 1) / kGraphRun;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < runs; r += gridDim.x * blockDim.x) {
-        float4 a = make_float4(INFINITY, INFINITY, INFINITY, 0.f), b = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-        for (int k = r * kGraphRun, e = min(n, (r + 1) * kGraphRun); k < e; ++k) {
-            const float4 p = nodes[k];
-            a.x = fminf(a.x, p.x); a.y = fminf(a.y, p.y); a.z = fminf(a.z, p.z);
-            b.x = fmaxf(b.x, p.x); b.y = fmaxf(b.y, p.y); b.z = fmaxf(b.z, p.z);
-        }
-        lo[r] = a;
-        hi[r] = b;
-    }
-}
-
 // UpdateNodeDistanceKernel + BuildNodeGraphKernel (libs/star/geometry/node_graph/NodeGraph.cu:10-101):
 // half-precision squared distances, k nearest including the node itself, __expf weights normalized.
 //
 // The reference fills an n x n table of half distances and scans a row of it in column order.
-// Here each node scans the other nodes in the same order but skips a run of kGraphRun whose
-// box is no nearer than the heap's current maximum.  Such a run cannot change the heap: the
-// per-axis gap to the box is at most each member's |dx| (a difference rounded to nearest is
-// monotone in its operands), the squared sum and the rounding to half are monotone too, so
-// the same expression on the gaps bounds every member's half distance from below, and the
-// heap only takes a distance strictly below its maximum.  Every heap update of the full scan
-// happens in the same order, so ids, weights and their ties come out the same.
-//
 // With node_status, a pair with a deleted node (status .y == kDeletedNodeStatus, NodeGraph.h:18)
 // gets the half of 1e6, which is infinite (NodeGraph.cu:20-35), so it never enters a heap; a
-// deleted node's own row keeps the heap's initial entries.  The boxes may still hold deleted
-// nodes: that only makes them larger, and the skip stays exact.  `normalize` divides the weights
+// deleted node's own row keeps the heap's initial entries.  `normalize` divides the weights
 // by their sum (USE_INTERPOLATE_WEIGHT_NORMALIZATION, NodeGraph.cu:87-99); without it they are the
 // raw __expf values, as the reference's geometry library compiles them.
 constexpr uint32_t kDeletedNodeStatus = 0xffffffffu;
@@ -417,46 +390,83 @@ __device__ __forceinline__ bool node_deleted(const uint2 *status, int i) {
     return status != nullptr && status[i].y == kDeletedNodeStatus;
 }
 
+__device__ __forceinline__ float graph_half_distance(float4 a, float4 b) {
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;   // the squares do not see the sign
+    return __half2float(__float2half_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)))));
+}
+
+// Row `a` of the node graph from its K neighbours in order (BuildNodeGraphPairKernel, NodeGraph.cu:103-118).
 template <int K>
-__global__ void k_node_graph(const float4 *nodes, const uint2 *status, int n, float r2, int normalize,
-                             const float4 *box_lo, const float4 *box_hi, uint16_t *knn, float *w, uint16_t *edges) {
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+__device__ __forceinline__ void graph_store(int a, const float *d, const uint16_t *id, float r2, int normalize, uint16_t *knn,
+                                            float *w, uint16_t *edges) {
+    float wv[K], sum = 0.f;
+#pragma unroll
+    for (int q = 0; q < K; ++q) wv[q] = __expf(-d[q] / (2 * r2));
+#pragma unroll
+    for (int q = 0; q < K; ++q) sum += wv[q];
+    const float inv = 1.0f / sum;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        knn[(size_t)a * K + q] = id[q];
+        w[(size_t)a * K + q] = normalize ? wv[q] * inv : wv[q];
+        edges[3 * ((size_t)a * K + q)] = (uint16_t)a;
+        edges[3 * ((size_t)a * K + q) + 1] = id[q];
+        edges[3 * ((size_t)a * K + q) + 2] = (uint16_t)q;
+    }
+}
+
+// The scan in column order, one warp per node: 32 nodes at a time, the heap in K lanes, its updates in node
+// order (a register maximum and two votes each).  Nodes
+// list[0 .. *count) (graphs of many nodes: those that k_node_graph_cells leaves open), or all n.
+constexpr int kGraphThreads = 128;
+template <int K>
+__global__ void __launch_bounds__(kGraphThreads) k_node_graph_ordered(const float4 *nodes, const uint2 *status, int n,
+                                                                      const uint32_t *list, const uint32_t *count, float r2,
+                                                                      int normalize, uint16_t *knn, float *w,
+                                                                      uint16_t *edges) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t rows = list ? min(*count, (uint32_t)n) : (uint32_t)n;
+    const uint32_t warps = gridDim.x * (kGraphThreads / 32);
+    for (uint32_t row = blockIdx.x * (kGraphThreads / 32) + (threadIdx.x >> 5); row < rows; row += warps) {
+        const int a = list ? (int)list[row] : (int)row;
         const float4 va = nodes[a];
-        Heap<K> h;
-        h.init(1e3f);
-        const bool a_deleted = node_deleted(status, a);
-        for (int r0 = 0, run = 0; r0 < n && !a_deleted; r0 += kGraphRun, ++run) {
-            const float4 lo = box_lo[run], hi = box_hi[run];
-            const float gx = fmaxf(fmaxf(lo.x - va.x, va.x - hi.x), 0.f);
-            const float gy = fmaxf(fmaxf(lo.y - va.y, va.y - hi.y), 0.f);
-            const float gz = fmaxf(fmaxf(lo.z - va.z, va.z - hi.z), 0.f);
-            const float bound = __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, __fmul_rn(gx, gx)));
-            if (__half2float(__float2half_rn(bound)) >= h.max_d) continue;
-            for (int b = r0, e = min(n, r0 + kGraphRun); b < e; ++b) {
-                const float4 vb = nodes[b];
-                const float4 hi_v = (a >= b) ? va : vb, lo_v = (a >= b) ? vb : va;
-                const float dx = hi_v.x - lo_v.x, dy = hi_v.y - lo_v.y, dz = hi_v.z - lo_v.z;
-                const float dist = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-                h.update((uint16_t)b, node_deleted(status, b) ? __half2float(__float2half_rn(1e6f))
-                                                               : __half2float(__float2half_rn(dist)));
+        // slot q of the heap in lane q; half distances are not negative, so their bits order like their values
+        uint32_t slot_d = lane < K ? __float_as_uint(1e3f) : 0u, top = __float_as_uint(1e3f);
+        int slot_id = 0;
+        if (!node_deleted(status, a))
+            for (int b0 = 0; b0 < n; b0 += 128) {
+                uint32_t d[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int b = b0 + 32 * q + lane;
+                    float v = INFINITY;   // deleted nodes, NaN and the end: enter no heap
+                    if (b < n && !node_deleted(status, b)) v = graph_half_distance(va, nodes[b]);
+                    d[q] = v < 1e3f ? __float_as_uint(v) : __float_as_uint(INFINITY);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    unsigned m = __ballot_sync(0xffffffffu, d[q] < top);
+                    while (m) {   // in node order; an entry replaces the first slot that holds the maximum
+                        const int l = __ffs(m) - 1;
+                        const uint32_t v = __shfl_sync(0xffffffffu, d[q], l);
+                        const unsigned full = __ballot_sync(0xffffffffu, lane < K && slot_d == top);
+                        if (lane == __ffs(full) - 1) {
+                            slot_d = v;
+                            slot_id = b0 + 32 * q + l;
+                        }
+                        top = __reduce_max_sync(0xffffffffu, slot_d);
+                        m &= __ballot_sync(0xffffffffu, d[q] < top) & (0xfffffffeu << l);
+                    }
+                }
             }
-        }
-        h.sort();
-        float wv[K], sum = 0.f;
-#pragma unroll
-        for (int q = 0; q < K; ++q) wv[q] = __expf(-h.d[q] / (2 * r2));
-#pragma unroll
-        for (int q = 0; q < K; ++q) sum += wv[q];
-        const float inv = 1.0f / sum;
+        Heap<K> h;
 #pragma unroll
         for (int q = 0; q < K; ++q) {
-            knn[(size_t)a * K + q] = h.id[q];
-            w[(size_t)a * K + q] = normalize ? wv[q] * inv : wv[q];
-            // BuildNodeGraphPairKernel (NodeGraph.cu:103-118)
-            edges[3 * ((size_t)a * K + q)] = (uint16_t)a;
-            edges[3 * ((size_t)a * K + q) + 1] = h.id[q];
-            edges[3 * ((size_t)a * K + q) + 2] = (uint16_t)q;
+            h.d[q] = __uint_as_float(__shfl_sync(0xffffffffu, slot_d, q));
+            h.id[q] = (uint16_t)__shfl_sync(0xffffffffu, slot_id, q);
         }
+        h.sort();
+        if (lane == 0) graph_store<K>(a, h.d, h.id, r2, normalize, knn, w, edges);
     }
 }
 
@@ -601,6 +611,96 @@ __device__ float skin_grid_build(const float4 *nodes, const uint2 *status, int n
     }
     __syncthreads();
     return h;
+}
+
+// Node graph over a grid of the nodes, for many nodes.  The scan in column order (k_node_graph_ordered) is
+// O(n^2) and, in voxel order, updates its heap all the way to the node (1673 us for 27k nodes, K = 8).  One
+// block puts the nodes into the cells of the skinning grid (k_graph_grid, 29 us); four lanes a node then keep
+// the K + 1 smallest half distances of the 3 x 3 x 3 cells around it (37 us at 23k).  Where they rise strictly and lie below the half distance of every node outside
+// (the rounding to half is monotone, so that of the squared distance to the cells' faces bounds theirs), the
+// ordered scan ends with the same K in the same order; the others (ties in half precision, 2-5% of the
+// nodes, deleted and far ones) go to a list for the ordered scan, whose longest warp is what is left (284 us).
+__global__ void __launch_bounds__(kSkinThreads, 1) k_graph_grid(const float4 *nodes, const uint2 *status, int n, float h0,
+                                                                float4 *cell_nodes, uint32_t *cell_end, float *h_out,
+                                                                uint32_t *count) {
+    extern __shared__ __align__(16) unsigned char skin_smem[];
+    uint32_t *ends = reinterpret_cast<uint32_t *>(skin_smem);
+    const float h = skin_grid_build(nodes, status, 0, n, h0, cell_nodes, ends);
+    for (int c = threadIdx.x; c < kSkinCells; c += kSkinThreads) cell_end[c] = ends[c];
+    if (threadIdx.x == 0) {
+        *h_out = h;
+        *count = 0;
+    }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kGraphThreads) k_node_graph_cells(const float4 *nodes, const uint2 *status, int n,
+                                                                    const float4 *cell_nodes, const uint32_t *cell_end,
+                                                                    const float *h_in, float r2, int normalize,
+                                                                    uint16_t *knn, float *w, uint16_t *edges,
+                                                                    uint32_t *list, uint32_t *count) {
+    // four lanes a node: lane q of them takes the rows q, q + 4, q + 8
+    const int a = min((int)(blockIdx.x * kGraphThreads + threadIdx.x) >> 2, n - 1), part_lane = threadIdx.x & 3;
+    const bool mine = (int)(blockIdx.x * kGraphThreads + threadIdx.x) >> 2 < n;
+    const float4 p = nodes[a];
+    const float h = *h_in, inv_h = 1.0f / h;
+    float ld[K + 1];
+    uint16_t lid[K + 1];
+#pragma unroll
+    for (int q = 0; q <= K; ++q) { ld[q] = 1e3f; lid[q] = 0; }
+    const float sx = skin_scaled(p.x, inv_h), sy = skin_scaled(p.y, inv_h), sz = skin_scaled(p.z, inv_h);
+    const int cx = __float2int_rd(sx), cy = __float2int_rd(sy), cz = __float2int_rd(sz);
+    const int x0 = (cx - 1) & (kSkinCellsX - 1), x1 = (cx + 1) & (kSkinCellsX - 1);
+    for (int row = part_lane; row < 9; row += 4) {
+        const int c0 = skin_cell(0, cy + row % 3 - 1, cz + row / 3 - 1);
+        for (int part = 0; part < (x0 <= x1 ? 1 : 2); ++part) {
+            const int lo = c0 + (x0 <= x1 || part == 0 ? x0 : 0);
+            const int hi = c0 + (x0 <= x1 || part == 1 ? x1 : kSkinCellsX - 1);
+            const uint32_t e = __ldg(cell_end + hi);
+            for (uint32_t k = lo > 0 ? __ldg(cell_end + lo - 1) : 0u; k < e; ++k) {
+                const float4 v = __ldg(cell_nodes + k);
+                const float dist = graph_half_distance(p, v);
+                if (dist < ld[K]) {
+                    const uint16_t b = (uint16_t)__float_as_int(v.w);
+#pragma unroll
+                    for (int q = K; q >= 0; --q) {   // shift the larger ones up
+                        const bool here = dist < ld[q], below = q > 0 && dist < ld[q > 0 ? q - 1 : 0];
+                        ld[q] = below ? ld[q > 0 ? q - 1 : 0] : (here ? dist : ld[q]);
+                        lid[q] = below ? lid[q > 0 ? q - 1 : 0] : (here ? b : lid[q]);
+                    }
+                }
+            }
+        }
+    }
+    // the four ascending lists into one: K + 1 times the smallest head (of equal ones the lowest lane's; ties
+    // go to the ordered scan anyway)
+    float d[K + 1];
+    uint16_t id[K + 1];
+#pragma unroll
+    for (int q = 0; q <= K; ++q) {
+        float m = ld[0];
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        const unsigned has = (__ballot_sync(0xffffffffu, ld[0] == m) >> (threadIdx.x & 28)) & 15u;
+        const int from = __ffs(has) - 1;
+        d[q] = m;
+        id[q] = (uint16_t)__shfl_sync(0xffffffffu, (int)lid[0], from, 4);
+        if (part_lane == from) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) { ld[k] = ld[k + 1]; lid[k] = lid[k + 1]; }
+            ld[K] = 1e3f;
+        }
+    }
+    if (!mine || part_lane != 0) return;
+    const float fx = sx - floorf(sx), fy = sy - floorf(sy), fz = sz - floorf(sz);
+    const float inside = fminf(fminf(fminf(fx, 1.f - fx), fminf(fy, 1.f - fy)), fminf(fz, 1.f - fz));
+    const float reach = (0.99f + inside) * h;
+    bool sure = fmaxf(fmaxf(fabsf(sx), fabsf(sy)), fabsf(sz)) <= 4096.f && !node_deleted(status, a) &&
+                d[K - 1] < __half2float(__float2half_rn(reach * reach));
+#pragma unroll
+    for (int q = 0; q < K; ++q) sure = sure && d[q] < d[q + 1];
+    if (sure) graph_store<K>(a, d, id, r2, normalize, knn, w, edges);
+    else list[atomicAdd(count, 1u)] = (uint32_t)a;
 }
 
 // One surfel's search: its five nearest so far, ascending, with the ids of four, and the distance up to
@@ -1149,28 +1249,59 @@ int ws_expand_nodes(const float *vertices, int num_vertices, float node_radius, 
     return WS_OK;
 }
 
+// Nodes from which the node graph goes over the grid (us, ordered scan of every node / grid; K = 4 and 8): 1843
+// nodes 40 / 65 and 50 / 76, 4117 72 / 91 and 91 / 109, 8247 170 / 134 and 240 / 151, 26865 1266 / 317 and
+// 1673 / 380.  With one thread a node and box-skipped runs these were 384 us at 1.7k nodes (K = 8) and 2961 at 23k.
+constexpr int kGraphGridFrom = 5000;
+
 int ws_build_node_graph_ex(const float *nodes, const uint32_t *node_status, int n, int k, float node_radius,
                            int normalize_weights, uint16_t *knn, float *w, uint16_t *edges, void *stream) {
     if (!nodes || n <= 0 || n > 65535 || !knn || !w || !edges || (k != 4 && k != 8)) return WS_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float r2 = node_radius * node_radius;
-    const int runs = (n + ws::kGraphRun - 1) / ws::kGraphRun;
-    // Run boxes from the stream-ordered pool: the call stays asynchronous.
-    float4 *boxes = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&boxes), 32ull * runs, st) != cudaSuccess) return WS_ERR_CUDA;
     const float4 *nd = reinterpret_cast<const float4 *>(nodes);
     const uint2 *status = reinterpret_cast<const uint2 *>(node_status);
     const int norm = normalize_weights ? 1 : 0;
-    ws::k_node_boxes<<<ws::grid_of(runs, 128), 128, 0, st>>>(nd, n, boxes, boxes + runs);
-    const int threads = 64;
-    const int grid = (n + threads - 1) / threads;
-    if (k == 4)
-        ws::k_node_graph<4><<<grid, threads, 0, st>>>(nd, status, n, r2, norm, boxes, boxes + runs, knn, w, edges);
-    else
-        ws::k_node_graph<8><<<grid, threads, 0, st>>>(nd, status, n, r2, norm, boxes, boxes + runs, knn, w, edges);
-    const cudaError_t launched = cudaGetLastError();
-    const cudaError_t freed = cudaFreeAsync(boxes, st);
-    return launched == cudaSuccess && freed == cudaSuccess ? WS_OK : WS_ERR_CUDA;
+    if (n < kGraphGridFrom || !(node_radius > 1e-6f && node_radius < 1e6f)) {
+        const int grid = std::min((n + 3) / 4, 148 * 16);
+        if (k == 4)
+            ws::k_node_graph_ordered<4><<<grid, ws::kGraphThreads, 0, st>>>(nd, status, n, nullptr, nullptr, r2, norm, knn,
+                                                                           w, edges);
+        else
+            ws::k_node_graph_ordered<8><<<grid, ws::kGraphThreads, 0, st>>>(nd, status, n, nullptr, nullptr, r2, norm, knn,
+                                                                           w, edges);
+        return cudaGetLastError() == cudaSuccess ? WS_OK : WS_ERR_CUDA;
+    }
+    // the grid and the list of open nodes from the stream-ordered pool: the call stays asynchronous
+    const size_t table = 4ull * ws::kSkinCells, placed = 16ull * n;
+    unsigned char *scratch = nullptr;
+    if (cudaMallocAsync(reinterpret_cast<void **>(&scratch), placed + table + 4ull * n + 16, st) != cudaSuccess)
+        return WS_ERR_CUDA;
+    float4 *cell_nodes = reinterpret_cast<float4 *>(scratch);
+    uint32_t *cell_end = reinterpret_cast<uint32_t *>(scratch + placed);
+    uint32_t *list = reinterpret_cast<uint32_t *>(scratch + placed + table), *count = list + n;
+    float *h = reinterpret_cast<float *>(count + 1);
+    cudaError_t e = cudaFuncSetAttribute(ws::k_graph_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)table);
+    if (e == cudaSuccess) {
+        // the K-th of 8 neighbours (itself among them) lies in the second ring around a node
+        const float h0 = (k == 4 ? 1.75f : 2.2f) * node_radius;
+        ws::k_graph_grid<<<1, ws::kSkinThreads, table, st>>>(nd, status, n, h0, cell_nodes, cell_end, h, count);
+        const int grid = (4 * n + ws::kGraphThreads - 1) / ws::kGraphThreads, open_grid = std::min((n + 3) / 4, 148 * 8);
+        if (k == 4) {
+            ws::k_node_graph_cells<4><<<grid, ws::kGraphThreads, 0, st>>>(nd, status, n, cell_nodes, cell_end, h, r2, norm,
+                                                                         knn, w, edges, list, count);
+            ws::k_node_graph_ordered<4><<<open_grid, ws::kGraphThreads, 0, st>>>(nd, status, n, list, count, r2, norm, knn,
+                                                                                w, edges);
+        } else {
+            ws::k_node_graph_cells<8><<<grid, ws::kGraphThreads, 0, st>>>(nd, status, n, cell_nodes, cell_end, h, r2, norm,
+                                                                         knn, w, edges, list, count);
+            ws::k_node_graph_ordered<8><<<open_grid, ws::kGraphThreads, 0, st>>>(nd, status, n, list, count, r2, norm, knn,
+                                                                                w, edges);
+        }
+        e = cudaGetLastError();
+    }
+    const cudaError_t freed = cudaFreeAsync(scratch, st);
+    return e == cudaSuccess && freed == cudaSuccess ? WS_OK : WS_ERR_CUDA;
 }
 
 int ws_build_node_graph(const float *nodes, int n, int k, float node_radius, uint16_t *knn, float *w, uint16_t *edges,
