@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -26,6 +27,12 @@ cudaError_t dalloc(T **p, size_t n) {
     *p = nullptr;
     if (n == 0) n = 1;
     return cudaMalloc(reinterpret_cast<void **>(p), n * sizeof(T));
+}
+
+// Solvers alive on a device (devices past the table share its last entry).
+std::atomic<int> &live_solvers(int device) {
+    static std::atomic<int> count[65];
+    return count[device >= 0 && device < 64 ? device : 64];
 }
 
 void free_all(ws::Workspace &w) {
@@ -227,16 +234,19 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
         delete h;
         return e == cudaErrorMemoryAllocation ? WS_ERR_CAPACITY : WS_ERR_CUDA;
     }
+    live_solvers(w.device).fetch_add(1);
     *out = h;
     return WS_OK;
 }
 
 int ws_destroy(ws_solver *h) {
     if (!h) return WS_ERR_INVALID_ARGUMENT;
-    cudaSetDevice(h->w.device);
+    const int device = h->w.device;
+    cudaSetDevice(device);
     if (h->w.last_stream) cudaStreamSynchronize(h->w.last_stream);
     free_all(h->w);
     delete h;
+    if (live_solvers(device).fetch_sub(1) == 1) ws::scratch_trim(device);
     return WS_OK;
 }
 

@@ -1063,9 +1063,50 @@ int noalloc_scratch(unsigned long long **out) {
     return WS_OK;
 }
 
-// Device temporaries of a node-growth call, from the stream-ordered pool of `st`: taken and
-// given back in stream order, so later calls reuse the pool's memory without a device-wide
-// synchronisation.
+// Scratch of the geometry calls, taken and given back in stream order from a pool of the library's own per
+// device.  The device's default pool returns its idle memory to the driver at every synchronisation, so the
+// first call after one mapped its scratch again: the solver-map pass of a frame took 479 us instead of 35,
+// and node construction, which synchronises itself, paid for it within each call.  This pool keeps up to
+// kScratchKeep idle bytes (node construction of 1M surfels holds about 50 MB); what is above goes back at the
+// next synchronisation, and all of it when the device's last solver is destroyed (scratch_trim).  In a
+// capture the allocation is the graph's own, as before.
+constexpr unsigned long long kScratchKeep = 64ull << 20;
+std::mutex g_scratch_mutex;
+cudaMemPool_t g_scratch_pool[kMaxDevices] = {};
+
+cudaMemPool_t scratch_pool() {   // null: none for this device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (!g_scratch_pool[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        unsigned long long keep = kScratchKeep;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            if (pool) cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        g_scratch_pool[dev] = pool;
+    }
+    return g_scratch_pool[dev];
+}
+
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (st && cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        capture = cudaStreamCaptureStatusNone;
+    }
+    cudaMemPool_t pool = capture == cudaStreamCaptureStatusNone ? scratch_pool() : nullptr;
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+}
+
+// Device temporaries of a node-growth call.
 struct DeviceBlocks {
     explicit DeviceBlocks(cudaStream_t s) : st(s) {}
     DeviceBlocks(const DeviceBlocks &) = delete;
@@ -1076,7 +1117,7 @@ struct DeviceBlocks {
     template <class T>
     T *get(size_t bytes) {
         void *p = nullptr;
-        if (err == cudaSuccess) err = cudaMallocAsync(&p, std::max<size_t>(bytes, 16), st);
+        if (err == cudaSuccess) err = scratch_alloc(&p, std::max<size_t>(bytes, 16), st);
         if (err != cudaSuccess) return nullptr;
         ptrs.push_back(p);
         return static_cast<T *>(p);
@@ -1186,6 +1227,16 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
 
 }  // namespace
 
+namespace ws {
+
+// Gives the idle scratch of `device` back to the driver.
+void scratch_trim(int device) {
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (g_scratch_pool[device] && cudaMemPoolTrimTo(g_scratch_pool[device], 0) != cudaSuccess) cudaGetLastError();
+}
+
+}  // namespace ws
 
 extern "C" {
 
@@ -1275,7 +1326,7 @@ int ws_build_node_graph_ex(const float *nodes, const uint32_t *node_status, int 
     // the grid and the list of open nodes from the stream-ordered pool: the call stays asynchronous
     const size_t table = 4ull * ws::kSkinCells, placed = 16ull * n;
     unsigned char *scratch = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&scratch), placed + table + 4ull * n + 16, st) != cudaSuccess)
+    if (scratch_alloc(reinterpret_cast<void **>(&scratch), placed + table + 4ull * n + 16, st) != cudaSuccess)
         return WS_ERR_CUDA;
     float4 *cell_nodes = reinterpret_cast<float4 *>(scratch);
     uint32_t *cell_end = reinterpret_cast<uint32_t *>(scratch + placed);
@@ -1388,7 +1439,7 @@ int ws_splat_maps(const float *verts, const float *attr_verts, const float *attr
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned long long *zbuf = nullptr;
     const size_t npix = (size_t)W * H;
-    if (cudaMallocAsync(&zbuf, 8 * npix, st) != cudaSuccess) return WS_ERR_CUDA;
+    if (scratch_alloc(reinterpret_cast<void **>(&zbuf), 8 * npix, st) != cudaSuccess) return WS_ERR_CUDA;
     if (cudaMemsetAsync(zbuf, 0xff, 8 * npix, st) != cudaSuccess) {
         cudaFreeAsync(zbuf, st);
         return WS_ERR_CUDA;
@@ -1443,7 +1494,7 @@ int ws_render_solver_maps(const float *vertex_confid, const float *normal_radius
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t npix = (size_t)p.width * p.height;
     unsigned long long *zbuf = nullptr;
-    if (cudaMallocAsync(&zbuf, 8 * npix, st) != cudaSuccess) return WS_ERR_CUDA;
+    if (scratch_alloc(reinterpret_cast<void **>(&zbuf), 8 * npix, st) != cudaSuccess) return WS_ERR_CUDA;
     if (cudaMemsetAsync(zbuf, 0xff, 8 * npix, st) != cudaSuccess) {
         cudaFreeAsync(zbuf, st);
         return WS_ERR_CUDA;
@@ -1474,7 +1525,7 @@ int ws_render_observation_maps(const float *vertex_confid, const float *normal_r
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t npix = (size_t)p.width * p.height;
     unsigned long long *zbuf = nullptr;
-    if (cudaMallocAsync(&zbuf, 8 * npix, st) != cudaSuccess) return WS_ERR_CUDA;
+    if (scratch_alloc(reinterpret_cast<void **>(&zbuf), 8 * npix, st) != cudaSuccess) return WS_ERR_CUDA;
     if (cudaMemsetAsync(zbuf, 0xff, 8 * npix, st) != cudaSuccess) {
         cudaFreeAsync(zbuf, st);
         return WS_ERR_CUDA;

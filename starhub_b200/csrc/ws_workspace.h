@@ -178,6 +178,8 @@ cudaError_t dedup_wait_selftest(int *flags, cudaStream_t st);
 cudaError_t gn_spmv_matrix_free(Workspace &w, const float *x, float *y, float *ux_dense, float *ux_reg,
                                 cudaStream_t st);
 int pcg_warps_per_block();
+// Gives the geometry calls' idle scratch on a device back to the driver (ws_graph.cu).
+void scratch_trim(int device);
 
 // Launch accounting for the measurement hooks.
 inline void count_launch(Workspace &w, int n = 1) { w.launches += n; }
