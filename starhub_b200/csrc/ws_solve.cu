@@ -221,7 +221,7 @@ __device__ __forceinline__ void reg_unit_jacobian(float3 a, float3 b, bool is_i,
     }
 }
 
-__device__ __forceinline__ int tri_index(int a, int c) {   // upper triangle (a <= c), row-major
+__device__ __forceinline__ constexpr int tri_index(int a, int c) {   // upper triangle (a <= c), row-major
     return a * 6 - (a * (a - 1)) / 2 + (c - a);
 }
 
@@ -351,7 +351,7 @@ __device__ __forceinline__ void fetch_records(float *stage, int lane, int groups
             }
         }
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
 // Dense record fields in the layout DenseLayout<C> (k_eval_dense).
@@ -457,8 +457,12 @@ __device__ __forceinline__ void accumulate_row(DAcc *D, DAcc *B, const float *ro
 
 // NT (threads per block) is chosen by the autotuner among 64, 128 and 256; the work of a
 // warp, and so every sum, is the same for all three.
-template <class DAcc, int NT, int C>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_node(const Scene *scenes, const Plan *plan,
+// A batch is two dependent trips to L2 (list words, then records) for little arithmetic, so two batches are
+// in flight (kBufs = 2): while one is summed, the next one's records are copied and the words of the one
+// after are loaded.  Per launch, one buffer and then two: 500 nodes with lists of about 1000 entries 73 -> 33
+// us, 3000 nodes with flow 178 -> 79, 1800 nodes 38 -> 20; 64 scenes 549 -> 480.
+template <class DAcc, int NT, int C, int kTPL, int kBufs>
+__global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble_node(const Scene *scenes, const Plan *plan,
                                                                      const uint32_t *node_scene, uint32_t total_nodes,
                                                                      const uint32_t *n2t_offset, const uint32_t *n2t_val,
                                                                      uint32_t cap_n2t, const float *drec, const float *rrec,
@@ -469,10 +473,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_node(const Scene *sc
     constexpr bool kCentred = sizeof(DAcc) == 8;   // mixed precision also uses node-centred twists
     constexpr int kSlot = kSlotWordsF32;             // per-lane partial sums at the end (27 floats)
     constexpr int kRec = record_stride<C>();
-    // at most 2 records per lane and 64 registers: 32 warps per SM, which this latency-bound
-    // kernel needs more than deeper batches
-    constexpr int kTPL = terms_per_lane(NT, kRec) < 2 ? terms_per_lane(NT, kRec) : 2;
-    __shared__ __align__(16) float stage[NT / 32][max_int(kTPL * 32 * kRec, 32 * kSlot)];
+    constexpr int kBatch = kTPL * 32 * kRec;         // words of one batch's records
+    __shared__ __align__(16) float stage[NT / 32][max_int(kBufs * kBatch, 32 * kSlot)];
     const int lane = threadIdx.x & 31;
     float *slots = stage[threadIdx.x >> 5];
     float *mine = slots + lane * kSlot;
@@ -483,8 +485,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_node(const Scene *sc
         const uint32_t s = node_scene[g];
         const uint32_t beg = n2t_offset[g], end = n2t_offset[g + 1];
         const float4 c4 = centers[g];
-        // the list past the first batch, into L2 ahead of the later batches' reads
-        if (lane == 0 && end > beg + 32u * kTPL) l2_prefetch_list(n2t_val, beg + 32u * kTPL, end, cap_n2t);
+        // the list past the first batches, into L2 ahead of the later batches' reads
+        if (lane == 0 && end > beg + 32u * kTPL * kBufs) l2_prefetch_list(n2t_val, beg + 32u * kTPL * kBufs, end, cap_n2t);
         const Scene &sc = scenes[s];
         const Plan &p = plan[s];
         const uint32_t nd = p.dense_count, ne = sc.num_edges, nn = sc.num_nodes;
@@ -498,38 +500,68 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_node(const Scene *sc
         for (int i = 0; i < 21; ++i) D[i] = 0.f;
 #pragma unroll
         for (int i = 0; i < 6; ++i) B[i] = 0.f;
-        for (uint32_t base = beg; base < end; base += 32 * kTPL) {
-            // 1 dense, 2 regularisation edge, 3 node motion; feature terms have a zero Jacobian
-            // (PreconditionerRhsBuilder.cu:214-219)
-            auto classify = [&](uint32_t term, const float4 *&src, int &parts) -> int {
-                src = nullptr;
-                parts = 0;
-                if (term < nd) {
-                    src = dbase + (size_t)(DenseLayout<C>::kFloats / 4) * term;
-                    parts = DenseLayout<C>::kFloats / 4;
-                    return 1;
-                }
-                if (term < nd + ne) {
-                    src = rbase + (size_t)(kRegRecord / 4) * (term - nd);
-                    parts = kRegRecord / 4;
-                    return 2;
-                }
-                return (term < nd + ne + nn && motion) ? 3 : 0;
-            };
-            const int groups = (int)min((uint32_t)kTPL, (end - base + 31) / 32);
-            fetch_records<kRec, C == 3 ? 8 : 4, kTPL>(slots, lane, groups, [&](int t, const float4 *&src, int &parts) {
+        // 1 dense, 2 regularisation edge, 3 node motion; feature terms have a zero Jacobian
+        // (PreconditionerRhsBuilder.cu:214-219)
+        auto classify = [&](uint32_t term, const float4 *&src, int &parts) -> int {
+            src = nullptr;
+            parts = 0;
+            if (term < nd) {
+                src = dbase + (size_t)(DenseLayout<C>::kFloats / 4) * term;
+                parts = DenseLayout<C>::kFloats / 4;
+                return 1;
+            }
+            if (term < nd + ne) {
+                src = rbase + (size_t)(kRegRecord / 4) * (term - nd);
+                parts = kRegRecord / 4;
+                return 2;
+            }
+            return (term < nd + ne + nn && motion) ? 3 : 0;
+        };
+        auto read_words = [&](uint32_t base, uint32_t (&w)[kTPL]) {
+#pragma unroll
+            for (int t = 0; t < kTPL; ++t) {
                 const uint32_t it = base + 32 * t + lane;
-                classify(it < end ? n2t_val[it] : kInvalidIndex, src, parts);
+                w[t] = it < end ? n2t_val[it] : kInvalidIndex;
+            }
+        };
+        auto fetch = [&](uint32_t base, const uint32_t (&w)[kTPL], float *buf) {   // an empty group past the list
+            const int groups = base < end ? (int)min((uint32_t)kTPL, (end - base + 31) / 32) : 0;
+            fetch_records<kRec, C == 3 ? 8 : 4, kTPL>(buf, lane, groups, [&](int t, const float4 *&src, int &parts) {
+                classify(w[t], src, parts);
             });
+        };
+        // kBufs = 2: a batch's records are copied while the batch before is summed, and the words of the
+        // batch after it are on their way
+        uint32_t words[kTPL], next[kTPL];
+        read_words(beg, words);
+        if constexpr (kBufs == 2) {
+            fetch(beg, words, slots);
+            read_words(beg + 32 * kTPL, next);
+        }
+        int parity = 0;
+        for (uint32_t base = beg; base < end; base += 32 * kTPL) {
+            const int groups = (int)min((uint32_t)kTPL, (end - base + 31) / 32);
+            const float *records = slots + parity * kBatch;
+            uint32_t after[kTPL];
+            if constexpr (kBufs == 2) {
+                parity ^= 1;
+                fetch(base + 32 * kTPL, next, slots + parity * kBatch);
+                read_words(base + 64 * kTPL, after);
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            } else {
+                fetch(base, words, slots);
+                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            }
             __syncwarp();
 #pragma unroll 1
             for (int t = 0; t < groups; ++t) {
-                const uint32_t it = base + 32 * t + lane;
-                const uint32_t term = it < end ? n2t_val[it] : kInvalidIndex;
+                uint32_t term = words[0];
+#pragma unroll
+                for (int k = 1; k < kTPL; ++k) term = t == k ? words[k] : term;
                 const float4 *src_unused;
                 int parts_unused;
                 const int kind = classify(term, src_unused, parts_unused);
-                const float *rec_t = slots + (32 * t + lane) * kRec;
+                const float *rec_t = records + (32 * t + lane) * kRec;
                 if (kind == 1) {
                     // point-to-plane + optical-flow rows (libs/star/opt/dense_image_jacobian.cuh:9-20)
                     float wk[4];
@@ -577,6 +609,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_node(const Scene *sc
                     }
                 }
             }
+            __syncwarp();
+            if constexpr (kBufs == 2) {
+#pragma unroll
+                for (int t = 0; t < kTPL; ++t) {
+                    words[t] = next[t];
+                    next[t] = after[t];
+                }
+            } else {
+                read_words(base + 32 * kTPL, words);
+            }
+        }
+        if constexpr (kBufs == 2) {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncwarp();
         }
         // lane partial sums -> slots; lane e sums entry e over the lanes in lane order
@@ -661,8 +706,8 @@ __device__ __forceinline__ float pick6(const float *v, int i) {
     return r;
 }
 
-template <int NT, int C>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_pair(
+template <int NT, int C, int kTPL, int kBufs>
+__global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble_pair(
     const Scene *scenes, const Plan *plan, const uint32_t *counts,
     const uint32_t *half_row, const uint32_t *half_col, const uint32_t *half_begin, const uint32_t *half_end,
     const uint32_t *half_scene, const uint32_t *pair_val, uint32_t cap_kv, const uint32_t *slot_up, const float *drec, const float *rrec,
@@ -670,10 +715,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_pair(
     constexpr int kSlot = kSlotWordsF32;   // per-lane partial sums at the end
     static_assert(kSlot >= 36, "a slot holds one lane's 36 partial sums");
     constexpr int kRec = record_stride<C>();
-    // at most 2 records per lane: the staging then leaves room for 32 warps per SM, which
-    // this latency-bound kernel needs more than deeper batches (pair lists are short)
-    constexpr int kTPL = terms_per_lane(NT, kRec) < 2 ? terms_per_lane(NT, kRec) : 2;
-    constexpr int kStageWords = max_int(kTPL * 32 * kRec, 32 * kSlot);
+    constexpr int kBatch = kTPL * 32 * kRec;       // words of one batch's records
+    constexpr int kStageWords = max_int(kBufs * kBatch, 32 * kSlot);
     constexpr int kStash = 4;   // smoothness terms per pair: one per edge direction, so at most 2
     __shared__ __align__(16) float stage[NT / 32][kStageWords + kStash * kRegRecord];
     const int lane = threadIdx.x & 31;
@@ -709,37 +752,73 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_pair(
 #pragma unroll
         for (int i = 0; i < 21; ++i) M[i] = 0.f;
         int nreg = 0;   // warp-uniform: smoothness records stashed so far
-        for (uint32_t base = beg; base < end; base += 32 * kTPL) {
-            // 1 dense, 2 regularisation edge (stashed, added after the dense sums); node-motion
-            // terms own no pairs
-            auto classify = [&](uint32_t term, const float4 *&src, int &parts) -> int {
-                src = nullptr;
-                parts = 0;
-                if (term < nd) {
-                    src = dbase + (size_t)(DenseLayout<C>::kFloats / 4) * term;
-                    parts = DenseLayout<C>::kFloats / 4;
-                    return 1;
-                }
-                if (term < nd + ne) {
-                    src = rbase + (size_t)(kRegRecord / 4) * (term - nd);
-                    parts = kRegRecord / 4;
-                    return 2;
-                }
-                return 0;
-            };
-            const int groups = (int)min((uint32_t)kTPL, (end - base + 31) / 32);
-            fetch_records<kRec, C == 3 ? 8 : 4, kTPL>(slots, lane, groups, [&](int t, const float4 *&src, int &parts) {
+        // 1 dense, 2 regularisation edge (stashed, added after the dense sums); node-motion
+        // terms own no pairs
+        auto classify = [&](uint32_t term, const float4 *&src, int &parts) -> int {
+            src = nullptr;
+            parts = 0;
+            if (term < nd) {
+                src = dbase + (size_t)(DenseLayout<C>::kFloats / 4) * term;
+                parts = DenseLayout<C>::kFloats / 4;
+                return 1;
+            }
+            if (term < nd + ne) {
+                src = rbase + (size_t)(kRegRecord / 4) * (term - nd);
+                parts = kRegRecord / 4;
+                return 2;
+            }
+            return 0;
+        };
+        auto read_words = [&](uint32_t base, uint32_t (&w)[kTPL]) {
+#pragma unroll
+            for (int t = 0; t < kTPL; ++t) {
                 const uint32_t it = base + 32 * t + lane;
-                classify(it < end ? pair_val[it] : kInvalidIndex, src, parts);
+                w[t] = it < end ? pair_val[it] : kInvalidIndex;
+            }
+        };
+        auto fetch = [&](uint32_t base, const uint32_t (&w)[kTPL], float *buf) {   // an empty group past the list
+            const int groups = base < end ? (int)min((uint32_t)kTPL, (end - base + 31) / 32) : 0;
+            fetch_records<kRec, C == 3 ? 8 : 4, kTPL>(buf, lane, groups, [&](int t, const float4 *&src, int &parts) {
+                classify(w[t], src, parts);
             });
+        };
+        // kBufs = 2: as in the node kernel, a batch's records are copied while the batch before is summed
+        uint32_t words[kTPL], next[kTPL];
+        if constexpr (kBufs == 2) {
+            read_words(beg, words);
+            fetch(beg, words, slots);
+            read_words(beg + 32 * kTPL, next);
+        }
+        int parity = 0;
+        for (uint32_t base = beg; base < end; base += 32 * kTPL) {
+            const int groups = (int)min((uint32_t)kTPL, (end - base + 31) / 32);
+            const float *records = slots + parity * kBatch;
+            uint32_t after[kTPL];
+            if constexpr (kBufs == 2) {
+                parity ^= 1;
+                fetch(base + 32 * kTPL, next, slots + parity * kBatch);
+                read_words(base + 64 * kTPL, after);
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            } else {
+                uint32_t now[kTPL];   // read again (from L1) when they are summed: fewer registers
+                read_words(base, now);
+                fetch(base, now, slots);
+                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            }
             __syncwarp();
 #pragma unroll 1
             for (int t = 0; t < groups; ++t) {
-                const uint32_t it = base + 32 * t + lane;
-                const float4 *src_unused;
-                int parts_unused;
-                const int kind = classify(it < end ? pair_val[it] : kInvalidIndex, src_unused, parts_unused);
-                const float *rec_t = slots + (32 * t + lane) * kRec;
+                uint32_t term;
+                if constexpr (kBufs == 2) {
+                    term = words[0];
+#pragma unroll
+                    for (int q = 1; q < kTPL; ++q) term = t == q ? words[q] : term;
+                } else {
+                    const uint32_t it = base + 32 * t + lane;
+                    term = it < end ? pair_val[it] : kInvalidIndex;
+                }
+                const int kind = term < nd ? 1 : (term < nd + ne ? 2 : 0);
+                const float *rec_t = records + (32 * t + lane) * kRec;
                 const unsigned regs = __ballot_sync(0xffffffffu, kind == 2);
                 if (kind == 2) {
                     const int k = nreg + __popc(regs & ((1u << lane) - 1u));
@@ -778,6 +857,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_assemble_pair(
                         for (int j = i; j < 6; ++j) M[tri_index(i, j)] += u[i] * g[j];
                 }
             }
+            __syncwarp();
+            if constexpr (kBufs == 2) {
+#pragma unroll
+                for (int t = 0; t < kTPL; ++t) {
+                    words[t] = next[t];
+                    next[t] = after[t];
+                }
+            }
+        }
+        if constexpr (kBufs == 2) {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncwarp();
         }
         // lane sums of M -> slots; lane e < 21 sums entry e over the lanes in lane order
@@ -2131,11 +2221,19 @@ void gn_eval(Workspace &w, cudaStream_t st) {
     }
 }
 
-template <class DAcc, int NT, int C>
-static void launch_assemble_node_c(Workspace &w, cudaStream_t st) {
-    k_assemble_node<DAcc, NT, C><<<grid_for(w.total_nodes * 32u, NT, w.num_sms, 32 * 128 / NT), NT, 0, st>>>(
+template <class DAcc, int NT, int C, int kTPL, int kBufs>
+static void launch_assemble_node_v(Workspace &w, cudaStream_t st) {
+    k_assemble_node<DAcc, NT, C, kTPL, kBufs><<<grid_for(w.total_nodes * 32u, NT, w.num_sms, 32 * 128 / NT), NT, 0, st>>>(
         w.scenes, w.plan, w.node_scene, w.total_nodes, w.n2t_offset, w.n2t_sorted_val, w.cap_n2t, w.d_record, w.r_record, w.se3,
         w.centers, w.item_ptr, w.cap_items, w.sym_blocks, w.diag64, w.jtr, w.error_flag);
+}
+template <class DAcc, int NT, int C>
+static void launch_assemble_node_c(Workspace &w, cudaStream_t st) {
+    // the deepest pipeline whose records fit in a block's 48 KB
+    constexpr int per_term = 4 * 32 * record_stride<C>() * (NT / 32);
+    if constexpr (4 * per_term <= 48 * 1024) launch_assemble_node_v<DAcc, NT, C, 2, 2>(w, st);
+    else if constexpr (2 * per_term <= 48 * 1024) launch_assemble_node_v<DAcc, NT, C, 1, 2>(w, st);
+    else launch_assemble_node_v<DAcc, NT, C, 1, 1>(w, st);
 }
 
 template <class DAcc, int NT>
@@ -2165,13 +2263,27 @@ void gn_assemble_node(Workspace &w, cudaStream_t st) {
     count_launch(w);
 }
 
-template <int NT, int C>
-static void launch_assemble_pair_c(Workspace &w, cudaStream_t st) {
-    k_assemble_pair<NT, C><<<grid_for(w.cap_half * 32u, NT, w.num_sms, 32 * 128 / NT), NT, 0, st>>>(
+template <int NT, int C, int kTPL, int kBufs>
+static void launch_assemble_pair_v(Workspace &w, cudaStream_t st) {
+    k_assemble_pair<NT, C, kTPL, kBufs><<<grid_for(w.cap_half * 32u, NT, w.num_sms, 32 * 128 / NT), NT, 0, st>>>(
         w.scenes, w.plan, w.counts, w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene,
         w.pair_sorted_val, w.cap_pair_kv,
         w.half_slot_up, w.d_record, w.r_record, w.centers, w.precision == WS_PREC_MIXED ? 1 : 0, w.sym_blocks,
         w.error_flag);
+}
+template <int NT, int C>
+static void launch_assemble_pair_c(Workspace &w, cudaStream_t st) {
+    // Pixels per node say how long the pairs' lists are (about 0.48 terms a pixel of a node).  Long lists gain
+    // from the pipeline (5 or 6 GN iterations, one buffer / two: 614 px a node 257 / 174 us, 307 with flow
+    // 502 / 442, 170 145 / 143); short ones of a batch from the warps that fit without it (120 px a node, 64
+    // scenes: 5.98 / 7.19 ms).
+    uint64_t pixels = 0;
+    for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s)
+        pixels += (uint64_t)w.h_scenes[s].width * w.h_scenes[s].height;
+    constexpr int kTPL = terms_per_lane(NT, record_stride<C>()) < 2 ? terms_per_lane(NT, record_stride<C>()) : 2;
+    constexpr int fit = C == 3 && NT > 128 ? 128 : NT;   // threads whose two buffers fit in 48 KB
+    if (pixels >= 150ull * w.total_nodes) launch_assemble_pair_v<fit, C, 1, 2>(w, st);
+    else launch_assemble_pair_v<NT, C, kTPL, 1>(w, st);
 }
 
 template <int NT>

@@ -26,8 +26,8 @@ struct Workspace {
     int pcg_clusters_active = 0;   // such clusters that run at once
     // launch shapes picked by ws_autotune (defaults until then); none of them changes a result
     struct Tuning {
-        int node_threads = 128;     // threads per block of the node assembly (64, 128, 256)
-        int pair_threads = 128;     // threads per block of the pair assembly
+        int node_threads = 64;      // threads per block of the node assembly (64, 128, 256)
+        int pair_threads = 64;      // threads per block of the pair assembly
         int pcg_blocks_per_sm = 64; // upper bound on PCG blocks per SM (capped by co-residency)
         bool tuned = false;
     } tune;

@@ -66,3 +66,28 @@ def test_scattered_node_order(ws, small_scene_k8):
         s.Sync()
         out.append(s.SolvedNodeSE3(c - 1).cpu().numpy().copy())
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nodes,lambda_of,precision", [(40, 0.0, 0), (255, 0.0, 1), (255, 0.1, 0), (500, 0.1, 1)])
+def test_long_and_short_list_assembly(ws, small_scene_k8, nodes, lambda_of, precision):
+    """Alone, the scene's lists are long (many pixels a node) and its pairs' records go through two buffers;
+    beside a scene with few pixels a node they go through one.  The sums run in the same order."""
+    import dataclasses
+    import torch
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    sc = dataclasses.replace(_cut(small_scene_k8, nodes, 7), lambda_of=lambda_of)
+    a, b = DeviceScene.from_scene(sc), DeviceScene.from_scene(small_scene_k8)
+    assert a.num_pixels >= 150 * a.num_nodes and a.num_pixels + b.num_pixels < 150 * (a.num_nodes + b.num_nodes)
+    out = []
+    for items in ([a], [a, b], [b, a]):
+        s = WarpSolver(max_nodes=sum(d.num_nodes for d in items), max_pixels=sum(d.num_pixels for d in items),
+                       max_edges=sum(d.num_edges for d in items), max_scenes=len(items), precision=precision)
+        for threads in (64, 128, 256):
+            s.set_tuning(threads, threads, 2)
+            s.SetBatchInputs(items)
+            s.SolveStreamed(2, 4, stream=torch.cuda.Stream())
+            s.Sync()
+            at = next(i for i, d in enumerate(items) if d is a)
+            out.append(s.SolvedNodeSE3(at).cpu().numpy().copy())
+    for x in out[1:]:
+        np.testing.assert_array_equal(out[0], x)
