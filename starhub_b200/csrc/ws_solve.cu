@@ -256,30 +256,41 @@ __device__ void gauss_jordan6(const float *in, float *out) {
         for (int i = 0; i < 6; ++i) out[6 * reloc[j] + i] = m[6 * i + j];
 }
 
-// Symmetric positive definite 6x6 inverse by Cholesky in FP64.
-__device__ void cholesky6_fp64(const double *in, float *out) {
+// Symmetric positive definite 6x6 inverse by Cholesky in FP64; `in` is the upper triangle, row-major
+// (tri_index).  Fully unrolled: with loops the factors lay in local memory, and a node's chain of square
+// roots and divisions, which is what bounds it, took 17 us.
+__device__ __forceinline__ void cholesky6_fp64(const double *in, float *out) {
     double L[21];   // packed lower triangle, row i holds i+1 entries
 #define LI(i, j) L[(i) * ((i) + 1) / 2 + (j)]
+#pragma unroll
     for (int i = 0; i < 6; ++i)
+#pragma unroll
         for (int j = 0; j <= i; ++j) {
-            double s = in[6 * i + j];
+            double s = in[tri_index(j, i)];
+#pragma unroll
             for (int k = 0; k < j; ++k) s -= LI(i, k) * LI(j, k);
             if (i == j) LI(i, i) = sqrt(s > 0.0 ? s : 1e-300);
             else LI(i, j) = s / LI(j, j);
         }
     double Linv[21];
 #define LV(i, j) Linv[(i) * ((i) + 1) / 2 + (j)]
+#pragma unroll
     for (int i = 0; i < 6; ++i) {
         LV(i, i) = 1.0 / LI(i, i);
+#pragma unroll
         for (int j = 0; j < i; ++j) {
             double s = 0.0;
+#pragma unroll
             for (int k = j; k < i; ++k) s -= LI(i, k) * LV(k, j);
             LV(i, j) = s / LI(i, i);
         }
     }
+#pragma unroll
     for (int i = 0; i < 6; ++i)
+#pragma unroll
         for (int j = i; j < 6; ++j) {
             double s = 0.0;
+#pragma unroll
             for (int k = j; k < 6; ++k) s += LV(k, i) * LV(k, j);
             out[6 * i + j] = (float)s;
             out[6 * j + i] = (float)s;
@@ -655,22 +666,16 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
 // accumulated block (mixed precision) or the reference's FP32 Gauss-Jordan with
 // partial pivoting of the stored block (BlockDiagonalPreconditionerInverse.cuh:14-73).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_block_inverse(const double *diag64, const float *sym_blocks,
+__global__ void __launch_bounds__(64) k_block_inverse(const double *diag64, const float *sym_blocks,
                                                        const uint32_t *item_ptr, uint32_t cap_items,
                                                        uint32_t total_nodes, int fp64, float *inv_diag) {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total_nodes; g += gridDim.x * blockDim.x) {
         float inv[36];
         if (fp64) {
-            double Dd[36];
+            double Dd[21];
             const double *src = diag64 + 21ull * g;
 #pragma unroll
-            for (int a = 0; a < 6; ++a)
-#pragma unroll
-                for (int c = a; c < 6; ++c) {
-                    const double v = src[tri_index(a, c)];
-                    Dd[6 * a + c] = v;
-                    Dd[6 * c + a] = v;
-                }
+            for (int i = 0; i < 21; ++i) Dd[i] = src[i];
             cholesky6_fp64(Dd, inv);
         } else {
             float full[36];
@@ -2257,7 +2262,7 @@ void gn_assemble_node(Workspace &w, cudaStream_t st) {
     if (w.precision == WS_PREC_FP32) launch_assemble_node_nt<float>(w, w.tune.node_threads, st);
     else launch_assemble_node_nt<double>(w, w.tune.node_threads, st);
     count_launch(w);
-    k_block_inverse<<<grid_for(w.total_nodes, 128, w.num_sms, 16), 128, 0, st>>>(
+    k_block_inverse<<<grid_for(w.total_nodes, 64, w.num_sms, 32), 64, 0, st>>>(
         w.diag64, w.sym_blocks, w.item_ptr, w.cap_items, w.total_nodes, w.precision == WS_PREC_MIXED ? 1 : 0,
         w.inv_diag);
     count_launch(w);
