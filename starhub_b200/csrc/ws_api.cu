@@ -205,7 +205,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     for (float **v : {&w.sd0, &w.sd1}) A(dalloc(v, (size_t)w.cap_nodes * ws::kSdStride));
     A(dalloc(&w.se3, (size_t)w.cap_nodes * 8));
     A(dalloc(&w.centers, w.cap_nodes));
-    A(dalloc(&w.chunk_partial, w.cap_chunks));
+    A(dalloc(&w.chunk_partial, 2 * (size_t)w.cap_chunks));
     A(dalloc(&w.scene_scalars, 8ull * w.cap_scenes));
     A(dalloc(&w.scene_counter, 64ull * w.cap_scenes));
     A(dalloc(&w.error_flag, 4));
@@ -224,9 +224,10 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
         A(dalloc(&w.pcg_tickets, 4));
         w.pcg_cluster = ws::pcg_cluster_max(&w.pcg_clusters_active);
         A(dalloc(&w.pcg_words, w.cap_items));
-        A(dalloc(&w.pcg_send, w.cap_half));
+        A(dalloc(&w.pcg_send, w.cap_items));
         A(dalloc(&w.pcg_send_count, w.cap_nodes));
-        A(dalloc(&w.pcg_halo, 16ull * w.cap_scenes));   // kResMaxCluster each
+        A(dalloc(&w.pcg_halo, 16ull * w.cap_scenes + 160));   // kResMaxCluster a scene, or kResMaxBlocks
+        w.pcg_grid_most = ws::pcg_grid_max(w.device);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -348,6 +349,7 @@ int ws_set_batch(ws_solver *h, const ws_inputs *scenes, int num_scenes) {
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return hs[a].num_nodes > hs[b].num_nodes; });
         for (int s = 0; s < num_scenes; ++s) hs[s].pcg_order = order[s];
     }
+    w.pcg_grid_blocks = ws::pcg_grid_blocks(hs, num_scenes, w.pcg_grid_most);
     w.h_scenes.assign(hs, hs + num_scenes);
     w.num_scenes = num_scenes;
     w.dense_channels = 1;
@@ -469,7 +471,7 @@ int ws_solve_graph(ws_solver *h, int gn_iters, int pcg_iters, void *stream) {
     const uint64_t key[] = {(uint64_t)gn_iters, (uint64_t)pcg_iters, (uint64_t)w.num_scenes, w.total_nodes,
                             w.total_edges, w.total_tiles, w.total_chunks, (uint64_t)w.node_bits,
                             (uint64_t)w.dense_channels, (uint64_t)ws::pcg_split_group(w),
-                            (uint64_t)ws::pcg_cluster_size(w)};
+                            (uint64_t)ws::pcg_mode(w), (uint64_t)w.pcg_grid_blocks};
     constexpr size_t kKey = sizeof(key) / sizeof(key[0]);
     bool same = w.graph_exec && w.graph_key.size() == kKey && std::equal(key, key + kKey, w.graph_key.begin());
     if (same) {
@@ -676,11 +678,11 @@ int ws_autotune(ws_solver *h, int pcg_iters, void *stream, ws_tuning *out) {
     const int max_per_sm = std::max(1, std::min(8, w.pcg_grid / std::max(1, w.num_sms)));
     int best_b = max_per_sm;
     float bb = 1e30f;
-    if (ws::pcg_cluster_size(w) > 0) {   // clusters run these inputs: blocks per SM stays at its bound
+    if (ws::pcg_mode(w) != ws::PcgMode::kStream) {   // k_pcg does not run these inputs: blocks per SM stays at its bound
         w.tune.pcg_blocks_per_sm = max_per_sm;
         out->pcg_ms[max_per_sm - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });
     }
-    for (int b = 1; b <= max_per_sm && ws::pcg_cluster_size(w) == 0; ++b) {
+    for (int b = 1; b <= max_per_sm && ws::pcg_mode(w) == ws::PcgMode::kStream; ++b) {
         w.tune.pcg_blocks_per_sm = b;
         ws::pcg_ranges(w, st);
         out->pcg_ms[b - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });

@@ -69,6 +69,7 @@ struct Scene {
     int tile_base, num_tiles;          // pixel tiles of this scene
     int chunk_base, num_chunks;        // PCG row groups (kRowsPerGroup nodes) of this scene
     int pcg_order;                     // entry k of the batch's table: the scene with the k-th most nodes
+    int pcg_block0, pcg_blocks;        // this scene's blocks of a PCG over the whole grid
 };
 
 // Per-scene counts derived on the device during the index build.

@@ -1,23 +1,28 @@
-// Block PCG with one thread-block cluster per scene, included by ws_solve.cu after the helpers it
-// shares with k_pcg (PcgArgs, matvec6, node_dot_group, twist_update_row, the bulk-copy helpers).
+// Block PCG that keeps a scene in the shared memory of its blocks, included by ws_solve.cu after the helpers
+// it shares with k_pcg (PcgArgs, matvec6, node_dot_group, twist_update_row, the bulk-copy helpers).
 //
-// What bounds a lone frame's PCG is not the matrix (1.6 MB at 1800 nodes) but the two scene-wide
-// reductions an iteration: through global tickets and polled generations each costs several microseconds
-// (22.8 us an iteration at 1800 nodes).  Here a scene's rows are split over the blocks of one cluster
-// (up to 16 SMs).  Each block keeps its rows' part of the symmetric store, the inverse diagonal and the
-// vectors in its shared memory for all iterations (what does not fit streams through a ring of bulk
-// copies, or is read from L2), a row's new s is pushed into the halos of the blocks whose items touch it,
-// transposed products go straight to the owning block, and the reductions are two hardware cluster
-// barriers an iteration: 7.4 us an iteration at 1800 nodes.  What is left is latency: barriers with
-// remote stores to drain (about 0.7 us each) and shared-memory traffic (192 KB a block and iteration).
-// Scenes of a batch are independent clusters, scheduled by the hardware, largest first.
+// What bounds a lone frame's PCG is not the matrix (1.6 MB at 1800 nodes, 7 MB at 8000) but the two
+// scene-wide reductions an iteration and the dependent trips to L2 around them: k_pcg takes 22.8 us an
+// iteration at 1800 nodes and 27.8 at 8000.  Here a scene's rows are split over blocks of one SM each.  A
+// block keeps its rows' part of the symmetric store, the inverse diagonal and the vectors in its shared memory
+// for all iterations (what does not fit streams through a ring of bulk copies, or is read from L2), and holds
+// s and d of the rows that its items touch elsewhere (its halo).
+//   * kGrid = false: the scene is one thread-block cluster (up to 16 SMs).  New s goes into the other blocks'
+//     halos and transposed products to the owning block through distributed shared memory, and the
+//     reductions are two hardware cluster barriers an iteration: 6.0 us an iteration at 500 nodes, 7.2 at
+//     1800.  What is left is latency and, with more rows a block, shared-memory traffic (192 KB a block and
+//     iteration at 1800 nodes).  A batch's scenes are independent clusters, the largest first.
+//   * kGrid = true: the scene has a share of all SMs.  Halos, transposed products and partials go through L2,
+//     and the blocks meet at a counter there: 9.8 us at 3000 nodes, 11.0 at 8000.  What is left are the two
+//     meetings (fence, atomic, poll: 2 to 3 us each) and the trips to L2 after them.
 //
 // The arithmetic is k_pcg's, operation by operation (products per item, row sums in item order,
 // contributions in column order, group partials over 16 rows, scene sums over groups in lane-strided
 // order), so both kernels give the same bits and a scene's result does not depend on which one ran.
 //
 // Waits: the cluster barriers are hardware barriers that every block of the scene reaches; a wait for a
-// bulk copy is bounded, sets WS_ERR_TIMEOUT and goes on, so that no block leaves the others waiting.
+// bulk copy is bounded, sets WS_ERR_TIMEOUT and goes on, so that no block leaves the others waiting.  A
+// meeting of the grid is bounded too; a block whose wait gives up sets WS_ERR_TIMEOUT and leaves.
 #pragma once
 
 namespace ws {
@@ -25,7 +30,8 @@ namespace ws {
 constexpr int kResMaxCluster = 16;
 constexpr int kResThreads = 512;
 constexpr int kResRows = kResThreads;   // rows of a block at most: one per thread
-constexpr uint32_t kResSmemBytes = 230400;
+constexpr uint32_t kResSmemBytes = 228864;   // beside 3 KB of static shared memory
+constexpr int kResMaxPolls = 1 << 22;   // polls of a meeting before it gives up (a second or more)
 constexpr uint32_t kResNodes = kResRows * kResMaxCluster;   // nodes of a scene at most
 constexpr int kPlanThreads = 512;
 static_assert(kResNodes <= 8192, "13-bit column numbers in an item word");
@@ -64,25 +70,29 @@ __device__ __forceinline__ void st_peer_f64(uint32_t a, double v) {
 
 // Item word of a block (built once per solve by k_pcg_plan): bits 0..8 the item's row in the block,
 // 9..21 its column as an index into the block's vectors (its own rows, then its halo: the other blocks'
-// rows that its items touch, in row order), 22..26 the rank of the block that owns the column, bit 31 a
+// rows that its items touch, in row order), 22..29 the rank of the block that owns the column, bit 31 a
 // diagonal item; the second word is the lower entry the transposed product goes to, counted from the
 // owning block's first (kInvalidIndex for none).
 constexpr uint32_t kResDiag = 0x80000000u;
 
 struct ResPlan {
     uint2 *words;          // [cap_items] item words
-    uint32_t *send;        // [cap_half] per row, from its first lower entry: (rank << 16) | halo index of the row there
-    uint32_t *send_count;  // [cap_nodes] blocks that hold the row in their halo
-    uint32_t *halo;        // [cap_scenes * kResMaxCluster] halo rows of each block
+    // clusters: [cap_half] per row, from its first lower entry: (rank << 16) | halo index of the row there;
+    // grid: [cap_items] per block, from its first item: the scene rows of its halo
+    uint32_t *send;
+    // [cap_nodes] clusters: blocks that hold the row in their halo; grid: lower entries from other blocks
+    uint32_t *send_count;
+    uint32_t *halo;        // halo rows of each block of the launch
 };
+constexpr int kResMaxBlocks = 160;   // blocks of a scene at most
 
 // The blocks' ranges of a scene: group, row, first item and first lower entry of every rank.
 struct ResRanges {
-    uint32_t group[kResMaxCluster + 1], row[kResMaxCluster + 1], item[kResMaxCluster + 1], low[kResMaxCluster + 1];
+    uint32_t group[kResMaxBlocks + 1], row[kResMaxBlocks + 1], item[kResMaxBlocks + 1], low[kResMaxBlocks + 1];
 };
 
 // Whole groups, balanced by items and rows (a row's own work is about four items').  Called by all
-// threads of a block (at least kResMaxCluster + 1); ends with a block barrier.
+// threads of a block (at least kResMaxBlocks + 1); ends with a block barrier.
 __device__ __forceinline__ void res_ranges(const PcgArgs &A, uint32_t nb, uint32_t nn, uint32_t groups, uint32_t size,
                                            ResRanges &R) {
     const uint32_t t = threadIdx.x;
@@ -113,22 +123,49 @@ __device__ __forceinline__ void res_ranges(const PcgArgs &A, uint32_t nb, uint32
 }
 
 __device__ __forceinline__ uint32_t res_rank_of(const ResRanges &R, uint32_t size, uint32_t row) {
-    uint32_t q = 0;
-    for (uint32_t k = 1; k < size; ++k) q += R.row[k] <= row ? 1u : 0u;
-    return q;
+    uint32_t lo = 0, hi = size - 1;   // the last block that starts at or before the row
+    while (lo < hi) {
+        const uint32_t m = (lo + hi + 1) >> 1;
+        if (R.row[m] <= row) lo = m;
+        else hi = m - 1;
+    }
+    return lo;
+}
+
+// Where a block of the launch belongs: its scene, and its rank among the scene's blocks.
+struct ResPlace {
+    uint32_t scene, rank, size;
+};
+template <bool kGrid>
+__device__ __forceinline__ ResPlace res_place(const PcgArgs &A) {
+    ResPlace p;
+    if constexpr (kGrid) {
+        uint32_t s = 0;   // the scenes' blocks follow one another in scene order
+        while (s + 1 < A.num_scenes && blockIdx.x >= (uint32_t)A.scenes[s + 1].pcg_block0) ++s;
+        p.scene = s;
+        p.rank = blockIdx.x - (uint32_t)A.scenes[s].pcg_block0;
+        p.size = (uint32_t)A.scenes[s].pcg_blocks;
+    } else {
+        p.rank = cluster_rank();
+        p.size = cluster_size();
+        p.scene = (uint32_t)A.scenes[blockIdx.x / p.size].pcg_order;
+    }
+    return p;
 }
 
 // Item words, halos and send lists of every block, once per solve (the structure is the same in every
 // Gauss-Newton iteration).  One cluster per scene, ranks as in k_pcg_cluster.  A block's halo is a bit
 // per scene row; a row's index in it is the number of set bits before it.  A row's lower entries name
 // the blocks whose items touch it, and so those its new s has to reach.
+template <bool kGrid>
 __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint32_t *colidx, ResPlan P) {
     __shared__ ResRanges R;
     __shared__ uint32_t bits[kResNodes / 32], before[kResNodes / 32], first_item[kResRows], warp_sums[kPlanThreads / 32];
     static_assert(kResNodes / 32 <= kPlanThreads, "a thread per bitmap word");
-    const uint32_t tid = threadIdx.x, lane = tid & 31, rank = cluster_rank(), size = cluster_size();
-    const uint32_t scene = (uint32_t)A.scenes[blockIdx.x / size].pcg_order;
-    const Scene &sc = A.scenes[scene];
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const ResPlace place = res_place<kGrid>(A);
+    const uint32_t rank = place.rank, size = place.size;
+    const Scene &sc = A.scenes[place.scene];
     const uint32_t nb = (uint32_t)sc.node_base, nn = (uint32_t)sc.num_nodes;
     res_ranges(A, nb, nn, (uint32_t)sc.num_chunks, size, R);
     const uint32_t row0 = R.row[rank], row1 = R.row[rank + 1], rows = row1 - row0;
@@ -155,7 +192,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
         uint32_t base = 0;
         for (uint32_t w = 0; w < (tid >> 5); ++w) base += warp_sums[w];
         if (tid < kResNodes / 32) before[tid] = base + inc - n;
-        if (tid == kPlanThreads - 1) P.halo[(size_t)kResMaxCluster * scene + rank] = base + inc;
+        if (tid == kPlanThreads - 1) P.halo[blockIdx.x] = base + inc;
     }
     __syncthreads();
     for (uint32_t k = tid; k < items; k += kPlanThreads) {
@@ -173,6 +210,19 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
         uint32_t slot = kInvalidIndex;
         if (!diag && it.y >= R.low[cr] && it.y < R.low[cr + 1]) slot = it.y - R.low[cr];
         P.words[item0 + k] = make_uint2(lo | (at << 9) | (cr << 22) | (diag ? kResDiag : 0u), slot);
+    }
+    if constexpr (kGrid) {
+        for (uint32_t c = tid; c < kResNodes; c += kPlanThreads)
+            if ((bits[c >> 5] >> (c & 31u)) & 1u)   // at most one halo row per item
+                P.send[item0 + before[c >> 5] + (uint32_t)__popc(bits[c >> 5] & ((1u << (c & 31u)) - 1u))] = nb + c;
+        for (uint32_t r = tid; r < rows; r += kPlanThreads) {
+            const uint32_t q0 = A.rowptr[row0 + r], p0 = A.item_ptr[row0 + r];
+            const uint32_t n = (A.rowptr[row0 + r + 1] - q0) - (A.item_ptr[row0 + r + 1] - p0);
+            uint32_t outside = 0;   // columns ascend, so those of other blocks come first
+            while (outside < n && q0 + 1u + outside < A.cap_blocks && __ldg(colidx + q0 + 1u + outside) < row0) ++outside;
+            P.send_count[row0 + r] = outside;
+        }
+        return;
     }
     cluster_arrive();
     cluster_wait();   // every block's bitmap is complete
@@ -198,18 +248,41 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
     cluster_wait();   // no block leaves while another reads its bitmap
 }
 
-// Sum of a scene's group partials, as reduce_scene takes it.
-__device__ __forceinline__ double res_reduce(const PcgArgs &A, const double *part, int groups, int lane) {
-    double v = 0.0;
-#pragma unroll 8
-    for (int c = lane; c < groups; c += 32) v += part[c];
-    v = warp_sum(v);
-    if (!A.fp64) v = (double)(float)v;
-    return v;
+// One thread's bounded wait for phase `parity` of `bar`.
+__device__ __forceinline__ void bulk_wait_one(unsigned long long *bar, unsigned parity) {
+    unsigned done = 0;
+    for (int i = 0; i < kBulkMaxPolls && done == 0; ++i)
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done)
+                     : "r"(smem_addr(bar)), "r"(parity)
+                     : "memory");
 }
 
-__global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPlan P) {
-    constexpr uint32_t kThreads = kResThreads, kWarps = kResThreads / 32, smem_bytes = kResSmemBytes;
+// Sum of a scene's group partials in the order of reduce_scene, eight of a lane's loads at a time.
+template <bool kGrid>
+__device__ __forceinline__ double res_reduce(const PcgArgs &A, const double *part, int groups, int lane) {
+    double v = 0.0;
+    for (int c0 = lane; c0 < groups; c0 += 256) {
+        double x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int c = min(c0 + 32 * k, groups - 1);
+            x[k] = kGrid ? __ldcg(part + c) : part[c];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (c0 + 32 * k < groups) v += x[k];
+    }
+    v = warp_sum(v);
+    return A.fp64 ? v : (double)(float)v;
+}
+
+// kGrid: a scene's blocks are blocks of a cooperative launch; they meet at a counter in L2 and exchange
+// halos, contributions and partials through L2.
+template <bool kGrid>
+__global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPlan P, uint32_t smem_bytes) {
+    constexpr uint32_t kThreads = kResThreads, kWarps = kResThreads / 32;
     constexpr uint32_t kChunkBytes = 32u * 144u;
     constexpr uint32_t kMaxRing = 24;
     extern __shared__ __align__(128) unsigned char res_smem[];
@@ -220,19 +293,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     const uint32_t tid = threadIdx.x;
     const int lane = tid & 31;
     const uint32_t warp = tid >> 5;
-    const uint32_t rank = cluster_rank(), size = cluster_size();
-    cluster_arrive();   // every block of the cluster has started once the matching wait returns
-    const uint32_t scene = (uint32_t)A.scenes[blockIdx.x / size].pcg_order;
-    const Scene &sc = A.scenes[scene];
+    __shared__ int s_left;   // grid: a wait gave up
+    if constexpr (!kGrid) cluster_arrive();   // every block of the cluster has started once the matching wait returns
+    const ResPlace place = res_place<kGrid>(A);
+    const uint32_t rank = place.rank, size = place.size;
+    const Scene &sc = A.scenes[place.scene];
     const uint32_t nb = (uint32_t)sc.node_base, nn = (uint32_t)sc.num_nodes, groups = (uint32_t)sc.num_chunks;
     res_ranges(A, nb, nn, groups, size, R);
-    uint32_t vmax = 0, lmax = 0, halo = 0;   // most vector rows (own and halo) and lower entries of a block
-    for (uint32_t k = 0; k < size; ++k) {
-        const uint32_t h = __ldg(P.halo + (size_t)kResMaxCluster * scene + k);
-        vmax = max(vmax, R.row[k + 1] - R.row[k] + h);
-        lmax = max(lmax, R.low[k + 1] - R.low[k]);
-        if (k == rank) halo = h;
-    }
+    // most vector rows (own and halo) and lower entries of a block: what peers write lies at the same offsets
+    const uint32_t halo = __ldg(P.halo + blockIdx.x);
+    uint32_t vmax = R.row[rank + 1] - R.row[rank] + halo, lmax = R.low[rank + 1] - R.low[rank];
+    if constexpr (!kGrid)
+        for (uint32_t k = 0; k < size; ++k) {
+            vmax = max(vmax, R.row[k + 1] - R.row[k] + __ldg(P.halo + (blockIdx.x - rank + k)));
+            lmax = max(lmax, R.low[k + 1] - R.low[k]);
+        }
     const uint32_t row0 = R.row[rank], rows = R.row[rank + 1] - row0;
     const uint32_t item0 = R.item[rank], items = R.item[rank + 1] - item0;
     const uint32_t low0 = R.low[rank], lows = R.low[rank + 1] - low0;
@@ -240,8 +315,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     const uint32_t chunks = (items + 31u) / 32u;
 
     // ---- shared memory: first what peers write (the same offsets in every block), then this block's ----
-    const uint32_t off_pa = 0, off_pb = 8u * groups;
-    uint32_t off = (16u * groups + 15u) & ~15u;
+    const uint32_t off_pa = 0, off_pb = 8u * groups;   // clusters: the partials of phases A and B
+    uint32_t off = kGrid ? 0u : (16u * groups + 15u) & ~15u;
     constexpr uint32_t kMinLocal = 32u * kThreads + 4u * kChunkBytes + 64u;   // product records and a small ring
     const uint32_t off_s = off, off_d = off + 24u * vmax;
     const bool vec_shared = off + 48u * vmax + kMinLocal <= smem_bytes;   // else s and d go through A.sd0 / A.sd1
@@ -252,9 +327,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     const bool words_shared = off + 8u * items + kMinLocal <= smem_bytes;
     uint2 *words = words_shared ? reinterpret_cast<uint2 *>(res_smem + off) : P.words + item0;
     if (words_shared) off = (off + 8u * items + 15u) & ~15u;
-    const bool send_shared = off + 4u * lows + kMinLocal <= smem_bytes;
-    uint32_t *send = send_shared ? reinterpret_cast<uint32_t *>(res_smem + off) : P.send + low0;
-    if (send_shared) off = (off + 4u * lows + 15u) & ~15u;
+    // clusters: where the rows' s goes; grid: the rows of the halo
+    const uint32_t send_n = kGrid ? halo : lows;
+    uint32_t *send_from = P.send + (kGrid ? item0 : low0);
+    const bool send_shared = off + 4u * send_n + kMinLocal <= smem_bytes;
+    uint32_t *send = send_shared ? reinterpret_cast<uint32_t *>(res_smem + off) : send_from;
+    if (send_shared) off = (off + 4u * send_n + 15u) & ~15u;
     // product records: of every item when everything fits, else of one item a thread
     const bool stage_all = off + 32u * items + 144u * rows + kChunkBytes * chunks <= smem_bytes;
     const uint32_t stage_items = stage_all ? max(32u * chunks, (uint32_t)kThreads) : (uint32_t)kThreads;
@@ -288,6 +366,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     if (tid == 0) {
         bulk_init(&s_bar, 1);
         if (ring > 0) bulk_init(s_ring, (int)ring);
+        for (uint32_t b = 0; b < kMaxRing; ++b) s_armed[b] = 0;
         const uint32_t block_bytes = 144u * min(32u * resident, items), bytes = block_bytes + (inv_shared ? 144u * rows : 0u);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(&s_bar)), "r"(bytes)
                      : "memory");
@@ -306,7 +385,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     if (words_shared)
         for (uint32_t k = tid; k < items; k += kThreads) words[k] = __ldg(P.words + item0 + k);
     if (send_shared)
-        for (uint32_t k = tid; k < lows; k += kThreads) send[k] = __ldg(P.send + low0 + k);
+        for (uint32_t k = tid; k < send_n; k += kThreads) send[k] = __ldg(send_from + k);
     // the thread's row: sixteen rows (a group) a warp while there are warps enough, so that the row loops of
     // a warp are as long as its longest of sixteen
     const bool sparse = rows <= kResRows / 2;
@@ -349,11 +428,49 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
             matvec6(A.inv_diag + 36ull * row, x, y);
         }
     };
-    // a group's partial to every block of the cluster: lane k of the group writes block k's copy
+    // a group's partial to every block of the cluster: lane k of the group writes block k's copy (grid: to L2)
     auto publish = [&](uint32_t off_part, double part) {
         const uint32_t g = r / kRowsPerGroup, k = r % kRowsPerGroup;
         static_assert(kRowsPerGroup >= kResMaxCluster, "a lane per block");
-        if (g < own_groups && k < size) st_peer_f64(peer_addr(smem_base + off_part + 8u * (group0 + g), k), part);
+        if constexpr (kGrid) {
+            if (g < own_groups && k == 0)
+                __stcg(A.group_partial + (off_part == off_pa ? 0u : A.total_groups) + sc.chunk_base + group0 + g, part);
+        } else {
+            if (g < own_groups && k < size) st_peer_f64(peer_addr(smem_base + off_part + 8u * (group0 + g), k), part);
+        }
+    };
+    // Every block of the scene has reached this point, and what it wrote before is visible; false when the
+    // wait gave up (grid only: WS_ERR_TIMEOUT is set, and the block leaves).
+    uint32_t meetings = 0;
+    auto meet = [&]() -> bool {
+        if constexpr (kGrid) {
+            ++meetings;
+            __syncthreads();
+            if (tid == 0) {
+                uint32_t *counter = A.scene_counter + (size_t)kSceneSync * place.scene;
+                __threadfence();
+                atomicAdd(counter, 1u);
+                bool ok = false;
+                for (int i = 0; i < kResMaxPolls && !ok; ++i) {
+                    ok = ld_acquire(counter) >= size * meetings;
+                    if (!ok && (i & 1023) == 1023 && *reinterpret_cast<volatile int *>(A.err) == WS_ERR_TIMEOUT) break;
+                }
+                if (!ok) set_err(A.err, WS_ERR_TIMEOUT);
+                s_left = ok ? 0 : 1;
+            }
+            __syncthreads();
+            return s_left == 0;
+        } else {
+            cluster_arrive();
+            cluster_wait();
+            return true;
+        }
+    };
+    // the scene's sum of group partials, in the block's first warp
+    auto reduce = [&](uint32_t off_part) -> double {
+        const double *part = kGrid ? A.group_partial + (off_part == off_pa ? 0u : A.total_groups) + sc.chunk_base
+                                   : reinterpret_cast<const double *>(res_smem + off_part);
+        return res_reduce<kGrid>(A, part, (int)groups, lane);
     };
     // s of the row into the block's vectors and into the halos that hold the row
     auto store_s = [&](const float *s, float *sd) {
@@ -362,7 +479,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
             p[0] = make_float2(s[0], s[1]);
             p[1] = make_float2(s[2], s[3]);
             p[2] = make_float2(s[4], s[5]);
-            for (uint32_t k = 0; k < sends; ++k) {
+            if constexpr (kGrid) {   // for the halos (A.r is free here)
+                __stcg(reinterpret_cast<float4 *>(A.r + 8ull * row), make_float4(s[0], s[1], s[2], s[3]));
+                __stcg(reinterpret_cast<float2 *>(A.r + 8ull * row + 4), make_float2(s[4], s[5]));
+            }
+            for (uint32_t k = 0; !kGrid && k < sends; ++k) {
                 const uint32_t to = send[l_begin + k];
                 const uint32_t a = peer_addr(smem_base + off_s + 24u * (to & 0xFFFFu), to >> 16);
                 st_peer2(a, s[0], s[1]);
@@ -378,7 +499,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     if (vec_shared)
         for (uint32_t k = tid; k < 3u * (rows + halo); k += kThreads)
             reinterpret_cast<float2 *>(res_smem + off_d)[k] = make_float2(0.f, 0.f);
-    cluster_wait();
+    if constexpr (!kGrid) cluster_wait();
     if (row_warp) {
         float s[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (has_row) {
@@ -388,21 +509,39 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
         }
         publish(off_pb, node_dot_group(A, rv, s, has_row));
     }
-    cluster_arrive();
-    cluster_wait();
-    // the scene's scalars: every block's first warp takes the sums (all blocks see the same partials)
+    bool here = meet();
+    // the scene's scalars: every block's last warp, the first to have no rows, takes the sums (all blocks see
+    // the same partials)
+    constexpr uint32_t kScalarWarp = kWarps - 1;
     double delta = 0.0;
-    if (warp == 0) delta = res_reduce(A, reinterpret_cast<const double *>(res_smem + off_pb), (int)groups, lane);
+    if (here && warp == kScalarWarp) delta = reduce(off_pb);
+    // grid: s of the thread's halo row, requested before beta is known
+    float halo_s[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (kGrid && here && vec_shared && tid < halo) load6(A.r + 8ull * send[tid], halo_s);
     float beta = 0.f;
 
-    for (int it = 0; it < A.pcg_iters; ++it) {
+    for (int it = 0; here && it < A.pcg_iters; ++it) {
         const float *sd_old = (it & 1) ? A.sd1 : A.sd0;
         float *sd_new = (it & 1) ? A.sd0 : A.sd1;
         // ---- phase A: d = s + beta d (own rows and halo), q = A d, <d, q> ----
         if (vec_shared) {
             const float2 *ps = reinterpret_cast<const float2 *>(res_smem + off_s);
             float2 *pd = reinterpret_cast<float2 *>(res_smem + off_d);
-            for (uint32_t k = tid; k < 3u * (rows + halo); k += kThreads) {
+            if constexpr (kGrid)
+                for (uint32_t k = tid; k < halo; k += kThreads) {
+                    float s[6];
+                    if (k == tid) {
+#pragma unroll
+                        for (int e = 0; e < 6; ++e) s[e] = halo_s[e];
+                    } else {
+                        load6(A.r + 8ull * send[k], s);
+                    }
+                    float2 *d = pd + 3u * (rows + k);
+#pragma unroll
+                    for (int e = 0; e < 3; ++e)
+                        d[e] = make_float2(s[2 * e] + beta * d[e].x, s[2 * e + 1] + beta * d[e].y);
+                }
+            for (uint32_t k = tid; k < 3u * (kGrid ? rows : rows + halo); k += kThreads) {
                 const float2 s = ps[k], d = pd[k];
                 pd[k] = make_float2(s.x + beta * d.x, s.y + beta * d.y);
             }
@@ -442,7 +581,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
                 }
                 if (!valid) continue;
                 float vr[6], vc[6];
-                const uint32_t cr = (w.x >> 22) & 31u;
+                const uint32_t cr = (w.x >> 22) & 255u;
                 if (vec_shared) {
                     const float2 *pr = reinterpret_cast<const float2 *>(res_smem + off_d) + 3u * (w.x & 511u);
                     const float2 *pc = reinterpret_cast<const float2 *>(res_smem + off_d) + 3u * ((w.x >> 9) & 8191u);
@@ -481,11 +620,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
                 }
                 const bool diag = (w.x & kResDiag) != 0;
                 if (w.y != kInvalidIndex) {
-                    if (!contrib_shared) {
+                    if (!contrib_shared || (kGrid && cr != rank)) {
                         store6_f2(A.contrib + 6ull * (R.low[cr] + w.y), t);
                     } else if (cr == rank) {
                         store6_f2(reinterpret_cast<float *>(res_smem + off_contrib + 24u * w.y), t);
-                    } else {
+                    } else if constexpr (!kGrid) {
                         const uint32_t ta = peer_addr(smem_base + off_contrib + 24u * w.y, cr);
                         st_peer2(ta, t[0], t[1]);
                         st_peer2(ta + 8u, t[2], t[3]);
@@ -551,20 +690,41 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
             }
             publish(off_pa, A.fp64 ? group_sum(dsum) : (double)group_sum((float)dsum));
         }
-        cluster_arrive();
-        cluster_wait();
+        here = meet();
+        if (!here) break;
         // ---- phase B: alpha; x += alpha d; r -= alpha q; s = M^-1 r; <r, s> ----
-        if (warp == 0) {
-            const double dq = res_reduce(A, reinterpret_cast<const double *>(res_smem + off_pa), (int)groups, lane);
+        if (warp == kScalarWarp) {
+            const double dq = reduce(off_pa);
             double alpha64 = dq != 0.0 ? delta / dq : 0.0;
             if (!A.fp64 && dq != 0.0) alpha64 = (double)((float)delta / (float)dq);
             if (lane == 0) s_scalar[0] = (float)alpha64;
         }
-        // the contributions do not need alpha: summed while the first warp takes it
+        // the contributions do not need alpha: summed while the last warp takes it
         if (has_row) {
             if (contrib_shared) {
                 const float2 *c = reinterpret_cast<const float2 *>(res_smem + off_contrib) + 3u * l_begin;
-                for (uint32_t k = 0; k < l_count; k += 4) {
+                uint32_t k0 = 0;
+                if constexpr (kGrid) {   // the first `sends` entries come from other blocks, through L2
+                    const float2 *g = reinterpret_cast<const float2 *>(A.contrib) + 3ull * (low0 + l_begin);
+                    for (; k0 < sends; k0 += 4) {
+                        float2 v[4][3];
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; ++e)
+#pragma unroll
+                            for (uint32_t h = 0; h < 3; ++h) v[e][h] = __ldcg(g + 3u * min(k0 + e, sends - 1u) + h);
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; ++e)
+                            if (k0 + e < sends) {
+#pragma unroll
+                                for (uint32_t h = 0; h < 3; ++h) {
+                                    q[2 * h] += v[e][h].x;
+                                    q[2 * h + 1] += v[e][h].y;
+                                }
+                            }
+                    }
+                    k0 = sends;
+                }
+                for (uint32_t k = k0; k < l_count; k += 4) {
                     float2 v[4][3];
 #pragma unroll
                     for (uint32_t e = 0; e < 4; ++e)
@@ -603,10 +763,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
             if (more) publish(off_pb, node_dot_group(A, rv, s, has_row));
         }
         if (more) {
-            cluster_arrive();
-            cluster_wait();
-            if (warp == 0) {
-                const double v = res_reduce(A, reinterpret_cast<const double *>(res_smem + off_pb), (int)groups, lane);
+            here = meet();
+            if (!here) break;
+            if (kGrid && vec_shared && tid < halo) load6(A.r + 8ull * send[tid], halo_s);
+            if (warp == kScalarWarp) {
+                const double v = reduce(off_pb);
                 double beta64 = delta != 0.0 ? v / delta : 0.0;
                 if (!A.fp64 && delta != 0.0) beta64 = (double)((float)v / (float)delta);
                 delta = v;
@@ -615,6 +776,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
             __syncthreads();
             beta = s_scalar[1];
         }
+    }
+    if (!here) {   // no block leaves with copies on their way into its shared memory
+        if (ring > 0 && tid == 0)
+            for (uint32_t b = 0; b < ring; ++b)
+                if (s_armed[b] > 0) bulk_wait_one(&s_ring[b], (s_armed[b] - 1u) & 1u);
+        __syncthreads();
+        return;
     }
     if (has_row) {
         store6(A.x + 8ull * row, xv);

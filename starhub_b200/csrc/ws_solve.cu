@@ -2379,12 +2379,12 @@ static void cluster_launch(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, i
 // Largest cluster the device can run k_pcg_cluster with (16, 8 or 0), and how many of them at once.
 int pcg_cluster_max(int *active) {
     *active = 0;
-    for (const void *k : {(const void *)k_pcg_cluster, (const void *)k_pcg_plan})
+    for (const void *k : {(const void *)k_pcg_cluster<false>, (const void *)k_pcg_plan<false>})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
-    if (cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemBytes) !=
+    if (cudaFuncSetAttribute(k_pcg_cluster<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemBytes) !=
         cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -2402,7 +2402,7 @@ int pcg_cluster_max(int *active) {
             cudaLaunchConfig_t cfg{};
             cudaLaunchAttribute attr{};
             cluster_launch(cfg, attr, size, 1, kResThreads, kResSmemBytes, nullptr);
-            if (cudaOccupancyMaxActiveClusters(&n, k_pcg_cluster, &cfg) == cudaSuccess && n >= 1) found = size;
+            if (cudaOccupancyMaxActiveClusters(&n, k_pcg_cluster<false>, &cfg) == cudaSuccess && n >= 1) found = size;
             else cudaGetLastError();
         }
         known[dev][0] = found + 1;
@@ -2412,24 +2412,70 @@ int pcg_cluster_max(int *active) {
     return known[dev][0] - 1;
 }
 
-// Blocks per scene of k_pcg_cluster, or 0 where k_pcg runs.  Both give the same bits; the rule is speed.
-// Per PCG iteration a scene of n thousand nodes takes a cluster of 16 about 3.6 + 3.1 n us (measured, with
-// the launch's load phase spread over 20 iterations: 6.8 us at 1k, 12 at 3k, 21 at 6k, 29 at 7k), and as
-// many scenes as clusters fit on the device (7) run side by side; k_pcg takes about 22 + 0.3 us per
-// thousand nodes of the whole batch (21 us at 1k, 23 at 3k, 27 at 6k, 28 at 7k, 71 at 163k).  Measured at
-// 5 x 20 iterations, k_pcg against clusters: lone 1k nodes 2.13 / 0.68 ms, 6k 2.71 / 2.11, 7k 2.85 / 2.94;
-// nodes log-uniform in [500, 8000], 8 scenes 3.54 / 2.49, 24 scenes 4.14 / 4.32, 64 scenes 7.1 / 10.9.
-int pcg_cluster_size(const Workspace &w) {
+// Most blocks of k_pcg_cluster<true> that run at once (one per SM), 0 without cooperative launches.
+int pcg_grid_max(int device) {
+    int per_sm = 0, sms = 0, coop = 0;
+    if (cudaFuncSetAttribute(k_pcg_cluster<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemBytes) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_cluster<true>, kResThreads, kResSmemBytes) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) {
+        cudaGetLastError();
+        return 0;
+    }
+    return std::min(kResMaxBlocks, per_sm * sms);
+}
+
+// Blocks of a batch's scenes in k_pcg_cluster<true>: one for every two row groups while that fits in `most`,
+// else in proportion to the nodes.  Returns their number, 0 where a scene does not fit.
+int pcg_grid_blocks(Scene *scenes, int num_scenes, int most) {
+    if (most <= 0 || num_scenes > most) return 0;
+    long long want = 0, nodes = 0;
+    for (int s = 0; s < num_scenes; ++s) {
+        want += (scenes[s].num_chunks + 1) / 2;
+        nodes += scenes[s].num_nodes;
+    }
+    int at = 0;
+    for (int s = 0; s < num_scenes; ++s) {
+        const long long share = (long long)(most - num_scenes) * scenes[s].num_nodes / std::max(1ll, nodes) + 1;
+        const int blocks = (int)std::max(1ll, want <= most ? (long long)(scenes[s].num_chunks + 1) / 2 : share);
+        if ((scenes[s].num_chunks + blocks - 1) / blocks * kRowsPerGroup > kResRows || scenes[s].num_nodes > (int)kResNodes)
+            return 0;
+        scenes[s].pcg_block0 = at;
+        scenes[s].pcg_blocks = blocks;
+        at += blocks;
+    }
+    return at <= most ? at : 0;
+}
+
+// How the batch's PCG runs.  All three give the same bits; the rule is speed, by what an iteration takes (us,
+// measured with the launch's load phase spread over 20 iterations):
+//   k_pcg            22 + 0.3 per thousand nodes of the batch (21 at 1k nodes, 23 at 4k, 28 at 8k, 71 at 163k);
+//   clusters         3.2 + 2.8 per thousand nodes of a scene (6.3 at 1k, 7.2 at 1.8k, 11.2 at 3k, 20 at 6k, 29 at
+//                    8k), the scenes side by side as far as clusters fit on the device (7 of 16 blocks);
+//   the whole grid   9.2 + 0.045 per row of its fullest block (9.7 at 1k to 3k nodes, 10.6 at 6k, 11.0 at 8k).
+// In ms of 5 x 20 iterations, k_pcg / clusters / grid: lone 1k nodes 2.11 / 0.63 / 0.97, 3k 2.28 / 1.12 / 0.98,
+// 8k 2.80 / 2.95 / 1.10; nodes log-uniform in [500, 8000], 4 scenes 2.86 / 1.89 / 1.22, 16 scenes 3.65 / 2.94 /
+// 2.28, 64 scenes 7.1 / 10.9 / does not fit.
+PcgMode pcg_mode(const Workspace &w) {
     const int size = w.pcg_cluster;
-    if (size <= 0 || w.pcg_clusters_active <= 0) return 0;
-    double most = 0.0, sum = 0.0;
+    double most = 0.0, sum = 0.0, rows = 0.0;
+    bool cluster_fits = size > 0 && w.pcg_clusters_active > 0;
     for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s) {
-        if (w.h_scenes[s].num_chunks > size * (kResRows / kRowsPerGroup)) return 0;
-        const double us = (3.6 + 3.1e-3 * w.h_scenes[s].num_nodes) * kResMaxCluster / size;
+        const Scene &sc = w.h_scenes[s];
+        if (sc.num_chunks > size * (kResRows / kRowsPerGroup)) cluster_fits = false;
+        const double us = (3.2 + 2.8e-3 * sc.num_nodes) * kResMaxCluster / std::max(1, size);
         most = std::max(most, us);
         sum += us;
+        if (w.pcg_grid_blocks > 0)
+            rows = std::max(rows, (double)kRowsPerGroup * ((sc.num_chunks + sc.pcg_blocks - 1) / sc.pcg_blocks));
     }
-    return std::max(most, sum / w.pcg_clusters_active) < 22.0 + 0.3e-3 * w.total_nodes ? size : 0;
+    const double stream = 22.0 + 0.3e-3 * w.total_nodes;
+    const double clusters = cluster_fits ? std::max(most, sum / w.pcg_clusters_active) : 1e30;
+    const double grid = w.pcg_grid_blocks > 0 ? 9.2 + 0.045 * rows : 1e30;
+    if (clusters <= grid) return clusters < stream ? PcgMode::kClusters : PcgMode::kStream;
+    return grid < stream ? PcgMode::kGrid : PcgMode::kStream;
 }
 
 static ResPlan res_plan(Workspace &w) {
@@ -2444,24 +2490,38 @@ static ResPlan res_plan(Workspace &w) {
 // Work distribution of the PCG, after the block CSR: the item words, halos and send lists of
 // k_pcg_cluster.
 cudaError_t pcg_plan(Workspace &w, cudaStream_t st) {
-    const int size = pcg_cluster_size(w);
-    if (size == 0) return cudaSuccess;
+    const PcgMode mode = pcg_mode(w);
+    if (mode == PcgMode::kStream) return cudaSuccess;
+    const PcgArgs a = pcg_args(w, 0);
+    count_launch(w);
+    if (mode == PcgMode::kGrid) {
+        k_pcg_plan<true><<<w.pcg_grid_blocks, kPlanThreads, 0, st>>>(a, w.colidx, res_plan(w));
+        return cudaGetLastError();
+    }
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
-    cluster_launch(cfg, attr, size, w.num_scenes, kPlanThreads, 0, st);
-    count_launch(w);
-    return cudaLaunchKernelEx(&cfg, k_pcg_plan, pcg_args(w, 0), (const uint32_t *)w.colidx, res_plan(w));
+    cluster_launch(cfg, attr, w.pcg_cluster, w.num_scenes, kPlanThreads, 0, st);
+    return cudaLaunchKernelEx(&cfg, k_pcg_plan<false>, a, (const uint32_t *)w.colidx, res_plan(w));
 }
 
 cudaError_t gn_pcg(Workspace &w, int pcg_iters, cudaStream_t st) {
     PcgArgs a = pcg_args(w, pcg_iters);
-    const int size = pcg_cluster_size(w);
-    if (size > 0) {
+    const PcgMode mode = pcg_mode(w);
+    if (mode == PcgMode::kClusters) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr{};
         count_launch(w);
-        cluster_launch(cfg, attr, size, w.num_scenes, kResThreads, kResSmemBytes, st);
-        return cudaLaunchKernelEx(&cfg, k_pcg_cluster, a, res_plan(w));
+        cluster_launch(cfg, attr, w.pcg_cluster, w.num_scenes, kResThreads, kResSmemBytes, st);
+        return cudaLaunchKernelEx(&cfg, k_pcg_cluster<false>, a, res_plan(w), kResSmemBytes);
+    }
+    if (mode == PcgMode::kGrid) {
+        cudaMemsetAsync(w.scene_counter, 0, sizeof(uint32_t) * kSceneSync * (size_t)w.num_scenes, st);
+        ResPlan plan = res_plan(w);
+        uint32_t smem = kResSmemBytes;
+        void *args[] = {&a, &plan, &smem};
+        count_launch(w);
+        return cudaLaunchCooperativeKernel((const void *)k_pcg_cluster<true>, dim3((unsigned)w.pcg_grid_blocks),
+                                           dim3(kResThreads), args, kResSmemBytes, st);
     }
     const int grid = pcg_launch_blocks(w);
     // tickets and generations start at zero every launch, so a launch that timed out half-way

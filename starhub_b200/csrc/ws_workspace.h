@@ -24,6 +24,8 @@ struct Workspace {
     int pcg_grid = 0;           // co-resident blocks for the persistent PCG kernel
     int pcg_cluster = 0;        // blocks per cluster of k_pcg_cluster on this device (16, 8; 0: none)
     int pcg_clusters_active = 0;   // such clusters that run at once
+    int pcg_grid_most = 0;      // blocks of k_pcg_cluster over the whole grid at most (one per SM; 0: none)
+    int pcg_grid_blocks = 0;    // those of the current batch (0: it does not fit)
     // launch shapes picked by ws_autotune (defaults until then); none of them changes a result
     struct Tuning {
         int node_threads = 64;      // threads per block of the node assembly (64, 128, 256)
@@ -105,8 +107,8 @@ struct Workspace {
                                                              // first row group of every PCG work unit, the
                                                              // group count, the first half's unit count
     uint4 *pcg_unit_info = nullptr;                          // [2 * PCG work units]: groups, rows, items, scenes
-    // work distribution of the cluster PCG (ResPlan): item words [cap_items], send lists [cap_half],
-    // sends per row [cap_nodes], halo rows per block [cap_scenes * 16]
+    // work distribution of k_pcg_cluster (ResPlan): item words and send or halo lists [cap_items], sends
+    // per row [cap_nodes], halo rows per block [cap_scenes * 16 + 160]
     uint2 *pcg_words = nullptr;
     uint32_t *pcg_send = nullptr, *pcg_send_count = nullptr, *pcg_halo = nullptr;
     uint32_t *pcg_tickets = nullptr;                         // [4]: [0] PCG work-unit tickets, zeroed per launch
@@ -122,7 +124,7 @@ struct Workspace {
     float *sd0 = nullptr, *sd1 = nullptr;
     float *se3 = nullptr;               // [cap_nodes * 8] current warp
     float4 *centers = nullptr;          // [cap_nodes] twist centre per node (current GN iteration)
-    double *chunk_partial = nullptr;    // [cap_chunks]
+    double *chunk_partial = nullptr;    // [2 * cap_chunks]
     double *scene_scalars = nullptr;    // [cap_scenes * 8]: delta, alpha, beta, dq ...
     uint32_t *scene_counter = nullptr;  // [cap_scenes * 64]: PCG tickets and generations per scene
     int *error_flag = nullptr;          // [4]
@@ -165,7 +167,10 @@ void init_warp(Workspace &w, cudaStream_t st);
 // Occupancy of the persistent PCG kernel.
 int pcg_max_blocks(int device);
 int pcg_cluster_max(int *active);
-int pcg_cluster_size(const Workspace &w);
+int pcg_grid_max(int device);
+int pcg_grid_blocks(Scene *scenes, int num_scenes, int most);
+enum class PcgMode { kStream = 0, kClusters = 1, kGrid = 2 };
+PcgMode pcg_mode(const Workspace &w);
 cudaError_t pcg_plan(Workspace &w, cudaStream_t st);
 int pcg_launch_blocks(const Workspace &w);
 void pcg_ranges(Workspace &w, cudaStream_t st);

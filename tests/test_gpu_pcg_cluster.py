@@ -91,3 +91,44 @@ def test_long_and_short_list_assembly(ws, small_scene_k8, nodes, lambda_of, prec
             out.append(s.SolvedNodeSE3(at).cpu().numpy().copy())
     for x in out[1:]:
         np.testing.assert_array_equal(out[0], x)
+
+
+@pytest.fixture(scope="module")
+def large_scene(orc):
+    """About 4500 nodes at 160x120: alone, its PCG runs on the whole grid."""
+    from starhub_b200 import scenes
+    spec = scenes.spec_for_nodes(5000, scenes.config_spec(0, width=160, height=120, focal=142.5), surfels_per_node=30)
+    return scenes.make_scene(spec, orc.OracleGeometry(), seed=21)
+
+
+@pytest.mark.parametrize("pcg,precision,scattered", [(0, 0, False), (1, 0, False), (12, 0, False), (7, 1, False),
+                                                     (6, 0, True)])
+def test_grid_equals_persistent(ws, large_scene, small_scene_k8, pcg, precision, scattered):
+    """The large scene alone and beside others (the whole grid), and in a batch that only k_pcg takes."""
+    import dataclasses
+    import torch
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    sc = large_scene
+    n = sc.num_nodes
+    if scattered:   # node ids in random order: halos of most of the scene
+        order = np.random.default_rng(9).permutation(n)
+        new_id = np.empty(n, int)
+        new_id[order] = np.arange(n)
+        e = sc.edges.astype(int).reshape(n, 8, 3)[order]
+        e = np.stack([new_id[e[..., 0]], new_id[e[..., 1]], e[..., 2]], -1).reshape(-1, 3)
+        sc = dataclasses.replace(sc, nodes=sc.nodes[order], node_cw=sc.node_cw[order], edges=e.astype(np.uint16),
+                                 surfel_knn=new_id[sc.surfel_knn.astype(int)].astype(np.uint16))
+    a = DeviceScene.from_scene(sc)
+    b, c = DeviceScene.from_scene(_cut(small_scene_k8, 17, 3)), DeviceScene.from_scene(small_scene_k8)
+    out = {}
+    for key, items in (("alone", [a]), ("few", [b, a, c]), ("other order", [c, a, b]), ("small alone", [c]),
+                       ("tiny alone", [b]), ("many", [a] * 40 + [b, c])):
+        s = WarpSolver(max_nodes=sum(d.num_nodes for d in items), max_pixels=sum(d.num_pixels for d in items),
+                       max_edges=sum(d.num_edges for d in items), max_scenes=len(items), precision=precision)
+        s.SetBatchInputs(items)
+        s.SolveStreamed(2, pcg, stream=torch.cuda.Stream())
+        s.Sync()
+        for i, d in enumerate(items):
+            name = "a" if d is a else "b" if d is b else "c"
+            got = s.SolvedNodeSE3(i).cpu().numpy()
+            np.testing.assert_array_equal(out.setdefault(name, got.copy()), got, err_msg=f"{name} in {key}")
