@@ -97,25 +97,31 @@ __device__ float3 orthogonal_unit(float3 v) {
     return v3(0.f, -v.z * inv, v.y * inv);
 }
 
-// Of the three cross products of the rows of M - lambda I, the longest one, normalised; its
-// squared length in len.
-__device__ float3 null_direction(const float3 row[3], float lambda, float &len) {
+// Of the three cross products of the rows of M - lambda I, the longest one (not yet normalised); its
+// squared length in len, that of the third product in len3.
+__device__ __forceinline__ float3 null_product(const float3 row[3], float lambda, float &len, float &len3) {
     float3 t0 = row[0], t1 = row[1], t2 = row[2];
     t0.x -= lambda;
     t1.y -= lambda;
     t2.z -= lambda;
     const float3 a = cross(t0, t1), b = cross(t0, t2), c = cross(t1, t2);
     const float la = dot(a, a), lb = dot(b, b), lc = dot(c, c);
+    len3 = lc;
     if (la >= lb && la >= lc) {
         len = la;
-        return scaled(a, inv_sqrt(la));
+        return a;
     }
     if (lb >= la && lb >= lc) {
         len = lb;
-        return scaled(b, inv_sqrt(lb));
+        return b;
     }
     len = lc;
-    return scaled(c, inv_sqrt(lc));
+    return c;
+}
+__device__ __forceinline__ float3 null_direction(const float3 row[3], float lambda) {
+    float len, len3;
+    const float3 v = null_product(row, lambda, len, len3);
+    return scaled(v, inv_sqrt(len));
 }
 
 // Eigenvector of the smallest eigenvalue of the symmetric matrix
@@ -133,35 +139,37 @@ __device__ float3 smallest_eigenvector(float m[6]) {
     float3 ev;
     cubic_roots(c0, c1, c2, ev);
     const float3 row[3] = {v3(m00, m01, m02), v3(m01, m11, m12), v3(m02, m12, m22)};
-    float len;
     if (ev.z - ev.x <= kFltEpsilon) return v3(1.f, 0.f, 0.f);   // a multiple of I
     if (ev.y - ev.x <= kFltEpsilon) {
         // the two smallest coincide: any unit vector orthogonal to the largest one's
-        const float3 e2 = null_direction(row, ev.z, len);
+        const float3 e2 = null_direction(row, ev.z);
         const float3 e1 = orthogonal_unit(e2);
         return cross(e1, e2);
     }
-    if (ev.z - ev.y <= kFltEpsilon) return null_direction(row, ev.x, len);   // the two largest coincide
+    if (ev.z - ev.y <= kFltEpsilon) return null_direction(row, ev.x);   // the two largest coincide
     // distinct eigenvalues: the directions for the largest, middle and smallest; the least
-    // reliable two (shortest cross products) are rebuilt as cross products of the others
-    float3 e[3];
-    float lens[3];
-    e[2] = null_direction(row, ev.z, lens[2]);
+    // reliable two (shortest cross products) are rebuilt as cross products of the others: first the shortest
+    // one, then the one in between.  Only what the smallest one's needs is normalised and rebuilt.
+    float l2, l1, l0, unused, third;
+    const float3 v2 = null_product(row, ev.z, l2, unused);
+    const float3 v1 = null_product(row, ev.y, l1, unused);
+    // the reference compares the third candidate's length for the smallest, whichever candidate won
+    const float3 v0 = null_product(row, ev.x, l0, third);
     int min_el = 2, max_el = 2;
-    e[1] = null_direction(row, ev.y, lens[1]);
-    if (lens[1] <= lens[min_el]) min_el = 1;
-    if (lens[1] > lens[max_el]) max_el = 1;
-    e[0] = null_direction(row, ev.x, lens[0]);
-    // the reference compares the third candidate's length here whichever candidate won
-    const float3 r1 = v3(row[1].x, row[1].y - ev.x, row[1].z), r2 = v3(row[2].x, row[2].y, row[2].z - ev.x);
-    const float3 c = cross(r1, r2);
-    const float len3 = dot(c, c);
-    if (len3 <= lens[min_el]) min_el = 0;
-    if (len3 > lens[max_el]) max_el = 0;
+    float shortest = l2, longest = l2;
+    if (l1 <= shortest) { min_el = 1; shortest = l1; }
+    if (l1 > longest) { max_el = 1; longest = l1; }
+    if (third <= shortest) min_el = 0;
+    if (third > longest) max_el = 0;
     const int mid_el = 3 - min_el - max_el;
-    e[min_el] = unit(cross(e[(min_el + 1) % 3], e[(min_el + 2) % 3]));
-    e[mid_el] = unit(cross(e[(mid_el + 1) % 3], e[(mid_el + 2) % 3]));
-    return e[0];
+    if (min_el != 0 && mid_el != 0) return scaled(v0, inv_sqrt(l0));
+    float3 e1 = scaled(v1, inv_sqrt(l1)), e2 = scaled(v2, inv_sqrt(l2));
+    if (min_el != 0) {   // the smallest one's lies in between: rebuilt from a rebuilt shortest one
+        const float3 e0 = scaled(v0, inv_sqrt(l0));
+        if (min_el == 1) e1 = unit(cross(e2, e0));
+        else e2 = unit(cross(e0, e1));
+    }
+    return unit(cross(e1, e2));
 }
 
 // compute_radius (normal_map.cu:10-23): the surfel radius in millimetres.
@@ -174,7 +182,8 @@ __device__ __forceinline__ float surfel_radius(float depth_m, float normal_z, fl
 // What bounds it is instruction issue: about 300 for the window's mean, 700 for its covariance (every product
 // and sum rounded on its own) and 1000 for the eigenvector, a pixel.  Vertices that count as zero are stored
 // as zeros, which add exactly nothing to the mean, and marked in a bit mask per tile row, so that the window
-// loops need no test of three components an element: 27.2 -> 26.1 us at 640x480, 70.3 -> 67.0 at 1280x720.
+// loops need no test of three components an element (27.2 -> 26.1 us at 640x480); only the eigenvector that is
+// returned is normalised and rebuilt (26.1 -> 25.2 us; 70.3 -> 64.4 in all at 1280x720).
 // Two and four pixels a thread, their windows read once, took 57 and 88 us: the unrolled sums need 164 and
 // 213 registers, and the eigenvector's chain of square roots and divisions needs the warps.
 __global__ void __launch_bounds__(kTileW *kTileH) k_measure_maps(const uint16_t *depth, int width, int height,
