@@ -875,16 +875,20 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncwarp();
         }
-        // lane sums of M -> slots; lane e < 21 sums entry e over the lanes in lane order
-#pragma unroll
-        for (int i = 0; i < 21; ++i) mine[i] = M[i];
-        __syncwarp();
+        // lane sums of M -> slots; lane e < 21 sums entry e over the lanes in lane order (those past the list
+        // hold zeros); nearly half of a scene's pairs have no dense term, and M is zero
         float m = 0.f;
-        if (lane < 21) {
+        if (end - beg > (uint32_t)nreg) {
+#pragma unroll
+            for (int i = 0; i < 21; ++i) mine[i] = M[i];
+            __syncwarp();
+            if (lane < 21) {
+                const int lanes = (int)min(32u, end - beg);
 #pragma unroll 8
-            for (int l = 0; l < 32; ++l) m += slots[l * kSlot + lane];
+                for (int l = 0; l < lanes; ++l) m += slots[l * kSlot + lane];
+            }
+            __syncwarp();
         }
-        __syncwarp();
         if (lane < 21) {   // the full symmetric M, row-major, in slots[0, 36)
             int ea = 0, ec = 0;
             tri_decode(lane, ea, ec);
