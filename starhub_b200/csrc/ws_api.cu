@@ -174,7 +174,11 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     A(dalloc(&w.n2t_val_alt, w.cap_n2t));
     A(dalloc(&w.n2t_offset, w.cap_nodes + 1));
     A(dalloc(&w.row_pair_cols, (size_t)w.cap_nodes * ws::kRowPairsMax));
-    A(dalloc(&w.row_pair_cnts, (size_t)w.cap_nodes * ws::kRowPairsMax));
+    {   // counts of a row's warps: up to 8 or 4 a row where the rows are few (pair_row_warps)
+        const uint32_t shares = std::max({w.cap_nodes, 4u * std::min(w.cap_nodes, ws::kRowWide4),
+                                          8u * std::min(w.cap_nodes, ws::kRowWide8)});
+        A(dalloc(&w.row_pair_cnts, (size_t)shares * ws::kRowPairsMax));
+    }
     A(dalloc(&w.row_pair_first, w.cap_nodes + 1));
     A(dalloc(&w.row_entry_first, w.cap_nodes + 1));
     A(dalloc(&w.pair_val, w.cap_pair_kv));

@@ -18,6 +18,8 @@ namespace ws {
 constexpr int kVecStride = 8;        // floats per node in PCG vectors
 constexpr int kSdStride = 12;        // floats per node in the PCG's s/d records
 constexpr int kRowPairsMax = 64;     // upper node pairs of one row in the pair map (WS_ERR_CAPACITY beyond)
+constexpr uint32_t kRowWide8 = 1184;   // nodes up to which the pair map may put 8 warps to a row (all resident at once)
+constexpr uint32_t kRowWide4 = 16384;  // and 4
 constexpr int kDenseRecord = 32;     // floats per dense-term record, largest layout (128 B)
 constexpr int kRegRecord = 16;       // floats per reg-term record (64 B)
 constexpr uint32_t kInvalidIndex = 0xFFFFFFFFu;

@@ -231,235 +231,329 @@ __global__ void k_n2t_offsets(const uint32_t *sorted_keys, const uint32_t *count
 // of the list, the term's nodes above i (every knn slot above i; the other end of an edge) yields
 // exactly row i's entries, each pair's in term order.  The pairs are sorted by (row, column), so
 // row i's pairs and entries are one contiguous range after those of the rows before it.
-// Pass 1 (one warp per row) counts each column's entries in a small hash table in shared memory
-// and keeps the row's columns sorted; two scans give every row its first pair and first entry;
-// pass 2 writes the pairs and places every entry at its pair's next free position.
+// Pass 1 counts each column's entries in a small hash table in shared memory and keeps the row's
+// columns sorted; two scans give every row its first pair and first entry; pass 2 writes the pairs
+// and places every entry at its pair's next free position.
+// What bounds them: the latency of a list's words and of its terms' nodes while rows are few, the
+// instructions per entry when there are many.  Hence W warps to a row where rows are few and long
+// (each takes a run of whole chunks and counts it apart, so that pass 2 knows where its entries of a
+// pair begin), the loads of the next two chunks in flight, and a table whose first probe nearly
+// always finds the column.  Both passes together, a warp a row without the pipeline / now: 500
+// nodes, lists of some 2000 entries 219 -> 35 us; 3000 nodes with 720p images 339 -> 84; 1800 nodes
+// 101 -> 30; 8000 nodes 78 -> 44; 64 scenes of 500 to 8000 nodes 1308 -> 909.
 // ---------------------------------------------------------------------------
-constexpr int kRowHash = 128;        // hash slots per warp (twice kRowPairsMax)
-constexpr int kRowWarps = 4;         // warps per block of the two row passes
-constexpr int kRowLanesEntries = 4;  // list entries per lane and pass (loads in flight)
+constexpr int kRowHash = 128;        // hash slots per row (twice kRowPairsMax)
+constexpr int kRowWarps = 4;         // warps per block when a warp has a row to itself
+constexpr int kRowBlocks = 10;       // such blocks per SM: 64 scenes 909 us; 8 blocks 941, 12 blocks 995
+constexpr int kRowLanesEntries = 2;  // list entries per lane and pass (loads in flight)
 constexpr int kRowChunk = 32 * kRowLanesEntries;   // list entries per pass
 constexpr int kRowStage = 3 * kRowChunk;           // their candidates (at most 3 each)
 
 constexpr uint32_t kNoCol = 0xFFFFFFFFu;
 
-// The columns above `row` that list entry `t` (scene-local term id) adds to row `row`'s pairs, in
-// c[0..2] (kNoCol where none); returns their number (at most 3).
-__device__ __forceinline__ int row_pair_columns(const Scene &sc, const Plan &p, const ushort4 *dense_knn,
-                                                uint32_t row, uint32_t t, uint32_t (&c)[3], int *err) {
-    const uint32_t nb = (uint32_t)sc.node_base, nd = p.dense_count, ne = (uint32_t)sc.num_edges,
-                   nn = (uint32_t)sc.num_nodes;
-    c[0] = c[1] = c[2] = kNoCol;
-    int n = 0;
-    auto push = [&](uint32_t v) {
-        c[0] = n == 0 ? v : c[0];
-        c[1] = n == 1 ? v : c[1];
-        c[2] = n == 2 ? v : c[2];
-        n = min(n + 1, 3);
-    };
-    if (t < nd || t >= nd + ne + nn) {   // dense or feature term: its knn slots above the row
-        const ushort4 k4 = t < nd ? dense_knn[p.dense_begin + t] : clamp_knn(sc.feature_knn[t - nd - ne - nn], sc, err);
-        if (nb + k4.x > row) push(nb + k4.x);
-        if (nb + k4.y > row) push(nb + k4.y);
-        if (nb + k4.z > row) push(nb + k4.z);
-        if (nb + k4.w > row) push(nb + k4.w);
-    } else if (t < nd + ne) {            // edge: its other end
+// List entry `t`'s (scene-local term id) nodes, local to the scene: a dense or feature term's four,
+// an edge's other end.  What adds no pair to the row (nothing there, a node-motion term, the
+// absent slots of an edge) is the row's own node, which is not above itself.
+__device__ __forceinline__ ushort4 row_entry_nodes(const Scene &sc, const Plan &p, const ushort4 *dense_knn,
+                                                   uint32_t local, uint32_t t, int *err) {
+    const uint32_t nd = p.dense_count, ne = (uint32_t)sc.num_edges, nn = (uint32_t)sc.num_nodes;
+    const uint16_t l = (uint16_t)local;
+    ushort4 k = make_ushort4(l, l, l, l);
+    if (t == kNoCol) return k;
+    if (t < nd) {
+        k = dense_knn[p.dense_begin + t];
+    } else if (t >= nd + ne + nn) {
+        k = clamp_knn(sc.feature_knn[t - nd - ne - nn], sc, err);
+    } else if (t < nd + ne) {
         uint16_t x, y;
         edge_ends(sc, t - nd, x, y, err);
-        const uint32_t other = (nb + x == row) ? nb + y : nb + x;
-        if (x != y && other > row) push(other);
+        k.x = x == l ? y : x;   // a self edge is in no list
     }
-    return n;
+    return k;
 }
 
-// Row `row`'s candidate columns of list entries base .. base + kRowChunk - 1 (below end), staged
-// in list order as (column, term); returns their number.  Lane l reads entries base + 32 q + l, so
-// every load instruction is coalesced and a lane has kRowLanesEntries gathers in flight.
-__device__ __forceinline__ uint32_t stage_row_candidates(const Scene &sc, const Plan &p, const ushort4 *dense_knn,
-                                                         const uint32_t *n2t_val, uint32_t row, uint32_t base,
-                                                         uint32_t end, uint32_t *st_col, uint32_t *st_term, int lane,
-                                                         int *err) {
-    uint32_t t[kRowLanesEntries];
+// A warp's share of a row's list, kRowChunk entries at a time: lane l has entries base + 32 q + l, so
+// every load instruction is coalesced and a lane has kRowLanesEntries gathers in flight.  The words
+// of the chunk after next and the nodes of the next one are on the way while a chunk is worked on:
+// both loads' latencies, some 1500 cycles together, otherwise stand before every chunk.
+__device__ __forceinline__ void row_words(uint32_t (&t)[kRowLanesEntries], const uint32_t *n2t_val, uint32_t base,
+                                          uint32_t end, int lane) {
 #pragma unroll
     for (int q = 0; q < kRowLanesEntries; ++q) {
         const uint32_t e = base + 32u * q + (uint32_t)lane;
         t[q] = e < end ? n2t_val[e] : kNoCol;
     }
-    uint32_t carry = 0;
+}
+
+// Calls use(t, k) for every chunk of entries beg .. end - 1, in order.
+template <class F>
+__device__ __forceinline__ void row_walk(const Scene &sc, const Plan &p, const ushort4 *dense_knn,
+                                         const uint32_t *n2t_val, uint32_t local, uint32_t beg, uint32_t end, int lane,
+                                         int *err, F &&use) {
+    if (beg >= end) return;
+    uint32_t t[kRowLanesEntries], t_next[kRowLanesEntries], t_after[kRowLanesEntries];
+    ushort4 k[kRowLanesEntries], k_next[kRowLanesEntries];
+    row_words(t, n2t_val, beg, end, lane);
+    const bool longer = beg + kRowChunk < end;
+    if (longer) row_words(t_next, n2t_val, beg + kRowChunk, end, lane);
 #pragma unroll
-    for (int q = 0; q < kRowLanesEntries; ++q) {
-        uint32_t col[3] = {kNoCol, kNoCol, kNoCol};
-        const int n = t[q] != kNoCol ? row_pair_columns(sc, p, dense_knn, row, t[q], col, err) : 0;
-        const uint32_t incl = warp_incl_scan_u32((uint32_t)n);
-        const uint32_t off = carry + incl - (uint32_t)n;
+    for (int q = 0; q < kRowLanesEntries; ++q) k[q] = row_entry_nodes(sc, p, dense_knn, local, t[q], err);
+    for (uint32_t base = beg;;) {
+        const bool more = base + kRowChunk < end;
+        if (more) {
+            row_words(t_after, n2t_val, base + 2 * kRowChunk, end, lane);
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (k < n) {
-                st_col[off + k] = col[k];
-                st_term[off + k] = t[q];
-            }
-        carry += __shfl_sync(0xffffffffu, incl, 31);
+            for (int q = 0; q < kRowLanesEntries; ++q)
+                k_next[q] = row_entry_nodes(sc, p, dense_knn, local, t_next[q], err);
+        }
+        use(t, k);
+        if (!more) return;
+        base += kRowChunk;
+#pragma unroll
+        for (int q = 0; q < kRowLanesEntries; ++q) {
+            t[q] = t_next[q];
+            t_next[q] = t_after[q];
+            k[q] = k_next[q];
+        }
     }
-    __syncwarp();
-    return carry;
+}
+
+// Entries beg .. end - 1 of a row's list that warp w of W walks: whole chunks, the same in both passes.
+template <int W>
+__device__ __forceinline__ void row_share(uint32_t &beg, uint32_t &end, int w) {
+    if (W == 1) return;
+    const uint32_t chunks = (end - beg + kRowChunk - 1) / kRowChunk, share = (chunks + W - 1) / W * kRowChunk;
+    const uint32_t b = beg + (uint32_t)w * share;
+    beg = min(b, end);
+    end = min(beg + share, end);
+}
+
+template <int W>
+__device__ __forceinline__ void row_sync() {
+    if (W == 1) __syncwarp();
+    else __syncthreads();
 }
 
 __device__ __forceinline__ uint32_t col_hash(uint32_t c) { return (c * 2654435761u) >> (32 - 7); }
 
-__global__ void __launch_bounds__(32 * kRowWarps) k_pair_rows_count(
+template <int W>
+__global__ void __launch_bounds__(32 * (W == 1 ? kRowWarps : W), (W == 1 ? kRowBlocks : 1)) k_pair_rows_count(
     const Scene *scenes, const Plan *plan, const uint32_t *node_scene, uint32_t total_nodes,
     const uint32_t *n2t_offset, const uint32_t *n2t_val, uint32_t cap_n2t, const ushort4 *dense_knn, uint32_t *row_cols,
     uint32_t *row_cnts, uint32_t *row_pairs, uint32_t *row_entries, int *err) {
     static_assert(kRowHash == 128, "col_hash gives 7 bits");
-    __shared__ uint32_t hkey[kRowWarps][kRowHash], hcnt[kRowWarps][kRowHash];
-    __shared__ uint32_t lcol[kRowWarps][kRowHash], lcnt[kRowWarps][kRowHash];
-    __shared__ uint32_t st_col[kRowWarps][kRowStage], st_term[kRowWarps][kRowStage];
+    constexpr int kRows = W == 1 ? kRowWarps : 1;   // rows a block has in hand
+    __shared__ uint32_t hkey[kRows][kRowHash], hcnt[kRows][W][kRowHash];
+    __shared__ uint32_t lcol[kRows][kRowHash], lslot[kRows][kRowHash];
+    __shared__ int hfull[kRows];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t *keys = hkey[wib], *cnts = hcnt[wib];
+    const int r = W == 1 ? wib : 0, w = W == 1 ? 0 : wib;
+    volatile uint32_t *keys = hkey[r];
+    uint32_t *cnts = hcnt[r][w];
     const unsigned lower = (1u << lane) - 1u;
-    const uint32_t warps = gridDim.x * kRowWarps;
-    for (uint32_t row = blockIdx.x * kRowWarps + wib; row < total_nodes; row += warps) {
+    for (uint32_t row = blockIdx.x * kRows + r; row < total_nodes; row += gridDim.x * kRows) {
         for (int k = lane; k < kRowHash; k += 32) {
-            keys[k] = kNoCol;
+            if (w == 0) keys[k] = kNoCol;
             cnts[k] = 0;
         }
-        __syncwarp();
+        if (w == 0 && lane == 0) hfull[r] = 0;
+        row_sync<W>();
         const uint32_t s = node_scene[row];
         const Scene &sc = scenes[s];
         const Plan &p = plan[s];
-        const uint32_t beg = n2t_offset[row], end = n2t_offset[row + 1];
+        const uint32_t nb = (uint32_t)sc.node_base, local = row - nb;
+        uint32_t beg = n2t_offset[row], end = n2t_offset[row + 1];
+        row_share<W>(beg, end, w);
         if (lane == 0 && end > beg + kRowChunk) l2_prefetch_list(n2t_val, beg + kRowChunk, end, cap_n2t);
-        bool full = false;
-        for (uint32_t base = beg; base < end; base += kRowChunk) {
-            const uint32_t total =
-                stage_row_candidates(sc, p, dense_knn, n2t_val, row, base, end, st_col[wib], st_term[wib], lane, err);
-            for (uint32_t v0 = 0; v0 < total; v0 += 32) {
-                const uint32_t v = v0 + (uint32_t)lane;
-                const uint32_t c = v < total ? st_col[wib][v] : kNoCol;
-                const unsigned peers = __match_any_sync(0xffffffffu, c);
-                if (c != kNoCol && (peers & lower) == 0) {   // one insertion per column and pass
-                    uint32_t slot = col_hash(c);
-                    bool placed = false;
-                    for (int probe = 0; probe < kRowHash && !placed; ++probe) {
-                        const uint32_t prev = atomicCAS(&keys[slot], kNoCol, c);
-                        if (prev == kNoCol || prev == c) {
-                            atomicAdd(&cnts[slot], (uint32_t)__popc(peers));
-                            placed = true;
-                        }
-                        slot = (slot + 1) & (kRowHash - 1);
-                    }
-                    if (!placed) full = true;
+        // almost every candidate finds its column at the first place it looks
+        auto count = [&](uint32_t node) {
+            uint32_t slot = col_hash(node);
+            uint32_t key = keys[slot];
+            const bool above = node > local;
+            if (above && key != node) {
+                int probe = 0;
+                for (; probe < kRowHash; ++probe) {
+                    if (key == kNoCol) key = atomicCAS(&hkey[r][slot], kNoCol, node);
+                    if (key == kNoCol || key == node) break;
+                    slot = (slot + 1) & (kRowHash - 1);
+                    key = keys[slot];
                 }
+                if (probe == kRowHash) hfull[r] = 1;
+            }
+            if (above) atomicAdd(&cnts[slot], 1u);
+        };
+        row_walk(sc, p, dense_knn, n2t_val, local, beg, end, lane, err,
+                 [&](const uint32_t (&)[kRowLanesEntries], const ushort4 (&k)[kRowLanesEntries]) {
+#pragma unroll
+                     for (int q = 0; q < kRowLanesEntries; ++q) {
+                         count(k[q].x);
+                         count(k[q].y);
+                         count(k[q].z);
+                         count(k[q].w);
+                     }
+                 });
+        row_sync<W>();
+        // the table's columns, compacted in slot order, then ranked by column
+        if (w == 0) {
+            uint32_t n_cols = 0;
+            for (int q = 0; q < kRowHash / 32; ++q) {
+                const uint32_t c = keys[32 * q + lane];
+                const unsigned occ = __ballot_sync(0xffffffffu, c != kNoCol);
+                if (c != kNoCol) {
+                    const uint32_t idx = n_cols + (uint32_t)__popc(occ & lower);
+                    lcol[r][idx] = c;
+                    lslot[r][idx] = (uint32_t)(32 * q + lane);
+                }
+                n_cols += (uint32_t)__popc(occ);
             }
             __syncwarp();
-        }
-        // the table's columns, compacted in slot order, then ranked by column
-        uint32_t n_cols = 0;
-        for (int q = 0; q < kRowHash / 32; ++q) {
-            const uint32_t c = keys[32 * q + lane];
-            const unsigned occ = __ballot_sync(0xffffffffu, c != kNoCol);
-            if (c != kNoCol) {
-                const uint32_t idx = n_cols + (uint32_t)__popc(occ & lower);
-                lcol[wib][idx] = c;
-                lcnt[wib][idx] = cnts[32 * q + lane];
+            const bool full = hfull[r] != 0 || n_cols > (uint32_t)kRowPairsMax;
+            if (full) {
+                if (lane == 0) set_error(err, WS_ERR_CAPACITY);
+                n_cols = 0;
             }
-            n_cols += (uint32_t)__popc(occ);
-        }
-        __syncwarp();
-        full = __any_sync(0xffffffffu, full) || n_cols > (uint32_t)kRowPairsMax;
-        if (full) {
-            if (lane == 0) set_error(err, WS_ERR_CAPACITY);
-            n_cols = 0;
-        }
-        uint32_t entries = 0;
-        for (uint32_t x = (uint32_t)lane; x < n_cols; x += 32) {
-            const uint32_t c = lcol[wib][x];
-            uint32_t rank = 0;
-            for (uint32_t y = 0; y < n_cols; ++y) rank += lcol[wib][y] < c ? 1u : 0u;
-            row_cols[(size_t)kRowPairsMax * row + rank] = c;
-            row_cnts[(size_t)kRowPairsMax * row + rank] = lcnt[wib][x];
-            entries += lcnt[wib][x];
-        }
+            uint32_t entries = 0;
+            for (uint32_t x = (uint32_t)lane; x < n_cols; x += 32) {
+                const uint32_t c = lcol[r][x];
+                uint32_t rank = 0;
+                for (uint32_t y = 0; y < n_cols; ++y) rank += lcol[r][y] < c ? 1u : 0u;
+                row_cols[(size_t)kRowPairsMax * row + rank] = nb + c;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) entries += __shfl_xor_sync(0xffffffffu, entries, o);
-        if (lane == 0) {
-            row_pairs[row] = n_cols;
-            row_entries[row] = full ? 0u : entries;
+                for (int v = 0; v < W; ++v) {
+                    const uint32_t n = hcnt[r][v][lslot[r][x]];
+                    row_cnts[((size_t)W * row + v) * kRowPairsMax + rank] = n;
+                    entries += n;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) entries += __shfl_xor_sync(0xffffffffu, entries, o);
+            if (lane == 0) {
+                row_pairs[row] = n_cols;
+                row_entries[row] = entries;
+            }
         }
-        __syncwarp();
+        row_sync<W>();
     }
 }
 
-__global__ void __launch_bounds__(32 * kRowWarps) k_pair_rows_fill(
+template <int W>
+__global__ void __launch_bounds__(32 * (W == 1 ? kRowWarps : W), (W == 1 ? kRowBlocks : 1)) k_pair_rows_fill(
     const Scene *scenes, const Plan *plan, const uint32_t *node_scene, uint32_t total_nodes,
     const uint32_t *n2t_offset, const uint32_t *n2t_val, uint32_t cap_n2t, const ushort4 *dense_knn, const uint32_t *row_cols,
     const uint32_t *row_cnts, const uint32_t *pair_first, const uint32_t *entry_first, uint32_t cap_half,
     uint32_t cap_kv, uint32_t *half_row, uint32_t *half_col, uint32_t *half_begin, uint32_t *half_end,
     uint32_t *half_scene, uint32_t *row_cnt_lo, uint32_t *pair_val, uint32_t *counts, int *err) {
-    __shared__ uint32_t s_col[kRowWarps][kRowPairsMax], s_next[kRowWarps][kRowPairsMax];
-    __shared__ uint32_t st_col[kRowWarps][kRowStage], st_term[kRowWarps][kRowStage];
+    constexpr int kWarps = W == 1 ? kRowWarps : W, kRows = W == 1 ? kRowWarps : 1;
+    __shared__ uint32_t hkey[kRows][kRowHash];   // place among the row's columns << 16 | node
+    __shared__ uint32_t s_next[kWarps][kRowPairsMax];
+    __shared__ uint32_t st_term[kWarps][kRowStage];
+    __shared__ uint16_t st_node[kWarps][kRowStage];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int r = W == 1 ? wib : 0, w = W == 1 ? 0 : wib;
+    uint32_t *next = s_next[wib], *term = st_term[wib];
+    uint16_t *node = st_node[wib];
     const unsigned lower = (1u << lane) - 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         counts[kCntHalf] = min(pair_first[total_nodes], cap_half);
         if (pair_first[total_nodes] > cap_half) set_error(err, WS_ERR_CAPACITY);
     }
-    const uint32_t warps = gridDim.x * kRowWarps;
-    for (uint32_t row = blockIdx.x * kRowWarps + wib; row < total_nodes; row += warps) {
+    for (uint32_t row = blockIdx.x * kRows + r; row < total_nodes; row += gridDim.x * kRows) {
         const uint32_t h0 = pair_first[row], n_cols = pair_first[row + 1] - h0;
+        if (n_cols == 0) continue;
         const uint32_t s = node_scene[row];
-        // the row's pairs: columns ascending, entry ranges one after another from the row's first
+        const Scene &sc = scenes[s];
+        const Plan &p = plan[s];
+        const uint32_t nb = (uint32_t)sc.node_base, local = row - nb;
+        if (w == 0)
+            for (int k = lane; k < kRowHash; k += 32) hkey[r][k] = kNoCol;
+        row_sync<W>();
+        // the row's pairs: columns ascending, entry ranges one after another from the row's first; in a
+        // pair's range the warps' shares one after another
         uint32_t carry = entry_first[row];
         for (uint32_t k0 = 0; k0 < n_cols; k0 += 32) {
             const uint32_t k = k0 + (uint32_t)lane;
             const uint32_t c = k < n_cols ? row_cols[(size_t)kRowPairsMax * row + k] : kNoCol;
-            const uint32_t n = k < n_cols ? row_cnts[(size_t)kRowPairsMax * row + k] : 0u;
+            uint32_t n = 0, before = 0;
+#pragma unroll
+            for (int v = 0; v < W; ++v) {
+                const uint32_t m = k < n_cols ? row_cnts[((size_t)W * row + v) * kRowPairsMax + k] : 0u;
+                before += v < w ? m : 0u;
+                n += m;
+            }
             const uint32_t incl = warp_incl_scan_u32(n);
             const uint32_t begin = carry + incl - n;
             carry += __shfl_sync(0xffffffffu, incl, 31);
             if (k < n_cols) {
-                s_col[wib][k] = c;
-                s_next[wib][k] = begin;
-                const uint32_t h = h0 + k;
-                if (h < cap_half) {
-                    half_row[h] = row;
-                    half_col[h] = c;
-                    half_begin[h] = begin;
-                    half_end[h] = begin + n;
-                    half_scene[h] = s;
-                    atomicAdd(&row_cnt_lo[c], 1u);
+                next[k] = begin + before;
+                if (w == 0) {
+                    uint32_t slot = col_hash(c - nb);
+                    for (int probe = 0; probe < kRowHash; ++probe) {
+                        if (atomicCAS(&hkey[r][slot], kNoCol, k << 16 | (c - nb)) == kNoCol) break;
+                        slot = (slot + 1) & (kRowHash - 1);
+                    }
+                    const uint32_t h = h0 + k;
+                    if (h < cap_half) {
+                        half_row[h] = row;
+                        half_col[h] = c;
+                        half_begin[h] = begin;
+                        half_end[h] = begin + n;
+                        half_scene[h] = s;
+                        atomicAdd(&row_cnt_lo[c], 1u);
+                    }
                 }
             }
         }
-        __syncwarp();
-        if (n_cols == 0) continue;
-        const Scene &sc = scenes[s];
-        const Plan &p = plan[s];
-        const uint32_t beg = n2t_offset[row], end = n2t_offset[row + 1];
+        row_sync<W>();
+        uint32_t beg = n2t_offset[row], end = n2t_offset[row + 1];
+        row_share<W>(beg, end, w);
         if (lane == 0 && end > beg + kRowChunk) l2_prefetch_list(n2t_val, beg + kRowChunk, end, cap_n2t);
-        for (uint32_t base = beg; base < end; base += kRowChunk) {
-            const uint32_t total =
-                stage_row_candidates(sc, p, dense_knn, n2t_val, row, base, end, st_col[wib], st_term[wib], lane, err);
+        row_walk(sc, p, dense_knn, n2t_val, local, beg, end, lane, err,
+                 [&](const uint32_t (&t)[kRowLanesEntries], const ushort4 (&k)[kRowLanesEntries]) {
+            // the chunk's candidates, staged in list order as (node, term)
+            uint32_t total = 0;
+#pragma unroll
+            for (int q = 0; q < kRowLanesEntries; ++q) {
+                const uint32_t n = min((uint32_t)(k[q].x > local) + (uint32_t)(k[q].y > local) +
+                                           (uint32_t)(k[q].z > local) + (uint32_t)(k[q].w > local), 3u);
+                const uint32_t incl = warp_incl_scan_u32(n), stop = total + incl;
+                uint32_t at = stop - n;
+                auto stage = [&](uint32_t v) {
+                    if (v > local && at < stop) {
+                        node[at] = (uint16_t)v;
+                        term[at] = t[q];
+                        ++at;
+                    }
+                };
+                stage(k[q].x);
+                stage(k[q].y);
+                stage(k[q].z);
+                stage(k[q].w);
+                total += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            __syncwarp();
             for (uint32_t v0 = 0; v0 < total; v0 += 32) {
                 const uint32_t v = v0 + (uint32_t)lane;
-                const uint32_t c = v < total ? st_col[wib][v] : kNoCol;
+                const uint32_t c = v < total ? (uint32_t)node[v] : kNoCol;
                 const unsigned peers = __match_any_sync(0xffffffffu, c);
-                uint32_t k = 0;
-                if (c != kNoCol) {   // the column's place among the row's (binary search)
-                    uint32_t lo = 0, hi = n_cols;
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if (s_col[wib][mid] < c) lo = mid + 1; else hi = mid;
+                uint32_t slot = col_hash(c), kk = kNoCol;
+                if (v < total) {
+                    uint32_t key = hkey[r][slot];
+                    for (int probe = 0; probe < kRowHash && (key & 0xFFFFu) != c && key != kNoCol; ++probe) {
+                        slot = (slot + 1) & (kRowHash - 1);
+                        key = hkey[r][slot];
                     }
-                    k = lo;
-                    const uint32_t pos = s_next[wib][min(k, n_cols - 1)] + (uint32_t)__popc(peers & lower);
-                    if (k < n_cols && s_col[wib][k] == c && pos < cap_kv) pair_val[pos] = st_term[wib][v];
+                    kk = (key & 0xFFFFu) == c ? key >> 16 : kNoCol;
+                }
+                if (kk < n_cols) {
+                    const uint32_t pos = next[kk] + (uint32_t)__popc(peers & lower);
+                    if (pos < cap_kv) pair_val[pos] = term[v];
                 }
                 __syncwarp();
-                if (c != kNoCol && (peers & lower) == 0 && k < n_cols) s_next[wib][k] += (uint32_t)__popc(peers);
+                if (kk < n_cols && (peers & lower) == 0) next[kk] += (uint32_t)__popc(peers);
                 __syncwarp();
             }
-        }
+        });
+        row_sync<W>();
     }
 }
 
@@ -600,30 +694,55 @@ __global__ void k_pcg_ranges(const uint32_t *item_ptr, const uint32_t *group_row
     }
 }
 
-static inline int grid_for(uint32_t n, int threads, int num_sms) {
+static inline int grid_for(uint32_t n, int threads, int num_sms, uint32_t per_sm = 8u) {
     const uint32_t want = (n + threads - 1) / threads;
-    const uint32_t cap = (uint32_t)num_sms * 8u;
+    const uint32_t cap = (uint32_t)num_sms * per_sm;
     return (int)std::max<uint32_t>(1u, std::min<uint32_t>(want, cap));
 }
 
+// Warps to a row of the pair map.  Several pay while rows are few and their lists long (pixels a node
+// say how long), one where rows fill the chip.  The whole index, 1 / 4 / 8 warps to a row, us:
+//   500 nodes, 614 px a node 372 / 263 / 239; 1000, 307 px 376 / 296 / 282; 1800, 171 px 341 / 292 / 296;
+//   3000, 102 px 341 / 304 / 318; 3000, 307 px 458 / 365 / 371; 5000, 184 px 429 / 382 / 410;
+//   8000, 38 px 334 / 360 / 407; 8000, 115 px 401 / 410 / 449; 8 x 500 nodes 538 / 464 / 470;
+//   20 x 500 nodes 879 / 812 / 867; 8 x 1800 nodes 521 / 540 / 620.
+static int pair_row_warps(const Workspace &w) {
+    uint64_t pixels = 0;
+    for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s)
+        pixels += (uint64_t)w.h_scenes[s].width * w.h_scenes[s].height;
+    const uint64_t n = w.total_nodes;
+    if (n <= kRowWide8 && pixels >= 250 * n) return 8;
+    if ((n <= 6000 && pixels >= 75 * n) || (n <= kRowWide4 && pixels >= 300 * n)) return 4;
+    return 1;
+}
+
 // Node pair -> term map, row by row from the node -> term map (see k_pair_rows_count).
-static void pair_index(Workspace &w, cudaStream_t st) {
+template <int W>
+static void pair_index_rows(Workspace &w, cudaStream_t st) {
     const uint32_t N = w.total_nodes;
-    const int grid = grid_for(N * 32u, 32 * kRowWarps, w.num_sms);
-    k_pair_rows_count<<<grid, 32 * kRowWarps, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset,
-                                                      w.n2t_sorted_val, w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts,
-                                                      w.row_cnt_up, w.row_entry_first, w.error_flag);
+    const int threads = 32 * (W == 1 ? kRowWarps : W);
+    const int grid = grid_for(N * 32u * W, threads, w.num_sms, 16);
+    k_pair_rows_count<W><<<grid, threads, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset, w.n2t_sorted_val,
+                                                   w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts, w.row_cnt_up,
+                                                   w.row_entry_first, w.error_flag);
     exclusive_scan(w.row_cnt_up, w.row_pair_first, nullptr, N, w.cap_nodes, w.scan_tmp, st);
     exclusive_scan(w.row_entry_first, w.row_entry_first, nullptr, N, w.cap_nodes, w.scan_tmp, st);
     cudaMemsetAsync(w.row_cnt_lo, 0, sizeof(uint32_t) * w.cap_nodes, st);
-    k_pair_rows_fill<<<grid, 32 * kRowWarps, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset,
-                                                     w.n2t_sorted_val, w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts,
-                                                     w.row_pair_first, w.row_entry_first, w.cap_half, w.cap_pair_kv,
-                                                     w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene,
-                                                     w.row_cnt_lo,
-                                                     w.pair_val, w.counts, w.error_flag);
-    w.pair_sorted_val = w.pair_val;
+    k_pair_rows_fill<W><<<grid, threads, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset, w.n2t_sorted_val,
+                                                  w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts,
+                                                  w.row_pair_first, w.row_entry_first, w.cap_half, w.cap_pair_kv,
+                                                  w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene,
+                                                  w.row_cnt_lo, w.pair_val, w.counts, w.error_flag);
     count_launch(w, 1 + 3 + 3 + 1);
+}
+
+static void pair_index(Workspace &w, cudaStream_t st) {
+    switch (pair_row_warps(w)) {
+        case 8: pair_index_rows<8>(w, st); break;
+        case 4: pair_index_rows<4>(w, st); break;
+        default: pair_index_rows<1>(w, st);
+    }
+    w.pair_sorted_val = w.pair_val;
 }
 
 void index_build(Workspace &w, cudaStream_t st) {

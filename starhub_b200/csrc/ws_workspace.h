@@ -74,7 +74,8 @@ struct Workspace {
 
     // pair->term, built row by row: per row its upper pairs' columns and entry counts (at most
     // kRowPairsMax a row), its first pair and first entry; pair_val holds every pair's term list
-    uint32_t *row_pair_cols = nullptr, *row_pair_cnts = nullptr;   // [cap_nodes * kRowPairsMax]
+    uint32_t *row_pair_cols = nullptr;                       // [cap_nodes * kRowPairsMax]
+    uint32_t *row_pair_cnts = nullptr;                       // [(row, warp of the row) * kRowPairsMax]
     uint32_t *row_pair_first = nullptr, *row_entry_first = nullptr;   // [cap_nodes + 1]
     uint32_t *pair_val = nullptr;                            // [cap_pair_kv]
     const uint32_t *pair_sorted_val = nullptr;
