@@ -703,12 +703,37 @@ __global__ void __launch_bounds__(64) k_block_inverse(const double *diag64, cons
 // pair, and the pair's smoothness terms (at most one per edge direction) are added last, in
 // list order, by the whole warp.
 // ---------------------------------------------------------------------------
-// v[i] for a run-time i < 6, by selects (no local-memory array).
-__device__ __forceinline__ float pick6(const float *v, int i) {
-    float r = v[0];
+// A smoothness term's rows for one of its nodes hold few different numbers (reg_unit_jacobian, recentred):
+// with d = (the term's point for the node) - (the node's centre), the three channels are
+//   (0, dz, -dy, 1, 0, 0), (-dz, 0, dx, 0, 1, 0), (dy, -dx, 0, 0, 0, 1), negated for the edge's second node.
+// They are kept as eight scaled words, 0, dx, dy, dz, -dx, -dy, -dz, 1, and this is the word of column q.  Building
+// both 3x6 Jacobians in every lane and picking from them took a seventh of the kernel's instructions (64 scenes,
+// 5 launches: 5.89 -> 5.77 ms without).
+__host__ __device__ constexpr int reg_word(int ch, int q) {
+    return q >= 3 ? (q - 3 == ch ? 7 : 0)
+         : ch == 0 ? (q == 1 ? 3 : q == 2 ? 5 : 0)
+         : ch == 1 ? (q == 0 ? 6 : q == 2 ? 1 : 0)
+                   : (q == 0 ? 2 : q == 1 ? 4 : 0);
+}
+// The words whose products make entry (r, c) of a term's block, at most two, in channel order:
+// row word | column word << 8 | row word << 16 | column word << 24 (word 0 is zero).
+__device__ __forceinline__ uint32_t reg_words(int r, int c) {
+    uint32_t w = 0;
+    int n = 0;
 #pragma unroll
-    for (int k = 1; k < 6; ++k) r = i == k ? v[k] : r;
-    return r;
+    for (int ch = 0; ch < 3; ++ch) {
+        int a = 0, b = 0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            a = r == q ? reg_word(ch, q) : a;
+            b = c == q ? reg_word(ch, q) : b;
+        }
+        if (a != 0 && b != 0) {
+            w |= (uint32_t)(a | b << 8) << (16 * n);
+            ++n;
+        }
+    }
+    return w;
 }
 
 template <int NT, int C, int kTPL, int kBufs>
@@ -730,6 +755,12 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     float *mine = slots + lane * kSlot;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nhalf = counts[kCntHalf];
+    // the lane's place in M (lane < 21) and the words of its block entries lane, 32 + lane (the latter in row 5,
+    // where only (5, 5) has a product)
+    int ea = 0, ec = 0;
+    tri_decode(lane, ea, ec);
+    const uint32_t m_at = (uint32_t)((6 * ea + ec) | (6 * ec + ea) << 8);
+    const uint32_t reg0 = reg_words(lane / 6, lane % 6);
     // grid-stride: at any time the warps work on neighbouring pairs, whose term records overlap,
     // so the records are read from DRAM about once and then from L2
     for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; h < nhalf; h += warps) {
@@ -875,63 +906,73 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncwarp();
         }
-        // lane sums of M -> slots; lane e < 21 sums entry e over the lanes in lane order (those past the list
-        // hold zeros); nearly half of a scene's pairs have no dense term, and M is zero
-        float m = 0.f;
+        float acc0 = 0.f, acc1 = 0.f;   // the block's entries lane, 32 + lane
+        // nearly half of a scene's pairs have no dense term: M is zero
         if (end - beg > (uint32_t)nreg) {
+            // lane sums of M -> slots; lane e < 21 sums entry e over the lanes in lane order (those past the
+            // list hold zeros)
 #pragma unroll
             for (int i = 0; i < 21; ++i) mine[i] = M[i];
             __syncwarp();
+            float m = 0.f;
             if (lane < 21) {
                 const int lanes = (int)min(32u, end - beg);
 #pragma unroll 8
                 for (int l = 0; l < lanes; ++l) m += slots[l * kSlot + lane];
             }
             __syncwarp();
+            if (lane < 21) {   // the full symmetric M, row-major, in slots[0, 36)
+                slots[m_at & 0xFFu] = m;
+                slots[m_at >> 8] = m;
+            }
+            __syncwarp();
+            // A = M S^T: A[:, 0:3] = M[:, 0:3] + M[:, 3:6] [c_col - c_row]x, A[:, 3:6] = M[:, 3:6]
+            const float3 dc = f3(c_col.x - c_row.x, c_col.y - c_row.y, c_col.z - c_row.z);
+            auto entry = [&](int e) -> float {
+                const int r = e / 6, c = e % 6;
+                float v = slots[e];
+                if (centred && c < 3) {
+                    const float *mr = slots + 6 * r + 3;
+                    // column c of [d]x = [[0, -dz, dy], [dz, 0, -dx], [-dy, dx, 0]]
+                    const float k0 = c == 0 ? 0.f : (c == 1 ? -dc.z : dc.y);
+                    const float k1 = c == 0 ? dc.z : (c == 1 ? 0.f : -dc.x);
+                    const float k2 = c == 0 ? -dc.y : (c == 1 ? dc.x : 0.f);
+                    v += mr[0] * k0 + mr[1] * k1 + mr[2] * k2;
+                }
+                return v;
+            };
+            acc0 = entry(lane);
+            acc1 = lane < 4 ? entry(32 + lane) : 0.f;
         }
-        if (lane < 21) {   // the full symmetric M, row-major, in slots[0, 36)
-            int ea = 0, ec = 0;
-            tri_decode(lane, ea, ec);
-            slots[6 * ea + ec] = m;
-            slots[6 * ec + ea] = m;
+        // smoothness rows (node_graph_reg_jacobian.cuh:85-106, 193-233), in list order: half a warp turns a
+        // stashed record into the words of its two nodes, then every lane multiplies its own
+        const int terms = min(nreg, kStash);
+        for (int k0 = 0; k0 < terms; k0 += 2) {
+            const int k = k0 + (lane >> 4), q = lane & 7;
+            float v = 0.f;
+            if (k < terms) {
+                const float *rec = stash + kRegRecord * k;
+                const bool second = (lane & 8) != 0;   // the pair's column node
+                const bool is_i = __float_as_uint(rec[8]) == (second ? col : row);
+                const int at = q < 4 ? q - 1 : q - 4;   // x, y, z for words 1 to 3 and 4 to 6
+                float d = 1.f;
+                if (q >= 1 && q < 7) {
+                    d = rec[(is_i ? 0 : 3) + at];
+                    const float3 c = second ? c_col : c_row;
+                    if (centred) d -= at == 0 ? c.x : (at == 1 ? c.y : c.z);
+                }
+                const float s1 = lam_r * rec[6] * d;
+                if (q != 0 && rec[7] != 0.f) v = ((q >= 4 && q < 7) == is_i) ? -s1 : s1;   // validity
+            }
+            __syncwarp();
+            if (k < terms) stash[kRegRecord * k + (lane & 15)] = v;
         }
         __syncwarp();
-        // A = M S^T: A[:, 0:3] = M[:, 0:3] + M[:, 3:6] [c_col - c_row]x, A[:, 3:6] = M[:, 3:6]
-        const float3 dc = f3(c_col.x - c_row.x, c_col.y - c_row.y, c_col.z - c_row.z);
-        auto entry = [&](int e) -> float {
-            const int r = e / 6, c = e % 6;
-            float v = slots[e];
-            if (centred && c < 3) {
-                const float *mr = slots + 6 * r + 3;
-                // column c of [d]x = [[0, -dz, dy], [dz, 0, -dx], [-dy, dx, 0]]
-                const float k0 = c == 0 ? 0.f : (c == 1 ? -dc.z : dc.y);
-                const float k1 = c == 0 ? dc.z : (c == 1 ? 0.f : -dc.x);
-                const float k2 = c == 0 ? -dc.y : (c == 1 ? dc.x : 0.f);
-                v += mr[0] * k0 + mr[1] * k1 + mr[2] * k2;
-            }
-            return v;
-        };
-        float acc0 = entry(lane), acc1 = lane < 4 ? entry(32 + lane) : 0.f;   // entries lane, 32 + lane
-        // smoothness rows (node_graph_reg_jacobian.cuh:85-106, 193-233), in list order
-        const int r0 = lane / 6, c0 = lane % 6, r1 = (32 + lane) / 6, c1 = (32 + lane) % 6;
-        for (int k = 0; k < min(nreg, kStash); ++k) {
-            const float *rec = stash + kRegRecord * k;
-            if (rec[7] == 0.f) continue;   // validity
-            const float3 a3 = f3(rec[0], rec[1], rec[2]), b3 = f3(rec[3], rec[4], rec[5]);
-            const uint32_t ei = __float_as_uint(rec[8]);
-            float Jr[3][6], Jc[3][6];
-            reg_unit_jacobian(a3, b3, row == ei, Jr);
-            reg_unit_jacobian(a3, b3, col == ei, Jc);
-            const float scale = lam_r * rec[6];
-#pragma unroll
-            for (int ch = 0; ch < 3; ++ch) {
-                if (centred) {
-                    recentre(Jr[ch], c_row);
-                    recentre(Jc[ch], c_col);
-                }
-                acc0 += (scale * pick6(Jr[ch], r0)) * (scale * pick6(Jc[ch], c0));
-                if (lane < 4) acc1 += (scale * pick6(Jr[ch], r1)) * (scale * pick6(Jc[ch], c1));
-            }
+        for (int k = 0; k < terms; ++k) {
+            const float *row_w = stash + kRegRecord * k, *col_w = row_w + 8;
+            acc0 += row_w[reg0 & 0xFFu] * col_w[reg0 >> 8 & 0xFFu];
+            acc0 += row_w[reg0 >> 16 & 0xFFu] * col_w[reg0 >> 24];
+            if (lane == 3) acc1 += row_w[7] * col_w[7];
         }
         __syncwarp();
         // item h + row + 1 of the symmetric store: the row's diagonal item and its earlier pairs
