@@ -218,6 +218,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     A(cudaEventCreateWithFlags(&w.tables_free, cudaEventDisableTiming));
     if (e == cudaSuccess) {
         A(cudaMemset(w.error_flag, 0, 4 * sizeof(int)));
+        A(cudaMemset(w.counts, 0, 8 * sizeof(uint32_t)));
         A(cudaMemset(w.scene_counter, 0, 64ull * w.cap_scenes * sizeof(uint32_t)));
         A(cudaMemset(w.se3, 0, (size_t)w.cap_nodes * 8 * sizeof(float)));
     }

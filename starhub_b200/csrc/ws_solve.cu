@@ -321,6 +321,7 @@ __device__ __forceinline__ void cholesky6_fp64(const double *in, float *out) {
 // lane (27 sums for a node, 21 or 36 for a pair); the stride keeps 16-byte accesses by
 // consecutive lanes on distinct banks.
 constexpr int kSlotWordsF32 = 36;
+constexpr uint32_t kTicketRun = 4;   // pairs of a run where there are many (64 scenes: 1 5.30, 2 5.06, 4 5.00, 8 5.07, 16 5.28 ms)
 
 // Staging of term records for the assembly kernels.  A batch holds kTPL records per lane:
 // record r = 32 t + l is lane l's t-th term, at stage + r * kRec (kRec words: a record plus
@@ -465,6 +466,43 @@ __device__ __forceinline__ void accumulate_row(DAcc *D, DAcc *B, const float *ro
         B[a] += dv * u[a];
     }
 }
+
+// The warps of the pair kernel draw their work, runs of `run` consecutive pairs, by tickets: the first by the
+// warp's number, the later ones from a counter.  Lists differ a lot in length, so with fixed shares many warps
+// end early (a quarter of the SMs' time); and neighbouring pairs are worked on at the same time over the whole
+// launch, so more of their records come from L2 (64 scenes, 5 launches: 5.77 -> 5.00 ms; the same for the node
+// kernel gained nothing).  The last warp to end puts the counters back to zero for the next launch.  Without
+// kDraw, for few pairs with long lists, the blocks' scheduling does as much: a fixed stride.
+template <bool kDraw>
+struct Tickets {
+    uint32_t *counter;   // [0] runs drawn beyond the first of every warp, [1] warps that have ended
+    uint32_t warps, n, run;
+    uint32_t at, stop;   // the current run
+    uint32_t next;       // lane 0: the next run, on its way
+
+    __device__ __forceinline__ Tickets(uint32_t *counter, uint32_t n, int lane) : counter(counter), n(n) {
+        warps = (gridDim.x * blockDim.x) >> 5;
+        run = kDraw && n > 16u * warps ? kTicketRun : 1u;
+        take((blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane);
+    }
+    __device__ __forceinline__ void take(uint32_t t, int lane) {
+        at = min(t, n) * run;   // t counts runs, so t * run may be past 32 bits only past n
+        stop = min(at + run, n);
+        if (kDraw && at < n && lane == 0) next = warps + atomicAdd(&counter[0], 1u);
+    }
+    __device__ __forceinline__ bool more() const { return at < n; }
+    __device__ __forceinline__ void advance(int lane) {
+        if constexpr (!kDraw) {
+            at += warps;
+            return;
+        }
+        if (++at < stop) return;
+        take(__shfl_sync(0xffffffffu, next, 0), lane);
+    }
+    __device__ __forceinline__ void finish(int lane) {
+        if (kDraw && lane == 0 && atomicAdd(&counter[1], 1u) == warps - 1) counter[0] = counter[1] = 0;
+    }
+};
 
 // NT (threads per block) is chosen by the autotuner among 64, 128 and 256; the work of a
 // warp, and so every sum, is the same for all three.
@@ -741,7 +779,7 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     const Scene *scenes, const Plan *plan, const uint32_t *counts,
     const uint32_t *half_row, const uint32_t *half_col, const uint32_t *half_begin, const uint32_t *half_end,
     const uint32_t *half_scene, const uint32_t *pair_val, uint32_t cap_kv, const uint32_t *slot_up, const float *drec, const float *rrec,
-    const float4 *centers, int centred, float *sym_blocks, int *err) {
+    const float4 *centers, int centred, float *sym_blocks, uint32_t *ticket, int *err) {
     constexpr int kSlot = kSlotWordsF32;   // per-lane partial sums at the end
     static_assert(kSlot >= 36, "a slot holds one lane's 36 partial sums");
     constexpr int kRec = record_stride<C>();
@@ -753,7 +791,6 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     float *slots = stage[threadIdx.x >> 5];
     float *stash = slots + kStageWords;   // the pair's smoothness records, in list order
     float *mine = slots + lane * kSlot;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nhalf = counts[kCntHalf];
     // the lane's place in M (lane < 21) and the words of its block entries lane, 32 + lane (the latter in row 5,
     // where only (5, 5) has a product)
@@ -761,20 +798,14 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     tri_decode(lane, ea, ec);
     const uint32_t m_at = (uint32_t)((6 * ea + ec) | (6 * ec + ea) << 8);
     const uint32_t reg0 = reg_words(lane / 6, lane % 6);
-    // grid-stride: at any time the warps work on neighbouring pairs, whose term records overlap,
+    // at any time the warps work on neighbouring pairs, whose term records overlap,
     // so the records are read from DRAM about once and then from L2
-    for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; h < nhalf; h += warps) {
+    Tickets<kBufs == 1> tickets(ticket, nhalf, lane);
+    for (; tickets.more(); tickets.advance(lane)) {
+        const uint32_t h = tickets.at;
         // the pair's words in one round of loads (its scene among them), then its slot check
         const uint32_t slot = slot_up[h], row = half_row[h], col = half_col[h], beg = half_begin[h],
                        end = half_end[h], s = half_scene[h];
-        // the term list of this warp's next pair, into L2 a pair ahead (its bounds come with this
-        // pair's words)
-        uint32_t next_beg = 0, next_end = 0;
-        if (lane == 0 && h + warps < nhalf) {
-            next_beg = half_begin[h + warps];
-            next_end = half_end[h + warps];
-        }
-        if (lane == 0 && next_end > next_beg) l2_prefetch_list(pair_val, next_beg, next_end, cap_kv);
         if (slot == kInvalidIndex) continue;   // capacity overflow, already flagged
         const Scene &sc = scenes[s];
         const Plan &p = plan[s];
@@ -981,6 +1012,7 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
         blk[lane] = acc0;
         if (lane < 4) blk[32 + lane] = acc1;
     }
+    tickets.finish(lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -2273,7 +2305,7 @@ void gn_eval(Workspace &w, cudaStream_t st) {
 
 template <class DAcc, int NT, int C, int kTPL, int kBufs>
 static void launch_assemble_node_v(Workspace &w, cudaStream_t st) {
-    k_assemble_node<DAcc, NT, C, kTPL, kBufs><<<grid_for(w.total_nodes * 32u, NT, w.num_sms, 32 * 128 / NT), NT, 0, st>>>(
+    k_assemble_node<DAcc, NT, C, kTPL, kBufs><<<grid_for(w.total_nodes * 32u, NT, w.num_sms, 64 * 128 / NT), NT, 0, st>>>(
         w.scenes, w.plan, w.node_scene, w.total_nodes, w.n2t_offset, w.n2t_sorted_val, w.cap_n2t, w.d_record, w.r_record, w.se3,
         w.centers, w.item_ptr, w.cap_items, w.sym_blocks, w.diag64, w.jtr, w.error_flag);
 }
@@ -2315,11 +2347,11 @@ void gn_assemble_node(Workspace &w, cudaStream_t st) {
 
 template <int NT, int C, int kTPL, int kBufs>
 static void launch_assemble_pair_v(Workspace &w, cudaStream_t st) {
-    k_assemble_pair<NT, C, kTPL, kBufs><<<grid_for(w.cap_half * 32u, NT, w.num_sms, 32 * 128 / NT), NT, 0, st>>>(
+    k_assemble_pair<NT, C, kTPL, kBufs><<<grid_for(w.cap_half * 32u, NT, w.num_sms, (kBufs == 1 ? 1024 : 4096) / NT), NT, 0, st>>>(
         w.scenes, w.plan, w.counts, w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene,
         w.pair_sorted_val, w.cap_pair_kv,
         w.half_slot_up, w.d_record, w.r_record, w.centers, w.precision == WS_PREC_MIXED ? 1 : 0, w.sym_blocks,
-        w.error_flag);
+        w.counts + kCntTicket, w.error_flag);
 }
 template <int NT, int C>
 static void launch_assemble_pair_c(Workspace &w, cudaStream_t st) {

@@ -191,6 +191,6 @@ void scratch_trim(int device);
 inline void count_launch(Workspace &w, int n = 1) { w.launches += n; }
 
 // Counters slot indices.
-enum { kCntDense = 0, kCntN2T = 1, kCntPairKV = 2, kCntHalf = 3, kCntPairValid = 4 };
+enum { kCntDense = 0, kCntN2T = 1, kCntPairKV = 2, kCntHalf = 3, kCntPairValid = 4, kCntTicket = 6 /* 2 */ };
 
 }  // namespace ws

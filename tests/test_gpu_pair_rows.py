@@ -68,3 +68,26 @@ def test_row_of_64_pairs(ws, small_scene_k8, pairs, wide):
     else:
         with pytest.raises(WarpSolveError):
             _solve(items, 1, 1)
+
+
+@pytest.mark.parametrize("precision,lambda_of", [(0, 0.0), (1, 0.1)])
+def test_pairs_drawn_in_runs(ws, small_scene_k8, precision, lambda_of):
+    """Past 16 pairs a warp the pair kernel's warps draw runs of four; launch after launch, and whatever the
+    blocks' size, every copy's result is the scene's own."""
+    import torch
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    a = DeviceScene.from_scene(dataclasses.replace(_cut(small_scene_k8, 1500), lambda_of=lambda_of))
+    copies = 73
+    out = []
+    for n in (1, copies):
+        s = WarpSolver(max_nodes=n * a.num_nodes, max_pixels=n * a.num_pixels, max_edges=n * a.num_edges, max_scenes=n,
+                       precision=precision)
+        for threads in (64, 128, 256, 64):
+            s.set_tuning(threads, threads, 2)
+            s.SetBatchInputs([a] * n)
+            s.SolveStreamed(2, 3, stream=torch.cuda.Stream())
+            s.Sync()
+            out += [s.SolvedNodeSE3(i).cpu().numpy().copy() for i in sorted({0, n // 3, n - 1})]
+    assert copies * len(s.node_pairs(0)["rows"]) > 16 * 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    for x in out[1:]:
+        np.testing.assert_array_equal(out[0], x)
