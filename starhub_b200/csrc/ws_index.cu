@@ -707,10 +707,7 @@ static inline int grid_for(uint32_t n, int threads, int num_sms, uint32_t per_sm
 //   8000, 38 px 334 / 360 / 407; 8000, 115 px 401 / 410 / 449; 8 x 500 nodes 538 / 464 / 470;
 //   20 x 500 nodes 879 / 812 / 867; 8 x 1800 nodes 521 / 540 / 620.
 static int pair_row_warps(const Workspace &w) {
-    uint64_t pixels = 0;
-    for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s)
-        pixels += (uint64_t)w.h_scenes[s].width * w.h_scenes[s].height;
-    const uint64_t n = w.total_nodes;
+    const uint64_t pixels = scene_pixels(w), n = w.total_nodes;
     if (n <= kRowWide8 && pixels >= 250 * n) return 8;
     if ((n <= 6000 && pixels >= 75 * n) || (n <= kRowWide4 && pixels >= 300 * n)) return 4;
     return 1;

@@ -452,18 +452,186 @@ __device__ __forceinline__ DAcc regulariser_entry(int a, int c, float3 cen, bool
     return -eps * v;
 }
 
-// D += u u^T (upper triangle) and b += v u for one scaled row.
-template <class DAcc>
-__device__ __forceinline__ void accumulate_row(DAcc *D, DAcc *B, const float *row, float scale, float v) {
-    DAcc u[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) u[q] = DAcc(scale * row[q]);
-    const DAcc dv = DAcc(v);
+// The part of a node's 27 sums that warp P of W has, as rows of D's upper triangle and entries of b: 7, 7, 7 and 6
+// sums for W = 4, 9 each for W = 3.
+template <int W, int P>
+__host__ __device__ constexpr bool part_row(int a) {
+    return W == 1 || P == (W == 4 ? (a < 2 ? a : a < 4 ? 2 : 3) : (a == 0 ? 0 : a < 3 ? 1 : 2));
+}
+template <int W, int P>
+__host__ __device__ constexpr bool part_rhs(int a) {
+    return W == 1 || P == (W == 4 ? (a == 0 ? 0 : a < 3 ? 1 : 3) : (a < 3 ? 0 : 2));
+}
+
+// D += u u^T (upper triangle) and b += v u for one scaled row, as far as warp P of W has them.
+template <int W, int P>
+__device__ __forceinline__ void accumulate(float *D, float *B, const float *u, float v) {
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
 #pragma unroll
-        for (int c = a; c < 6; ++c) D[tri_index(a, c)] += u[a] * u[c];
-        B[a] += dv * u[a];
+        for (int c = a; c < 6; ++c)
+            if (part_row<W, P>(a)) D[tri_index(a, c)] += u[a] * u[c];
+        if (part_rhs<W, P>(a)) B[a] += v * u[a];
+    }
+}
+
+template <int W, int P>
+__device__ __forceinline__ void accumulate_row(float *D, float *B, const float *row, float scale, float v) {
+    float u[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) u[q] = scale * row[q];
+    accumulate<W, P>(D, B, u, v);
+}
+
+// What the terms of one node's list need.
+template <int C>
+struct NodeTerms {
+    const Scene &sc;
+    const float4 *dbase, *rbase;
+    const float *se3;
+    uint32_t g, nd, ne, nn;
+    float3 cen;
+    float lam_d, lam_of, lam_r, lam_n;
+    bool motion;
+
+    __device__ NodeTerms(const Scene &sc, const Plan &p, uint32_t g, float4 c4, const float *drec, const float *rrec,
+                         const float *se3)
+        : sc(sc), se3(se3), g(g) {
+        nd = p.dense_count;
+        ne = sc.num_edges;
+        nn = sc.num_nodes;
+        cen = f3(c4.x, c4.y, c4.z);
+        lam_d = sc.lam_depth;
+        lam_of = sc.lam_of;
+        lam_r = sc.lam_reg;
+        lam_n = sc.lam_node;
+        motion = lam_n != 0.f && sc.node_motion != nullptr;
+        dbase = reinterpret_cast<const float4 *>(drec + (size_t)DenseLayout<C>::kFloats * p.dense_begin);
+        rbase = reinterpret_cast<const float4 *>(rrec + (size_t)kRegRecord * sc.edge_base);
+    }
+    // 1 dense, 2 regularisation edge, 3 node motion; feature terms have a zero Jacobian
+    // (PreconditionerRhsBuilder.cu:214-219)
+    __device__ __forceinline__ int classify(uint32_t term, const float4 *&src, int &parts) const {
+        src = nullptr;
+        parts = 0;
+        if (term < nd) {
+            src = dbase + (size_t)(DenseLayout<C>::kFloats / 4) * term;
+            parts = DenseLayout<C>::kFloats / 4;
+            return 1;
+        }
+        if (term < nd + ne) {
+            src = rbase + (size_t)(kRegRecord / 4) * (term - nd);
+            parts = kRegRecord / 4;
+            return 2;
+        }
+        return (term < nd + ne + nn && motion) ? 3 : 0;
+    }
+    // a dense term's scaled rows, row(ch, g, scale, v):
+    // point-to-plane + optical-flow rows (libs/star/opt/dense_image_jacobian.cuh:9-20)
+    template <bool kCentred, class F>
+    __device__ __forceinline__ void dense_rows(const float *rec_t, F &&row) const {
+        float wk[4];
+        uint32_t ids[4];
+        read_weights<C>(rec_t, wk, ids);
+        float w = wk[0];   // weight of the last slot whose node is g
+#pragma unroll
+        for (int k = 1; k < 4; ++k) if (ids[k] == g) w = wk[k];
+#pragma unroll
+        for (int ch = 0; ch < C; ++ch) {
+            float gl[6];
+            const float res = read_channel<C>(rec_t, ch, gl);
+            if (kCentred) recentre(gl, cen);
+            const float scale = (ch == 0 ? lam_d : lam_of) * w;
+            row(ch, gl, scale, -(scale * res));
+        }
+    }
+    // the record in place: channel ch's scaled row u and its v at 8 ch, for all warps of a node
+    template <bool kCentred>
+    __device__ __forceinline__ void scale_dense(float *rec_t) const {
+        float4 out[2 * C];
+        dense_rows<kCentred>(rec_t, [&](int ch, const float *gl, float scale, float v) {
+            out[2 * ch] = make_float4(scale * gl[0], scale * gl[1], scale * gl[2], scale * gl[3]);
+            out[2 * ch + 1] = make_float4(scale * gl[4], scale * gl[5], v, 0.f);
+        });
+#pragma unroll
+        for (int q = 0; q < 2 * C; ++q) reinterpret_cast<float4 *>(rec_t)[q] = out[q];
+    }
+    template <int W, int P>
+    static __device__ __forceinline__ void add_scaled(const float *rec_t, float *D, float *B) {
+#pragma unroll
+        for (int ch = 0; ch < C; ++ch) {
+            const float4 a = reinterpret_cast<const float4 *>(rec_t)[2 * ch], b = reinterpret_cast<const float4 *>(rec_t)[2 * ch + 1];
+            const float u[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+            accumulate<W, P>(D, B, u, b.z);
+        }
+    }
+    // one term's products; kScaled: dense records are scaled already
+    template <int W, int P, bool kCentred, bool kScaled>
+    __device__ __forceinline__ void add(uint32_t term, const float *rec_t, float *D, float *B) const {
+        const float4 *src_unused;
+        int parts_unused;
+        const int kind = classify(term, src_unused, parts_unused);
+        if (kind == 1) {
+            if constexpr (kScaled)
+                add_scaled<W, P>(rec_t, D, B);
+            else
+                dense_rows<kCentred>(rec_t, [&](int, const float *gl, float scale, float v) {
+                    accumulate_row<W, P>(D, B, gl, scale, v);
+                });
+        } else if (kind == 2) {
+            // regularisation rows (node_graph_reg_jacobian.cuh:85-106, 193-233)
+            float rec[kRegRecord];
+            read_slot<kRegRecord / 4>(rec_t, rec);
+            if (rec[7] != 0.f) {
+                const float3 a3 = f3(rec[0], rec[1], rec[2]), b3 = f3(rec[3], rec[4], rec[5]);
+                float J[3][6];
+                reg_unit_jacobian(a3, b3, __float_as_uint(rec[8]) == g, J);
+                const float scale = lam_r * rec[6];
+#pragma unroll
+                for (int ch = 0; ch < 3; ++ch) {
+                    if (kCentred) recentre(J[ch], cen);
+                    accumulate_row<W, P>(D, B, J[ch], scale, -(scale * rec[10 + ch]));
+                }
+            }
+        } else if (kind == 3) {
+            // node-motion rows (node_motion_jacobian.cuh:7-36), lambda_node = 0 by default
+            const uint32_t nl = term - nd - ne;
+            const float4 pred = sc.node_motion[nl];
+            const SE3f T = dq_se3(load_dq(se3 + 8ull * (sc.node_base + nl)));
+            const float res3[3] = {T.t.x - pred.x, T.t.y - pred.y, T.t.z - pred.z};
+            const float scale = lam_n * pred.w;
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) {
+                float J[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                J[3 + ch] = 1.f;
+                if (kCentred) recentre(J, cen);
+                accumulate_row<W, P>(D, B, J, scale, -(scale * res3[ch]));
+            }
+        }
+    }
+};
+
+// The end of a node's list: lane e < 27 of a warp sums entry e of the lanes' partial sums in lane order and stores
+// it, lanes 0 to 20 D(ea, ec), lanes 21 to 26 b.
+template <class DAcc>
+__device__ __forceinline__ void finish_node(const float *slots, int lane, int ea, int ec, uint32_t g, float3 cen, const uint32_t *item_ptr,
+                                            uint32_t cap_items, float *sym_blocks, double *diag64, float *jtr, int *err) {
+    constexpr bool kCentred = sizeof(DAcc) == 8;
+    DAcc acc = DAcc(0);
+    if (lane < 27) {
+#pragma unroll 8
+        for (int l = 0; l < 32; ++l) acc += DAcc(slots[l * kSlotWordsF32 + lane]);
+    }
+    if (lane < 21) {
+        acc += regulariser_entry<DAcc>(ea, ec, cen, kCentred);
+        float *blk = sym_blocks + 36ull * min(item_ptr[g], cap_items - 1);   // the row's first item
+        blk[6 * ea + ec] = (float)acc;
+        blk[6 * ec + ea] = (float)acc;
+        if (kCentred) diag64[21ull * g + lane] = (double)acc;
+    } else if (lane < 29) {
+        const float bq = lane < 27 ? (float)acc : 0.f;
+        jtr[8ull * g + (lane - 21)] = bq;
+        if (isnan(bq)) set_err(err, WS_ERR_NAN);
     }
 }
 
@@ -527,7 +695,7 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     const int lane = threadIdx.x & 31;
     float *slots = stage[threadIdx.x >> 5];
     float *mine = slots + lane * kSlot;
-    int ea = 0, ec = 0;   // lanes 0..20 finish D(ea, ec), lanes 21..26 finish b
+    int ea = 0, ec = 0;
     tri_decode(lane, ea, ec);
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < total_nodes; g += warps) {
@@ -536,36 +704,12 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
         const float4 c4 = centers[g];
         // the list past the first batches, into L2 ahead of the later batches' reads
         if (lane == 0 && end > beg + 32u * kTPL * kBufs) l2_prefetch_list(n2t_val, beg + 32u * kTPL * kBufs, end, cap_n2t);
-        const Scene &sc = scenes[s];
-        const Plan &p = plan[s];
-        const uint32_t nd = p.dense_count, ne = sc.num_edges, nn = sc.num_nodes;
-        const float lam_d = sc.lam_depth, lam_of = sc.lam_of, lam_r = sc.lam_reg, lam_n = sc.lam_node;
-        const bool motion = lam_n != 0.f && sc.node_motion != nullptr;
-        const float4 *dbase = reinterpret_cast<const float4 *>(drec + (size_t)DenseLayout<C>::kFloats * p.dense_begin);
-        const float4 *rbase = reinterpret_cast<const float4 *>(rrec + (size_t)kRegRecord * sc.edge_base);
-        const float3 cen = f3(c4.x, c4.y, c4.z);
+        const NodeTerms<C> terms(scenes[s], plan[s], g, c4, drec, rrec, se3);
         float D[21], B[6];
 #pragma unroll
         for (int i = 0; i < 21; ++i) D[i] = 0.f;
 #pragma unroll
         for (int i = 0; i < 6; ++i) B[i] = 0.f;
-        // 1 dense, 2 regularisation edge, 3 node motion; feature terms have a zero Jacobian
-        // (PreconditionerRhsBuilder.cu:214-219)
-        auto classify = [&](uint32_t term, const float4 *&src, int &parts) -> int {
-            src = nullptr;
-            parts = 0;
-            if (term < nd) {
-                src = dbase + (size_t)(DenseLayout<C>::kFloats / 4) * term;
-                parts = DenseLayout<C>::kFloats / 4;
-                return 1;
-            }
-            if (term < nd + ne) {
-                src = rbase + (size_t)(kRegRecord / 4) * (term - nd);
-                parts = kRegRecord / 4;
-                return 2;
-            }
-            return (term < nd + ne + nn && motion) ? 3 : 0;
-        };
         auto read_words = [&](uint32_t base, uint32_t (&w)[kTPL]) {
 #pragma unroll
             for (int t = 0; t < kTPL; ++t) {
@@ -576,7 +720,7 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
         auto fetch = [&](uint32_t base, const uint32_t (&w)[kTPL], float *buf) {   // an empty group past the list
             const int groups = base < end ? (int)min((uint32_t)kTPL, (end - base + 31) / 32) : 0;
             fetch_records<kRec, C == 3 ? 8 : 4, kTPL>(buf, lane, groups, [&](int t, const float4 *&src, int &parts) {
-                classify(w[t], src, parts);
+                terms.classify(w[t], src, parts);
             });
         };
         // kBufs = 2: a batch's records are copied while the batch before is summed, and the words of the
@@ -607,56 +751,7 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
                 uint32_t term = words[0];
 #pragma unroll
                 for (int k = 1; k < kTPL; ++k) term = t == k ? words[k] : term;
-                const float4 *src_unused;
-                int parts_unused;
-                const int kind = classify(term, src_unused, parts_unused);
-                const float *rec_t = records + (32 * t + lane) * kRec;
-                if (kind == 1) {
-                    // point-to-plane + optical-flow rows (libs/star/opt/dense_image_jacobian.cuh:9-20)
-                    float wk[4];
-                    uint32_t ids[4];
-                    read_weights<C>(rec_t, wk, ids);
-                    float w = wk[0];   // weight of the last slot whose node is g
-#pragma unroll
-                    for (int k = 1; k < 4; ++k) if (ids[k] == g) w = wk[k];
-#pragma unroll
-                    for (int ch = 0; ch < C; ++ch) {
-                        float gl[6];
-                        const float res = read_channel<C>(rec_t, ch, gl);
-                        if (kCentred) recentre(gl, cen);
-                        const float scale = (ch == 0 ? lam_d : lam_of) * w;
-                        accumulate_row(D, B, gl, scale, -(scale * res));
-                    }
-                } else if (kind == 2) {
-                    // regularisation rows (node_graph_reg_jacobian.cuh:85-106, 193-233)
-                    float rec[kRegRecord];
-                    read_slot<kRegRecord / 4>(rec_t, rec);
-                    if (rec[7] != 0.f) {
-                        const float3 a3 = f3(rec[0], rec[1], rec[2]), b3 = f3(rec[3], rec[4], rec[5]);
-                        float J[3][6];
-                        reg_unit_jacobian(a3, b3, __float_as_uint(rec[8]) == g, J);
-                        const float scale = lam_r * rec[6];
-#pragma unroll
-                        for (int ch = 0; ch < 3; ++ch) {
-                            if (kCentred) recentre(J[ch], cen);
-                            accumulate_row(D, B, J[ch], scale, -(scale * rec[10 + ch]));
-                        }
-                    }
-                } else if (kind == 3) {
-                    // node-motion rows (node_motion_jacobian.cuh:7-36), lambda_node = 0 by default
-                    const uint32_t nl = term - nd - ne;
-                    const float4 pred = sc.node_motion[nl];
-                    const SE3f T = dq_se3(load_dq(se3 + 8ull * (sc.node_base + nl)));
-                    const float res3[3] = {T.t.x - pred.x, T.t.y - pred.y, T.t.z - pred.z};
-                    const float scale = lam_n * pred.w;
-#pragma unroll
-                    for (int ch = 0; ch < 3; ++ch) {
-                        float J[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                        J[3 + ch] = 1.f;
-                        if (kCentred) recentre(J, cen);
-                        accumulate_row(D, B, J, scale, -(scale * res3[ch]));
-                    }
-                }
+                terms.template add<1, 0, kCentred, false>(term, records + (32 * t + lane) * kRec, D, B);
             }
             __syncwarp();
             if constexpr (kBufs == 2) {
@@ -679,23 +774,120 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
 #pragma unroll
         for (int i = 0; i < 6; ++i) mine[21 + i] = B[i];
         __syncwarp();
-        DAcc acc = DAcc(0);
-        if (lane < 27) {
-#pragma unroll 8
-            for (int l = 0; l < 32; ++l) acc += DAcc(slots[l * kSlot + lane]);
-        }
+        finish_node<DAcc>(slots, lane, ea, ec, g, terms.cen, item_ptr, cap_items, sym_blocks, diag64, jtr, err);
         __syncwarp();
-        if (lane < 21) {
-            acc += regulariser_entry<DAcc>(ea, ec, cen, kCentred);
-            float *blk = sym_blocks + 36ull * min(item_ptr[g], cap_items - 1);   // the row's first item
-            blk[6 * ea + ec] = (float)acc;
-            blk[6 * ec + ea] = (float)acc;
-            if (kCentred) diag64[21ull * g + lane] = (double)acc;
-        } else if (lane < 29) {
-            const float bq = lane < 27 ? (float)acc : 0.f;
-            jtr[8ull * g + (lane - 21)] = bq;
-            if (isnan(bq)) set_err(err, WS_ERR_NAN);
+    }
+}
+
+// Few nodes with long lists: a block of W warps has a node.  A lone warp is bound by its own chain of instructions
+// (some 1000 cycles for 64 terms, one or two warps to a scheduler), so the work of a batch of 32 W terms is shared:
+// every warp copies 32 records and turns them into scaled rows in place, once for all, and every warp adds its part
+// of the 27 sums over all of the rows, so lane l of each meets the terms l, 32 + l, ... in the order that one warp
+// would, and the results are the same bits.  Scaling the next batch runs beside summing this one, and kBufs - 1
+// batches are on their way.  Per launch, one warp / a block to a node: 500 nodes, 614 px a node 34 -> 18 us; 3000
+// nodes with flow, 307 px a node 75 -> 64 us.  Three warps with flow: three buffers then fit in 48 KB.
+// The warps run different instances of wide_list, so they meet at a named barrier.
+template <int W>
+__device__ __forceinline__ void warps_meet() { asm volatile("bar.sync 1, %0;\n" ::"n"(32 * W) : "memory"); }
+
+template <class DAcc, int C, int W, int kBufs, int P>
+__device__ __forceinline__ void wide_list(const NodeTerms<C> &terms, uint32_t beg, uint32_t end, const uint32_t *n2t_val,
+                                          float *stage, uint32_t (*s_word)[32 * W], int lane) {
+    constexpr bool kCentred = sizeof(DAcc) == 8;
+    constexpr int kRec = record_stride<C>(), kTerms = 32 * W, kBatch = kTerms * kRec;
+    float D[21], B[6];
+#pragma unroll
+    for (int i = 0; i < 21; ++i) D[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) B[i] = 0.f;
+    auto read_word = [&](uint32_t base) {
+        const uint32_t it = base + 32 * P + lane;
+        return it < end ? n2t_val[it] : kInvalidIndex;
+    };
+    auto fetch = [&](uint32_t base, uint32_t word, int buf) {
+        s_word[buf][32 * P + lane] = word;
+        fetch_records<kRec, C == 3 ? 8 : 4, 1>(stage + buf * kBatch + 32 * P * kRec, lane, base + 32 * P < end ? 1 : 0,
+                                               [&](int, const float4 *&src, int &parts) {
+                                                   terms.classify(word, src, parts);
+                                               });
+    };
+    auto scale = [&](int buf) {   // the warp's own part of a batch, once it is there
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kBufs - 2) : "memory");
+        __syncwarp();
+        return s_word[buf][32 * P + lane] < terms.nd;
+    };
+    uint32_t ahead = read_word(beg);
+#pragma unroll
+    for (int b = 0; b < kBufs - 1; ++b) {
+        const uint32_t word = ahead;
+        ahead = read_word(beg + kTerms * (b + 1));
+        fetch(beg + kTerms * b, word, b);
+    }
+    if (scale(0)) terms.template scale_dense<kCentred>(stage + (32 * P + lane) * kRec);
+    int buf = 0;
+    for (uint32_t base = beg; base < end; base += kTerms) {
+        const int following = buf == kBufs - 1 ? 0 : buf + 1;
+        warps_meet<W>();   // the batch is there, scaled, and all warps are done with the one before it
+        const uint32_t word = ahead;
+        ahead = read_word(base + kTerms * kBufs);
+        fetch(base + kTerms * (kBufs - 1), word, buf == 0 ? kBufs - 1 : buf - 1);
+        const bool dense = scale(following);
+        const int groups = (int)min((uint32_t)W, (end - base + 31) / 32);
+        const float *records = stage + buf * kBatch + lane * kRec;
+        // a list is in term order, the dense terms first: a batch whose last word is one has no others
+        if (s_word[buf][kTerms - 1] < terms.nd) {
+#pragma unroll
+            for (int t = 0; t < W; ++t) terms.template add_scaled<W, P>(records + 32 * t * kRec, D, B);
+        } else {
+#pragma unroll 1
+            for (int t = 0; t < groups; ++t)
+                terms.template add<W, P, kCentred, true>(s_word[buf][32 * t + lane], records + 32 * t * kRec, D, B);
         }
+        if (dense) terms.template scale_dense<kCentred>(stage + following * kBatch + (32 * P + lane) * kRec);
+        buf = following;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    warps_meet<W>();
+    float *mine = stage + lane * kSlotWordsF32;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+#pragma unroll
+        for (int c = a; c < 6; ++c)
+            if (part_row<W, P>(a)) mine[tri_index(a, c)] = D[tri_index(a, c)];
+        if (part_rhs<W, P>(a)) mine[21 + a] = B[a];
+    }
+    warps_meet<W>();
+}
+
+template <class DAcc, int C, int W, int kBufs>
+__global__ void __launch_bounds__(32 * W, 5) k_assemble_node_wide(const Scene *scenes, const Plan *plan,
+                                                                  const uint32_t *node_scene, uint32_t total_nodes,
+                                                                  const uint32_t *n2t_offset, const uint32_t *n2t_val,
+                                                                  uint32_t cap_n2t, const float *drec, const float *rrec,
+                                                                  const float *se3, const float4 *centers,
+                                                                  const uint32_t *item_ptr, uint32_t cap_items,
+                                                                  float *sym_blocks, double *diag64, float *jtr, int *err) {
+    static_assert(W == 3 || W == 4, "parts for three or four warps");
+    __shared__ __align__(16) float stage[kBufs * 32 * W * record_stride<C>()];
+    __shared__ uint32_t s_word[kBufs][32 * W];
+    const int lane = threadIdx.x & 31;
+    int ea = 0, ec = 0;
+    tri_decode(lane, ea, ec);
+    for (uint32_t g = blockIdx.x; g < total_nodes; g += gridDim.x) {
+        const uint32_t s = node_scene[g];
+        const uint32_t beg = n2t_offset[g], end = n2t_offset[g + 1];
+        if (threadIdx.x == 0 && end > beg + 32u * W * kBufs)
+            l2_prefetch_list(n2t_val, beg + 32u * W * kBufs, end, cap_n2t);
+        const NodeTerms<C> terms(scenes[s], plan[s], g, centers[g], drec, rrec, se3);
+        switch (threadIdx.x >> 5) {
+            case 0: wide_list<DAcc, C, W, kBufs, 0>(terms, beg, end, n2t_val, stage, s_word, lane); break;
+            case 1: wide_list<DAcc, C, W, kBufs, 1>(terms, beg, end, n2t_val, stage, s_word, lane); break;
+            case 2: wide_list<DAcc, C, W, kBufs, 2>(terms, beg, end, n2t_val, stage, s_word, lane); break;
+            default: wide_list<DAcc, C, W, kBufs, W - 1>(terms, beg, end, n2t_val, stage, s_word, lane);
+        }
+        if (threadIdx.x < 32)
+            finish_node<DAcc>(stage, lane, ea, ec, g, terms.cen, item_ptr, cap_items, sym_blocks, diag64, jtr, err);
+        __syncthreads();
     }
 }
 
@@ -2318,6 +2510,13 @@ static void launch_assemble_node_c(Workspace &w, cudaStream_t st) {
     else launch_assemble_node_v<DAcc, NT, C, 1, 1>(w, st);
 }
 
+template <class DAcc, int C, int W, int kBufs>
+static void launch_assemble_node_wide(Workspace &w, cudaStream_t st) {
+    k_assemble_node_wide<DAcc, C, W, kBufs><<<w.total_nodes, 32 * W, 0, st>>>(
+        w.scenes, w.plan, w.node_scene, w.total_nodes, w.n2t_offset, w.n2t_sorted_val, w.cap_n2t, w.d_record, w.r_record, w.se3,
+        w.centers, w.item_ptr, w.cap_items, w.sym_blocks, w.diag64, w.jtr, w.error_flag);
+}
+
 template <class DAcc, int NT>
 static void launch_assemble_node(Workspace &w, cudaStream_t st) {
     if (w.dense_channels == 3) launch_assemble_node_c<DAcc, NT, 3>(w, st);
@@ -2336,7 +2535,20 @@ static void launch_assemble_node_nt(Workspace &w, int nt, cudaStream_t st) {
 }
 
 void gn_assemble_node(Workspace &w, cudaStream_t st) {
-    if (w.precision == WS_PREC_FP32) launch_assemble_node_nt<float>(w, w.tune.node_threads, st);
+    // A block to a node pays while the nodes fit the chip at once and their lists are long.  Node kernel and
+    // inverse, a warp / a block to a node, us: 500 nodes with 614 px a node 48 / 34, 1400 with 219 40 / 32, 1800
+    // with 171 34 / 34, 3000 with 307 59 / 55, 3 x 500 with 614 58 / 48, 8 x 500 78 / 87, 20 x 500 135 / 177; with
+    // flow 1500 with 205 56 / 43, 1500 with 614 150 / 94, 3000 with 102 39 / 45, 3000 with 307 89 / 82, 5000 with
+    // 184 71 / 87.
+    if (w.total_nodes <= 3200 && scene_pixels(w) >= 200ull * w.total_nodes) {
+        if (w.precision == WS_PREC_FP32) {
+            if (w.dense_channels == 3) launch_assemble_node_wide<float, 3, 3, 3>(w, st);
+            else launch_assemble_node_wide<float, 1, 4, 4>(w, st);
+        } else {
+            if (w.dense_channels == 3) launch_assemble_node_wide<double, 3, 3, 3>(w, st);
+            else launch_assemble_node_wide<double, 1, 4, 4>(w, st);
+        }
+    } else if (w.precision == WS_PREC_FP32) launch_assemble_node_nt<float>(w, w.tune.node_threads, st);
     else launch_assemble_node_nt<double>(w, w.tune.node_threads, st);
     count_launch(w);
     k_block_inverse<<<grid_for(w.total_nodes, 64, w.num_sms, 32), 64, 0, st>>>(
@@ -2359,12 +2571,9 @@ static void launch_assemble_pair_c(Workspace &w, cudaStream_t st) {
     // from the pipeline (5 or 6 GN iterations, one buffer / two: 614 px a node 257 / 174 us, 307 with flow
     // 502 / 442, 170 145 / 143); short ones of a batch from the warps that fit without it (120 px a node, 64
     // scenes: 5.98 / 7.19 ms).
-    uint64_t pixels = 0;
-    for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s)
-        pixels += (uint64_t)w.h_scenes[s].width * w.h_scenes[s].height;
     constexpr int kTPL = terms_per_lane(NT, record_stride<C>()) < 2 ? terms_per_lane(NT, record_stride<C>()) : 2;
     constexpr int fit = C == 3 && NT > 128 ? 128 : NT;   // threads whose two buffers fit in 48 KB
-    if (pixels >= 150ull * w.total_nodes) launch_assemble_pair_v<fit, C, 1, 2>(w, st);
+    if (scene_pixels(w) >= 150ull * w.total_nodes) launch_assemble_pair_v<fit, C, 1, 2>(w, st);
     else launch_assemble_pair_v<NT, C, kTPL, 1>(w, st);
 }
 

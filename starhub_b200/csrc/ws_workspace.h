@@ -190,6 +190,14 @@ void scratch_trim(int device);
 // Launch accounting for the measurement hooks.
 inline void count_launch(Workspace &w, int n = 1) { w.launches += n; }
 
+// Pixels of all scenes' images: with the nodes, how long the term lists are.
+inline uint64_t scene_pixels(const Workspace &w) {
+    uint64_t pixels = 0;
+    for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s)
+        pixels += (uint64_t)w.h_scenes[s].width * w.h_scenes[s].height;
+    return pixels;
+}
+
 // Counters slot indices.
 enum { kCntDense = 0, kCntN2T = 1, kCntPairKV = 2, kCntHalf = 3, kCntPairValid = 4, kCntTicket = 6 /* 2 */ };
 
