@@ -145,7 +145,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     w.cap_half = std::min<uint32_t>(w.cap_half, (0xFFFFFFF0u - w.cap_nodes) / 2u);
     w.cap_blocks = w.cap_nodes + 2u * w.cap_half;
     w.cap_items = w.cap_nodes + w.cap_half;
-    const uint32_t sort_cap = std::max(w.cap_n2t, w.cap_half);
+    const int sort_tiles = std::max(ws::sort_max_tiles(w.cap_n2t), ws::sort_max_tiles(w.cap_half));
     const uint32_t scan_cap = std::max(w.cap_nodes, w.cap_tiles) + 1;
     cudaError_t e = cudaSuccess;
     auto A = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
@@ -159,7 +159,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     A(dalloc(&w.chunk_scene, w.cap_chunks));
     A(dalloc(&w.chunk_row, w.cap_chunks));
     A(dalloc(&w.scan_tmp, scan_cap / ws::kScanTile + 4));
-    A(dalloc(&w.sort_hist, (size_t)ws::kSortMaxDigits * ws::sort_max_tiles(sort_cap)));
+    A(dalloc(&w.sort_hist, (size_t)ws::kSortMaxDigits * sort_tiles));
     A(dalloc(&w.sort_digit, ws::kSortMaxDigits));
     A(dalloc(&w.d_pixels, w.cap_pixels));
     A(dalloc(&w.d_knn, w.cap_pixels));

@@ -14,8 +14,11 @@
 namespace ws {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortRounds = 16;
-constexpr int kSortTile = kSortThreads * kSortRounds;   // 4096 keys per tile
+// Keys per thread of a tile: 8, or 16 from a capacity of 4 M keys.  A frame's keys fill few tiles (500 k in all; two
+// passes' scatter of 500 nodes 12.9 / 15.4 us, 8000 nodes 25.5 / 31.5), a batch's tables of tiles are read and
+// written for all digits (64 scenes, all three kernels 859 / 627 us).
+constexpr int kSortRoundsSmall = 8, kSortRoundsLarge = 16;
+inline int sort_rounds(uint32_t cap) { return cap <= (4u << 20) ? kSortRoundsSmall : kSortRoundsLarge; }
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;    // 2048 elements per tile
@@ -128,23 +131,32 @@ inline void exclusive_scan(const uint32_t *in, uint32_t *out, const uint32_t *n_
 
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort of (key, u32 value), D = 8 or 9 bits per pass (256 or 512 digits; each
-// thread of a 256-thread block looks after one or two of them).
+// thread of a 256-thread block looks after one or two of them).  A tile has R keys per thread.
 // hist layout: hist[digit * max_tiles + tile].
 // ---------------------------------------------------------------------------
-template <class K, int D>
-__global__ void k_radix_upsweep(const K *keys, const uint32_t *n_dev, uint32_t n_static, int shift,
-                                uint32_t *hist, int max_tiles) {
+// Counts a tile's digits: all keys of a thread are read before the first is counted (64 scenes, all passes 258 -> 182
+// us).  Shared atomics merge equal digits of a warp well enough: merging them by matching takes 226 us.
+// A warp has R * 32 consecutive keys of the tile, lane l the keys 32 r + l.
+template <class K, int D, int R>
+__global__ void __launch_bounds__(kSortThreads) k_radix_upsweep(const K *keys, const uint32_t *n_dev, uint32_t n_static,
+                                                                int shift, uint32_t *hist, int max_tiles) {
     constexpr uint32_t kDigits = 1u << D;
     __shared__ uint32_t h[kDigits];
     const uint32_t n = n_dev ? *n_dev : n_static;
+    const uint32_t base = blockIdx.x * (uint32_t)(kSortThreads * R);
     for (uint32_t d = threadIdx.x; d < kDigits; d += kSortThreads) h[d] = 0;
+    const int lane = threadIdx.x & 31;
+    const uint32_t first = base + (threadIdx.x >> 5) * (32u * R) + (uint32_t)lane;
+    K key[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) key[r] = first + 32u * r < n ? keys[first + 32u * r] : K(0);
     __syncthreads();
-    const uint32_t base = blockIdx.x * (uint32_t)kSortTile;
     if (base < n) {
-#pragma unroll 4
-        for (int r = 0; r < kSortRounds; ++r) {
-            const uint32_t idx = base + r * kSortThreads + threadIdx.x;
-            if (idx < n) atomicAdd(&h[(uint32_t)(keys[idx] >> shift) & (kDigits - 1u)], 1u);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool valid = first + 32u * r < n;
+            const uint32_t d = (uint32_t)(key[r] >> shift) & (kDigits - 1u);
+            if (valid) atomicAdd(&h[d], 1u);
         }
     }
     __syncthreads();
@@ -153,11 +165,11 @@ __global__ void k_radix_upsweep(const K *keys, const uint32_t *n_dev, uint32_t n
 
 // Exclusive scan of one digit's tile counts (one block per digit) over the tiles in use,
 // 1024 consecutive counts per pass (4 per thread), with the running total carried along.
-static __global__ void k_radix_scan(uint32_t *hist, int max_tiles, const uint32_t *n_dev, uint32_t n_static,
+static __global__ void k_radix_scan(uint32_t *hist, int max_tiles, uint32_t tile, const uint32_t *n_dev, uint32_t n_static,
                                     uint32_t *digit_total) {
     __shared__ uint32_t sm[32];
     const uint32_t n = n_dev ? *n_dev : n_static;
-    const int used = min(max_tiles, (int)((n + kSortTile - 1) / kSortTile));
+    const int used = min(max_tiles, (int)((n + tile - 1) / tile));
     uint32_t *row = hist + (size_t)blockIdx.x * max_tiles;
     uint32_t carry = 0;
     for (int base = 0; base < used; base += 4 * (int)blockDim.x) {
@@ -179,24 +191,41 @@ static __global__ void k_radix_scan(uint32_t *hist, int max_tiles, const uint32_
     if (threadIdx.x == 0) digit_total[blockIdx.x] = carry;
 }
 
-template <class K, int D>
+// Places a tile's keys and values, all of them read at once.  What bounds it is the ranking (every key's place among its digit's) and the
+// writes: a warp ranks its own run of keys against counters of its own, with nothing shared until all are ranked,
+// and the tile goes through shared memory in digit order, so that a digit's keys are written side by side.  Ranking by rounds of the whole block, four barriers a round, and
+// writing each key where it belongs took, for all passes of 64 scenes' lists 613 us, now 412; 8000 nodes' 58, now
+// 26; 200 k voxels 52, now 18.  Ranking by ballots of the digit's bits instead of matching: 585 us for 64 scenes.
+template <class K, int D, int R>
 __global__ void __launch_bounds__(kSortThreads)
 k_radix_scatter(const K *keys_in, const uint32_t *vals_in, K *keys_out, uint32_t *vals_out,
                 const uint32_t *n_dev, uint32_t n_static, int shift,
                 const uint32_t *hist, int max_tiles, const uint32_t *digit_total) {
     constexpr uint32_t kDigits = 1u << D;
     constexpr int kPer = (int)kDigits / kSortThreads;   // digits per thread
+    constexpr int kWarps = kSortThreads / 32;
     static_assert(kPer == 1 || kPer == 2, "8- or 9-bit digits");
-    __shared__ uint32_t digit_base[kDigits];
-    __shared__ uint32_t run[kDigits];
-    __shared__ uint16_t wcount[kSortThreads / 32][kDigits];
+    __shared__ uint32_t delta[kDigits];                 // digit -> its first place in the output less that in the tile
+    __shared__ uint16_t wcount[kWarps][kDigits];
+    __shared__ K s_key[kSortThreads * R];
+    __shared__ uint32_t s_val[kSortThreads * R];
     __shared__ uint32_t sm[32];
     const uint32_t n = n_dev ? *n_dev : n_static;
-    const uint32_t base = blockIdx.x * (uint32_t)kSortTile;
+    const uint32_t base = blockIdx.x * (uint32_t)(kSortThreads * R);
     if (base >= n) return;                      // uniform for the whole block
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t first = base + (uint32_t)warp * (32u * R) + (uint32_t)lane;
+    K key[R];
+    uint32_t val[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t idx = first + 32u * r;
+        key[r] = idx < n ? keys_in[idx] : K(0);
+        val[r] = idx < n ? vals_in[idx] : 0u;
+    }
+    // thread t owns digits kPer t .. kPer t + kPer - 1
+    uint32_t global[kPer];
     {
-        // thread t owns digits kPer t .. kPer t + kPer - 1
         uint32_t tot[kPer], sum = 0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
@@ -206,54 +235,82 @@ k_radix_scatter(const K *keys_in, const uint32_t *vals_in, K *keys_out, uint32_t
         uint32_t ex = block_excl_scan_u32(sum, nullptr, sm);
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const uint32_t d = (uint32_t)(kPer * t + k);
-            digit_base[d] = ex + hist[(size_t)d * max_tiles + blockIdx.x];
-            run[d] = 0;
+            global[k] = ex + hist[(size_t)(kPer * t + k) * max_tiles + blockIdx.x];
             ex += tot[k];
         }
     }
-    for (int r = 0; r < kSortRounds; ++r) {
-        const uint32_t idx = base + r * kSortThreads + t;
-        const bool valid = idx < n;
-        K key = 0;
-        uint32_t val = 0;
-        uint32_t d = kDigits;
-        if (valid) {
-            key = keys_in[idx];
-            val = vals_in[idx];
-            d = (uint32_t)(key >> shift) & (kDigits - 1u);
-        }
-        __syncthreads();
+    for (uint32_t d = (uint32_t)lane; d < kDigits; d += 32) wcount[warp][d] = 0;
+    __syncwarp();
+    uint16_t rank[R];
 #pragma unroll
-        for (int w = 0; w < kSortThreads / 32; ++w)
-#pragma unroll
-            for (int k = 0; k < kPer; ++k) wcount[w][kPer * t + k] = 0;
-        __syncthreads();
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank_w = __popc(peers & ((1u << lane) - 1u));
-        if (valid && rank_w == 0) wcount[warp][d] = (uint16_t)__popc(peers);
-        __syncthreads();
-        if (valid) {
-            uint32_t pre = 0;
-            for (int w = 0; w < warp; ++w) pre += wcount[w][d];
-            const uint32_t pos = digit_base[d] + run[d] + pre + (uint32_t)rank_w;
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-        }
-        __syncthreads();
+    for (int r = 0; r < R; ++r) {
+        const bool valid = first + 32u * r < n;
+        const uint32_t d = (uint32_t)(key[r] >> shift) & (kDigits - 1u);
+        const unsigned peers = __match_any_sync(0xffffffffu, valid ? d : kDigits);
+        const uint32_t before = wcount[warp][d];
+        const uint32_t lower = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        rank[r] = (uint16_t)(before + lower);
+        __syncwarp();
+        if (valid && lower == 0) wcount[warp][d] = (uint16_t)(before + (uint32_t)__popc(peers));
+        __syncwarp();
+    }
+    __syncthreads();
+    {
+        uint32_t tot[kPer], sum = 0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            uint32_t tot = 0;
+            tot[k] = 0;
 #pragma unroll
-            for (int w = 0; w < kSortThreads / 32; ++w) tot += wcount[w][kPer * t + k];
-            run[kPer * t + k] += tot;
+            for (int w = 0; w < kWarps; ++w) tot[k] += wcount[w][kPer * t + k];
+            sum += tot[k];
         }
-        if (base + (uint32_t)(r + 1) * kSortThreads >= n) break;   // uniform
+        uint32_t at = block_excl_scan_u32(sum, nullptr, sm);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            delta[kPer * t + k] = global[k] - at;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const uint32_t c = wcount[w][kPer * t + k];
+                wcount[w][kPer * t + k] = (uint16_t)at;
+                at += c;
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (first + 32u * r < n) {
+            const uint32_t d = (uint32_t)(key[r] >> shift) & (kDigits - 1u);
+            const uint32_t at = (uint32_t)wcount[warp][d] + rank[r];
+            s_key[at] = key[r];
+            s_val[at] = val[r];
+        }
+    }
+    __syncthreads();
+    const uint32_t count = min((uint32_t)(kSortThreads * R), n - base);
+#pragma unroll 4
+    for (uint32_t i = (uint32_t)t; i < count; i += kSortThreads) {
+        const K k = s_key[i];
+        const uint32_t at = delta[(uint32_t)(k >> shift) & (kDigits - 1u)] + i;
+        keys_out[at] = k;
+        vals_out[at] = s_val[i];
     }
 }
 
-inline int sort_max_tiles(uint32_t cap) { return (int)((cap + kSortTile - 1) / kSortTile) + 1; }
+inline int sort_max_tiles(uint32_t cap) {
+    const uint32_t tile = (uint32_t)(kSortThreads * sort_rounds(cap));
+    return (int)((cap + tile - 1) / tile) + 1;
+}
 constexpr int kSortMaxDigits = 512;
+
+template <class K, int D, int R>
+inline void radix_pass(const K *ki, const uint32_t *vi, K *ko, uint32_t *vo, const uint32_t *n_dev, uint32_t n_static,
+                       int shift, uint32_t *hist, int max_tiles, uint32_t *digit_total, cudaStream_t st) {
+    k_radix_upsweep<K, D, R><<<max_tiles, kSortThreads, 0, st>>>(ki, n_dev, n_static, shift, hist, max_tiles);
+    k_radix_scan<<<1 << D, 256, 0, st>>>(hist, max_tiles, (uint32_t)(kSortThreads * R), n_dev, n_static, digit_total);
+    k_radix_scatter<K, D, R><<<max_tiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n_dev, n_static, shift, hist, max_tiles,
+                                                                  digit_total);
+}
 
 // Sorts `bits` low bits of the keys, 9 bits per pass when that saves a pass over 8 bits.
 // Buffers a/b ping-pong; returns true when the result ended in the `alt` buffers.  hist needs
@@ -264,23 +321,16 @@ inline bool radix_sort(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_alt,
                        uint32_t *hist, uint32_t *digit_total, cudaStream_t st) {
     const int max_tiles = sort_max_tiles(cap);
     const int step = ((bits + 8) / 9 < (bits + 7) / 8) ? 9 : 8;
+    const bool small = sort_rounds(cap) == kSortRoundsSmall;
     bool in_alt = false;
     for (int shift = 0; shift < bits; shift += step) {
         K *ki = in_alt ? keys_alt : keys;
         uint32_t *vi = in_alt ? vals_alt : vals;
         K *ko = in_alt ? keys : keys_alt;
         uint32_t *vo = in_alt ? vals : vals_alt;
-        if (step == 9) {
-            k_radix_upsweep<K, 9><<<max_tiles, kSortThreads, 0, st>>>(ki, n_dev, n_static, shift, hist, max_tiles);
-            k_radix_scan<<<512, 256, 0, st>>>(hist, max_tiles, n_dev, n_static, digit_total);
-            k_radix_scatter<K, 9><<<max_tiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n_dev, n_static, shift, hist,
-                                                                       max_tiles, digit_total);
-        } else {
-            k_radix_upsweep<K, 8><<<max_tiles, kSortThreads, 0, st>>>(ki, n_dev, n_static, shift, hist, max_tiles);
-            k_radix_scan<<<256, 256, 0, st>>>(hist, max_tiles, n_dev, n_static, digit_total);
-            k_radix_scatter<K, 8><<<max_tiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n_dev, n_static, shift, hist,
-                                                                       max_tiles, digit_total);
-        }
+        auto pass = step == 9 ? (small ? radix_pass<K, 9, kSortRoundsSmall> : radix_pass<K, 9, kSortRoundsLarge>)
+                              : (small ? radix_pass<K, 8, kSortRoundsSmall> : radix_pass<K, 8, kSortRoundsLarge>);
+        pass(ki, vi, ko, vo, n_dev, n_static, shift, hist, max_tiles, digit_total, st);
         in_alt = !in_alt;
     }
     return in_alt;
