@@ -1151,7 +1151,7 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
         const bool alt = ws::radix_sort<uint32_t>(keys, vals, keys2, vals2, nullptr, n, n, 30, hist, digit, st);
         const uint32_t *sk = alt ? keys2 : keys, *sv = alt ? vals2 : vals;
         ws::k_voxel_marks<<<ws::grid_of(n, 256), 256, 0, st>>>(sk, n, heads);
-        ws::exclusive_scan(heads, heads, nullptr, n, n, tmp, st);
+        ws::exclusive_scan(heads, heads, n, tmp, st);
         ws::k_voxel_sample<<<ws::grid_of(n, 256), 256, 0, st>>>(sk, sv, heads, n, pts, voxel, cand);
         if (cudaMemcpyAsync(&nv, heads + n, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return WS_ERR_CUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return WS_ERR_CUDA;
@@ -1181,11 +1181,11 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
         cudaMemsetAsync(table, 0, 4ull * ws::kDedupTable, st) != cudaSuccess)
         return WS_ERR_CUDA;
     ws::k_dedup_count<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, table, err);
-    ws::exclusive_scan(table, table, nullptr, ws::kDedupTable, ws::kDedupTable, tmp, st);
+    ws::exclusive_scan(table, table, ws::kDedupTable, tmp, st);
     ws::k_dedup_place<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, table, placed);
     ws::k_dedup_neighbours<false><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, thr, cnt,
                                                                        nullptr, 0, err);
-    ws::exclusive_scan(cnt, cnt, nullptr, nv, nv, tmp, st);
+    ws::exclusive_scan(cnt, cnt, nv, tmp, st);
     uint32_t count = 0;
     for (int attempt = 0;; ++attempt) {
         ws::k_dedup_neighbours<true><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, thr, cnt,
@@ -1201,7 +1201,7 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
             return WS_ERR_CUDA;
         }
         ws::k_dedup_flags<<<ws::grid_of(nv, 256), 256, 0, st>>>(decision, nv, pos);
-        ws::exclusive_scan(pos, pos, nullptr, nv, nv, tmp, st);
+        ws::exclusive_scan(pos, pos, nv, tmp, st);
         ws::k_dedup_emit<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, decision, pos, nv, *nodes);
         if (cudaGetLastError() != cudaSuccess) return WS_ERR_CUDA;
         uint32_t total = 0;

@@ -722,15 +722,14 @@ static void pair_index_rows(Workspace &w, cudaStream_t st) {
     k_pair_rows_count<W><<<grid, threads, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset, w.n2t_sorted_val,
                                                    w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts, w.row_cnt_up,
                                                    w.row_entry_first, w.error_flag);
-    exclusive_scan(w.row_cnt_up, w.row_pair_first, nullptr, N, w.cap_nodes, w.scan_tmp, st);
-    exclusive_scan(w.row_entry_first, w.row_entry_first, nullptr, N, w.cap_nodes, w.scan_tmp, st);
+    count_launch(w, exclusive_scan2(w.row_cnt_up, w.row_pair_first, w.row_entry_first, w.row_entry_first, N, w.scan_tmp, st));
     cudaMemsetAsync(w.row_cnt_lo, 0, sizeof(uint32_t) * w.cap_nodes, st);
     k_pair_rows_fill<W><<<grid, threads, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset, w.n2t_sorted_val,
                                                   w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts,
                                                   w.row_pair_first, w.row_entry_first, w.cap_half, w.cap_pair_kv,
                                                   w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene,
                                                   w.row_cnt_lo, w.pair_val, w.counts, w.error_flag);
-    count_launch(w, 1 + 3 + 3 + 1);
+    count_launch(w, 1 + 1);
 }
 
 static void pair_index(Workspace &w, cudaStream_t st) {
@@ -748,8 +747,7 @@ void index_build(Workspace &w, cudaStream_t st) {
     const uint32_t N = w.total_nodes;
     // 1. compaction of potential pixels
     k_pixel_count<<<T, kPixTileThreads, 0, st>>>(w.scenes, w.tile_scene, T, w.tile_count);
-    exclusive_scan(w.tile_count, w.tile_count, nullptr, (uint32_t)T, w.cap_tiles, w.scan_tmp, st);
-    count_launch(w, 1 + 3);
+    count_launch(w, 1 + exclusive_scan(w.tile_count, w.tile_count, (uint32_t)T, w.scan_tmp, st));
     k_plan<<<1, 32, 0, st>>>(w.scenes, S, w.tile_count, T, w.plan, w.counts, w.cap_n2t, w.cap_pair_kv, w.error_flag);
     k_pixel_compact<<<T, kPixTileThreads, 0, st>>>(w.scenes, w.tile_scene, T, w.tile_count, w.d_pixels, w.d_knn,
                                                    w.d_sw, w.d_cw, w.d_scene, w.cap_pixels, w.error_flag);
@@ -772,12 +770,11 @@ void index_build(Workspace &w, cudaStream_t st) {
     // 4. block CSR
     k_row_first<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(w.half_row, w.counts, w.row_first);
     k_row_len<<<grid_for(N, 256, w.num_sms), 256, 0, st>>>(w.row_cnt_up, w.row_cnt_lo, N, w.rowptr, w.item_ptr);
-    exclusive_scan(w.rowptr, w.rowptr, nullptr, N, w.cap_nodes, w.scan_tmp, st);
-    exclusive_scan(w.item_ptr, w.item_ptr, nullptr, N, w.cap_nodes, w.scan_tmp, st);
+    count_launch(w, exclusive_scan2(w.rowptr, w.rowptr, w.item_ptr, w.item_ptr, N, w.scan_tmp, st));
     k_col_kv<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(w.half_col, w.counts, w.col_key, w.col_val);
     const bool col_alt = radix_sort<uint32_t>(w.col_key, w.col_val, w.col_key_alt, w.col_val_alt, w.counts + kCntHalf,
                                               0, w.cap_half, w.node_bits, w.sort_hist, w.sort_digit, st);
-    count_launch(w, 1 + 1 + 3 + 3 + 1 + 3 * radix_passes(w.node_bits));
+    count_launch(w, 1 + 1 + 1 + 3 * radix_passes(w.node_bits));
     const uint32_t *scol = col_alt ? w.col_key_alt : w.col_key;
     const uint32_t *sh = col_alt ? w.col_val_alt : w.col_val;
     k_slots<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(scol, sh, w.counts, w.half_row, w.half_col,
