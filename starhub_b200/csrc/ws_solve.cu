@@ -671,10 +671,11 @@ struct Tickets {
     uint32_t at, stop;   // the current run
     uint32_t next;       // lane 0: the next run, on its way
 
-    __device__ __forceinline__ Tickets(uint32_t *counter, uint32_t n, int lane) : counter(counter), n(n) {
-        warps = (gridDim.x * blockDim.x) >> 5;
+    // of the launch's blocks from first_block on
+    __device__ __forceinline__ Tickets(uint32_t *counter, uint32_t n, uint32_t first_block, int lane) : counter(counter), n(n) {
+        warps = ((gridDim.x - first_block) * blockDim.x) >> 5;
         run = kDraw && n > 16u * warps ? kTicketRun : 1u;
-        take((blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane);
+        take(((blockIdx.x - first_block) * blockDim.x + threadIdx.x) >> 5, lane);
     }
     __device__ __forceinline__ void take(uint32_t t, int lane) {
         at = min(t, n) * run;   // t counts runs, so t * run may be past 32 bits only past n
@@ -918,29 +919,38 @@ __global__ void __launch_bounds__(32 * W, 5) k_assemble_node_wide(const Scene *s
 // Block-diagonal preconditioner, one thread per node: FP64 Cholesky of the FP64
 // accumulated block (mixed precision) or the reference's FP32 Gauss-Jordan with
 // partial pivoting of the stored block (BlockDiagonalPreconditionerInverse.cuh:14-73).
+// The inverses are a chain of FP64 latencies, 8 to 10 us whatever the number of nodes, and need only the
+// diagonal blocks: the pair kernel's first blocks take them, beside the pairs, instead of a launch between the two.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(64) k_block_inverse(const double *diag64, const float *sym_blocks,
-                                                       const uint32_t *item_ptr, uint32_t cap_items,
-                                                       uint32_t total_nodes, int fp64, float *inv_diag) {
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total_nodes; g += gridDim.x * blockDim.x) {
+struct InverseArgs {
+    const double *diag64;
+    const float *sym_blocks;
+    const uint32_t *item_ptr;
+    uint32_t cap_items, total_nodes, blocks;   // blocks of the launch that take it
+    int fp64;
+    float *inv_diag;
+};
+__device__ __noinline__ void invert_blocks(const InverseArgs &a) {
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < a.total_nodes; g += a.blocks * blockDim.x) {
         float inv[36];
-        if (fp64) {
+        if (a.fp64) {
             double Dd[21];
-            const double *src = diag64 + 21ull * g;
+            const double *src = a.diag64 + 21ull * g;
 #pragma unroll
             for (int i = 0; i < 21; ++i) Dd[i] = src[i];
             cholesky6_fp64(Dd, inv);
         } else {
             float full[36];
 #pragma unroll
-            for (int i = 0; i < 36; ++i) full[i] = sym_blocks[36ull * min(item_ptr[g], cap_items - 1) + i];
+            for (int i = 0; i < 36; ++i) full[i] = a.sym_blocks[36ull * min(a.item_ptr[g], a.cap_items - 1) + i];
             gauss_jordan6(full, inv);
         }
-        float4 *o = reinterpret_cast<float4 *>(inv_diag + 36ull * g);
+        float4 *o = reinterpret_cast<float4 *>(a.inv_diag + 36ull * g);
 #pragma unroll
         for (int i = 0; i < 9; ++i) o[i] = make_float4(inv[4 * i], inv[4 * i + 1], inv[4 * i + 2], inv[4 * i + 3]);
     }
 }
+__global__ void __launch_bounds__(64) k_block_inverse(InverseArgs a) { invert_blocks(a); }
 
 // ---------------------------------------------------------------------------
 // Off-diagonal blocks, once per unordered node pair (i < j) over the pair's term list
@@ -989,12 +999,12 @@ __device__ __forceinline__ uint32_t reg_words(int r, int c) {
     return w;
 }
 
-template <int NT, int C, int kTPL, int kBufs>
+template <int NT, int C, int kTPL, int kBufs, bool kInverse>
 __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble_pair(
     const Scene *scenes, const Plan *plan, const uint32_t *counts,
     const uint32_t *half_row, const uint32_t *half_col, const uint32_t *half_begin, const uint32_t *half_end,
     const uint32_t *half_scene, const uint32_t *pair_val, uint32_t cap_kv, const uint32_t *slot_up, const float *drec, const float *rrec,
-    const float4 *centers, int centred, float *sym_blocks, uint32_t *ticket, int *err) {
+    const float4 *centers, int centred, float *sym_blocks, uint32_t *ticket, InverseArgs inverse, int *err) {
     constexpr int kSlot = kSlotWordsF32;   // per-lane partial sums at the end
     static_assert(kSlot >= 36, "a slot holds one lane's 36 partial sums");
     constexpr int kRec = record_stride<C>();
@@ -1002,6 +1012,11 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     constexpr int kStageWords = max_int(kBufs * kBatch, 32 * kSlot);
     constexpr int kStash = 4;   // smoothness terms per pair: one per edge direction, so at most 2
     __shared__ __align__(16) float stage[NT / 32][kStageWords + kStash * kRegRecord];
+    if constexpr (kInverse)
+        if (blockIdx.x < inverse.blocks) {
+            invert_blocks(inverse);
+            return;
+        }
     const int lane = threadIdx.x & 31;
     float *slots = stage[threadIdx.x >> 5];
     float *stash = slots + kStageWords;   // the pair's smoothness records, in list order
@@ -1015,7 +1030,7 @@ __global__ void __launch_bounds__(NT, (kBufs == 1 ? 1024 : 512) / NT) k_assemble
     const uint32_t reg0 = reg_words(lane / 6, lane % 6);
     // at any time the warps work on neighbouring pairs, whose term records overlap,
     // so the records are read from DRAM about once and then from L2
-    Tickets<kBufs == 1> tickets(ticket, nhalf, lane);
+    Tickets<kBufs == 1> tickets(ticket, nhalf, kInverse ? inverse.blocks : 0u, lane);
     for (; tickets.more(); tickets.advance(lane)) {
         const uint32_t h = tickets.at;
         // the pair's words in one round of loads (its scene among them), then its slot check
@@ -2574,19 +2589,31 @@ void gn_assemble_node(Workspace &w, cudaStream_t st) {
     } else if (w.precision == WS_PREC_FP32) launch_assemble_node_nt<float>(w, w.tune.node_threads, st);
     else launch_assemble_node_nt<double>(w, w.tune.node_threads, st);
     count_launch(w);
-    k_block_inverse<<<grid_for(w.total_nodes, 64, w.num_sms, 32), 64, 0, st>>>(
-        w.diag64, w.sym_blocks, w.item_ptr, w.cap_items, w.total_nodes, w.precision == WS_PREC_MIXED ? 1 : 0,
-        w.inv_diag);
-    count_launch(w);
 }
 
-template <int NT, int C, int kTPL, int kBufs>
-static void launch_assemble_pair_v(Workspace &w, cudaStream_t st) {
-    k_assemble_pair<NT, C, kTPL, kBufs><<<grid_for(w.cap_half * 32u, NT, w.num_sms, (kBufs == 1 ? 1024 : 4096) / NT), NT, 0, st>>>(
+static InverseArgs inverse_args(const Workspace &w, uint32_t blocks) {
+    return {w.diag64, w.sym_blocks, w.item_ptr, w.cap_items, w.total_nodes, blocks, w.precision == WS_PREC_MIXED ? 1 : 0,
+            w.inv_diag};
+}
+// Nodes up to which the pair kernel takes the inverses: the launch saved is worth 12 us an iteration or more (500
+// nodes, 6 iterations: 1021 -> 947 us in all; 4 x 1500 141 -> 129 us an iteration, 8 x 4000 296 -> 287).  The call
+// in it costs the kernel's registers 4 % with very many pairs (64 scenes: 5.0 -> 5.2 ms).
+constexpr uint32_t kInverseInPairs = 32768;
+
+template <int NT, int C, int kTPL, int kBufs, bool kInverse>
+static void launch_assemble_pair_i(Workspace &w, cudaStream_t st) {
+    const InverseArgs inverse = inverse_args(w, kInverse ? (w.total_nodes + NT - 1) / NT : 0u);
+    const uint32_t pairs = (uint32_t)grid_for(w.cap_half * 32u, NT, w.num_sms, (kBufs == 1 ? 1024 : 4096) / NT);
+    k_assemble_pair<NT, C, kTPL, kBufs, kInverse><<<inverse.blocks + pairs, NT, 0, st>>>(
         w.scenes, w.plan, w.counts, w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene,
         w.pair_sorted_val, w.cap_pair_kv,
         w.half_slot_up, w.d_record, w.r_record, w.centers, w.precision == WS_PREC_MIXED ? 1 : 0, w.sym_blocks,
-        w.counts + kCntTicket, w.error_flag);
+        w.counts + kCntTicket, inverse, w.error_flag);
+}
+template <int NT, int C, int kTPL, int kBufs>
+static void launch_assemble_pair_v(Workspace &w, cudaStream_t st) {
+    if (w.total_nodes <= kInverseInPairs) launch_assemble_pair_i<NT, C, kTPL, kBufs, true>(w, st);
+    else launch_assemble_pair_i<NT, C, kTPL, kBufs, false>(w, st);
 }
 template <int NT, int C>
 static void launch_assemble_pair_c(Workspace &w, cudaStream_t st) {
@@ -2607,6 +2634,11 @@ static void launch_assemble_pair(Workspace &w, cudaStream_t st) {
 }
 
 void gn_assemble_pair(Workspace &w, cudaStream_t st) {
+    if (w.total_nodes > kInverseInPairs) {
+        const uint32_t blocks = (uint32_t)grid_for(w.total_nodes, 64, w.num_sms, 32);
+        k_block_inverse<<<blocks, 64, 0, st>>>(inverse_args(w, blocks));
+        count_launch(w);
+    }
     if (w.tune.pair_threads == 64) launch_assemble_pair<64>(w, st);
     else if (w.tune.pair_threads == 256) launch_assemble_pair<256>(w, st);
     else launch_assemble_pair<128>(w, st);
