@@ -553,7 +553,7 @@ def main():
     kv = sum(c["n2t_kv"] for c in counts)
     index_bytes = 2 * (kv * 8 + 6 * nd_tot * 12)
     per_launch = {"pcg": (pcg_bytes, phase_ms["pcg"] / GN_ITERS, "k_pcg"),
-                  "eval": (eval_bytes, phase_ms["eval"] / GN_ITERS, "k_eval_dense"),
+                  "eval": (eval_bytes, phase_ms["eval"] / GN_ITERS, "k_eval"),
                   "assemble_node": (asm_node_bytes, phase_ms["assemble_node"] / GN_ITERS, "k_assemble_node"),
                   "assemble_pair": (asm_pair_bytes, phase_ms["assemble_pair"] / GN_ITERS, "k_assemble_pair"),
                   "index": (index_bytes, phase_ms["index"], "index build")}
