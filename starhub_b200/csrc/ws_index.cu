@@ -159,10 +159,12 @@ __device__ __forceinline__ ushort4 clamp_knn(ushort4 k, const Scene &sc, int *er
 // sit at plan.n2t_base as [4 per dense term | 2 per edge | 1 per node | 4 per feature].  One
 // thread per dense term writes that term's 4 entries (its scene from the compaction), and
 // one block row per scene writes the scene's other entries, so no entry searches for its scene.
-__global__ void k_n2t_kv_dense(const Scene *scenes, const Plan *plan, const uint32_t *counts,
-                               const uint32_t *term_scene, const ushort4 *dense_knn, uint32_t *keys, uint32_t *vals) {
+constexpr uint32_t kTailBlocks = 16;
+__device__ __forceinline__ void n2t_kv_dense(uint32_t block, uint32_t blocks, const Scene *scenes, const Plan *plan,
+                                             const uint32_t *counts, const uint32_t *term_scene,
+                                             const ushort4 *dense_knn, uint32_t *keys, uint32_t *vals) {
     const uint32_t n = counts[kCntDense];
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    for (uint32_t t = block * blockDim.x + threadIdx.x; t < n; t += blocks * blockDim.x) {
         const uint32_t s = term_scene[t];
         const Plan &p = plan[s];
         const uint32_t lt = t - p.dense_begin, base = p.n2t_base + 4u * lt, nb = scenes[s].node_base;
@@ -175,13 +177,13 @@ __global__ void k_n2t_kv_dense(const Scene *scenes, const Plan *plan, const uint
     }
 }
 
-__global__ void k_n2t_kv_tail(const Scene *scenes, const Plan *plan, uint32_t *keys, uint32_t *vals,
-                              uint32_t invalid_key, int *err) {
-    const Scene &sc = scenes[blockIdx.y];
-    const Plan &p = plan[blockIdx.y];
+__device__ __forceinline__ void n2t_kv_tail(uint32_t s, uint32_t block, const Scene *scenes, const Plan *plan,
+                                            uint32_t *keys, uint32_t *vals, uint32_t invalid_key, int *err) {
+    const Scene &sc = scenes[s];
+    const Plan &p = plan[s];
     const uint32_t nd = p.dense_count, ne = sc.num_edges, nn = sc.num_nodes, nf = sc.num_features;
     const uint32_t len = 2u * ne + nn + 4u * nf, base = p.n2t_base + 4u * nd;
-    for (uint32_t j0 = blockIdx.x * blockDim.x + threadIdx.x; j0 < len; j0 += gridDim.x * blockDim.x) {
+    for (uint32_t j0 = block * blockDim.x + threadIdx.x; j0 < len; j0 += kTailBlocks * blockDim.x) {
         uint32_t j = j0, key, val;
         if (j < 2u * ne) {
             const uint32_t e = j >> 1;
@@ -206,11 +208,25 @@ __global__ void k_n2t_kv_tail(const Scene *scenes, const Plan *plan, uint32_t *k
     }
 }
 
+// The first kTailBlocks blocks of every scene write its edge, node and feature entries, the others the dense ones.
+__global__ void __launch_bounds__(256) k_n2t_kv(const Scene *scenes, int num_scenes, const Plan *plan,
+                                                const uint32_t *counts, const uint32_t *term_scene,
+                                                const ushort4 *dense_knn, uint32_t *keys, uint32_t *vals,
+                                                uint32_t invalid_key, int *err) {
+    const uint32_t tails = kTailBlocks * (uint32_t)num_scenes;
+    if (blockIdx.x < tails)
+        n2t_kv_tail(blockIdx.x / kTailBlocks, blockIdx.x % kTailBlocks, scenes, plan, keys, vals, invalid_key, err);
+    else
+        n2t_kv_dense(blockIdx.x - tails, gridDim.x - tails, scenes, plan, counts, term_scene, dense_knn, keys, vals);
+}
+
 // computeTermOffsetKernel (Node2TermsIndex.cu:78-121) as a lower bound per node.
+// Also clears the pairs' counts below the diagonal for the pair map.
 __global__ void k_n2t_offsets(const uint32_t *sorted_keys, const uint32_t *counts, uint32_t total_nodes,
-                              uint32_t *offsets) {
+                              uint32_t *offsets, uint32_t *row_cnt_lo) {
     const uint32_t n = counts[kCntN2T];
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g <= total_nodes; g += gridDim.x * blockDim.x) {
+        if (g < total_nodes) row_cnt_lo[g] = 0;
         uint32_t lo = 0, hi = n;
         while (lo < hi) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -557,23 +573,18 @@ __global__ void __launch_bounds__(32 * (W == 1 ? kRowWarps : W), (W == 1 ? kRowB
     }
 }
 
-__global__ void k_row_first(const uint32_t *half_row, const uint32_t *counts, uint32_t *row_first) {
-    const uint32_t n = counts[kCntHalf];
-    for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x)
-        if (h == 0 || half_row[h - 1] != half_row[h]) row_first[half_row[h]] = h;
-}
-
-__global__ void k_row_len(const uint32_t *up, const uint32_t *lo, uint32_t total_nodes, uint32_t *len,
-                          uint32_t *items) {
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total_nodes; g += gridDim.x * blockDim.x) {
+// For the block CSR: every row's first pair and lengths, and the pairs keyed by column for their sort.
+__global__ void k_csr_rows(const uint32_t *half_row, const uint32_t *half_col, const uint32_t *counts, const uint32_t *up,
+                           const uint32_t *lo, uint32_t total_nodes, uint32_t *row_first, uint32_t *len, uint32_t *items,
+                           uint32_t *keys, uint32_t *vals) {
+    const uint32_t n = counts[kCntHalf], first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (uint32_t g = first; g < total_nodes; g += stride) {
         len[g] = 1u + up[g] + lo[g];
         items[g] = 1u + up[g];   // stored blocks of the row: the diagonal and the upper pairs
     }
-}
-
-__global__ void k_col_kv(const uint32_t *half_col, const uint32_t *counts, uint32_t *keys, uint32_t *vals) {
-    const uint32_t n = counts[kCntHalf];
-    for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x) {
+    for (uint32_t h = first; h < n; h += stride) {
+        const uint32_t row = half_row[h];
+        if (h == 0 || half_row[h - 1] != row) row_first[row] = h;
         keys[h] = half_col[h];
         vals[h] = h;
     }
@@ -585,11 +596,14 @@ __global__ void k_col_kv(const uint32_t *half_col, const uint32_t *counts, uint3
 // Bin-Blocked CSR (NodePairRowColumnIndex.cu:110-124).  Also the item record of every pair
 // h = (row, col) of the symmetric store (item h + row + 1): its lower entry is its position
 // k among the pairs sorted by column (then row).
+// Then the diagonal slot of every row, and the item records of the row's diagonal item (the row, marked
+// as a row start, and its scene).
 __global__ void k_slots(const uint32_t *sorted_col, const uint32_t *sorted_h, const uint32_t *counts,
                         const uint32_t *half_row, const uint32_t *half_col, const uint32_t *row_first,
                         const uint32_t *row_cnt_lo, const uint32_t *rowptr, uint32_t cap_blocks,
                         uint32_t *slot_up, uint32_t *slot_lo, uint32_t *colidx, uint2 *item_info,
-                        uint32_t *item_col, int *err) {
+                        uint32_t *item_col, const uint32_t *item_ptr, const uint32_t *node_scene, uint32_t total_nodes,
+                        int *err) {
     const uint32_t n = counts[kCntHalf];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t col = sorted_col[k];
@@ -615,13 +629,6 @@ __global__ void k_slots(const uint32_t *sorted_col, const uint32_t *sorted_h, co
         item_info[h + row + 1u] = make_uint2(half_col[h], k);
         item_col[h + row + 1u] = half_col[h];
     }
-}
-
-// Diagonal slot of every row, and the item records of the row's diagonal item (the row, marked
-// as a row start, and its scene).
-__global__ void k_diag_cols(const uint32_t *rowptr, const uint32_t *item_ptr, const uint32_t *node_scene,
-                            uint32_t total_nodes, uint32_t cap_blocks, uint32_t *colidx, uint2 *item_info,
-                            uint32_t *item_col, int *err) {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total_nodes; g += gridDim.x * blockDim.x) {
         const uint32_t s = rowptr[g];
         if (s < cap_blocks) colidx[s] = g;
@@ -723,7 +730,6 @@ static void pair_index_rows(Workspace &w, cudaStream_t st) {
                                                    w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts, w.row_cnt_up,
                                                    w.row_entry_first, w.error_flag);
     count_launch(w, exclusive_scan2(w.row_cnt_up, w.row_pair_first, w.row_entry_first, w.row_entry_first, N, w.scan_tmp, st));
-    cudaMemsetAsync(w.row_cnt_lo, 0, sizeof(uint32_t) * w.cap_nodes, st);
     k_pair_rows_fill<W><<<grid, threads, 0, st>>>(w.scenes, w.plan, w.node_scene, N, w.n2t_offset, w.n2t_sorted_val,
                                                   w.cap_n2t, w.d_knn, w.row_pair_cols, w.row_pair_cnts,
                                                   w.row_pair_first, w.row_entry_first, w.cap_half, w.cap_pair_kv,
@@ -754,36 +760,33 @@ void index_build(Workspace &w, cudaStream_t st) {
     count_launch(w, 2);
     // 2. node -> term
     const uint32_t n2t_invalid = (1u << w.node_bits) - 1u;
-    k_n2t_kv_dense<<<grid_for(w.cap_pixels, 256, w.num_sms), 256, 0, st>>>(w.scenes, w.plan, w.counts, w.d_scene,
-                                                                            w.d_knn, w.n2t_key, w.n2t_val);
-    k_n2t_kv_tail<<<dim3(16, S), 256, 0, st>>>(w.scenes, w.plan, w.n2t_key, w.n2t_val, n2t_invalid, w.error_flag);
+    k_n2t_kv<<<kTailBlocks * S + grid_for(w.cap_pixels, 256, w.num_sms), 256, 0, st>>>(
+        w.scenes, S, w.plan, w.counts, w.d_scene, w.d_knn, w.n2t_key, w.n2t_val, n2t_invalid, w.error_flag);
     count_launch(w);
     const bool n2t_alt = radix_sort<uint32_t>(w.n2t_key, w.n2t_val, w.n2t_key_alt, w.n2t_val_alt, w.counts + kCntN2T, 0,
                                               w.cap_n2t, w.node_bits, w.sort_hist, w.sort_digit, st);
-    count_launch(w, 1 + 3 * radix_passes(w.node_bits));
+    count_launch(w, 3 * radix_passes(w.node_bits));
     w.n2t_sorted_key = n2t_alt ? w.n2t_key_alt : w.n2t_key;
     w.n2t_sorted_val = n2t_alt ? w.n2t_val_alt : w.n2t_val;
-    k_n2t_offsets<<<grid_for(N + 1, 256, w.num_sms), 256, 0, st>>>(w.n2t_sorted_key, w.counts, N, w.n2t_offset);
+    k_n2t_offsets<<<grid_for(N + 1, 256, w.num_sms), 256, 0, st>>>(w.n2t_sorted_key, w.counts, N, w.n2t_offset,
+                                                                  w.row_cnt_lo);
     count_launch(w);
     // 3. node pair -> term
     pair_index(w, st);
     // 4. block CSR
-    k_row_first<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(w.half_row, w.counts, w.row_first);
-    k_row_len<<<grid_for(N, 256, w.num_sms), 256, 0, st>>>(w.row_cnt_up, w.row_cnt_lo, N, w.rowptr, w.item_ptr);
+    k_csr_rows<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(w.half_row, w.half_col, w.counts, w.row_cnt_up,
+                                                                     w.row_cnt_lo, N, w.row_first, w.rowptr, w.item_ptr,
+                                                                     w.col_key, w.col_val);
     count_launch(w, exclusive_scan2(w.rowptr, w.rowptr, w.item_ptr, w.item_ptr, N, w.scan_tmp, st));
-    k_col_kv<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(w.half_col, w.counts, w.col_key, w.col_val);
     const bool col_alt = radix_sort<uint32_t>(w.col_key, w.col_val, w.col_key_alt, w.col_val_alt, w.counts + kCntHalf,
                                               0, w.cap_half, w.node_bits, w.sort_hist, w.sort_digit, st);
-    count_launch(w, 1 + 1 + 1 + 3 * radix_passes(w.node_bits));
+    count_launch(w, 1 + 3 * radix_passes(w.node_bits));
     const uint32_t *scol = col_alt ? w.col_key_alt : w.col_key;
     const uint32_t *sh = col_alt ? w.col_val_alt : w.col_val;
-    k_slots<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(scol, sh, w.counts, w.half_row, w.half_col,
-                                                                    w.row_first, w.row_cnt_lo, w.rowptr,
-                                                                    w.cap_blocks, w.half_slot_up, w.half_slot_lo, w.colidx,
-                                                                    w.item_info, w.item_col, w.error_flag);
-    k_diag_cols<<<grid_for(N, 256, w.num_sms), 256, 0, st>>>(w.rowptr, w.item_ptr, w.node_scene, N, w.cap_blocks,
-                                                             w.colidx, w.item_info, w.item_col, w.error_flag);
-    count_launch(w, 2);
+    k_slots<<<grid_for(w.cap_half, 256, w.num_sms), 256, 0, st>>>(
+        scol, sh, w.counts, w.half_row, w.half_col, w.row_first, w.row_cnt_lo, w.rowptr, w.cap_blocks, w.half_slot_up,
+        w.half_slot_lo, w.colidx, w.item_info, w.item_col, w.item_ptr, w.node_scene, N, w.error_flag);
+    count_launch(w);
     pcg_ranges(w, st);
     pcg_plan(w, st);
 }
