@@ -86,6 +86,8 @@ int validate(const ws_inputs &in) {
 
 }  // namespace
 
+void ws::pcg_allow_resident(ws_solver *h, bool allow) { h->w.pcg_resident = allow; }
+
 extern "C" {
 
 int ws_version(void) { return 1; }

@@ -78,6 +78,7 @@ struct ws_server {
     std::unordered_map<unsigned long long, Request> requests;
     std::map<int, Resident> scenes;
     std::vector<Executor> execs;
+    int busy = 0;   // executors with a batch on the device
     cudaStream_t control = nullptr;
     bool stop = false;
     unsigned long long next_id = 1;
@@ -181,6 +182,12 @@ void executor_loop(ws_server *s, int index) {
             }
             ++s->batches;
             s->batch_scene_sum += batch.size();
+            // The resident PCG takes all shared memory of its SMs, so batches beside it wait: it is for a batch
+            // that starts on an idle device with no frame waiting.  The results are the same bits.  32 streams, 840
+            // frames/s, three executors, p50 / p99 ms: always by size 11.3 / 22.5, never 7.5 / 16.3, this 7.8 / 16.8;
+            // a lone batch, p50 2.0, 3.6, 2.0.
+            ws::pcg_allow_resident(x.solver, s->busy == 0 && s->waiting.empty());
+            ++s->busy;
             if (has_ready(s)) s->cv_work.notify_one();   // frames left over for another free executor
         }
         // launch outside the lock; resident warps are only written by the executor whose
@@ -212,6 +219,7 @@ void executor_loop(ws_server *s, int index) {
         const Clock::time_point t = Clock::now();
         {
             std::lock_guard<std::mutex> lk(s->m);
+            --s->busy;
             for (unsigned long long id : batch) {
                 Request &r = s->requests.at(id);
                 r.status = st;

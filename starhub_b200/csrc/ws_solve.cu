@@ -2826,6 +2826,7 @@ int pcg_grid_blocks(Scene *scenes, int num_scenes, int most) {
 // 8k 2.80 / 2.95 / 1.10; nodes log-uniform in [500, 8000], 4 scenes 2.86 / 1.89 / 1.22, 16 scenes 3.65 / 2.94 /
 // 2.28, 64 scenes 7.1 / 10.9 / does not fit.
 PcgMode pcg_mode(const Workspace &w) {
+    if (!w.pcg_resident) return PcgMode::kStream;
     const int size = w.pcg_cluster;
     double most = 0.0, sum = 0.0, rows = 0.0;
     bool cluster_fits = size > 0 && w.pcg_clusters_active > 0;

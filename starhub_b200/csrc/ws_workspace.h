@@ -24,6 +24,7 @@ struct Workspace {
     int pcg_grid = 0;           // co-resident blocks for the persistent PCG kernel
     int pcg_cluster = 0;        // blocks per cluster of k_pcg_cluster on this device (16, 8; 0: none)
     int pcg_clusters_active = 0;   // such clusters that run at once
+    bool pcg_resident = true;   // k_pcg_cluster may be used: it fills the shared memory of the SMs it runs on
     int pcg_grid_most = 0;      // blocks of k_pcg_cluster over the whole grid at most (one per SM; 0: none)
     int pcg_grid_blocks = 0;    // those of the current batch (0: it does not fit)
     // launch shapes picked by ws_autotune (defaults until then); none of them changes a result
@@ -186,6 +187,8 @@ cudaError_t gn_spmv_matrix_free(Workspace &w, const float *x, float *y, float *u
 int pcg_warps_per_block();
 // Gives the geometry calls' idle scratch on a device back to the driver (ws_graph.cu).
 void scratch_trim(int device);
+// Whether the solver's next solves may use the resident PCG (ws_api.cu).
+void pcg_allow_resident(::ws_solver *h, bool allow);
 
 // Launch accounting for the measurement hooks.
 inline void count_launch(Workspace &w, int n = 1) { w.launches += n; }
