@@ -196,8 +196,8 @@ int ws_expand_nodes(const float *vertices, int num_vertices, float node_radius, 
                     void *stream);
 /* UpdateNodeDistanceKernel + BuildNodeGraphKernel + BuildNodeGraphPairKernel
  * (NodeGraph.cu:10-118): device in/out; k = 4 or 8; edges gets (i, knn[i][k], k).  The
- * n x n half-distance table is not built: each node scans runs of 32 nodes and skips the runs
- * whose bounding box cannot enter its heap (same results).  Asynchronous on `stream`. */
+ * n x n half-distance table is not built: a warp scans the nodes in order, from 5000 nodes on only those
+ * of the cells around its own (same results).  Asynchronous on `stream`. */
 int ws_build_node_graph(const float *nodes, int num_nodes, int k, float node_radius,
                         uint16_t *knn, float *spatial_w, uint16_t *edges, void *stream);
 /* SkinnerKernel (libs/star/geometry/node_graph/Skinner.cu:10-94): device in/out, weights divided

@@ -229,11 +229,12 @@ static __global__ void k_radix_scan(uint32_t *hist, int max_tiles, uint32_t tile
     if (threadIdx.x == 0) digit_total[blockIdx.x] = carry;
 }
 
-// Places a tile's keys and values, all of them read at once.  What bounds it is the ranking (every key's place among its digit's) and the
-// writes: a warp ranks its own run of keys against counters of its own, with nothing shared until all are ranked,
-// and the tile goes through shared memory in digit order, so that a digit's keys are written side by side.  Ranking by rounds of the whole block, four barriers a round, and
-// writing each key where it belongs took, for all passes of 64 scenes' lists 613 us, now 412; 8000 nodes' 58, now
-// 26; 200 k voxels 52, now 18.  Ranking by ballots of the digit's bits instead of matching: 585 us for 64 scenes.
+// Places a tile's keys and values, all of them read at once.  What bounds it is the ranking (every key's place among
+// its digit's) and the writes: a warp ranks its own run of keys against counters of its own, with nothing shared
+// until all are ranked, and the tile goes through shared memory in digit order, so that a digit's keys are written
+// side by side.  Ranking by rounds of the whole block, four barriers a round, and writing each key where it belongs
+// took, for all passes of 64 scenes' lists 613 us, now 412; 8000 nodes' 58, now 26; 200 k voxels 52, now 18.
+// Ranking by ballots of the digit's bits instead of matching: 585 us for 64 scenes.
 template <class K, int D, int R>
 __global__ void __launch_bounds__(kSortThreads)
 k_radix_scatter(const K *keys_in, const uint32_t *vals_in, K *keys_out, uint32_t *vals_out,
