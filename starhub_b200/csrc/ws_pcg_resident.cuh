@@ -319,7 +319,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     uint32_t off = kGrid ? 0u : (16u * groups + 15u) & ~15u;
     constexpr uint32_t kMinLocal = 32u * kThreads + 4u * kChunkBytes + 64u;   // product records and a small ring
     const uint32_t off_s = off, off_d = off + 24u * vmax;
-    const bool vec_shared = off + 48u * vmax + kMinLocal <= smem_bytes;   // else s and d go through A.sd0 / A.sd1
+    // s and d in shared memory, else in A.sd0 / A.sd1.  One answer for the scene, since blocks that have them there
+    // publish s by another way than blocks that have not: vmax is a cluster's largest; on the grid thread t looks
+    // at the scene's block t
+    bool vec_shared = off + 48u * vmax + kMinLocal <= smem_bytes;
+    if constexpr (kGrid) {
+        static_assert(kResThreads >= kResMaxBlocks, "a thread per block of the scene");
+        if (tid < size)
+            vec_shared = off + 48u * (R.row[tid + 1] - R.row[tid] + __ldg(P.halo + (blockIdx.x - rank + tid))) + kMinLocal <=
+                         smem_bytes;
+        vec_shared = __syncthreads_and(vec_shared);
+    }
     if (vec_shared) off = (off + 48u * vmax + 15u) & ~15u;
     const uint32_t off_contrib = off;
     const bool contrib_shared = off + 24u * lmax + kMinLocal <= smem_bytes;   // else through A.contrib
