@@ -422,7 +422,7 @@ int ws_server_get_stats(ws_server *s, ws_server_stats *stats);
 typedef struct ws_tuning {
     int node_threads;           /* chosen threads per block, node assembly */
     int pair_threads;           /* chosen threads per block, pair assembly */
-    int pcg_blocks_per_sm;      /* chosen PCG blocks per SM */
+    int pcg_blocks_per_sm;      /* chosen PCG blocks per SM (streamed form only, see ws_set_pcg_form) */
     float node_ms[3];           /* per candidate 64 / 128 / 256 threads; < 0 = not offered */
     float pair_ms[3];
     float pcg_ms[8];            /* per candidate 1..8 blocks per SM; < 0 = not offered */
@@ -430,6 +430,24 @@ typedef struct ws_tuning {
 int ws_autotune(ws_solver *solver, int pcg_iters, void *stream, ws_tuning *result);
 /* Applies a tuning (e.g. one stored from an earlier ws_autotune on the same workload). */
 int ws_set_tuning(ws_solver *solver, const ws_tuning *tuning);
+
+/* ---- Form of the PCG --------------------------------------------------------------------
+ * No reference counterpart.  The PCG of a batch runs in one of three forms, with the same bits: streamed (a
+ * persistent kernel of up to pcg_blocks_per_sm blocks on every SM), one thread-block cluster per scene, or the
+ * scenes side by side over the whole device.  The last two keep the matrix in shared memory, up to all of an
+ * SM's, on every SM they run on: they do not follow pcg_blocks_per_sm, and another solver's kernels wait for
+ * them.  WS_PCG_AUTO, the default, takes the form that is fastest for a solver that has the device to itself; a
+ * program whose solvers work side by side on several streams of one device is served best by WS_PCG_STREAMED. */
+#define WS_PCG_AUTO 0
+#define WS_PCG_STREAMED 1
+#define WS_PCG_CLUSTERS 2           /* at most 8192 nodes a scene */
+#define WS_PCG_GRID 3               /* at most 8192 nodes a scene, and 512 rows a block of the device's */
+/* Sets the form of the solver's later solves.  A batch that does not fit the form asked for is solved streamed.
+ * shared_bytes: dynamic shared memory a block of the last two forms may use, 49152 to 228864, 0 = all of it (what
+ * does not fit is read from L2). */
+int ws_set_pcg_form(ws_solver *solver, int form, int shared_bytes);
+/* The form (not WS_PCG_AUTO) that a solve of the inputs set takes; WS_ERR_NOT_READY without inputs. */
+int ws_get_pcg_form(ws_solver *solver, int *form);
 
 /* Library version / build identification. */
 int ws_version(void);

@@ -24,6 +24,11 @@ WS_ERR_NO_DEVICE = -7
 WS_PREC_MIXED = 0
 WS_PREC_FP32 = 1
 
+WS_PCG_AUTO = 0
+WS_PCG_STREAMED = 1
+WS_PCG_CLUSTERS = 2
+WS_PCG_GRID = 3
+
 WS_NOALLOC_MAX_PIXELS = 1280 * 720
 
 # Every symbol include/warpsolve.h declares.
@@ -39,7 +44,7 @@ EXPORTED = [
     "ws_selftest_wait_timeout", "ws_selftest_grid_barrier_timeout", "ws_render_solver_maps",
     "ws_render_observation_maps",
     "ws_build_node_graph_ex", "ws_skinning_ex", "ws_skinning_incremental",
-    "ws_set_tuning",
+    "ws_set_tuning", "ws_set_pcg_form", "ws_get_pcg_form",
 ]
 
 
@@ -192,6 +197,8 @@ def load() -> C.CDLL:
         "ws_skinning_incremental": (i, [vp, vp, i, i, vp, i, i, f, i, vp, vp, vp, vp]),
         "ws_autotune": (i, [vp, i, vp, C.POINTER(WsTuning)]),
         "ws_set_tuning": (i, [vp, C.POINTER(WsTuning)]),
+        "ws_set_pcg_form": (i, [vp, i, i]),
+        "ws_get_pcg_form": (i, [vp, C.POINTER(i)]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)

@@ -86,8 +86,6 @@ int validate(const ws_inputs &in) {
 
 }  // namespace
 
-void ws::pcg_allow_resident(ws_solver *h, bool allow) { h->w.pcg_resident = allow; }
-
 extern "C" {
 
 int ws_version(void) { return 1; }
@@ -235,6 +233,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
         A(dalloc(&w.pcg_send_count, w.cap_nodes));
         A(dalloc(&w.pcg_halo, 16ull * w.cap_scenes + 160));   // kResMaxCluster a scene, or kResMaxBlocks
         w.pcg_grid_most = ws::pcg_grid_max(w.device);
+        w.pcg_smem = ws::pcg_smem_max();
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -478,7 +477,7 @@ int ws_solve_graph(ws_solver *h, int gn_iters, int pcg_iters, void *stream) {
     const uint64_t key[] = {(uint64_t)gn_iters, (uint64_t)pcg_iters, (uint64_t)w.num_scenes, w.total_nodes,
                             w.total_edges, w.total_tiles, w.total_chunks, (uint64_t)w.node_bits,
                             (uint64_t)w.dense_channels, (uint64_t)ws::pcg_split_group(w),
-                            (uint64_t)ws::pcg_mode(w), (uint64_t)w.pcg_grid_blocks};
+                            (uint64_t)ws::pcg_mode(w), (uint64_t)w.pcg_grid_blocks, w.pcg_smem};
     constexpr size_t kKey = sizeof(key) / sizeof(key[0]);
     bool same = w.graph_exec && w.graph_key.size() == kKey && std::equal(key, key + kKey, w.graph_key.begin());
     if (same) {
@@ -630,6 +629,22 @@ int ws_set_tuning(ws_solver *h, const ws_tuning *t) {
     w.tune.pcg_blocks_per_sm = t->pcg_blocks_per_sm;
     w.tune.tuned = true;
     drop_graph(w);
+    return WS_OK;
+}
+
+int ws_set_pcg_form(ws_solver *h, int form, int shared_bytes) {
+    if (!h || form < WS_PCG_AUTO || form > WS_PCG_GRID) return WS_ERR_INVALID_ARGUMENT;
+    if (shared_bytes != 0 && (shared_bytes < (int)ws::pcg_smem_min() || shared_bytes > (int)ws::pcg_smem_max()))
+        return WS_ERR_INVALID_ARGUMENT;
+    h->w.pcg_form = form;
+    h->w.pcg_smem = shared_bytes == 0 ? ws::pcg_smem_max() : (uint32_t)shared_bytes & ~127u;
+    return WS_OK;
+}
+
+int ws_get_pcg_form(ws_solver *h, int *form) {
+    if (!h || !form) return WS_ERR_INVALID_ARGUMENT;
+    if (!h->w.have_inputs) return WS_ERR_NOT_READY;
+    *form = (int)ws::pcg_mode(h->w);
     return WS_OK;
 }
 

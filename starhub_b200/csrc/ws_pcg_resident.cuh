@@ -31,6 +31,7 @@ constexpr int kResMaxCluster = 16;
 constexpr int kResThreads = 512;
 constexpr int kResRows = kResThreads;   // rows of a block at most: one per thread
 constexpr uint32_t kResSmemBytes = 228864;   // beside 3 KB of static shared memory
+constexpr uint32_t kResSmemMin = 49152;      // a cluster's partials (8 KB at most), product records and a ring of four
 constexpr int kResMaxPolls = 1 << 22;   // polls of a meeting before it gives up (a second or more)
 constexpr uint32_t kResNodes = kResRows * kResMaxCluster;   // nodes of a scene at most
 constexpr int kPlanThreads = 512;

@@ -186,7 +186,7 @@ void executor_loop(ws_server *s, int index) {
             // that starts on an idle device with no frame waiting.  The results are the same bits.  32 streams, 840
             // frames/s, three executors, p50 / p99 ms: always by size 11.3 / 22.5, never 7.5 / 16.3, this 7.8 / 16.8;
             // a lone batch, p50 2.0, 3.6, 2.0.
-            ws::pcg_allow_resident(x.solver, s->busy == 0 && s->waiting.empty());
+            ws_set_pcg_form(x.solver, s->busy == 0 && s->waiting.empty() ? WS_PCG_AUTO : WS_PCG_STREAMED, 0);
             ++s->busy;
             if (has_ready(s)) s->cv_work.notify_one();   // frames left over for another free executor
         }

@@ -2779,6 +2779,9 @@ int pcg_cluster_max(int *active) {
     return known[dev][0] - 1;
 }
 
+uint32_t pcg_smem_max() { return kResSmemBytes; }
+uint32_t pcg_smem_min() { return kResSmemMin; }
+
 // Most blocks of k_pcg_cluster<true> that run at once (one per SM), 0 without cooperative launches.
 int pcg_grid_max(int device) {
     int per_sm = 0, sms = 0, coop = 0;
@@ -2826,7 +2829,7 @@ int pcg_grid_blocks(Scene *scenes, int num_scenes, int most) {
 // 8k 2.80 / 2.95 / 1.10; nodes log-uniform in [500, 8000], 4 scenes 2.86 / 1.89 / 1.22, 16 scenes 3.65 / 2.94 /
 // 2.28, 64 scenes 7.1 / 10.9 / does not fit.
 PcgMode pcg_mode(const Workspace &w) {
-    if (!w.pcg_resident) return PcgMode::kStream;
+    if (w.pcg_form == WS_PCG_STREAMED) return PcgMode::kStream;
     const int size = w.pcg_cluster;
     double most = 0.0, sum = 0.0, rows = 0.0;
     bool cluster_fits = size > 0 && w.pcg_clusters_active > 0;
@@ -2839,6 +2842,8 @@ PcgMode pcg_mode(const Workspace &w) {
         if (w.pcg_grid_blocks > 0)
             rows = std::max(rows, (double)kRowsPerGroup * ((sc.num_chunks + sc.pcg_blocks - 1) / sc.pcg_blocks));
     }
+    if (w.pcg_form == WS_PCG_CLUSTERS) return cluster_fits ? PcgMode::kClusters : PcgMode::kStream;
+    if (w.pcg_form == WS_PCG_GRID) return w.pcg_grid_blocks > 0 ? PcgMode::kGrid : PcgMode::kStream;
     const double stream = 22.0 + 0.3e-3 * w.total_nodes;
     const double clusters = cluster_fits ? std::max(most, sum / w.pcg_clusters_active) : 1e30;
     const double grid = w.pcg_grid_blocks > 0 ? 9.2 + 0.045 * rows : 1e30;
@@ -2879,17 +2884,17 @@ cudaError_t gn_pcg(Workspace &w, int pcg_iters, cudaStream_t st) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr{};
         count_launch(w);
-        cluster_launch(cfg, attr, w.pcg_cluster, w.num_scenes, kResThreads, kResSmemBytes, st);
-        return cudaLaunchKernelEx(&cfg, k_pcg_cluster<false>, a, res_plan(w), kResSmemBytes);
+        cluster_launch(cfg, attr, w.pcg_cluster, w.num_scenes, kResThreads, w.pcg_smem, st);
+        return cudaLaunchKernelEx(&cfg, k_pcg_cluster<false>, a, res_plan(w), w.pcg_smem);
     }
     if (mode == PcgMode::kGrid) {
         cudaMemsetAsync(w.scene_counter, 0, sizeof(uint32_t) * kSceneSync * (size_t)w.num_scenes, st);
         ResPlan plan = res_plan(w);
-        uint32_t smem = kResSmemBytes;
+        uint32_t smem = w.pcg_smem;
         void *args[] = {&a, &plan, &smem};
         count_launch(w);
         return cudaLaunchCooperativeKernel((const void *)k_pcg_cluster<true>, dim3((unsigned)w.pcg_grid_blocks),
-                                           dim3(kResThreads), args, kResSmemBytes, st);
+                                           dim3(kResThreads), args, smem, st);
     }
     const int grid = pcg_launch_blocks(w);
     // tickets and generations start at zero every launch, so a launch that timed out half-way

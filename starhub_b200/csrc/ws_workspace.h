@@ -24,7 +24,8 @@ struct Workspace {
     int pcg_grid = 0;           // co-resident blocks for the persistent PCG kernel
     int pcg_cluster = 0;        // blocks per cluster of k_pcg_cluster on this device (16, 8; 0: none)
     int pcg_clusters_active = 0;   // such clusters that run at once
-    bool pcg_resident = true;   // k_pcg_cluster may be used: it fills the shared memory of the SMs it runs on
+    int pcg_form = WS_PCG_AUTO;    // the caller's choice (ws_set_pcg_form)
+    uint32_t pcg_smem = 0;         // dynamic shared memory of a block of k_pcg_cluster
     int pcg_grid_most = 0;      // blocks of k_pcg_cluster over the whole grid at most (one per SM; 0: none)
     int pcg_grid_blocks = 0;    // those of the current batch (0: it does not fit)
     // launch shapes picked by ws_autotune (defaults until then); none of them changes a result
@@ -171,7 +172,9 @@ int pcg_max_blocks(int device);
 int pcg_cluster_max(int *active);
 int pcg_grid_max(int device);
 int pcg_grid_blocks(Scene *scenes, int num_scenes, int most);
-enum class PcgMode { kStream = 0, kClusters = 1, kGrid = 2 };
+uint32_t pcg_smem_max();
+uint32_t pcg_smem_min();
+enum class PcgMode { kStream = WS_PCG_STREAMED, kClusters = WS_PCG_CLUSTERS, kGrid = WS_PCG_GRID };
 PcgMode pcg_mode(const Workspace &w);
 cudaError_t pcg_plan(Workspace &w, cudaStream_t st);
 int pcg_launch_blocks(const Workspace &w);
@@ -187,8 +190,6 @@ cudaError_t gn_spmv_matrix_free(Workspace &w, const float *x, float *y, float *u
 int pcg_warps_per_block();
 // Gives the geometry calls' idle scratch on a device back to the driver (ws_graph.cu).
 void scratch_trim(int device);
-// Whether the solver's next solves may use the resident PCG (ws_api.cu).
-void pcg_allow_resident(::ws_solver *h, bool allow);
 
 // Launch accounting for the measurement hooks.
 inline void count_launch(Workspace &w, int n = 1) { w.launches += n; }

@@ -236,6 +236,16 @@ class WarpSolver:
         t.node_threads, t.pair_threads, t.pcg_blocks_per_sm = node_threads, pair_threads, pcg_blocks_per_sm
         check(self._lib.ws_set_tuning(self._h, C.byref(t)), "ws_set_tuning")
 
+    def set_pcg_form(self, form: int = _lib.WS_PCG_AUTO, shared_bytes: int = 0) -> None:
+        """Form of the PCG of the later solves (ws_set_pcg_form); no form changes a result."""
+        check(self._lib.ws_set_pcg_form(self._h, form, shared_bytes), "ws_set_pcg_form")
+
+    def pcg_form(self) -> int:
+        """The form that a solve of the inputs set takes (ws_get_pcg_form)."""
+        f = C.c_int()
+        check(self._lib.ws_get_pcg_form(self._h, C.byref(f)), "ws_get_pcg_form")
+        return f.value
+
     # -- measurement ---------------------------------------------------------
     def set_profiling(self, enable: bool) -> None:
         check(self._lib.ws_set_profiling(self._h, 1 if enable else 0), "ws_set_profiling")

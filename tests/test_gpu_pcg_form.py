@@ -1,0 +1,44 @@
+"""ws_set_pcg_form: a program whose solvers share a device can keep a solver's PCG on the streamed form, and every
+form gives the same bits."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+
+def test_arguments():
+    from starhub_b200 import _lib, build
+    build.build()
+    lib = _lib.load()
+    form = C.c_int()
+    assert lib.ws_set_pcg_form(None, 0, 0) == _lib.WS_ERR_INVALID_ARGUMENT
+    assert lib.ws_get_pcg_form(None, C.byref(form)) == _lib.WS_ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [False, True])
+def test_streamed_on_request(ws, small_scene, tiny_scene, graph):
+    import torch
+    from starhub_b200 import _lib
+    from starhub_b200._lib import WarpSolveError
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    ds = [DeviceScene.from_scene(s) for s in (small_scene, tiny_scene)]
+    s = WarpSolver(max_nodes=sum(d.num_nodes for d in ds), max_pixels=sum(d.num_pixels for d in ds),
+                   max_edges=sum(d.num_edges for d in ds), max_scenes=2)
+    with pytest.raises(WarpSolveError):
+        s.pcg_form()   # no inputs yet
+    for bad in ((-1, 0), (4, 0), (0, 49151), (0, 228865), (0, -1)):
+        with pytest.raises(WarpSolveError):
+            s.set_pcg_form(*bad)
+    s.SetBatchInputs(ds)
+    out, stream = {}, torch.cuda.Stream()
+    for form in (_lib.WS_PCG_AUTO, _lib.WS_PCG_STREAMED, _lib.WS_PCG_CLUSTERS, _lib.WS_PCG_GRID, _lib.WS_PCG_AUTO):
+        s.set_pcg_form(form)
+        ran = s.pcg_form()
+        assert ran == form if form != _lib.WS_PCG_AUTO else ran != _lib.WS_PCG_STREAMED
+        for _ in range(2):
+            s.SolveStreamed(2, 7, stream=stream, graph=graph)
+        s.Sync()
+        for i in range(2):
+            got = s.SolvedNodeSE3(i).cpu().numpy()
+            np.testing.assert_array_equal(out.setdefault(i, got.copy()), got, err_msg=f"form {form}")
