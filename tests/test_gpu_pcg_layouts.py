@@ -96,3 +96,48 @@ def test_grid_blocks_that_do_not_all_fit(ws, scenes, nodes, touches, many):
     assert np.isfinite(want).all() and np.abs(want - np.float32([0, 0, 0, 1, 0, 0, 0, 0])).max() > 1e-6
     for i in range(scenes):
         np.testing.assert_array_equal(few.SolvedNodeSE3(i).cpu().numpy(), want)
+
+
+# What a block keeps in shared memory and what it leaves outside, by its budget: at 49152 bytes next to nothing fits
+# (products one item a thread, a ring of four or five buffers, vectors, contributions, words, send lists and
+# inverses in L2), at 228864 everything of the small scenes.
+BUDGETS = (49152, 65536, 100000, 160000, 0)
+
+
+def compare_forms(items, gn, pcg, precision, forms):
+    """Every form and budget against k_pcg, scene by scene."""
+    import torch
+    from starhub_b200 import _lib
+    from starhub_b200.solver import WarpSolver
+    s = WarpSolver(max_nodes=sum(d.num_nodes for d in items), max_pixels=sum(d.num_pixels for d in items),
+                   max_edges=sum(d.num_edges for d in items), max_scenes=len(items), precision=precision)
+    s.SetBatchInputs(items)
+    want = None
+    for form, budget in [(_lib.WS_PCG_STREAMED, 0)] + [(f, b) for f in forms for b in BUDGETS]:
+        s.set_pcg_form(form, budget)
+        assert s.pcg_form() == form
+        s.SolveStreamed(gn, pcg, stream=torch.cuda.Stream())
+        s.Sync()
+        got = [s.SolvedNodeSE3(i).cpu().numpy().copy() for i in range(len(items))]
+        if want is None:
+            want = got
+            assert all(np.isfinite(g).all() for g in got)
+        for i, (a, b) in enumerate(zip(want, got)):
+            np.testing.assert_array_equal(a, b, err_msg=f"form {form}, {budget} bytes, scene {i}")
+
+
+# one group; a partial group; more than 256 rows a cluster block (a thread a row); 512 rows a block; random and band
+@pytest.mark.parametrize("nodes,touches,pcg,precision", [
+    (16, 3, 3, 0), (37, 2, 4, 1), (900, 8, 1, 0), (900, 8, 0, 0), (2500, 3, 6, 0), (2500, 12, 5, 1), (4200, 6, 4, 0),
+    (8192, 2, 3, 0)])
+def test_one_scene_in_every_layout(ws, nodes, touches, pcg, precision):
+    compare_forms([random_scene(nodes, touches, seed=nodes)], 2, pcg, precision, (2, 3))
+
+
+# on the grid: many rows a block (up to 512), blocks of very different lengths, the equal split of the groups; as
+# clusters: more scenes than run at once
+@pytest.mark.parametrize("sizes,touches,pcg,precision", [
+    ([4500] * 9 + [300, 17, 4500], 5, 5, 0), ([8000, 1200, 8000, 40], 9, 4, 1), ([3000, 2000] * 5, 10, 7, 0)])
+def test_batches_in_every_layout(ws, sizes, touches, pcg, precision):
+    by_size = {n: random_scene(n, touches, seed=n) for n in set(sizes)}
+    compare_forms([by_size[n] for n in sizes], 2, pcg, precision, (2, 3))
