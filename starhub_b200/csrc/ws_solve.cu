@@ -2820,33 +2820,38 @@ int pcg_grid_blocks(Scene *scenes, int num_scenes, int most) {
 }
 
 // How the batch's PCG runs.  All three give the same bits; the rule is speed, by what an iteration takes (us,
-// measured with the launch's load phase spread over 20 iterations):
-//   k_pcg            22 + 0.3 per thousand nodes of the batch (21 at 1k nodes, 23 at 4k, 28 at 8k, 71 at 163k);
-//   clusters         3.2 + 2.8 per thousand nodes of a scene (6.3 at 1k, 7.2 at 1.8k, 11.2 at 3k, 20 at 6k, 29 at
-//                    8k), the scenes side by side as far as clusters fit on the device (7 of 16 blocks);
-//   the whole grid   9.2 + 0.045 per row of its fullest block (9.7 at 1k to 3k nodes, 10.6 at 6k, 11.0 at 8k).
-// In ms of 5 x 20 iterations, k_pcg / clusters / grid: lone 1k nodes 2.11 / 0.63 / 0.97, 3k 2.28 / 1.12 / 0.98,
-// 8k 2.80 / 2.95 / 1.10; nodes log-uniform in [500, 8000], 4 scenes 2.86 / 1.89 / 1.22, 16 scenes 3.65 / 2.94 /
-// 2.28, 64 scenes 7.1 / 10.9 / does not fit.
+// measured with the launch's load phase spread over 20 iterations, about 5 upper pairs a row):
+//   k_pcg            22 + 0.3 per thousand nodes of the batch (21 at 1k nodes, 23 at 4k, 28.5 at 8k, 39 at 72k);
+//   clusters         4.4 + 1.5 per thousand nodes of a scene while its matrix fits in shared memory (5.3 at 500 nodes,
+//                    6.2 at 1k, 7.1 at 1.8k), beyond 4.9 + 2.4 (10.1 at 2.3k, 11.1 at 3k, 13.4 at 4k, 18.4 at 5.5k);
+//                    as many scenes side by side as clusters fit on the device (7 of 16 blocks), the others after
+//                    them (1.8k nodes: 7 scenes 7.3, 20 scenes 21.3);
+//   the whole grid   8.9 + 0.041 per row of its fullest block (10.0 at 32 rows, 11.2 at 64, 18 at 224, 22 at 336, 28 at
+//                    448).
+// us an iteration, k_pcg / clusters / grid: lone 1k nodes 21.1 / 6.2 / 10.0, 3k 22.6 / 11.1 / 10.0, 8k 28.6 / 30.1 / 11.2;
+// 7 x 3k 25.5 / 11.3 / 14.6, 8 x 1k 21.2 / 12.3 / 10.4, 8 x 4k 27.8 / 26.9 / 18.7, 8 x 8k 38.4 / 60.8 / 27.8, 20 x 1.8k
+// 30.6 / 21.3 / 18.8, 32 of 500 to 8k 50.8 / 57.3 / does not fit.
 PcgMode pcg_mode(const Workspace &w) {
     if (w.pcg_form == WS_PCG_STREAMED) return PcgMode::kStream;
-    const int size = w.pcg_cluster;
-    double most = 0.0, sum = 0.0, rows = 0.0;
-    bool cluster_fits = size > 0 && w.pcg_clusters_active > 0;
-    for (int s = 0; s < w.num_scenes && s < (int)w.h_scenes.size(); ++s) {
-        const Scene &sc = w.h_scenes[s];
+    const int size = w.pcg_cluster, slots = w.pcg_clusters_active;
+    double rows = 0.0, clusters = 0.0;
+    bool cluster_fits = size > 0 && slots > 0;
+    double busy[64] = {};   // when the places of clusters side by side are free again
+    for (int k = 0; k < w.num_scenes && k < (int)w.h_scenes.size(); ++k) {
+        const Scene &sc = w.h_scenes[w.h_scenes[k].pcg_order];   // the order in which the clusters start
         if (sc.num_chunks > size * (kResRows / kRowsPerGroup)) cluster_fits = false;
-        const double us = (3.2 + 2.8e-3 * sc.num_nodes) * kResMaxCluster / std::max(1, size);
-        most = std::max(most, us);
-        sum += us;
+        const double n = 1e-3 * sc.num_nodes * kResMaxCluster / std::max(1, size);
+        double *place = std::min_element(busy, busy + std::min(std::max(slots, 1), 64));
+        *place += n <= 2.1 ? 4.4 + 1.5 * n : 4.9 + 2.4 * n;
+        clusters = std::max(clusters, *place);
         if (w.pcg_grid_blocks > 0)
             rows = std::max(rows, (double)kRowsPerGroup * ((sc.num_chunks + sc.pcg_blocks - 1) / sc.pcg_blocks));
     }
     if (w.pcg_form == WS_PCG_CLUSTERS) return cluster_fits ? PcgMode::kClusters : PcgMode::kStream;
     if (w.pcg_form == WS_PCG_GRID) return w.pcg_grid_blocks > 0 ? PcgMode::kGrid : PcgMode::kStream;
     const double stream = 22.0 + 0.3e-3 * w.total_nodes;
-    const double clusters = cluster_fits ? std::max(most, sum / w.pcg_clusters_active) : 1e30;
-    const double grid = w.pcg_grid_blocks > 0 ? 9.2 + 0.045 * rows : 1e30;
+    const double grid = w.pcg_grid_blocks > 0 ? 8.9 + 0.041 * rows : 1e30;
+    if (!cluster_fits) clusters = 1e30;
     if (clusters <= grid) return clusters < stream ? PcgMode::kClusters : PcgMode::kStream;
     return grid < stream ? PcgMode::kGrid : PcgMode::kStream;
 }

@@ -42,3 +42,18 @@ def test_streamed_on_request(ws, small_scene, tiny_scene, graph):
         for i in range(2):
             got = s.SolvedNodeSE3(i).cpu().numpy()
             np.testing.assert_array_equal(out.setdefault(i, got.copy()), got, err_msg=f"form {form}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scenes,nodes,form", [(1, 500, 2), (1, 1800, 2), (7, 3000, 2), (1, 8000, 3), (8, 1000, 3),
+                                               (8, 4000, 3), (8, 8000, 3), (40, 4000, 1)])
+def test_form_by_size(ws, scenes, nodes, form):
+    """Scenes that do not fit beside one another run in rounds: eight clusters on a device that holds seven take
+    twice a cluster's time (8 x 8000 nodes: 60.8 us an iteration, 27.8 over the whole grid, 38.4 streamed)."""
+    from starhub_b200.solver import WarpSolver
+    from test_gpu_pcg_layouts import random_scene
+    a = random_scene(nodes, 1)
+    s = WarpSolver(max_nodes=scenes * nodes, max_pixels=scenes * a.num_pixels, max_edges=scenes * a.num_edges,
+                   max_scenes=scenes)
+    s.SetBatchInputs([a] * scenes)
+    assert s.pcg_form() == form
