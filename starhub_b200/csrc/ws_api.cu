@@ -43,7 +43,7 @@ void free_all(ws::Workspace &w) {
                     w.row_entry_first, w.pair_val, w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene, w.half_slot_up,
                     w.half_slot_lo, w.row_cnt_up, w.row_cnt_lo, w.row_first, w.rowptr, w.col_key, w.col_val,
                     w.col_key_alt, w.col_val_alt, w.colidx, w.item_ptr, w.item_info, w.item_col, w.sym_blocks, w.contrib, w.pcg_warp_groups, w.pcg_unit_info, w.pcg_words, w.pcg_send,
-                    w.pcg_send_count, w.pcg_halo, w.pcg_tickets, w.mf_ux, w.inv_diag, w.diag64, w.jtr, w.x, w.r, w.q,
+                    w.pcg_send_count, w.pcg_halo, w.pcg_vec, w.pcg_tickets, w.mf_ux, w.inv_diag, w.diag64, w.jtr, w.x, w.r, w.q,
                     w.sd0, w.sd1, w.se3, w.centers, w.chunk_partial, w.scene_scalars, w.scene_counter,
                     w.error_flag};
     for (void *p : ptrs)
@@ -232,6 +232,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
         A(dalloc(&w.pcg_send, w.cap_items));
         A(dalloc(&w.pcg_send_count, w.cap_nodes));
         A(dalloc(&w.pcg_halo, 16ull * w.cap_scenes + 160));   // kResMaxCluster a scene, or kResMaxBlocks
+        A(dalloc(&w.pcg_vec, w.cap_scenes));
         w.pcg_grid_most = ws::pcg_grid_max(w.device);
         w.pcg_smem = ws::pcg_smem_max();
     }

@@ -104,7 +104,7 @@ __global__ void k_pixel_compact(const Scene *scenes, const uint32_t *tile_scene,
 // Per-scene counts and key/value ranges (term_offset_types.h:62-82 size2offset),
 // computed after the compaction scan.
 __global__ void k_plan(const Scene *scenes, int num_scenes, const uint32_t *tile_offset, int total_tiles,
-                       Plan *plan, uint32_t *counts, uint32_t cap_n2t, uint32_t cap_pair, int *err) {
+                       Plan *plan, uint32_t *counts, uint32_t *pcg_vec, uint32_t cap_n2t, uint32_t cap_pair, int *err) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     uint32_t n2t = 0, pair = 0;
     for (int s = 0; s < num_scenes; ++s) {
@@ -120,6 +120,7 @@ __global__ void k_plan(const Scene *scenes, int num_scenes, const uint32_t *tile
         n2t += p.n2t_count;
         pair += p.pair_count;
         plan[s] = p;
+        pcg_vec[s] = 0;   // raised by k_pcg_plan
     }
     if (n2t > cap_n2t || pair > cap_pair) {
         set_error(err, WS_ERR_CAPACITY);
@@ -754,7 +755,7 @@ void index_build(Workspace &w, cudaStream_t st) {
     // 1. compaction of potential pixels
     k_pixel_count<<<T, kPixTileThreads, 0, st>>>(w.scenes, w.tile_scene, T, w.tile_count);
     count_launch(w, 1 + exclusive_scan(w.tile_count, w.tile_count, (uint32_t)T, w.scan_tmp, st));
-    k_plan<<<1, 32, 0, st>>>(w.scenes, S, w.tile_count, T, w.plan, w.counts, w.cap_n2t, w.cap_pair_kv, w.error_flag);
+    k_plan<<<1, 32, 0, st>>>(w.scenes, S, w.tile_count, T, w.plan, w.counts, w.pcg_vec, w.cap_n2t, w.cap_pair_kv, w.error_flag);
     k_pixel_compact<<<T, kPixTileThreads, 0, st>>>(w.scenes, w.tile_scene, T, w.tile_count, w.d_pixels, w.d_knn,
                                                    w.d_sw, w.d_cw, w.d_scene, w.cap_pixels, w.error_flag);
     count_launch(w, 2);

@@ -84,6 +84,7 @@ struct ResPlan {
     // [cap_nodes] clusters: blocks that hold the row in their halo; grid: lower entries from other blocks
     uint32_t *send_count;
     uint32_t *halo;        // halo rows of each block of the launch
+    uint32_t *vec;         // grid: most own and halo rows of a block, per scene (zero before the plan)
 };
 constexpr int kResMaxBlocks = 160;   // blocks of a scene at most
 
@@ -193,7 +194,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
         uint32_t base = 0;
         for (uint32_t w = 0; w < (tid >> 5); ++w) base += warp_sums[w];
         if (tid < kResNodes / 32) before[tid] = base + inc - n;
-        if (tid == kPlanThreads - 1) P.halo[blockIdx.x] = base + inc;
+        if (tid == kPlanThreads - 1) {
+            P.halo[blockIdx.x] = base + inc;
+            if constexpr (kGrid) atomicMax(P.vec + place.scene, rows + base + inc);
+        }
     }
     __syncthreads();
     for (uint32_t k = tid; k < items; k += kPlanThreads) {
@@ -279,22 +283,32 @@ __device__ __forceinline__ double res_reduce(const PcgArgs &A, const double *par
     return A.fp64 ? v : (double)(float)v;
 }
 
+constexpr uint32_t kResChunkBytes = 32u * 144u;   // matrix blocks of 32 items
+constexpr uint32_t kResMaxRing = 24;
+constexpr uint32_t kResMinLocal = 32u * kResThreads + 4u * kResChunkBytes + 64u;   // product records and a small ring
+
+struct ResShared {
+    ResRanges R;
+    __align__(8) unsigned long long bar, ring[kResMaxRing];
+    volatile uint32_t armed[kResMaxRing];   // copies armed on each ring buffer so far
+    float scalar[2];                        // alpha and beta
+    int left;                               // grid: a wait gave up
+};
+
 // kGrid: a scene's blocks are blocks of a cooperative launch; they meet at a counter in L2 and exchange
 // halos, contributions and partials through L2.
-template <bool kGrid>
-__global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPlan P, uint32_t smem_bytes) {
+// kVec: s and d are in shared memory (1) or in A.sd0 / A.sd1 (0) for all of the scene's blocks, since blocks that
+// have them in shared memory publish s by another way than blocks that have not; -1: a cluster, which sees by its
+// largest block.  (As a run-time answer on the grid it costs registers the kernel has not: frames of 8000 nodes 1780 -> 1820 us.)
+template <bool kGrid, int kVec>
+__device__ __forceinline__ void pcg_resident(const PcgArgs &A, const ResPlan &P, uint32_t smem_bytes, ResShared &S) {
     constexpr uint32_t kThreads = kResThreads, kWarps = kResThreads / 32;
-    constexpr uint32_t kChunkBytes = 32u * 144u;
-    constexpr uint32_t kMaxRing = 24;
+    constexpr uint32_t kChunkBytes = kResChunkBytes, kMaxRing = kResMaxRing, kMinLocal = kResMinLocal;
     extern __shared__ __align__(128) unsigned char res_smem[];
-    __shared__ ResRanges R;
-    __shared__ __align__(8) unsigned long long s_bar, s_ring[kMaxRing];
-    __shared__ volatile uint32_t s_armed[kMaxRing];   // copies armed on each ring buffer so far
-    __shared__ float s_scalar[2];                      // alpha and beta
+    ResRanges &R = S.R;
     const uint32_t tid = threadIdx.x;
     const int lane = tid & 31;
     const uint32_t warp = tid >> 5;
-    __shared__ int s_left;   // grid: a wait gave up
     if constexpr (!kGrid) cluster_arrive();   // every block of the cluster has started once the matching wait returns
     const ResPlace place = res_place<kGrid>(A);
     const uint32_t rank = place.rank, size = place.size;
@@ -318,19 +332,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     // ---- shared memory: first what peers write (the same offsets in every block), then this block's ----
     const uint32_t off_pa = 0, off_pb = 8u * groups;   // clusters: the partials of phases A and B
     uint32_t off = kGrid ? 0u : (16u * groups + 15u) & ~15u;
-    constexpr uint32_t kMinLocal = 32u * kThreads + 4u * kChunkBytes + 64u;   // product records and a small ring
     const uint32_t off_s = off, off_d = off + 24u * vmax;
-    // s and d in shared memory, else in A.sd0 / A.sd1.  One answer for the scene, since blocks that have them there
-    // publish s by another way than blocks that have not: vmax is a cluster's largest; on the grid thread t looks
-    // at the scene's block t
-    bool vec_shared = off + 48u * vmax + kMinLocal <= smem_bytes;
-    if constexpr (kGrid) {
-        static_assert(kResThreads >= kResMaxBlocks, "a thread per block of the scene");
-        if (tid < size)
-            vec_shared = off + 48u * (R.row[tid + 1] - R.row[tid] + __ldg(P.halo + (blockIdx.x - rank + tid))) + kMinLocal <=
-                         smem_bytes;
-        vec_shared = __syncthreads_and(vec_shared);
-    }
+    const bool vec_shared = kVec >= 0 ? kVec != 0 : off + 48u * vmax + kMinLocal <= smem_bytes;
     if (vec_shared) off = (off + 48u * vmax + 15u) & ~15u;
     const uint32_t off_contrib = off;
     const bool contrib_shared = off + 24u * lmax + kMinLocal <= smem_bytes;   // else through A.contrib
@@ -364,29 +367,29 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
     auto stream_chunk = [&](uint32_t n) {
         const uint32_t first = 32u * (resident + n % streamed), bytes = 144u * min(32u, items - first), b = n % ring;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(&s_ring[b])), "r"(bytes)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(&S.ring[b])), "r"(bytes)
                      : "memory");
-        s_armed[b] = n / ring + 1u;
+        S.armed[b] = n / ring + 1u;
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
                          smem_addr(blk_s) + kChunkBytes * (resident + b)),
-                     "l"(A.sym_blocks + 36ull * (item0 + first)), "r"(bytes), "r"(smem_addr(&s_ring[b]))
+                     "l"(A.sym_blocks + 36ull * (item0 + first)), "r"(bytes), "r"(smem_addr(&S.ring[b]))
                      : "memory");
     };
 
     // ---- load: blocks and inverse diagonals by bulk copies, words and send lists by plain loads ----
     if (tid == 0) {
-        bulk_init(&s_bar, 1);
-        if (ring > 0) bulk_init(s_ring, (int)ring);
-        for (uint32_t b = 0; b < kMaxRing; ++b) s_armed[b] = 0;
+        bulk_init(&S.bar, 1);
+        if (ring > 0) bulk_init(S.ring, (int)ring);
+        for (uint32_t b = 0; b < kMaxRing; ++b) S.armed[b] = 0;
         const uint32_t block_bytes = 144u * min(32u * resident, items), bytes = block_bytes + (inv_shared ? 144u * rows : 0u);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(&s_bar)), "r"(bytes)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(&S.bar)), "r"(bytes)
                      : "memory");
         auto copy = [&](const float *src, float *dst, uint32_t n) {   // n bytes, a multiple of 16
             for (uint32_t at = 0; at < n; at += 18432u)
                 asm volatile(
                     "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
                         smem_addr(dst) + at),
-                    "l"(reinterpret_cast<const char *>(src) + at), "r"(min(18432u, n - at)), "r"(smem_addr(&s_bar))
+                    "l"(reinterpret_cast<const char *>(src) + at), "r"(min(18432u, n - at)), "r"(smem_addr(&S.bar))
                     : "memory");
         };
         if (inv_shared) copy(A.inv_diag + 36ull * row0, inv_s, 144u * rows);
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
         load6(A.jtr + 8ull * row, rv);
     }
     __syncthreads();   // the mbarriers are initialised, the words and send lists written
-    if (!bulk_wait(&s_bar, 0) && lane == 0) set_err(A.err, WS_ERR_TIMEOUT);
+    if (!bulk_wait(&S.bar, 0) && lane == 0) set_err(A.err, WS_ERR_TIMEOUT);
 
     // y = M^-1 x of the thread's row
     auto precondition = [&](const float *x, float *y) {
@@ -467,10 +470,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
                     if (!ok && (i & 1023) == 1023 && *reinterpret_cast<volatile int *>(A.err) == WS_ERR_TIMEOUT) break;
                 }
                 if (!ok) set_err(A.err, WS_ERR_TIMEOUT);
-                s_left = ok ? 0 : 1;
+                S.left = ok ? 0 : 1;
             }
             __syncthreads();
-            return s_left == 0;
+            return S.left == 0;
         } else {
             cluster_arrive();
             cluster_wait();
@@ -575,10 +578,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
                     // the copy is armed by the warp that used the buffer before; a parity wait is only
                     // meaningful once it is
                     bool armed = false;
-                    for (int i = 0; i < kBulkMaxPolls && !armed; ++i) armed = s_armed[n % ring] > n / ring;
+                    for (int i = 0; i < kBulkMaxPolls && !armed; ++i) armed = S.armed[n % ring] > n / ring;
                     armed = __all_sync(0xffffffffu, armed);
                     __syncwarp();
-                    if ((!armed || !bulk_wait(&s_ring[n % ring], (n / ring) & 1u)) && lane == 0)
+                    if ((!armed || !bulk_wait(&S.ring[n % ring], (n / ring) & 1u)) && lane == 0)
                         set_err(A.err, WS_ERR_TIMEOUT);
                 }
                 if (valid) {
@@ -708,7 +711,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
             const double dq = reduce(off_pa);
             double alpha64 = dq != 0.0 ? delta / dq : 0.0;
             if (!A.fp64 && dq != 0.0) alpha64 = (double)((float)delta / (float)dq);
-            if (lane == 0) s_scalar[0] = (float)alpha64;
+            if (lane == 0) S.scalar[0] = (float)alpha64;
         }
         // the contributions do not need alpha: summed while the last warp takes it
         if (has_row) {
@@ -758,7 +761,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
         __syncthreads();
         const bool more = it + 1 < A.pcg_iters;
         if (row_warp) {
-            const float alpha = s_scalar[0];
+            const float alpha = S.scalar[0];
             float s[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (has_row) {
 #pragma unroll
@@ -782,22 +785,36 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPl
                 double beta64 = delta != 0.0 ? v / delta : 0.0;
                 if (!A.fp64 && delta != 0.0) beta64 = (double)((float)v / (float)delta);
                 delta = v;
-                if (lane == 0) s_scalar[1] = (float)beta64;
+                if (lane == 0) S.scalar[1] = (float)beta64;
             }
             __syncthreads();
-            beta = s_scalar[1];
+            beta = S.scalar[1];
         }
     }
     if (!here) {   // no block leaves with copies on their way into its shared memory
         if (ring > 0 && tid == 0)
             for (uint32_t b = 0; b < ring; ++b)
-                if (s_armed[b] > 0) bulk_wait_one(&s_ring[b], (s_armed[b] - 1u) & 1u);
+                if (S.armed[b] > 0) bulk_wait_one(&S.ring[b], (S.armed[b] - 1u) & 1u);
         __syncthreads();
         return;
     }
     if (has_row) {
         store6(A.x + 8ull * row, xv);
         twist_update_row(A, row, xv);
+    }
+}
+
+template <bool kGrid>
+__global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPlan P, uint32_t smem_bytes) {
+    __shared__ ResShared S;
+    if constexpr (kGrid) {
+        // the widest of the scene's blocks decides for all of them
+        if (48u * __ldg(P.vec + res_place<true>(A).scene) + kResMinLocal <= smem_bytes)
+            pcg_resident<true, 1>(A, P, smem_bytes, S);
+        else
+            pcg_resident<true, 0>(A, P, smem_bytes, S);
+    } else {
+        pcg_resident<false, -1>(A, P, smem_bytes, S);
     }
 }
 

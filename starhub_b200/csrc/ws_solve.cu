@@ -2862,6 +2862,7 @@ static ResPlan res_plan(Workspace &w) {
     p.send = w.pcg_send;
     p.send_count = w.pcg_send_count;
     p.halo = w.pcg_halo;
+    p.vec = w.pcg_vec;
     return p;
 }
 

@@ -114,6 +114,7 @@ struct Workspace {
     // per row [cap_nodes], halo rows per block [cap_scenes * 16 + 160]
     uint2 *pcg_words = nullptr;
     uint32_t *pcg_send = nullptr, *pcg_send_count = nullptr, *pcg_halo = nullptr;
+    uint32_t *pcg_vec = nullptr;                             // [cap_scenes] zeroed by k_plan
     uint32_t *pcg_tickets = nullptr;                         // [4]: [0] PCG work-unit tickets, zeroed per launch
     float *mf_ux = nullptr;             // matrix-free SpMV scratch: J x per dense term and edge (float4),
                                         // allocated on first use

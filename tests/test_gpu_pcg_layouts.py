@@ -72,14 +72,16 @@ def vector_rows(scene, blocks):
 FITS = (228864 - (32 * 512 + 4 * 4608 + 64)) // 48   # vector rows that fit beside the product records and the ring
 
 
-def solve(items, gn, pcg, precision=0):
+def solve(items, gn, pcg, form):
     import torch
     from starhub_b200.solver import WarpSolver
     s = WarpSolver(max_nodes=sum(d.num_nodes for d in items), max_pixels=sum(d.num_pixels for d in items),
-                   max_edges=sum(d.num_edges for d in items), max_scenes=len(items), precision=precision)
+                   max_edges=sum(d.num_edges for d in items), max_scenes=len(items))
+    s.set_pcg_form(form)
     s.SetBatchInputs(items)
     s.SolveStreamed(gn, pcg, stream=torch.cuda.Stream())
     s.Sync()
+    assert s.pcg_form() == form
     return s
 
 
@@ -91,7 +93,7 @@ def test_grid_blocks_that_do_not_all_fit(ws, scenes, nodes, touches, many):
     blocks = (148 - scenes) // scenes + 1
     v = vector_rows(a, blocks)
     assert (v > FITS).any() and (v <= FITS).any(), (v.max(), v.min())
-    few, k_pcg = solve([a] * scenes, 2, 8), solve([a] * many, 2, 8)
+    few, k_pcg = solve([a] * scenes, 2, 8, 3), solve([a] * many, 2, 8, 1)
     want = k_pcg.SolvedNodeSE3(0).cpu().numpy()
     assert np.isfinite(want).all() and np.abs(want - np.float32([0, 0, 0, 1, 0, 0, 0, 0])).max() > 1e-6
     for i in range(scenes):
