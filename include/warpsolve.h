@@ -446,7 +446,9 @@ int ws_set_tuning(ws_solver *solver, const ws_tuning *tuning);
  * shared_bytes: dynamic shared memory a block of the last two forms may use, 49152 to 228864, 0 = all of it (what
  * does not fit is read from L2). */
 int ws_set_pcg_form(ws_solver *solver, int form, int shared_bytes);
-/* The form (not WS_PCG_AUTO) that a solve of the inputs set takes; WS_ERR_NOT_READY without inputs. */
+/* The form (not WS_PCG_AUTO) that a solve of the inputs set takes; WS_ERR_NOT_READY without inputs.  For some sizes
+ * WS_PCG_AUTO depends on the node pairs, which the device counts: before the inputs' first solve this is then the
+ * form by size, afterwards the one that the last solve took (synchronises its stream). */
 int ws_get_pcg_form(ws_solver *solver, int *form);
 
 /* Library version / build identification. */

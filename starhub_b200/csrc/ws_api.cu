@@ -43,8 +43,8 @@ void free_all(ws::Workspace &w) {
                     w.row_entry_first, w.pair_val, w.half_row, w.half_col, w.half_begin, w.half_end, w.half_scene, w.half_slot_up,
                     w.half_slot_lo, w.row_cnt_up, w.row_cnt_lo, w.row_first, w.rowptr, w.col_key, w.col_val,
                     w.col_key_alt, w.col_val_alt, w.colidx, w.item_ptr, w.item_info, w.item_col, w.sym_blocks, w.contrib, w.pcg_warp_groups, w.pcg_unit_info, w.pcg_words, w.pcg_send,
-                    w.pcg_send_count, w.pcg_halo, w.pcg_vec, w.pcg_tickets, w.mf_ux, w.inv_diag, w.diag64, w.jtr, w.x, w.r, w.q,
-                    w.sd0, w.sd1, w.se3, w.centers, w.chunk_partial, w.scene_scalars, w.scene_counter,
+                    w.pcg_send_count, w.pcg_halo, w.pcg_vec, w.pcg_sync, w.mf_ux, w.inv_diag, w.diag64, w.jtr, w.x, w.r, w.q,
+                    w.sd0, w.sd1, w.se3, w.centers, w.chunk_partial, w.scene_scalars,
                     w.error_flag};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -151,7 +151,7 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     auto A = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     A(dalloc(&w.scenes, w.cap_scenes));
     A(dalloc(&w.plan, w.cap_scenes));
-    A(dalloc(&w.counts, 8));
+    A(dalloc(&w.counts, ws::kCounts));
     A(dalloc(&w.tile_scene, w.cap_tiles));
     A(dalloc(&w.tile_count, w.cap_tiles + 1));
     A(dalloc(&w.node_scene, w.cap_nodes));
@@ -211,22 +211,23 @@ int ws_create(const ws_config *cfg, ws_solver **out) {
     A(dalloc(&w.centers, w.cap_nodes));
     A(dalloc(&w.chunk_partial, 2 * (size_t)w.cap_chunks));
     A(dalloc(&w.scene_scalars, 8ull * w.cap_scenes));
-    A(dalloc(&w.scene_counter, 64ull * w.cap_scenes));
+    A(dalloc(&w.pcg_sync, 64ull * (1 + w.cap_scenes)));
+    w.pcg_tickets = w.pcg_sync;
+    w.scene_counter = w.pcg_sync ? w.pcg_sync + 64 : nullptr;
     A(dalloc(&w.error_flag, 4));
     w.h_tables_bytes = sizeof(ws::Scene) * w.cap_scenes + 4ull * (w.cap_tiles + w.cap_nodes + w.cap_edges + 2ull * w.cap_chunks);
     A(cudaMallocHost(&w.h_tables, w.h_tables_bytes));
     A(cudaEventCreateWithFlags(&w.tables_free, cudaEventDisableTiming));
     if (e == cudaSuccess) {
         A(cudaMemset(w.error_flag, 0, 4 * sizeof(int)));
-        A(cudaMemset(w.counts, 0, 8 * sizeof(uint32_t)));
-        A(cudaMemset(w.scene_counter, 0, 64ull * w.cap_scenes * sizeof(uint32_t)));
+        A(cudaMemset(w.counts, 0, ws::kCounts * sizeof(uint32_t)));
+        A(cudaMemset(w.pcg_sync, 0, 64ull * (1 + w.cap_scenes) * sizeof(uint32_t)));
         A(cudaMemset(w.se3, 0, (size_t)w.cap_nodes * 8 * sizeof(float)));
     }
     if (e == cudaSuccess) {
         w.pcg_grid = ws::pcg_max_blocks(w.device);
         A(dalloc(&w.pcg_warp_groups, (size_t)ws::kPcgUnitsPerWarp * w.pcg_grid * ws::pcg_warps_per_block() + 2));
         A(dalloc(&w.pcg_unit_info, 2 * (size_t)ws::kPcgUnitsPerWarp * w.pcg_grid * ws::pcg_warps_per_block()));
-        A(dalloc(&w.pcg_tickets, 4));
         w.pcg_cluster = ws::pcg_cluster_max(&w.pcg_clusters_active);
         A(dalloc(&w.pcg_words, w.cap_items));
         A(dalloc(&w.pcg_send, w.cap_items));
@@ -475,10 +476,12 @@ int ws_solve_graph(ws_solver *h, int gn_iters, int pcg_iters, void *stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (!st) return WS_ERR_INVALID_ARGUMENT;   // the legacy stream cannot be captured
     w.last_stream = st;
+    const ws::PcgChoice choice = ws::pcg_choice(w);
     const uint64_t key[] = {(uint64_t)gn_iters, (uint64_t)pcg_iters, (uint64_t)w.num_scenes, w.total_nodes,
                             w.total_edges, w.total_tiles, w.total_chunks, (uint64_t)w.node_bits,
                             (uint64_t)w.dense_channels, (uint64_t)ws::pcg_split_group(w),
-                            (uint64_t)ws::pcg_mode(w), (uint64_t)w.pcg_grid_blocks, w.pcg_smem};
+                            (uint64_t)choice.mode, (uint64_t)choice.sure, (uint64_t)choice.rounds,
+                            (uint64_t)w.pcg_grid_blocks, w.pcg_smem};
     constexpr size_t kKey = sizeof(key) / sizeof(key[0]);
     bool same = w.graph_exec && w.graph_key.size() == kKey && std::equal(key, key + kKey, w.graph_key.begin());
     if (same) {
@@ -645,7 +648,7 @@ int ws_set_pcg_form(ws_solver *h, int form, int shared_bytes) {
 int ws_get_pcg_form(ws_solver *h, int *form) {
     if (!h || !form) return WS_ERR_INVALID_ARGUMENT;
     if (!h->w.have_inputs) return WS_ERR_NOT_READY;
-    *form = (int)ws::pcg_mode(h->w);
+    *form = (int)(h->w.have_solution ? ws::pcg_ran(h->w) : ws::pcg_choice(h->w).mode);
     return WS_OK;
 }
 
@@ -701,11 +704,11 @@ int ws_autotune(ws_solver *h, int pcg_iters, void *stream, ws_tuning *out) {
     const int max_per_sm = std::max(1, std::min(8, w.pcg_grid / std::max(1, w.num_sms)));
     int best_b = max_per_sm;
     float bb = 1e30f;
-    if (ws::pcg_mode(w) != ws::PcgMode::kStream) {   // k_pcg does not run these inputs: blocks per SM stays at its bound
+    if (ws::pcg_choice(w).mode != ws::PcgMode::kStream) {   // k_pcg does not run these inputs: blocks per SM stays at its bound
         w.tune.pcg_blocks_per_sm = max_per_sm;
         out->pcg_ms[max_per_sm - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });
     }
-    for (int b = 1; b <= max_per_sm && ws::pcg_mode(w) == ws::PcgMode::kStream; ++b) {
+    for (int b = 1; b <= max_per_sm && ws::pcg_choice(w).mode == ws::PcgMode::kStream; ++b) {
         w.tune.pcg_blocks_per_sm = b;
         ws::pcg_ranges(w, st);
         out->pcg_ms[b - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });

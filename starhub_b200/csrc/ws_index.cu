@@ -130,6 +130,7 @@ __global__ void k_plan(const Scene *scenes, int num_scenes, const uint32_t *tile
     counts[kCntDense] = tile_offset[total_tiles];
     counts[kCntN2T] = n2t;
     counts[kCntPairKV] = pair;
+    counts[kCntPcgCost] = counts[kCntPcgCost + 1] = 0;   // raised by k_pcg_plan
 }
 
 // Node-graph edge endpoints clamped into the scene (an out-of-range id flags WS_ERR_INVALID_ARGUMENT).

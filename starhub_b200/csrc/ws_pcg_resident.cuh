@@ -85,6 +85,10 @@ struct ResPlan {
     uint32_t *send_count;
     uint32_t *halo;        // halo rows of each block of the launch
     uint32_t *vec;         // grid: most own and halo rows of a block, per scene (zero before the plan)
+    // where the device chooses the form (resident_pays; else null): ns an iteration of the launch's slowest block in
+    // phase A and in phase B
+    uint32_t *cost;
+    uint32_t smem;         // bytes that a block of k_pcg_cluster will have
 };
 constexpr int kResMaxBlocks = 160;   // blocks of a scene at most
 
@@ -155,6 +159,29 @@ __device__ __forceinline__ ResPlace res_place(const PcgArgs &A) {
     return p;
 }
 
+// What bounds a block, in ns an iteration: least squares over launches of 1 to 30 scenes of 500 to 8000 nodes with 5 to
+// 30 upper pairs a row, within 15 % of what was measured (5.3 to 180 us).  Phase A: the block's items, on the grid
+// twice beyond some 3900 of them, in a cluster also the products sent to other blocks.
+// Phase B: the contributions that rows read from L2.
+template <bool kGrid>
+__device__ __forceinline__ void res_cost(const ResPlan &P, uint32_t vec_rows, uint32_t items, uint32_t lows,
+                                         uint32_t crossing, uint32_t outside, uint32_t groups) {
+    if (P.cost == nullptr) return;
+    const uint32_t vec = 48u * vec_rows + 35000u + (kGrid ? 0u : 16u * groups);   // beside records and a small ring
+    const bool vec_fits = vec <= P.smem, low_fits = vec + 24u * lows <= P.smem;
+    const float i = (float)items;
+    float a, b;
+    if (kGrid) {
+        a = 7.f * i + 7.2f * fmaxf(i - 3900.f, 0.f) + (vec_fits ? 0.f : 6.f * i);
+        b = 4.8f * (float)outside + (low_fits ? 0.f : 0.6f * (float)lows);
+    } else {
+        a = 3.5f * i + 6.5f * (float)crossing + (vec + 24u * lows + 144u * items > P.smem ? 2500.f : 0.f);
+        b = low_fits ? 0.f : 4.6f * (float)lows;
+    }
+    atomicMax(P.cost, (uint32_t)a);
+    atomicMax(P.cost + 1, (uint32_t)b);
+}
+
 // Item words, halos and send lists of every block, once per solve (the structure is the same in every
 // Gauss-Newton iteration).  One cluster per scene, ranks as in k_pcg_cluster.  A block's halo is a bit
 // per scene row; a row's index in it is the number of set bits before it.  A row's lower entries name
@@ -163,6 +190,7 @@ template <bool kGrid>
 __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint32_t *colidx, ResPlan P) {
     __shared__ ResRanges R;
     __shared__ uint32_t bits[kResNodes / 32], before[kResNodes / 32], first_item[kResRows], warp_sums[kPlanThreads / 32];
+    __shared__ uint32_t s_crossing, s_outside;   // items with a column in another block, contributions from other blocks
     static_assert(kResNodes / 32 <= kPlanThreads, "a thread per bitmap word");
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     const ResPlace place = res_place<kGrid>(A);
@@ -172,13 +200,17 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
     res_ranges(A, nb, nn, (uint32_t)sc.num_chunks, size, R);
     const uint32_t row0 = R.row[rank], row1 = R.row[rank + 1], rows = row1 - row0;
     const uint32_t item0 = R.item[rank], items = R.item[rank + 1] - item0;
+    if (tid == 0) s_crossing = s_outside = 0;
     if (tid < kResNodes / 32) bits[tid] = 0;
     for (uint32_t r = tid; r < rows; r += kPlanThreads) first_item[r] = min(A.item_ptr[row0 + r], A.cap_items) - item0;
     __syncthreads();
     auto column = [&](uint32_t word) { return min(max(word & ~kItemRowStart, nb), nb + nn - 1); };
     for (uint32_t k = tid; k < items; k += kPlanThreads) {
         const uint32_t col = column(__ldg(A.item_col + item0 + k));
-        if (col < row0 || col >= row1) atomicOr(&bits[(col - nb) >> 5], 1u << ((col - nb) & 31u));
+        const bool crosses = col < row0 || col >= row1;
+        if (crosses) atomicOr(&bits[(col - nb) >> 5], 1u << ((col - nb) & 31u));
+        const unsigned active = __activemask(), crossing = __ballot_sync(active, crosses);
+        if (P.cost != nullptr && lane == (uint32_t)__ffs(active) - 1u) atomicAdd(&s_crossing, (uint32_t)__popc(crossing));
     }
     __syncthreads();
     {   // halo rows before each bitmap word
@@ -226,11 +258,23 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
             uint32_t outside = 0;   // columns ascend, so those of other blocks come first
             while (outside < n && q0 + 1u + outside < A.cap_blocks && __ldg(colidx + q0 + 1u + outside) < row0) ++outside;
             P.send_count[row0 + r] = outside;
+            if (P.cost != nullptr) atomicAdd(&s_outside, outside);
         }
+        __syncthreads();
+        if (tid == 0) res_cost<kGrid>(P, rows + P.halo[blockIdx.x], items, R.low[rank + 1] - R.low[rank], s_crossing, s_outside,
+                                      (uint32_t)sc.num_chunks);
         return;
     }
     cluster_arrive();
     cluster_wait();   // every block's bitmap is complete
+    if (tid == 0) {   // a cluster lays its blocks out alike: by its most vector rows and contributions
+        uint32_t most = 0, lows = 0;
+        for (uint32_t k = 0; k < size; ++k) {
+            most = max(most, R.row[k + 1] - R.row[k] + __ldcg(P.halo + (blockIdx.x - rank + k)));
+            lows = max(lows, R.low[k + 1] - R.low[k]);
+        }
+        res_cost<kGrid>(P, most, items, lows, s_crossing, 0, (uint32_t)sc.num_chunks);
+    }
     for (uint32_t r = tid; r < rows; r += kPlanThreads) {
         const uint32_t row = row0 + r, c = row - nb;
         const uint32_t q0 = A.rowptr[row], p0 = A.item_ptr[row];
@@ -807,6 +851,7 @@ __device__ __forceinline__ void pcg_resident(const PcgArgs &A, const ResPlan &P,
 template <bool kGrid>
 __global__ void __launch_bounds__(kResThreads, 1) k_pcg_cluster(PcgArgs A, ResPlan P, uint32_t smem_bytes) {
     __shared__ ResShared S;
+    if (A.cost != nullptr && !resident_pays(A)) return;   // k_pcg runs
     if constexpr (kGrid) {
         // the widest of the scene's blocks decides for all of them
         if (48u * __ldg(P.vec + res_place<true>(A).scene) + kResMinLocal <= smem_bytes)

@@ -1343,7 +1343,28 @@ struct PcgArgs {
     const float4 *centers;
     int pcg_iters;
     int fp64;                 // FP64 reductions and node-centred twists
+    // where the device chooses between a resident form and k_pcg (else null): the costs that k_pcg_plan found
+    const uint32_t *cost;
+    uint32_t cost_base, cost_rounds;   // ns; in 1024ths
 };
+
+// Whether a batch's resident form (k_pcg_cluster) is faster than k_pcg, in ns an iteration.  The host does not know
+// how many node pairs the rows have; k_pcg_plan does: it leaves the largest costs of a block in phase A and phase B
+// (res_cost), beside `base` for the meetings.  k_pcg: 11 us, 2 for every upper pair a row (the chains of the row sums)
+// and 36 ns per thousand items of the batch.  us an iteration, k_pcg and the form by size, at 5 pairs a row (a
+// surface) / 7.5 / 15 / 30 (pairs anywhere in the scene): 4 x 8000 on the grid 32.2 17.4 / 38.4 33.9 / 59.3 105 / 99.9
+// 239; 16 x 4500 on the grid 39.2 36.1 / 48.2 95.5 / 82.8 236 / 148 546; 4 x 3000 in clusters 24 11.1 / 29.0 20.3 /
+// 47.2 86.9 / 81.2 144.  In whole numbers, since both kernels and the host have to come to the same answer.
+__host__ __device__ inline bool resident_pays(uint32_t base, uint32_t rounds_1024, uint32_t phase_a, uint32_t phase_b,
+                                              uint32_t items, uint32_t nodes) {
+    const unsigned long long it = items, n = nodes > 0 ? nodes : 1u, resident = (unsigned long long)base + phase_a + phase_b;
+    // 6 % in favour of the form by size: large batches of surface scenes are near the line, and on its side
+    return (rounds_1024 * resident * 94ull / 100ull) >> 10 <= 11000ull + (it > n ? 2000ull * (it - n) / n : 0ull) + 36ull * it / 1000ull;
+}
+__device__ __forceinline__ bool resident_pays(const PcgArgs &A) {
+    return resident_pays(A.cost_base, A.cost_rounds, __ldg(A.cost), __ldg(A.cost + 1), __ldg(A.item_ptr + A.total_nodes),
+                         A.total_nodes);
+}
 
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;   // requested sleep, about two seconds
 constexpr int kSceneSync = 64;        // words per scene in scene_counter (tickets and generations on separate lines)
@@ -2026,6 +2047,7 @@ __device__ __forceinline__ void twist_update_row(const PcgArgs &A, uint32_t row,
 
 __global__ void __launch_bounds__(kPcgThreads, 3) k_pcg(PcgArgs A) {
     extern __shared__ __align__(16) float pcg_smem[];
+    if (A.cost != nullptr && resident_pays(A)) return;   // the resident form has run
     const int lane = threadIdx.x & 31;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     float *wsm = pcg_smem + (threadIdx.x >> 5) * kPcgWarpFloats;
@@ -2686,7 +2708,7 @@ uint32_t pcg_split_group(const Workspace &w) {
 }
 
 static PcgArgs pcg_args(Workspace &w, int pcg_iters) {
-    PcgArgs a;
+    PcgArgs a{};
     a.scenes = w.scenes;
     a.group_scene = w.chunk_scene;
     a.group_row = w.chunk_row;
@@ -2831,33 +2853,61 @@ int pcg_grid_blocks(Scene *scenes, int num_scenes, int most) {
 // us an iteration, k_pcg / clusters / grid: lone 1k nodes 21.1 / 6.2 / 10.0, 3k 22.6 / 11.1 / 10.0, 8k 28.6 / 30.1 / 11.2;
 // 7 x 3k 25.5 / 11.3 / 14.6, 8 x 1k 21.2 / 12.3 / 10.4, 8 x 4k 27.8 / 26.9 / 18.7, 8 x 8k 38.4 / 60.8 / 27.8, 20 x 1.8k
 // 30.6 / 21.3 / 18.8, 32 of 500 to 8k 50.8 / 57.3 / does not fit.
-PcgMode pcg_mode(const Workspace &w) {
-    if (w.pcg_form == WS_PCG_STREAMED) return PcgMode::kStream;
+// Rows with many pairs make the resident forms slow (what does not fit in shared memory, and contributions from
+// other blocks).  Up to kSureRows a block of the grid and kSureNodes a cluster (all of a surface's matrix in shared
+// memory) the size decides: with 15 pairs a row anywhere in the scene those are still 0.4 to 1.1 of k_pcg's time.
+// Beyond, both kernels are launched and the device says which one runs (resident_pays), for the 5 us of a launch that
+// ends at once, in 200 us or more.
+constexpr int kSureNodes = 2100, kSureRows = 96;
+PcgChoice pcg_choice(const Workspace &w) {
+    constexpr PcgChoice stream_only{PcgMode::kStream, true, 1024};
+    if (w.pcg_form == WS_PCG_STREAMED) return stream_only;
     const int size = w.pcg_cluster, slots = w.pcg_clusters_active;
-    double rows = 0.0, clusters = 0.0;
+    double rows = 0.0, clusters = 0.0, largest = 0.0;
+    int nodes = 0;
     bool cluster_fits = size > 0 && slots > 0;
     double busy[64] = {};   // when the places of clusters side by side are free again
     for (int k = 0; k < w.num_scenes && k < (int)w.h_scenes.size(); ++k) {
         const Scene &sc = w.h_scenes[w.h_scenes[k].pcg_order];   // the order in which the clusters start
         if (sc.num_chunks > size * (kResRows / kRowsPerGroup)) cluster_fits = false;
+        nodes = std::max(nodes, sc.num_nodes);
         const double n = 1e-3 * sc.num_nodes * kResMaxCluster / std::max(1, size);
+        const double us = n <= 2.1 ? 4.4 + 1.5 * n : 4.9 + 2.4 * n;
         double *place = std::min_element(busy, busy + std::min(std::max(slots, 1), 64));
-        *place += n <= 2.1 ? 4.4 + 1.5 * n : 4.9 + 2.4 * n;
+        *place += us;
+        largest = std::max(largest, us);
         clusters = std::max(clusters, *place);
         if (w.pcg_grid_blocks > 0)
             rows = std::max(rows, (double)kRowsPerGroup * ((sc.num_chunks + sc.pcg_blocks - 1) / sc.pcg_blocks));
     }
-    if (w.pcg_form == WS_PCG_CLUSTERS) return cluster_fits ? PcgMode::kClusters : PcgMode::kStream;
-    if (w.pcg_form == WS_PCG_GRID) return w.pcg_grid_blocks > 0 ? PcgMode::kGrid : PcgMode::kStream;
+    const PcgChoice by_clusters{PcgMode::kClusters, nodes <= kSureNodes, (uint32_t)(1024.0 * clusters / std::max(largest, 1.0))};
+    const PcgChoice by_grid{PcgMode::kGrid, rows <= kSureRows, 1024};
+    if (w.pcg_form == WS_PCG_CLUSTERS) return cluster_fits ? PcgChoice{PcgMode::kClusters, true, 1024} : stream_only;
+    if (w.pcg_form == WS_PCG_GRID) return w.pcg_grid_blocks > 0 ? PcgChoice{PcgMode::kGrid, true, 1024} : stream_only;
     const double stream = 22.0 + 0.3e-3 * w.total_nodes;
     const double grid = w.pcg_grid_blocks > 0 ? 8.9 + 0.041 * rows : 1e30;
     if (!cluster_fits) clusters = 1e30;
-    if (clusters <= grid) return clusters < stream ? PcgMode::kClusters : PcgMode::kStream;
-    return grid < stream ? PcgMode::kGrid : PcgMode::kStream;
+    if (std::min(clusters, grid) >= stream) return stream_only;
+    return clusters <= grid ? by_clusters : by_grid;
 }
 
-static ResPlan res_plan(Workspace &w) {
+// ns of an iteration beside the blocks' work: the meetings and the scalars.
+static uint32_t pcg_base_cost(PcgMode mode) { return mode == PcgMode::kGrid ? 6400u : 3200u; }
+
+PcgMode pcg_ran(Workspace &w) {
+    const PcgChoice c = pcg_choice(w);
+    uint32_t cost[2] = {0, 0}, items = 0;
+    if (c.mode == PcgMode::kStream || c.sure || cudaStreamSynchronize(w.last_stream) != cudaSuccess ||
+        cudaMemcpy(cost, w.counts + kCntPcgCost, sizeof(cost), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(&items, w.item_ptr + w.total_nodes, sizeof(items), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return c.mode;
+    return resident_pays(pcg_base_cost(c.mode), c.rounds, cost[0], cost[1], items, w.total_nodes) ? c.mode : PcgMode::kStream;
+}
+
+static ResPlan res_plan(Workspace &w, const PcgChoice &c) {
     ResPlan p;
+    p.cost = c.sure ? nullptr : w.counts + kCntPcgCost;
+    p.smem = w.pcg_smem;
     p.words = w.pcg_words;
     p.send = w.pcg_send;
     p.send_count = w.pcg_send_count;
@@ -2869,44 +2919,50 @@ static ResPlan res_plan(Workspace &w) {
 // Work distribution of the PCG, after the block CSR: the item words, halos and send lists of
 // k_pcg_cluster.
 cudaError_t pcg_plan(Workspace &w, cudaStream_t st) {
-    const PcgMode mode = pcg_mode(w);
-    if (mode == PcgMode::kStream) return cudaSuccess;
+    const PcgChoice c = pcg_choice(w);
+    if (c.mode == PcgMode::kStream) return cudaSuccess;
     const PcgArgs a = pcg_args(w, 0);
     count_launch(w);
-    if (mode == PcgMode::kGrid) {
-        k_pcg_plan<true><<<w.pcg_grid_blocks, kPlanThreads, 0, st>>>(a, w.colidx, res_plan(w));
+    if (c.mode == PcgMode::kGrid) {
+        k_pcg_plan<true><<<w.pcg_grid_blocks, kPlanThreads, 0, st>>>(a, w.colidx, res_plan(w, c));
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
     cluster_launch(cfg, attr, w.pcg_cluster, w.num_scenes, kPlanThreads, 0, st);
-    return cudaLaunchKernelEx(&cfg, k_pcg_plan<false>, a, (const uint32_t *)w.colidx, res_plan(w));
+    return cudaLaunchKernelEx(&cfg, k_pcg_plan<false>, a, (const uint32_t *)w.colidx, res_plan(w, c));
 }
 
 cudaError_t gn_pcg(Workspace &w, int pcg_iters, cudaStream_t st) {
     PcgArgs a = pcg_args(w, pcg_iters);
-    const PcgMode mode = pcg_mode(w);
-    if (mode == PcgMode::kClusters) {
+    const PcgChoice c = pcg_choice(w);
+    ResPlan plan = res_plan(w, c);
+    if (!c.sure) {
+        a.cost = plan.cost;
+        a.cost_base = pcg_base_cost(c.mode);
+        a.cost_rounds = c.rounds;
+    }
+    // the counters that the blocks meet at, and those of k_pcg: each launch that uses them starts from zero, so one
+    // that timed out half-way cannot leak into the next
+    if (c.mode != PcgMode::kClusters || !c.sure)
+        cudaMemsetAsync(w.pcg_sync, 0, sizeof(uint32_t) * kSceneSync * (1 + (size_t)w.num_scenes), st);
+    cudaError_t e = cudaSuccess;
+    if (c.mode == PcgMode::kClusters) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr{};
-        count_launch(w);
         cluster_launch(cfg, attr, w.pcg_cluster, w.num_scenes, kResThreads, w.pcg_smem, st);
-        return cudaLaunchKernelEx(&cfg, k_pcg_cluster<false>, a, res_plan(w), w.pcg_smem);
-    }
-    if (mode == PcgMode::kGrid) {
-        cudaMemsetAsync(w.scene_counter, 0, sizeof(uint32_t) * kSceneSync * (size_t)w.num_scenes, st);
-        ResPlan plan = res_plan(w);
+        e = cudaLaunchKernelEx(&cfg, k_pcg_cluster<false>, a, plan, w.pcg_smem);
+    } else if (c.mode == PcgMode::kGrid) {
         uint32_t smem = w.pcg_smem;
         void *args[] = {&a, &plan, &smem};
+        e = cudaLaunchCooperativeKernel((const void *)k_pcg_cluster<true>, dim3((unsigned)w.pcg_grid_blocks),
+                                        dim3(kResThreads), args, smem, st);
+    }
+    if (c.mode != PcgMode::kStream) {
         count_launch(w);
-        return cudaLaunchCooperativeKernel((const void *)k_pcg_cluster<true>, dim3((unsigned)w.pcg_grid_blocks),
-                                           dim3(kResThreads), args, smem, st);
+        if (c.sure || e != cudaSuccess) return e;
     }
     const int grid = pcg_launch_blocks(w);
-    // tickets and generations start at zero every launch, so a launch that timed out half-way
-    // cannot leak into the next
-    cudaMemsetAsync(w.scene_counter, 0, sizeof(uint32_t) * kSceneSync * (size_t)w.num_scenes, st);
-    cudaMemsetAsync(w.pcg_tickets, 0, sizeof(uint32_t), st);
     void *args[] = {&a};
     count_launch(w);
     return cudaLaunchCooperativeKernel((const void *)k_pcg, dim3(grid), dim3(kPcgThreads), args, kPcgSmemBytes, st);

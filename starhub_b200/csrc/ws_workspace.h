@@ -115,7 +115,9 @@ struct Workspace {
     uint2 *pcg_words = nullptr;
     uint32_t *pcg_send = nullptr, *pcg_send_count = nullptr, *pcg_halo = nullptr;
     uint32_t *pcg_vec = nullptr;                             // [cap_scenes] zeroed by k_plan
-    uint32_t *pcg_tickets = nullptr;                         // [4]: [0] PCG work-unit tickets, zeroed per launch
+    // [(1 + cap_scenes) * 64], zeroed by one memset before a launch that meets by them: [0] PCG work-unit tickets, then
+    // the scenes' counters
+    uint32_t *pcg_sync = nullptr, *pcg_tickets = nullptr;
     float *mf_ux = nullptr;             // matrix-free SpMV scratch: J x per dense term and edge (float4),
                                         // allocated on first use
 
@@ -176,7 +178,13 @@ int pcg_grid_blocks(Scene *scenes, int num_scenes, int most);
 uint32_t pcg_smem_max();
 uint32_t pcg_smem_min();
 enum class PcgMode { kStream = WS_PCG_STREAMED, kClusters = WS_PCG_CLUSTERS, kGrid = WS_PCG_GRID };
-PcgMode pcg_mode(const Workspace &w);
+struct PcgChoice {
+    PcgMode mode;
+    bool sure;      // by size alone; else the device compares the mode with k_pcg, once it knows the node pairs
+    uint32_t rounds;   // clusters: the batch's time over that of its largest scene, in 1024ths
+};
+PcgChoice pcg_choice(const Workspace &w);
+PcgMode pcg_ran(Workspace &w);   // the mode of the last solve (synchronises its stream where the device chose)
 cudaError_t pcg_plan(Workspace &w, cudaStream_t st);
 int pcg_launch_blocks(const Workspace &w);
 void pcg_ranges(Workspace &w, cudaStream_t st);
@@ -204,6 +212,7 @@ inline uint64_t scene_pixels(const Workspace &w) {
 }
 
 // Counters slot indices.
-enum { kCntDense = 0, kCntN2T = 1, kCntPairKV = 2, kCntHalf = 3, kCntPairValid = 4, kCntTicket = 6 /* 2 */ };
+enum { kCntDense = 0, kCntN2T = 1, kCntPairKV = 2, kCntHalf = 3, kCntPairValid = 4, kCntTicket = 6 /* 2 */,
+       kCntPcgCost = 8 /* 2 */, kCounts = 10 };
 
 }  // namespace ws

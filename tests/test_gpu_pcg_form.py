@@ -57,3 +57,36 @@ def test_form_by_size(ws, scenes, nodes, form):
                    max_scenes=scenes)
     s.SetBatchInputs([a] * scenes)
     assert s.pcg_form() == form
+
+
+# touches: 1 gives about 4.5 upper pairs a row, 8 about 15, anywhere in the scene
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("sizes,sparse,dense", [([4000] * 8, 3, 1), ([8000, 3000] * 3, 3, 1), ([3000] * 4, 2, 1)])
+def test_form_by_pairs(ws, sizes, sparse, dense, graph):
+    """Where the size does not settle it, the device takes the streamed form for rows with many pairs (16 x 4500 nodes
+    with 15 pairs a row: 238 us an iteration over the whole grid, 83 streamed); one solver meets both."""
+    import torch
+    from starhub_b200 import _lib
+    from starhub_b200.solver import WarpSolver
+    from test_gpu_pcg_layouts import random_scene
+    by_size = {(n, t): random_scene(n, t) for n in set(sizes) for t in (1, 10)}
+    most = [by_size[n, 10] for n in sizes]
+    stream = torch.cuda.Stream()
+    s = WarpSolver(max_nodes=sum(sizes), max_pixels=sum(a.num_pixels for a in most),
+                   max_edges=sum(a.num_edges for a in most), max_scenes=len(sizes))
+    for touches, form in ((10, dense), (1, sparse), (10, dense)):
+        items = [by_size[n, touches] for n in sizes]
+        out = []
+        for ask in (_lib.WS_PCG_AUTO, _lib.WS_PCG_STREAMED):
+            s.set_pcg_form(ask)
+            s.SetBatchInputs(items)
+            for _ in range(2):
+                s.SolveStreamed(2, 3, stream=stream, graph=graph)
+            s.Sync()
+            if ask == _lib.WS_PCG_AUTO:
+                assert s.pcg_form() == form, touches
+            out.append([s.SolvedNodeSE3(i).cpu().numpy().copy() for i in range(len(items))])
+        for a, b in zip(*out):
+            assert np.isfinite(a).all()
+            np.testing.assert_array_equal(a, b)
