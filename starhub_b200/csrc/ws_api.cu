@@ -704,16 +704,16 @@ int ws_autotune(ws_solver *h, int pcg_iters, void *stream, ws_tuning *out) {
     const int max_per_sm = std::max(1, std::min(8, w.pcg_grid / std::max(1, w.num_sms)));
     int best_b = max_per_sm;
     float bb = 1e30f;
-    if (ws::pcg_choice(w).mode != ws::PcgMode::kStream) {   // k_pcg does not run these inputs: blocks per SM stays at its bound
-        w.tune.pcg_blocks_per_sm = max_per_sm;
-        out->pcg_ms[max_per_sm - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });
-    }
-    for (int b = 1; b <= max_per_sm && ws::pcg_choice(w).mode == ws::PcgMode::kStream; ++b) {
+    // blocks per SM of k_pcg, also where these inputs run resident: later inputs may not
+    const int form = w.pcg_form;
+    w.pcg_form = WS_PCG_STREAMED;
+    for (int b = 1; b <= max_per_sm; ++b) {
         w.tune.pcg_blocks_per_sm = b;
         ws::pcg_ranges(w, st);
         out->pcg_ms[b - 1] = time_ms([&] { ws::gn_pcg(w, pcg_iters, st); });
         if (out->pcg_ms[b - 1] < bb) { bb = out->pcg_ms[b - 1]; best_b = b; }
     }
+    w.pcg_form = form;
     w.tune.pcg_blocks_per_sm = best_b;
     w.tune.tuned = true;
     ws::pcg_ranges(w, st);
