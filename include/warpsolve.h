@@ -132,6 +132,13 @@ int ws_spmv(ws_solver *solver, const float *x, float *y, void *stream);
  * WS_ERR_TIMEOUT after about two seconds of requested sleep when the bound works (the device
  * stays usable), WS_ERR_CUDA if a CUDA call fails.  Synchronises `stream`. */
 int ws_selftest_wait_timeout(void *stream);
+/* Failure-detection self-test of the waits of the PCG over the whole device (ws_set_pcg_form), no reference
+ * counterpart: a wait for a copy that nobody started, and the PCG of the last solve's system launched without its
+ * last block, so that the others' meeting runs out and they leave.  Returns WS_ERR_TIMEOUT after a few seconds when
+ * the bounds work (the device stays usable), WS_OK if a wait ended otherwise, WS_ERR_NOT_READY before a solve or for
+ * a batch that does not take that form.  The solution is lost; the next solve starts as usual.  Synchronises
+ * `stream`. */
+int ws_selftest_resident_timeout(ws_solver *solver, void *stream);
 /* Failure-detection self-test of the wait that node construction and growth use in their overlap
  * check (ws_init_nodes, ws_expand_nodes), where a candidate waits for the decisions on earlier
  * ones; no reference counterpart (the reference runs that check on the host).  A candidate waits

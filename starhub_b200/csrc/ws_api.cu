@@ -595,6 +595,21 @@ int ws_selftest_wait_timeout(void *stream) {
     return status == 0 ? WS_OK : status;
 }
 
+int ws_selftest_resident_timeout(ws_solver *h, void *stream) {
+    if (!h) return WS_ERR_INVALID_ARGUMENT;
+    ws::Workspace &w = h->w;
+    if (!w.have_solution) return WS_ERR_NOT_READY;
+    cudaSetDevice(w.device);
+    int status = 0;
+    if (w.last_stream) cudaStreamSynchronize(w.last_stream);
+    if (ws::pcg_resident_selftest(w, &status, (cudaStream_t)stream) != cudaSuccess) {
+        cudaGetLastError();
+        return WS_ERR_CUDA;
+    }
+    if (status != WS_ERR_NOT_READY) w.have_solution = false;   // some scenes' warps were updated, others not
+    return status;
+}
+
 int ws_selftest_grid_barrier_timeout(void *stream) {
     int flags = 0;
     if (ws::dedup_wait_selftest(&flags, (cudaStream_t)stream) != cudaSuccess) return WS_ERR_CUDA;

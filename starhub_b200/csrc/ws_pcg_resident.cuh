@@ -297,15 +297,25 @@ __global__ void __launch_bounds__(kPlanThreads) k_pcg_plan(PcgArgs A, const uint
     cluster_wait();   // no block leaves while another reads its bitmap
 }
 
-// One thread's bounded wait for phase `parity` of `bar`.
-__device__ __forceinline__ void bulk_wait_one(unsigned long long *bar, unsigned parity) {
+// One thread's bounded wait for phase `parity` of `bar`; false when the polls ran out.
+__device__ __forceinline__ bool bulk_wait_one(unsigned long long *bar, unsigned parity, int polls = kBulkMaxPolls) {
     unsigned done = 0;
-    for (int i = 0; i < kBulkMaxPolls && done == 0; ++i)
+    for (int i = 0; i < polls && done == 0; ++i)
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(done)
                      : "r"(smem_addr(bar)), "r"(parity)
                      : "memory");
+    return done != 0;
+}
+
+// Self-test: a wait for a copy that nobody has started runs out.
+__global__ void k_bulk_wait_selftest(int *err) {
+    __shared__ __align__(8) unsigned long long bar;
+    if (threadIdx.x == 0) {
+        bulk_init(&bar, 1);
+        if (!bulk_wait_one(&bar, 0, 256)) set_err(err, WS_ERR_TIMEOUT);
+    }
 }
 
 // Sum of a scene's group partials in the order of reduce_scene, eight of a lane's loads at a time.

@@ -2987,6 +2987,37 @@ cudaError_t gn_spmv_matrix_free(Workspace &w, const float *x, float *y, float *u
     return cudaGetLastError();
 }
 
+cudaError_t pcg_resident_selftest(Workspace &w, int *status, cudaStream_t st) {
+    *status = WS_ERR_NOT_READY;
+    const int form = w.pcg_form;
+    w.pcg_form = WS_PCG_GRID;
+    const PcgChoice c = pcg_choice(w);
+    cudaError_t e = cudaSuccess;
+    if (c.mode == PcgMode::kGrid && w.h_scenes[w.num_scenes - 1].pcg_blocks > 1) {
+        // what the launches leave in the error flag: first of the copy's wait, then of the meeting
+        int flag[2] = {0, 0};
+        auto A = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+        A(cudaMemsetAsync(w.error_flag, 0, sizeof(int), st));
+        k_bulk_wait_selftest<<<1, 32, 0, st>>>(w.error_flag);
+        A(cudaGetLastError());
+        A(cudaMemcpyAsync(&flag[0], w.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        A(cudaMemsetAsync(w.error_flag, 0, sizeof(int), st));
+        A(cudaMemsetAsync(w.pcg_vec, 0, sizeof(uint32_t) * w.num_scenes, st));
+        A(pcg_plan(w, st));
+        A(cudaMemsetAsync(w.pcg_sync, 0, sizeof(uint32_t) * kSceneSync * (1 + (size_t)w.num_scenes), st));
+        if (e == cudaSuccess) {   // every block but the last
+            k_pcg_cluster<true><<<w.pcg_grid_blocks - 1, kResThreads, w.pcg_smem, st>>>(pcg_args(w, 3), res_plan(w, c), w.pcg_smem);
+            A(cudaGetLastError());
+        }
+        A(cudaMemcpyAsync(&flag[1], w.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        A(cudaMemsetAsync(w.error_flag, 0, sizeof(int), st));
+        A(cudaStreamSynchronize(st));
+        *status = flag[0] == WS_ERR_TIMEOUT && flag[1] == WS_ERR_TIMEOUT ? WS_ERR_TIMEOUT : WS_OK;
+    }
+    w.pcg_form = form;
+    return e;
+}
+
 cudaError_t gn_spmv(Workspace &w, const float *x, float *y, cudaStream_t st) {
     const PcgArgs a = pcg_args(w, 0);
     const cudaError_t attr =

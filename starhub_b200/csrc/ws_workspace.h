@@ -193,6 +193,9 @@ uint32_t pcg_split_group(const Workspace &w);
 cudaError_t gn_spmv(Workspace &w, const float *x, float *y, cudaStream_t st);
 // Runs the PCG's bounded scene wait on a generation nothing advances; *status gets the flag it left.
 cudaError_t pcg_wait_selftest(int *status, cudaStream_t st);
+// Runs the waits of the PCG over the whole grid out: *status gets WS_ERR_TIMEOUT when both gave up as they should,
+// WS_ERR_NOT_READY where the batch does not take that form with two blocks or more in its last scene.
+cudaError_t pcg_resident_selftest(Workspace &w, int *status, cudaStream_t st);
 cudaError_t dedup_wait_selftest(int *flags, cudaStream_t st);
 cudaError_t gn_spmv_matrix_free(Workspace &w, const float *x, float *y, float *ux_dense, float *ux_reg,
                                 cudaStream_t st);

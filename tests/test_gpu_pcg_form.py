@@ -90,3 +90,30 @@ def test_form_by_pairs(ws, sizes, sparse, dense, graph):
         for a, b in zip(*out):
             assert np.isfinite(a).all()
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("budget", [0, 49152])   # without and with a ring whose copies are on their way
+def test_resident_waits_give_up_and_the_device_stays_usable(ws, small_scene_k8, budget):
+    """The waits of the PCG over the whole grid are bounded: for a copy that nobody starts, and at a meeting that one
+    block never reaches, where the others leave with WS_ERR_TIMEOUT.  A solve afterwards equals one before."""
+    import time
+    import torch
+    from starhub_b200 import _lib
+    from starhub_b200.solver import DeviceScene, WarpSolver
+    ds = DeviceScene.from_scene(small_scene_k8)
+    s = WarpSolver(max_nodes=ds.num_nodes, max_pixels=ds.num_pixels, max_edges=ds.num_edges)
+    s.set_pcg_form(_lib.WS_PCG_GRID, budget)
+    s.SetSolverInputs(ds)
+    lib, stream = _lib.load(), torch.cuda.Stream()
+    assert lib.ws_selftest_resident_timeout(s._h, None) == _lib.WS_ERR_NOT_READY
+    out = []
+    for _ in range(2):
+        s.SolveStreamed(2, 6, stream=stream)
+        s.Sync()
+        out.append(s.SolvedNodeSE3(0).cpu().numpy().copy())
+        if len(out) == 1:
+            t0 = time.perf_counter()
+            assert lib.ws_selftest_resident_timeout(s._h, C.c_void_p(stream.cuda_stream)) == _lib.WS_ERR_TIMEOUT
+            assert 0.05 < time.perf_counter() - t0 < 60.0
+    np.testing.assert_array_equal(*out)
