@@ -434,7 +434,7 @@ cudaError_t enqueue_solve(ws::Workspace &w, int gn, int pcg, cudaStream_t st) {
         if (w.init_ptrs[s])
             A(cudaMemcpyAsync(w.se3 + 8ull * w.h_scenes[s].node_base, w.init_ptrs[s],
                               32ull * w.h_scenes[s].num_nodes, cudaMemcpyDeviceToDevice, st));
-    ws::index_build(w, st);
+    A(ws::index_build(w, st));
     mark(0);
     for (int it = 0; it < gn && e == cudaSuccess; ++it) {
         ws::gn_eval(w, st);

@@ -749,7 +749,7 @@ static void pair_index(Workspace &w, cudaStream_t st) {
     w.pair_sorted_val = w.pair_val;
 }
 
-void index_build(Workspace &w, cudaStream_t st) {
+cudaError_t index_build(Workspace &w, cudaStream_t st) {
     const int S = w.num_scenes;
     const int T = (int)w.total_tiles;
     const uint32_t N = w.total_nodes;
@@ -790,7 +790,7 @@ void index_build(Workspace &w, cudaStream_t st) {
         w.half_slot_lo, w.colidx, w.item_info, w.item_col, w.item_ptr, w.node_scene, N, w.error_flag);
     count_launch(w);
     pcg_ranges(w, st);
-    pcg_plan(w, st);
+    return pcg_plan(w, st);
 }
 
 void pcg_ranges(Workspace &w, cudaStream_t st) {

@@ -160,7 +160,7 @@ struct Workspace {
 };
 
 // Index build (ws_index.cu): compaction, node->term, pair->term, block CSR.
-void index_build(Workspace &w, cudaStream_t st);
+cudaError_t index_build(Workspace &w, cudaStream_t st);
 // One Gauss-Newton iteration (ws_solve.cu): term evaluation, assembly, PCG, update,
 // and its four phases.
 cudaError_t gn_iteration(Workspace &w, int pcg_iters, cudaStream_t st);
