@@ -179,7 +179,13 @@ int ws_get_system(ws_solver *solver, int scene, uint32_t *rowptr, uint32_t *cols
 int ws_get_dense_jacobian(ws_solver *solver, int scene, float *residual, float *gradient,
                           int capacity, int *count);
 
-/* ---- Node graph, skinning and warp (bit-exact to the reference's integer outputs) ---- */
+/* ---- Node graph, skinning and warp (bit-exact to the reference's integer outputs) ----
+ * The calls below take their scratch from a pool of the library's own on the current device, in stream order.  The
+ * pool keeps up to 64 MB of idle memory from one call for the next, until the device's last solver is destroyed or
+ * ws_trim_scratch is called. */
+
+/* Gives the scratch of `device` back to the driver.  Synchronises the device. */
+int ws_trim_scratch(int device);
 
 /* NodeGraph::InitializeNodeGraphFromVertex (libs/star/geometry/node_graph/NodeGraph.cu:460-498):
  * voxel subsample (VoxelSubsamplerSorting.cu:8-96) and the greedy overlap check of

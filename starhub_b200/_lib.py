@@ -45,6 +45,7 @@ EXPORTED = [
     "ws_render_observation_maps",
     "ws_build_node_graph_ex", "ws_skinning_ex", "ws_skinning_incremental",
     "ws_set_tuning", "ws_set_pcg_form", "ws_get_pcg_form", "ws_selftest_resident_timeout",
+    "ws_trim_scratch",
 ]
 
 
@@ -198,6 +199,7 @@ def load() -> C.CDLL:
         "ws_autotune": (i, [vp, i, vp, C.POINTER(WsTuning)]),
         "ws_set_tuning": (i, [vp, C.POINTER(WsTuning)]),
         "ws_set_pcg_form": (i, [vp, i, i]),
+        "ws_trim_scratch": (i, [i]),
         "ws_selftest_resident_timeout": (i, [vp, vp]),
         "ws_get_pcg_form": (i, [vp, C.POINTER(i)]),
     }

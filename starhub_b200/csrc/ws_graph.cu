@@ -1068,7 +1068,8 @@ int noalloc_scratch(unsigned long long **out) {
 // first call after one mapped its scratch again: the solver-map pass of a frame took 479 us instead of 35,
 // and node construction, which synchronises itself, paid for it within each call.  This pool keeps up to
 // kScratchKeep idle bytes (node construction of 1M surfels holds about 50 MB); what is above goes back at the
-// next synchronisation, and all of it when the device's last solver is destroyed (scratch_trim).  In a
+// next synchronisation, and all of it when the device's last solver is destroyed or the program asks for it
+// (ws_trim_scratch: a program may use the geometry calls without a solver).  In a
 // capture the allocation is the graph's own, as before.
 constexpr unsigned long long kScratchKeep = 64ull << 20;
 std::mutex g_scratch_mutex;
@@ -1229,16 +1230,32 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
 
 namespace ws {
 
-// Gives the idle scratch of `device` back to the driver.
-void scratch_trim(int device) {
-    if (device < 0 || device >= kMaxDevices) return;
+// Gives the idle scratch of `device` back to the driver; false when the device refuses.
+bool scratch_trim(int device) {
+    if (device < 0 || device >= kMaxDevices) return true;   // such devices have no pool
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (g_scratch_pool[device] && cudaMemPoolTrimTo(g_scratch_pool[device], 0) != cudaSuccess) cudaGetLastError();
+    if (!g_scratch_pool[device] || cudaMemPoolTrimTo(g_scratch_pool[device], 0) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
 }
 
 }  // namespace ws
 
 extern "C" {
+
+int ws_trim_scratch(int device) {
+    int devices = 0;
+    if (cudaGetDeviceCount(&devices) != cudaSuccess) {
+        cudaGetLastError();
+        return WS_ERR_NO_DEVICE;
+    }
+    if (device < 0 || device >= devices) return WS_ERR_INVALID_ARGUMENT;
+    // scratch is given back to the pool in stream order: it is idle once the device has come that far
+    int here = 0;
+    if (cudaGetDevice(&here) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return WS_ERR_CUDA;
+    const bool done = cudaDeviceSynchronize() == cudaSuccess && ws::scratch_trim(device);
+    return cudaSetDevice(here) == cudaSuccess && done ? WS_OK : WS_ERR_CUDA;
+}
 
 int ws_init_nodes(const float *surfels, int n, float node_radius, float *nodes_host, int cap, int *num_nodes,
                   void *stream) {

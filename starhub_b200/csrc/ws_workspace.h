@@ -201,7 +201,7 @@ cudaError_t gn_spmv_matrix_free(Workspace &w, const float *x, float *y, float *u
                                 cudaStream_t st);
 int pcg_warps_per_block();
 // Gives the geometry calls' idle scratch on a device back to the driver (ws_graph.cu).
-void scratch_trim(int device);
+bool scratch_trim(int device);
 
 // Launch accounting for the measurement hooks.
 inline void count_launch(Workspace &w, int n = 1) { w.launches += n; }
