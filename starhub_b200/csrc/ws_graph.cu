@@ -541,8 +541,9 @@ __global__ void __launch_bounds__(256) k_skinning(const float4 *nodes, const uin
 // Result: exactly k_skinning's.  When the four nearest found are strictly below the fifth and below
 // every node outside the cells (by the distance to their faces, with a margin of a hundredth of a cell
 // for the rounding of the scaled coordinates, |cell| <= 4096), and differ from one another, the ordered
-// scan ends with the same four in the same order.  Otherwise (ties, far or few nodes, NaN) the surfel's
-// warp repeats the ordered scan itself, 32 nodes at a time with the heap updates in node order.
+// scan ends with the same four in the same order.  Otherwise (ties, far or few nodes, NaN) the surfel is
+// open: its warp repeats the ordered scan for it, 32 nodes at a time with the heap updates in node order,
+// or, where it has many of them, every lane for its own (skin_open).
 constexpr int kSkinThreads = 1024;
 constexpr int kSkinCellsX = 32, kSkinCellsY = 32, kSkinCellsZ = 16;
 constexpr int kSkinCells = kSkinCellsX * kSkinCellsY * kSkinCellsZ;
@@ -709,6 +710,23 @@ struct SkinNearest {
     float d[5] = {1e6f, 1e6f, 1e6f, 1e6f, 1e6f};
     int id[4] = {0, 0, 0, 0};
     float reach = 1e30f;
+    __device__ __forceinline__ void insert(float dist, int node) {   // dist < d[4]
+        const bool b0 = dist < d[0], b1 = dist < d[1], b2 = dist < d[2], b3 = dist < d[3];
+        d[4] = b3 ? d[3] : dist;
+        d[3] = b2 ? d[2] : (b3 ? dist : d[3]);
+        id[3] = b2 ? id[2] : (b3 ? node : id[3]);
+        d[2] = b1 ? d[1] : (b2 ? dist : d[2]);
+        id[2] = b1 ? id[1] : (b2 ? node : id[2]);
+        d[1] = b0 ? d[0] : (b1 ? dist : d[1]);
+        id[1] = b0 ? id[0] : (b1 ? node : id[1]);
+        d[0] = b0 ? dist : d[0];
+        id[0] = b0 ? node : id[0];
+    }
+    // the nearest four are distinct, nearer than the fifth and than every node outside the cells: any order of the
+    // nodes gives them
+    __device__ __forceinline__ bool sure() const {
+        return d[0] < d[1] && d[1] < d[2] && d[2] < d[3] && d[3] < d[4] && reach > 0.f && d[3] < reach * reach;
+    }
 };
 
 __device__ __forceinline__ void skin_grid_search(float4 p, float h, const float4 *cell_nodes, const uint32_t *cell_end,
@@ -727,19 +745,7 @@ __device__ __forceinline__ void skin_grid_search(float4 p, float h, const float4
             for (uint32_t k = lo > 0 ? cell_end[lo - 1] : 0u; k < e; ++k) {
                 const float4 q = cell_nodes[k];
                 const float dist = sq3_fused(p.x - q.x, p.y - q.y, p.z - q.z);
-                if (dist < b.d[4]) {
-                    const int id = __float_as_int(q.w);
-                    const bool b0 = dist < b.d[0], b1 = dist < b.d[1], b2 = dist < b.d[2], b3 = dist < b.d[3];
-                    b.d[4] = b3 ? b.d[3] : dist;
-                    b.d[3] = b2 ? b.d[2] : (b3 ? dist : b.d[3]);
-                    b.id[3] = b2 ? b.id[2] : (b3 ? id : b.id[3]);
-                    b.d[2] = b1 ? b.d[1] : (b2 ? dist : b.d[2]);
-                    b.id[2] = b1 ? b.id[1] : (b2 ? id : b.id[2]);
-                    b.d[1] = b0 ? b.d[0] : (b1 ? dist : b.d[1]);
-                    b.id[1] = b0 ? b.id[0] : (b1 ? id : b.id[1]);
-                    b.d[0] = b0 ? dist : b.d[0];
-                    b.id[0] = b0 ? id : b.id[0];
-                }
+                if (dist < b.d[4]) b.insert(dist, __float_as_int(q.w));
             }
         }
     }
@@ -750,35 +756,151 @@ __device__ __forceinline__ void skin_grid_search(float4 p, float h, const float4
     b.reach = near ? fminf(b.reach, (0.99f + inside) * h) : -1.f;
 }
 
+constexpr float kSkinOpen = -1.f;   // a connect weight, until the surfel's turn comes
+constexpr int kSkinMany = 6;   // open surfels of a warp from which on every lane looks at all nodes for its own (skin_open)
+
+struct SkinOut {
+    float r2;
+    int normalize;
+    ushort4 *knn;
+    float4 *sw, *cw;
+};
+__device__ __forceinline__ void skin_store(const SkinOut &o, int v, const float (&d)[4], const int (&id)[4]) {
+    float wv[4], sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        wv[i] = __expf(-d[i] / (2.f * o.r2));
+        sum += wv[i];
+    }
+    const float inv = 1.f / sum;
+    o.knn[v] = make_ushort4((uint16_t)id[0], (uint16_t)id[1], (uint16_t)id[2], (uint16_t)id[3]);
+    o.sw[v] = o.normalize ? make_float4(inv * wv[0], inv * wv[1], inv * wv[2], inv * wv[3])
+                          : make_float4(wv[0], wv[1], wv[2], wv[3]);
+    o.cw[v] = make_float4(1.f, 1.f, 1.f, 1.f);
+}
+
+// The ordered scan for the surfel at p of lane `who`, by the whole warp, 32 nodes at a time.
+__device__ __forceinline__ void skin_scan_one(const float4 *nodes, const uint2 *status, int n_nodes, float4 p, int who,
+                                              Heap<4> &heap) {
+    const int lane = threadIdx.x & 31;
+    const float px = __shfl_sync(0xffffffffu, p.x, who), py = __shfl_sync(0xffffffffu, p.y, who),
+                pz = __shfl_sync(0xffffffffu, p.z, who);
+    heap.init(1e6f);
+    for (int i0 = 0; i0 < n_nodes; i0 += 32) {
+        const int i = i0 + lane;
+        float dist = 1e6f;
+        if (i < n_nodes && !node_deleted(status, i)) {
+            const float4 q = nodes[i];
+            dist = sq3_fused(px - q.x, py - q.y, pz - q.z);
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, dist < heap.max_d); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            heap.update((uint16_t)(i0 + l), __shfl_sync(0xffffffffu, dist, l));
+        }
+    }
+    heap.sort();
+}
+
+// Many open surfels of a warp: the ordered scan by every lane for its own, 32 nodes at a time from global memory, the
+// next 32 on their way.  us, one surfel after another / this / k_skinning, which the grid is not to lose to: surfels far
+// from all nodes, 200k on 8000 nodes 5569 / 1376 / 1787, 300 on 8000 2328 / 511 / 622; all tied, 195k on 8000 10445 /
+// 1303 / 2072, on 1000 3625 / 350 / 325.
+__device__ __forceinline__ void skin_open(const float4 *nodes, const uint2 *status, int n_nodes, float4 p, int v, unsigned open,
+                                          const SkinOut &o) {
+    const int lane = threadIdx.x & 31;
+    const bool mine = (open >> lane) & 1u;
+    Heap<4> heap;
+    heap.init(1e6f);
+    float4 q = nodes[min(lane, n_nodes - 1)];
+    bool here = lane < n_nodes && !node_deleted(status, lane);
+    for (int i0 = 0; i0 < n_nodes; i0 += 32) {
+        const float4 now = q;
+        const unsigned alive = __ballot_sync(0xffffffffu, here);
+        const int next = i0 + 32 + lane;
+        q = nodes[min(next, n_nodes - 1)];
+        here = next < n_nodes && !node_deleted(status, next);
+        // the distance to the 32 nodes' box, rounded as theirs are, bounds them: what lies beyond enters no heap
+        const bool in = (alive >> lane) & 1u;
+        float lo[3] = {in ? now.x : INFINITY, in ? now.y : INFINITY, in ? now.z : INFINITY};
+        float hi[3] = {in ? now.x : -INFINITY, in ? now.y : -INFINITY, in ? now.z : -INFINITY};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+                hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+            }
+        const float box = sq3_fused(fmaxf(fmaxf(lo[0] - p.x, p.x - hi[0]), 0.f), fmaxf(fmaxf(lo[1] - p.y, p.y - hi[1]), 0.f),
+                                    fmaxf(fmaxf(lo[2] - p.z, p.z - hi[2]), 0.f));
+        if (!__any_sync(0xffffffffu, mine && box < heap.max_d)) continue;
+#pragma unroll 4
+        for (int l = 0; l < 32; ++l) {
+            const float x = __shfl_sync(0xffffffffu, now.x, l), y = __shfl_sync(0xffffffffu, now.y, l),
+                        z = __shfl_sync(0xffffffffu, now.z, l);
+            const float dist = (alive >> l) & 1u ? sq3_fused(p.x - x, p.y - y, p.z - z) : 1e6f;
+            if (__any_sync(0xffffffffu, mine && dist < heap.max_d)) heap.update((uint16_t)(i0 + l), dist);
+        }
+    }
+    heap.sort();
+    if (mine) {
+        float d[4];
+        int ids[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            ids[i] = heap.id[i];
+            const float4 q = nodes[min(ids[i], n_nodes - 1)];
+            d[i] = sq3_fused(p.x - q.x, p.y - q.y, p.z - q.z);
+        }
+        skin_store(o, v, d, ids);
+    }
+}
+
+// A warp's rounds of 32 surfels: whole rounds of the launch by blocks (neighbouring memory), the last one, or few
+// surfels, over all blocks (200k surfels 66 -> 59 us, 3000 on 8000 nodes 110 -> 82).
+struct SkinRounds {
+    int base, full, stride, shift;
+    uint32_t bit = 1;   // of the round, modulo 32
+    __device__ __forceinline__ SkinRounds(int first_vert, int n_verts) {
+        const int by_block = (int)(blockIdx.x * (kSkinThreads / 32) + (threadIdx.x >> 5)),
+                  spread = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+        stride = 32 * (int)(gridDim.x * (kSkinThreads / 32));
+        full = (n_verts - first_vert) / stride;
+        shift = 32 * (spread - by_block);
+        base = first_vert + 32 * by_block + (full == 0 ? shift : 0);
+    }
+    __device__ __forceinline__ void next() {
+        base += stride;
+        if (--full == 0) base += shift;
+        bit = __funnelshift_l(bit, bit, 1);
+    }
+};
+
+// The rounds (modulo 32) of a warp that left many surfels open.  Last: in the loop its code costs the usual case 2 %.
+__device__ __forceinline__ void skin_later(const float4 *nodes, const uint2 *status, int n_nodes, const float4 *verts, int first_vert,
+                                           int n_verts, uint32_t rounds, const SkinOut &out) {
+    const int lane = threadIdx.x & 31;
+    for (SkinRounds r(first_vert, n_verts); r.base < n_verts; r.next()) {
+        if ((rounds & r.bit) == 0) continue;
+        const int v = r.base + lane;
+        const unsigned open = __ballot_sync(0xffffffffu, v < n_verts && out.cw[v].x == kSkinOpen);
+        if (open) skin_open(nodes, status, n_nodes, verts[min(v, n_verts - 1)], v, open, out);
+    }
+}
+
 // The surfels of a warp (lane's surfel v at p): the ordered scan where the search does not settle the
 // result, then ids and weights.
-__device__ __forceinline__ void skin_grid_finish(const float4 *nodes, const uint2 *status, int n_nodes, float4 p, int v,
-                                                 bool live, SkinNearest &b, float r2, int normalize, ushort4 *knn,
-                                                 float4 *sw, float4 *cw) {
+// Many open surfels are left out and returned; until skin_open's turn their connect weight says so.
+__device__ __forceinline__ unsigned skin_grid_finish(const float4 *nodes, const uint2 *status, int n_nodes, float4 p, int v,
+                                                     bool live, SkinNearest &b, const SkinOut &o) {
     const int lane = threadIdx.x & 31;
-    const bool sure = b.d[0] < b.d[1] && b.d[1] < b.d[2] && b.d[2] < b.d[3] && b.d[3] < b.d[4] && b.reach > 0.f &&
-                      b.d[3] < b.reach * b.reach;
-    unsigned open = __ballot_sync(0xffffffffu, live && !sure);
+    unsigned open = __ballot_sync(0xffffffffu, live && !b.sure());
+    const unsigned many = __popc(open) >= kSkinMany ? open : 0u;
+    open &= ~many;
     while (open) {
         const int who = __ffs(open) - 1;
         open &= open - 1;
-        const float px = __shfl_sync(0xffffffffu, p.x, who), py = __shfl_sync(0xffffffffu, p.y, who),
-                    pz = __shfl_sync(0xffffffffu, p.z, who);
         Heap<4> heap;
-        heap.init(1e6f);
-        for (int i0 = 0; i0 < n_nodes; i0 += 32) {
-            const int i = i0 + lane;
-            float dist = 1e6f;
-            if (i < n_nodes && !node_deleted(status, i)) {
-                const float4 q = nodes[i];
-                dist = sq3_fused(px - q.x, py - q.y, pz - q.z);
-            }
-            for (unsigned m = __ballot_sync(0xffffffffu, dist < heap.max_d); m; m &= m - 1) {
-                const int l = __ffs(m) - 1;
-                heap.update((uint16_t)(i0 + l), __shfl_sync(0xffffffffu, dist, l));
-            }
-        }
-        heap.sort();
+        skin_scan_one(nodes, status, n_nodes, p, who, heap);
         if (lane == who) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -788,33 +910,27 @@ __device__ __forceinline__ void skin_grid_finish(const float4 *nodes, const uint
             }
         }
     }
-    if (!live) return;
-    float wv[4], sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        wv[i] = __expf(-b.d[i] / (2.f * r2));
-        sum += wv[i];
+    if (live && ((many >> lane) & 1u) == 0) {
+        const float d[4] = {b.d[0], b.d[1], b.d[2], b.d[3]};
+        skin_store(o, v, d, b.id);
+    } else if (live) {
+        o.cw[v].x = kSkinOpen;
     }
-    const float inv = 1.f / sum;
-    knn[v] = make_ushort4((uint16_t)b.id[0], (uint16_t)b.id[1], (uint16_t)b.id[2], (uint16_t)b.id[3]);
-    sw[v] = normalize ? make_float4(inv * wv[0], inv * wv[1], inv * wv[2], inv * wv[3])
-                      : make_float4(wv[0], wv[1], wv[2], wv[3]);
-    cw[v] = make_float4(1.f, 1.f, 1.f, 1.f);
+    return many;
 }
 
 // kChunked: more than kSkinGridNodes nodes; a launch then covers at most 32 surfels a warp.
 template <bool kChunked>
 __global__ void __launch_bounds__(kSkinThreads, 1) k_skinning_grid(const float4 *nodes, const uint2 *status, int n_nodes,
                                                                    const float4 *verts, int first_vert, int n_verts,
-                                                                   float radius, float r2, int normalize, ushort4 *knn,
-                                                                   float4 *sw, float4 *cw) {
+                                                                   float radius, const SkinOut out) {
     extern __shared__ __align__(16) unsigned char skin_smem[];
     float4 *cell_nodes = reinterpret_cast<float4 *>(skin_smem);                                    // one chunk's
     uint32_t *cell_end = reinterpret_cast<uint32_t *>(skin_smem + 16 * (size_t)min(n_nodes, kSkinGridNodes));
-    const int lane = threadIdx.x & 31, warps = gridDim.x * (kSkinThreads / 32);
-    const int first = first_vert + 32 * (blockIdx.x * (kSkinThreads / 32) + (threadIdx.x >> 5));
+    const int lane = threadIdx.x & 31;
+    SkinRounds r(first_vert, n_verts);
     if constexpr (kChunked) {
-        const int v = first + lane;
+        const int v = r.base + lane;
         const bool live = v < n_verts;
         const float4 p = live ? verts[v] : make_float4(0.f, 0.f, 0.f, 0.f);
         SkinNearest b;
@@ -823,17 +939,24 @@ __global__ void __launch_bounds__(kSkinThreads, 1) k_skinning_grid(const float4 
                                             cell_nodes, cell_end);
             if (live) skin_grid_search(p, h, cell_nodes, cell_end, b);
         }
-        skin_grid_finish(nodes, status, n_nodes, p, v, live, b, r2, normalize, knn, sw, cw);
+        const unsigned many = skin_grid_finish(nodes, status, n_nodes, p, v, live, b, out);
+        if (many) skin_open(nodes, status, n_nodes, p, v, many, out);
     } else {
         const float h = skin_grid_build(nodes, status, 0, n_nodes, 1.75f * radius, cell_nodes, cell_end);
-        for (int base = first; base < n_verts; base += 32 * warps) {
-            const int v = base + lane;
+        __shared__ uint32_t s_later[kSkinThreads / 32];
+        uint32_t &later = s_later[threadIdx.x >> 5];
+        if (lane == 0) later = 0;
+        for (; r.base < n_verts; r.next()) {
+            const int v = r.base + lane;
             const bool live = v < n_verts;
             const float4 p = live ? verts[v] : make_float4(0.f, 0.f, 0.f, 0.f);
             SkinNearest b;
             if (live) skin_grid_search(p, h, cell_nodes, cell_end, b);
-            skin_grid_finish(nodes, status, n_nodes, p, v, live, b, r2, normalize, knn, sw, cw);
+            if (skin_grid_finish(nodes, status, n_nodes, p, v, live, b, out) && lane == 0) later |= r.bit;
         }
+        __syncwarp();
+        if (later != 0)
+            skin_later(nodes, status, n_nodes, verts, first_vert, n_verts, later, out);
     }
 }
 
@@ -1406,11 +1529,12 @@ int ws_skinning_incremental(const float *nodes, const uint32_t *node_status, int
         const int slab = chunked ? sms * ws::kSkinThreads : count;   // surfels of a launch
         for (long long v0 = num_remaining_surfels; v0 < num_verts; v0 += slab) {
             const int v1 = (int)std::min<long long>(num_verts, v0 + slab);
-            const int grid = (int)std::min<long long>(sms, (v1 - v0 + ws::kSkinThreads - 1) / ws::kSkinThreads);
+            const int grid = (int)std::min<long long>(sms, (v1 - v0 + 31) / 32);
             kernel<<<grid, ws::kSkinThreads, smem, st>>>(
                 reinterpret_cast<const float4 *>(nodes), reinterpret_cast<const uint2 *>(node_status), num_nodes,
-                reinterpret_cast<const float4 *>(verts), (int)v0, v1, node_radius, r2, normalize_weights ? 1 : 0,
-                reinterpret_cast<ushort4 *>(knn), reinterpret_cast<float4 *>(sw), reinterpret_cast<float4 *>(cw));
+                reinterpret_cast<const float4 *>(verts), (int)v0, v1, node_radius,
+                ws::SkinOut{r2, normalize_weights ? 1 : 0, reinterpret_cast<ushort4 *>(knn), reinterpret_cast<float4 *>(sw),
+                            reinterpret_cast<float4 *>(cw)});
         }
         return cudaGetLastError() == cudaSuccess ? WS_OK : WS_ERR_CUDA;
     }
