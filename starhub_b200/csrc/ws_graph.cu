@@ -188,39 +188,42 @@ __global__ void k_voxel_sample(const uint32_t *keys, const uint32_t *perm, const
 // differ by at most r (1 + 2^-22) per axis, i.e. 0.889 cells; the scaled coordinates are
 // clamped to +-2^18 cells, where a float resolves 1/32 of a cell, so their rounding adds at most
 // 1/32 and such candidates lie in the same or adjacent cells.  Cell coordinates wrap at
-// kDedupCells per axis, which only adds far candidates that the distance test turns away.  The
+// `cells` per axis, a power of two, which only adds far candidates that the distance test turns away.  The
 // candidates are put in cell order by counting (a table of all cells, counts, a scan, placement): their
 // order within a cell is left open, since no decision depends on it.  Sorting them by a 30-bit cell key
 // and searching it took 13 launches and 18 binary searches a candidate.
 constexpr float kDedupCellScale = 1.125f;
-constexpr int kDedupCells = 64;                                              // per axis
-constexpr uint32_t kDedupTable = kDedupCells * kDedupCells * kDedupCells;
+// Cells per axis: 64, and 128 from as many candidates as that table has cells (988k candidates spread over 12 m, R =
+// 0.025: 3044 / 2758 us in all, 2.9M 12569 / 7869; the table is cleared and scanned, which few candidates would not pay).
+constexpr int kDedupCellsMost = 128;
+constexpr int dedup_cells(uint32_t nv) { return nv <= (1u << 18) ? 64 : kDedupCellsMost; }
+constexpr uint32_t dedup_table(int cells) { return (uint32_t)cells * cells * cells; }
 
 __device__ __forceinline__ int dedup_cell(float v, float inv_cell) {
     return __float2int_rd(fminf(fmaxf(__fmul_rn(v, inv_cell), -262144.f), 262144.f));
 }
 
-__device__ __forceinline__ uint32_t dedup_key(int x, int y, int z) {
-    constexpr int m = kDedupCells - 1;
-    return (uint32_t)(x & m) + kDedupCells * ((uint32_t)(y & m) + kDedupCells * (uint32_t)(z & m));
+__device__ __forceinline__ uint32_t dedup_key(int x, int y, int z, int cells) {
+    const int m = cells - 1;
+    return (uint32_t)(x & m) + (uint32_t)cells * ((uint32_t)(y & m) + (uint32_t)cells * (uint32_t)(z & m));
 }
-__device__ __forceinline__ uint32_t dedup_key_of(float4 p, float inv_cell) {
-    return dedup_key(dedup_cell(p.x, inv_cell), dedup_cell(p.y, inv_cell), dedup_cell(p.z, inv_cell));
+__device__ __forceinline__ uint32_t dedup_key_of(float4 p, float inv_cell, int cells) {
+    return dedup_key(dedup_cell(p.x, inv_cell), dedup_cell(p.y, inv_cell), dedup_cell(p.z, inv_cell), cells);
 }
 
-__global__ void k_dedup_count(const float4 *cand, uint32_t nv, float inv_cell, uint32_t *table, int *err) {
+__global__ void k_dedup_count(const float4 *cand, uint32_t nv, float inv_cell, int cells, uint32_t *table, int *err) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
         const float4 p = cand[i];
         if (isnan(p.x) || isnan(p.y) || isnan(p.z)) atomicOr(err, 1);
-        atomicAdd(table + dedup_key_of(p, inv_cell), 1u);
+        atomicAdd(table + dedup_key_of(p, inv_cell, cells), 1u);
     }
 }
 
 // table: first position of every cell; on return the end of every cell (the next one's first).
-__global__ void k_dedup_place(const float4 *cand, uint32_t nv, float inv_cell, uint32_t *table, float4 *placed) {
+__global__ void k_dedup_place(const float4 *cand, uint32_t nv, float inv_cell, int cells, uint32_t *table, float4 *placed) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
         const float4 p = cand[i];
-        placed[atomicAdd(table + dedup_key_of(p, inv_cell), 1u)] = make_float4(p.x, p.y, p.z, __uint_as_float(i));
+        placed[atomicAdd(table + dedup_key_of(p, inv_cell, cells), 1u)] = make_float4(p.x, p.y, p.z, __uint_as_float(i));
     }
 }
 
@@ -229,18 +232,19 @@ __global__ void k_dedup_place(const float4 *cand, uint32_t nv, float inv_cell, u
 // kFill = true writes their indices from offset `cnt[i]` of `nbr`.
 template <bool kFill>
 __global__ void k_dedup_neighbours(const float4 *cand, const uint32_t *cell_end, const float4 *placed, uint32_t nv,
-                                   float inv_cell, float thr, uint32_t *cnt, uint32_t *nbr, uint32_t cap, int *err) {
+                                   float inv_cell, int cells, float thr, uint32_t *cnt, uint32_t *nbr, uint32_t cap,
+                                   int *err) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
         const float4 p = cand[i];
         const int cx = dedup_cell(p.x, inv_cell), cy = dedup_cell(p.y, inv_cell), cz = dedup_cell(p.z, inv_cell);
-        const uint32_t x0 = (uint32_t)(cx - 1) & (kDedupCells - 1), x1 = (uint32_t)(cx + 1) & (kDedupCells - 1);
+        const uint32_t x0 = (uint32_t)((cx - 1) & (cells - 1)), x1 = (uint32_t)((cx + 1) & (cells - 1));
         const int ranges = x0 < x1 ? 1 : 2;
         uint32_t c = 0, out = kFill ? cnt[i] : 0u;
         for (int row = 0; row < 9; ++row) {
-            const uint32_t c0 = dedup_key(0, cy + row % 3 - 1, cz + row / 3 - 1);
+            const uint32_t c0 = dedup_key(0, cy + row % 3 - 1, cz + row / 3 - 1, cells);
             for (int q = 0; q < ranges; ++q) {
                 const uint32_t lo = c0 + (ranges == 1 || q == 0 ? x0 : 0u);
-                const uint32_t hi = c0 + (ranges == 1 || q == 1 ? x1 : (uint32_t)(kDedupCells - 1));
+                const uint32_t hi = c0 + (ranges == 1 || q == 1 ? x1 : (uint32_t)(cells - 1));
                 const uint32_t e = __ldg(cell_end + hi);
                 for (uint32_t b = lo > 0 ? __ldg(cell_end + lo - 1) : 0u; b < e; ++b) {
                     const float4 o = placed[b];
@@ -259,11 +263,12 @@ __global__ void k_dedup_neighbours(const float4 *cand, const uint32_t *cell_end,
         if (!kFill) cnt[i] = c;
     }
 }
-// Overlapping pairs per candidate: a candidate is the only one of its voxel (0.7 R), and a ball of 0.85 R
-// around one meets at most 4^3 voxels, so it has at most 63 neighbours and half of them are earlier.  (Far
-// from the origin, where floats are coarser than that, `err` gets 8 and the lists are made again as long as
-// they need to be.)
-constexpr uint32_t kDedupPairsPerCandidate = 32;
+// Overlapping pairs kept per candidate.  A candidate is the only one of its voxel (0.7 R), so a ball of 0.85 R around
+// one holds about 7.5 (a volume filled at random; eight voxels' candidates in a common corner see 7 each), half of them
+// earlier.  (Where there are more, `err` gets 8 and the lists are made again as long as they need to be; a candidate
+// has at most 63 neighbours.)  32 a candidate went past the scratch that the pool keeps: 988k candidates 2758 / 1923
+// us, 2.9M 7869 / 5691.
+constexpr uint32_t kDedupPairsPerCandidate = 8;
 
 // The decisions, without rounds: thread t takes candidates t, t + T, ... (T threads in all) in turn and
 // re-reads a candidate's open earlier neighbours until one is kept (rejected) or none is open (kept).
@@ -1329,7 +1334,7 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
     uint32_t *keys = mem.get<uint32_t>(4ull * (n + 1)), *vals = mem.get<uint32_t>(4ull * (n + 1));
     uint32_t *keys2 = mem.get<uint32_t>(4ull * (n + 1)), *vals2 = mem.get<uint32_t>(4ull * (n + 1));
     uint32_t *heads = mem.get<uint32_t>(4ull * (n + 1));
-    uint32_t *tmp = mem.get<uint32_t>(4ull * (std::max(n, ws::kDedupTable) / ws::kScanTile + 4));
+    uint32_t *tmp = mem.get<uint32_t>(4ull * (std::max(n, ws::dedup_table(ws::kDedupCellsMost)) / ws::kScanTile + 4));
     uint32_t *hist = mem.get<uint32_t>(4ull * 256 * ws::sort_max_tiles(n));
     uint32_t *digit = mem.get<uint32_t>(4ull * 256);
     float4 *cand = mem.get<float4>(16ull * n);
@@ -1356,7 +1361,9 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
     const float inv_cell = 1.0f / (ws::kDedupCellScale * r);
     uint32_t *cnt = heads, *pos = vals2;   // free again: the candidates are written
     uint32_t pairs = (uint32_t)std::min<uint64_t>((uint64_t)ws::kDedupPairsPerCandidate * nv, 0xFFFFFFF0ull);
-    uint32_t *table = mem.get<uint32_t>(4ull * (ws::kDedupTable + 1));
+    const int cells = ws::dedup_cells(nv);
+    const uint32_t table_cells = ws::dedup_table(cells);
+    uint32_t *table = mem.get<uint32_t>(4ull * (table_cells + 1));
     float4 *placed = mem.get<float4>(16ull * nv);
     uint32_t *nbr = mem.get<uint32_t>(4ull * pairs);
     uint8_t *decision = mem.get<uint8_t>(nv);
@@ -1368,17 +1375,17 @@ int grow_nodes(const float4 *pts, uint32_t n, float node_radius, DeviceBlocks &m
         per_sm < 1)
         return WS_ERR_CUDA;
     if (cudaMemsetAsync(err, 0, 4, st) != cudaSuccess || cudaMemsetAsync(decision, 0, nv, st) != cudaSuccess ||
-        cudaMemsetAsync(table, 0, 4ull * ws::kDedupTable, st) != cudaSuccess)
+        cudaMemsetAsync(table, 0, 4ull * table_cells, st) != cudaSuccess)
         return WS_ERR_CUDA;
-    ws::k_dedup_count<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, table, err);
-    ws::exclusive_scan(table, table, ws::kDedupTable, tmp, st);
-    ws::k_dedup_place<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, table, placed);
-    ws::k_dedup_neighbours<false><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, thr, cnt,
+    ws::k_dedup_count<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, cells, table, err);
+    ws::exclusive_scan(table, table, table_cells, tmp, st);
+    ws::k_dedup_place<<<ws::grid_of(nv, 256), 256, 0, st>>>(cand, nv, inv_cell, cells, table, placed);
+    ws::k_dedup_neighbours<false><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, cells, thr, cnt,
                                                                        nullptr, 0, err);
     ws::exclusive_scan(cnt, cnt, nv, tmp, st);
     uint32_t count = 0;
     for (int attempt = 0;; ++attempt) {
-        ws::k_dedup_neighbours<true><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, thr, cnt,
+        ws::k_dedup_neighbours<true><<<ws::grid_of(nv, 128), 128, 0, st>>>(cand, table, placed, nv, inv_cell, cells, thr, cnt,
                                                                           nbr, pairs, err);
         const long long want = ((long long)nv + ws::kDedupThreads - 1) / ws::kDedupThreads;
         const int grid = (int)std::min<long long>(want, (long long)per_sm * sms);
