@@ -161,7 +161,7 @@ __device__ __forceinline__ ResPlace res_place(const PcgArgs &A) {
 
 // What bounds a block, in ns an iteration: least squares over launches of 1 to 30 scenes of 500 to 8000 nodes with 5 to
 // 30 upper pairs a row, within 15 % of what was measured (5.3 to 180 us).  Phase A: the block's items, on the grid
-// twice beyond some 3900 of them, in a cluster also the products sent to other blocks.
+// twice beyond some 4600 of them, in a cluster also the products sent to other blocks.
 // Phase B: the contributions that rows read from L2.
 template <bool kGrid>
 __device__ __forceinline__ void res_cost(const ResPlan &P, uint32_t vec_rows, uint32_t items, uint32_t lows,
@@ -172,7 +172,7 @@ __device__ __forceinline__ void res_cost(const ResPlan &P, uint32_t vec_rows, ui
     const float i = (float)items;
     float a, b;
     if (kGrid) {
-        a = 7.f * i + 7.2f * fmaxf(i - 3900.f, 0.f) + (vec_fits ? 0.f : 6.f * i);
+        a = 7.f * i + 7.2f * fmaxf(i - 4600.f, 0.f) + (vec_fits ? 0.f : 6.f * i);
         b = 4.8f * (float)outside + (low_fits ? 0.f : 0.6f * (float)lows);
     } else {
         a = 3.5f * i + 6.5f * (float)crossing + (vec + 24u * lows + 144u * items > P.smem ? 2500.f : 0.f);
