@@ -9,16 +9,18 @@
 // s and d of the rows that its items touch elsewhere (its halo).
 //   * kGrid = false: the scene is one thread-block cluster (up to 16 SMs).  New s goes into the other blocks'
 //     halos and transposed products to the owning block through distributed shared memory, and the
-//     reductions are two hardware cluster barriers an iteration: 6.0 us an iteration at 500 nodes, 7.2 at
-//     1800.  What is left is latency and, with more rows a block, shared-memory traffic (192 KB a block and
-//     iteration at 1800 nodes).  A batch's scenes are independent clusters, the largest first.
+//     reductions are two hardware cluster barriers an iteration: 5.3 us an iteration at 500 nodes, 7.1 at
+//     1800 (launches of 20, their load phase included).  What is left is latency and, with more rows a block,
+//     shared-memory traffic (192 KB a block and iteration at 1800 nodes).  A batch's scenes are independent
+//     clusters, the largest first.
 //   * kGrid = true: the scene has a share of all SMs.  Halos, transposed products and partials go through L2,
-//     and the blocks meet at a counter there: 9.8 us at 3000 nodes, 11.0 at 8000.  What is left are the two
-//     meetings (fence, atomic, poll: 2 to 3 us each) and the trips to L2 after them.
+//     and the blocks meet at a counter there: 9.6 us at 3000 nodes, 10.7 at 8000.  What is left are the two
+//     meetings (fence, atomic, poll: 1.3 us each with 148 blocks) and the dependent trips to L2 after them.
 //
 // The arithmetic is k_pcg's, operation by operation (products per item, row sums in item order,
 // contributions in column order, group partials over 16 rows, scene sums over groups in lane-strided
-// order), so both kernels give the same bits and a scene's result does not depend on which one ran.
+// order), so all forms give the same bits and a scene's result does not depend on which one ran, nor on what
+// found room in shared memory.
 //
 // Waits: the cluster barriers are hardware barriers that every block of the scene reaches; a wait for a
 // bulk copy is bounded, sets WS_ERR_TIMEOUT and goes on, so that no block leaves the others waiting.  A
