@@ -51,8 +51,8 @@ struct Heap {
 #pragma unroll
             for (int i = 0; i < CAP; ++i)
                 if (i == max_id) { d[i] = dist; id[i] = idx; }
+            refresh();
         }
-        refresh();
     }
     // Ascending order.  Distinct distances have one: a sorting network in registers.  With ties the
     // order is that of the reference's quicksort.
@@ -84,9 +84,10 @@ struct Heap {
         }
     }
     // Lomuto quicksort on strict <, iterative form of the reference's recursion
-    // (same partitions in the same order); kept out of line, since its run-time indices put the arrays in
-    // local memory.
-    static __device__ __noinline__ void quicksort_arrays(float *d, uint16_t *id) {
+    // (same partitions in the same order), on copies, since its run-time indices put the arrays in local memory
+    // (as a call it cost the loops around it their registers: 300k surfels on 2000 new nodes 615 -> 660 us; inlined,
+    // and with the maximum sought again only when a node has entered, 402).
+    static __device__ __forceinline__ void quicksort_arrays(float *d, uint16_t *id) {
         int lo_stack[2 * CAP + 2], hi_stack[2 * CAP + 2];
         int top = 0;
         lo_stack[0] = 0;
