@@ -1575,9 +1575,9 @@ int ws_build_node_graph(const float *nodes, int n, int k, float node_radius, uin
     return ws_build_node_graph_ex(nodes, nullptr, n, k, node_radius, 1, knn, w, edges, stream);
 }
 
-// Nodes from which a full skinning goes over the grid (building it takes about 20 us; both sides measured,
-// k_skinning / grid, at 3000 and 260k surfels: 104 nodes 18 / 40 and 64 / 72 us, 248 nodes 36 / 42 and
-// 134 / 74 us, 305 nodes 42 / 40 and 161 / 71 us, 525 nodes 68 / 38 and 259 / 68 us).
+// Nodes from which a full skinning goes over the grid (building it takes about 20 us; both sides measured as replayed
+// kernels, k_skinning / grid, at 3000 and 260k surfels of a torus, us: 302 nodes 33 / 28 and 146 / 65, 366 nodes 38 / 28
+// and 171 / 65, 535 nodes 54 / 26 and 237 / 63; below, k_skinning takes 13 and 56 at 97 nodes, 27 and 127 at 258).
 constexpr int kSkinGridFrom = 300;
 
 int ws_skinning_incremental(const float *nodes, const uint32_t *node_status, int num_nodes, int num_prev_nodes,
